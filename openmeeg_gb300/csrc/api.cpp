@@ -379,28 +379,29 @@ void assemble_headmat_internal(omg_geometry g, const omg_integrator& integ, doub
         if (same && m1 == skip_self_mesh) continue;
         const int64_t t1b = h.tbeg[m1], t1e = h.tbeg[m1 + 1], t2b = h.tbeg[m2], t2e = h.tbeg[m2 + 1];
         const int64_t v1b = h.vbeg[m1], v1e = h.vbeg[m1 + 1], v2b = h.vbeg[m2], v2e = h.vbeg[m2 + 1];
-        double Scoeff = 0.0;
-        if (same ? !h.barrier[m1] : (!h.barrier[m1] && !h.barrier[m2])) {   // set_S_block
-            launch_S_block(d, t1b, t1e, t2b, t2e, same, p.cS, order, hm, ld, nullptr, ctx->d_err, s);
-            Scoeff = p.cS;
+        const int64_t n1 = t1e - t1b, n2 = t2e - t2b;
+        // S, on the analytic triangles of mesh 1 and the points of mesh 2, with the D (D*) block of the same roles
+        const bool sInHM = same ? !h.barrier[m1] : (!h.barrier[m1] && !h.barrier[m2]);   // set_S_block
+        const bool wantD21 = !h.barrier[m2];                                             // set_Dstar_block (D: same)
+        {
+            DevBuf stmp(sInHM ? 0 : (size_t)n1 * n2 * 8, s), d21(wantD21 ? (size_t)n1 * n2 * 24 : 0, s);
+            launch_SD_block(d, t1b, t1e, v1b, v1e, t2b, t2e, same, order, true, p.cS, sInHM ? hm : nullptr, ld,
+                            stmp.as<double>(), d21.as<double>(), s);
+            if (sInHM)   // set_N_block from the S already in the matrix
+                launch_N_block(d, v1b, v1e, t1b, t1e, v2b, v2e, t2b, t2e, same, p.cN / p.cS, hm, ld, nullptr, hm, s,
+                               false, s_along_b(h, m1, m2));
+            else         // ... or from a temporary unit S block (current barriers)
+                launch_N_block(d, v1b, v1e, t1b, t1e, v2b, v2e, t2b, t2e, same, p.cN, nullptr, ld, stmp.as<double>(),
+                               hm, s, false, true);
+            if (wantD21)
+                launch_D_gather(d, t2b, t2e, t1b, t1e, v1b, v1e, p.cD, d21.as<double>(), hm, ld, s);
         }
-        if (Scoeff != 0.0) {   // set_N_block from the S already in the matrix
-            launch_N_block(d, v1b, v1e, t1b, t1e, v2b, v2e, t2b, t2e, same, p.cN / Scoeff, hm, ld, nullptr, hm, s,
-                           false, s_along_b(h, m1, m2));
-        } else {               // ... or from a temporary unit S block (current barriers)
-            DevBuf tmp((size_t)(t1e - t1b) * (t2e - t2b) * 8, s);
-            launch_S_block(d, t1b, t1e, t2b, t2e, same, 1.0, order, nullptr, 0, tmp.as<double>(), ctx->d_err, s);
-            launch_N_block(d, v1b, v1e, t1b, t1e, v2b, v2e, t2b, t2e, same, p.cN, nullptr, ld, tmp.as<double>(), hm, s,
-                           false, true);
+        if (!same && !h.barrier[m1]) {   // set_D_block
+            DevBuf d12((size_t)n1 * n2 * 24, s);
+            launch_SD_block(d, t2b, t2e, v2b, v2e, t1b, t1e, false, order, false, 0.0, nullptr, 0, nullptr,
+                            d12.as<double>(), s);
+            launch_D_gather(d, t1b, t1e, t2b, t2e, v2b, v2e, p.cD, d12.as<double>(), hm, ld, s);
         }
-        auto dblock = [&](int ma, int mb) {
-            const int64_t tab = h.tbeg[ma], tae = h.tbeg[ma + 1], tbb = h.tbeg[mb], tbe = h.tbeg[mb + 1];
-            DevBuf tmp((size_t)(tae - tab) * (tbe - tbb) * 3 * 8, s);
-            launch_D_block(d, tab, tae, tbb, tbe, order, tmp.as<double>(), ctx->d_err, s);
-            launch_D_gather(d, tab, tae, tbb, tbe, h.vbeg[mb], h.vbeg[mb + 1], p.cD, tmp.as<double>(), hm, ld, s);
-        };
-        if (!h.barrier[m1]) dblock(m1, m2);                 // set_D_block
-        if (!same && !h.barrier[m2]) dblock(m2, m1);        // set_Dstar_block
     }
     // deflate (assembleHeadMat.cpp:27-60)
     for (const auto& part : h.part_outermost) {
@@ -1711,14 +1712,15 @@ int omg_surfsourcemat_dev(omg_context ctx, omg_geometry geo, const double* verts
             const int64_t t1b = h.tbeg[m], t1e = h.tbeg[m + 1], n1 = t1e - t1b;
             {
                 DevBuf S((size_t)n1 * n_tris * 8, s);   // unit-coefficient S block (the source is no unknown)
-                launch_S_block(u.d, t1b, t1e, tsb, tse, false, 1.0, it.order, nullptr, 0, S.as<double>(),
-                               ctx->d_err, s);
+                launch_SD_block(u.d, t1b, t1e, h.vbeg[m], h.vbeg[m + 1], tsb, tse, false, it.order, true, 1.0, nullptr,
+                                0, S.as<double>(), nullptr, s);
                 launch_N_block(u.d, h.vbeg[m], h.vbeg[m + 1], t1b, t1e, vsb, vse, tsb, tse, false, coeffN, nullptr,
                                Nint, S.as<double>(), out.as<double>(), s, true, true);
             }
             if (!h.barrier[m]) {
                 DevBuf D((size_t)n1 * n_tris * 24, s);
-                launch_D_block(u.d, t1b, t1e, tsb, tse, it.order, D.as<double>(), ctx->d_err, s);
+                launch_SD_block(u.d, tsb, tse, vsb, vse, t1b, t1e, false, it.order, false, 0.0, nullptr, 0, nullptr,
+                                D.as<double>(), s);
                 launch_D_gather(u.d, t1b, t1e, tsb, tse, vsb, vse, coeffN * L, D.as<double>(), out.as<double>(), Nint,
                                 s, true);
             }

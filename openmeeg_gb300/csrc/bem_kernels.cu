@@ -195,118 +195,325 @@ __device__ __forceinline__ int64_t lower_at(int64_t a, int64_t b, int64_t ld) {
 }
 
 // ---------------------------------------------------------------------------
-// S block (DiagonalBlock::S operators.h:209-237, NonDiagonalBlock::S :391-425):
-// S(t1,t2) = coeff * integral over t2 (Gauss rule) of OperatorS(t1).
-// One CTA per TI x TJ tile; t1 OperatorS records and t2 quadrature records
-// are bulk-copied into shared memory.  One thread per (t1,t2) pair.
+// S and D blocks (DiagonalBlock::S operators.h:209-237, NonDiagonalBlock::S
+// :391-425, BlocksBase::D :83-115) in FP64:
+//   S(b, a) = integral over a (Gauss rule) of OperatorS(b),
+//   D(a, b, j) = integral over a of P1SingleLayerPotential(b)_j,
+// for the analytic triangles b of one mesh and the rule points of the
+// triangles a of another (or the same) one.
+//
+// The FP64 pipe bounds these blocks (one thread per pair evaluating both closed
+// forms from their vertices kept it 88% busy: ~270 operations per single-layer
+// value, ~300 per double-layer one), so the operations are shared as far as the
+// closed forms allow, and memory traffic, which FP64 leaves nearly idle, is spent
+// for it.  For a batch of points, three launches fill and read global tables:
+//   1. d[v][x] = |x - v| for every vertex of the analytic mesh (half a vertex per
+//      triangle, instead of three distances per triangle);
+//   2. l[e][x] = (integral over the edge of 1/|x - y|) / length
+//      = 2 atanh(len / (d_a + d_b)) / len for every edge (1.5 per triangle instead
+//      of three logarithms each in S and in D: D's log((d_b + r_b.u)/(d_a + r_a.u))
+//      is the same integral);
+//   3. per (triangle, point): the heights h = n.(p0 - x), E_j = n.(r_j+1 x r_j+2)
+//      (linear in x; E_0 + E_1 + E_2 = 2A), the solid angle
+//      W = 2 atan(2 A h / (d0 d1 d2 + sum d_i r_j.r_k)) with r_j.r_k from the tabled
+//      distances and the edge lengths, then
+//        S = sum_i E_opp(i) l_i - h W,
+//        D_j = (W E_j + h sum_i (D_j+1 . D_i) l_i) / 2A, D_0 + D_1 + D_2 = W.
+// About 80 FP64 operations per (triangle, point) for S and D together.  The
+// arctangent and the logarithm take their series where the argument is small
+// (|x| <= 1/16 or 1/4, by the far terms' size against 2^-55) and the library
+// functions elsewhere; square roots and reciprocals are the hardware
+// approximations refined by one third-order Newton step.
+// Measured: 27.4 ms for the blocks of a 4486-unknown head (131 M values; 20 ms at the
+// 529 G FMA/s of the FP64 pipe) against 121 ms for one thread per pair without
+// tables; the 4-layer head of 7 / 9 / 10 / 11-frequency spheres 73 ms against 320 ms.
+// Lanes run over the triangles a at the same rule point, so every table read is
+// coalesced, the triangle b is uniform in a warp, and the sum over the rule stays
+// in registers (no shuffles, which cost FP64 additions).
 // ---------------------------------------------------------------------------
-constexpr int S_TI = 16, S_TJ = 64, S_THREADS = 256;
+constexpr int TGEO = 22;   // p0, -n, m0 = n x D0, m2 = n x D2 (3 each), 2A, |D_i|^2 (3), D0.D1 D1.D2 D2.D0, |D_i| (3)
 
-__global__ void __launch_bounds__(S_THREADS) s_block_kernel(const double* __restrict__ srec,
-                                                            const double* __restrict__ qrec, int64_t t1b, int64_t n1,
-                                                            int64_t t2b, int64_t n2, int same, double coeff,
-                                                            int order, const int32_t* __restrict__ tpos, double* hm,
-                                                            int64_t ld, double* tmp, int* err) {
-    extern __shared__ __align__(16) double smem[];
-    __shared__ __align__(8) uint64_t bar;
-    const int64_t i0 = (int64_t)blockIdx.y * S_TI, j0 = (int64_t)blockIdx.x * S_TJ;
-    if (same && j0 + S_TJ <= i0) return;   // tile strictly below the diagonal
-    const int ni = (int)(n1 - i0 < (int64_t)S_TI ? n1 - i0 : (int64_t)S_TI), nj = (int)(n2 - j0 < (int64_t)S_TJ ? n2 - j0 : (int64_t)S_TJ);
-    double* sS = smem;                 // ni x SREC
-    double* sQ = smem + S_TI * SREC;   // nj x QREC
-    if (!dev::stage_two(sS, srec + (t1b + i0) * SREC, (uint32_t)(ni * SREC * 8), sQ, qrec + (t2b + j0) * QREC,
-                        (uint32_t)(nj * QREC * 8), &bar, err))
-        return;
+__global__ void sd_geometry_kernel(int64_t t0, int64_t nt, const double* __restrict__ V,
+                                   const int32_t* __restrict__ T, const int32_t* __restrict__ v2t_beg,
+                                   const int32_t* __restrict__ v2t_tri, double* tgeo, int32_t* eown) {
+    const int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (it >= nt) return;
+    const int32_t* tv = T + 3 * (t0 + it);
+    const d3 p0 = dev::ld3(V + 3 * (int64_t)tv[0]), p1 = dev::ld3(V + 3 * (int64_t)tv[1]),
+             p2 = dev::ld3(V + 3 * (int64_t)tv[2]);
+    const d3 D0 = p1 - p0, D1 = p2 - p1, D2 = p0 - p2;
+    d3 nn = dev::cross(D0, p2 - p0);
+    const double nrm = dev::norm(nn);
+    const d3 n = nn * (1.0 / nrm);
+    const d3 m0 = dev::cross(n, D0), m2 = dev::cross(n, D2);
+    double* g = tgeo + it * TGEO;
+    g[0] = p0.x; g[1] = p0.y; g[2] = p0.z;
+    g[3] = -n.x; g[4] = -n.y; g[5] = -n.z;
+    g[6] = m0.x; g[7] = m0.y; g[8] = m0.z;
+    g[9] = m2.x; g[10] = m2.y; g[11] = m2.z;
+    g[12] = nrm;
+    g[13] = dev::dot(D0, D0); g[14] = dev::dot(D1, D1); g[15] = dev::dot(D2, D2);
+    g[16] = dev::dot(D0, D1); g[17] = dev::dot(D1, D2); g[18] = dev::dot(D2, D0);
+    g[19] = sqrt(g[13]); g[20] = sqrt(g[14]); g[21] = sqrt(g[15]);
+    // table row of edge i (corners i, i + 1): the slot 3 t + i of the first triangle of the range that has it
+    for (int i = 0; i < 3; ++i) {
+        const int32_t a = tv[i], b = tv[(i + 1) % 3];
+        int32_t own = (int32_t)(3 * it + i);
+        for (int k = v2t_beg[a]; k < v2t_beg[a + 1]; ++k) {
+            const int64_t t = v2t_tri[k];
+            if (t < t0 || t >= t0 + it) continue;   // (triangles around a vertex are listed in increasing order)
+            const int32_t* u = T + 3 * t;
+            int found = -1;
+            for (int j = 0; j < 3; ++j)
+                if ((u[j] == a && u[(j + 1) % 3] == b) || (u[j] == b && u[(j + 1) % 3] == a)) found = j;
+            if (found >= 0) {
+                own = (int32_t)(3 * (t - t0) + found);
+                break;
+            }
+        }
+        eown[3 * it + i] = own;
+    }
+}
+
+// 1/x to about an ulp: the hardware approximation and one third-order Newton step.
+__device__ __forceinline__ double sd_rcp(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(fma(e, e, e), y, y);
+}
+// sqrt(x) to about an ulp (x > 0), likewise from the approximate reciprocal square root.
+__device__ __forceinline__ double sd_sqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double g = x * y;
+    const double e = fma(-g, y, 1.0);
+    return fma(g * e, fma(0.375, e, 0.5), g);
+}
+// |x| < 1e-10 on the integer pipe.
+__device__ __forceinline__ bool sd_flat(double x) {
+    return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) < __double_as_longlong(1e-10);
+}
+// |x| < 2^k by the exponent field (integer pipe; NaN and infinity compare false).
+__device__ __forceinline__ bool sd_below(double x, int k) {
+    return ((__double2hiint(x) >> 20) & 0x7FF) < 1023 + k;
+}
+
+constexpr int SD_V = 16;      // vertices per CTA of the distance table
+constexpr int SD_E = 8;       // triangles per CTA of the edge table
+constexpr int SD_THREADS = 256;
+
+// Point x = q na + ia of a batch of na triangles from a0: point q of triangle a0 + ia.  Row 0..2 of pts:
+// coordinates; d[v * npt + x]: distance to vertex vb + v.
+__global__ void __launch_bounds__(SD_THREADS) sd_distance_kernel(const double* __restrict__ qrec, int64_t a0, int na,
+                                                                 int npt, const double* __restrict__ V, int64_t vb,
+                                                                 int nv, double* __restrict__ pts,
+                                                                 double* __restrict__ d) {
+    const int x = blockIdx.x * SD_THREADS + threadIdx.x;
+    if (x >= npt) return;
+    const int q = x / na, ia = x - q * na;
+    const double* src = qrec + (a0 + ia) * QREC + 3 * q;
+    const double px = src[0], py = src[1], pz = src[2];
+    if (blockIdx.y == 0) {
+        pts[x] = px;
+        pts[(int64_t)npt + x] = py;
+        pts[2 * (int64_t)npt + x] = pz;
+    }
+    const int v1 = min(nv, (int)(blockIdx.y + 1) * SD_V);
+#pragma unroll 4
+    for (int v = blockIdx.y * SD_V; v < v1; ++v) {
+        const double* p = V + 3 * (vb + v);
+        const double rx = p[0] - px, ry = p[1] - py, rz = p[2] - pz;
+        d[(int64_t)v * npt + x] = sd_sqrt(fma(rx, rx, fma(ry, ry, rz * rz)));
+    }
+}
+
+// 2 atanh(len / R) / len, R = d_a + d_b.  With y = 1/R and z = len y: 2 y (1 + z^2/3 + z^4/5 + ...); the last
+// term kept is above 2^-55 at each limit.
+__device__ __forceinline__ double sd_edge(double R, double len) {
+    const double y = sd_rcp(R);
+    const double z = len * y, w = z * z;
+    double p;
+    if (sd_below(z, -4)) {          // z < 1/16
+        p = fma(w, 1.0 / 13, 1.0 / 11);
+    } else if (sd_below(z, -3)) {   // z < 1/8
+        p = fma(w, 1.0 / 17, 1.0 / 15);
+        p = fma(w, p, 1.0 / 13);
+        p = fma(w, p, 1.0 / 11);
+    } else if (sd_below(z, -2)) {   // z < 1/4
+        p = fma(w, 1.0 / 27, 1.0 / 25);
+        p = fma(w, p, 1.0 / 23);
+        p = fma(w, p, 1.0 / 21);
+        p = fma(w, p, 1.0 / 19);
+        p = fma(w, p, 1.0 / 17);
+        p = fma(w, p, 1.0 / 15);
+        p = fma(w, p, 1.0 / 13);
+        p = fma(w, p, 1.0 / 11);
+    } else {
+        return 2.0 * atanh(len / R) / len;
+    }
+    p = fma(w, p, 1.0 / 9);
+    p = fma(w, p, 1.0 / 7);
+    p = fma(w, p, 1.0 / 5);
+    p = fma(w, p, 1.0 / 3);
+    return 2.0 * fma(w * p, y, y);
+}
+
+// The solid angle, 2 atan2(num, den): its series where num / den < 1/16 (den > 0).
+__device__ __forceinline__ double sd_angle(double num, double den) {
+    const double t = num * sd_rcp(den);
+    if (__double2hiint(den) < 0 || !sd_below(t, -4)) return 2.0 * atan2(num, den);
+    const double w = t * t;
+    double p;
+    if (sd_below(t, -7)) {
+        p = fma(w, -1.0 / 7, 1.0 / 5);
+    } else {
+        p = fma(w, 1.0 / 13, -1.0 / 11);
+        p = fma(w, p, 1.0 / 9);
+        p = fma(w, p, -1.0 / 7);
+        p = fma(w, p, 1.0 / 5);
+    }
+    p = fma(w, p, -1.0 / 3);
+    return fma(w * p, t + t, t + t);
+}
+
+// l[3 b + i]: edge i (corners i, i + 1) of triangle b, in the rows that own their edge.
+__global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb, int npt, const int32_t* __restrict__ T,
+                                                             int64_t vb, const double* __restrict__ tgeo,
+                                                             const int32_t* __restrict__ eown,
+                                                             const double* __restrict__ d, double* __restrict__ l) {
+    const int x = blockIdx.x * SD_THREADS + threadIdx.x;
+    if (x >= npt) return;
+    const int b1 = min(nb, (int)(blockIdx.y + 1) * SD_E);
+    for (int b = blockIdx.y * SD_E; b < b1; ++b) {
+        const int32_t* tv = T + 3 * (tb + b);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            if (eown[3 * b + i] != 3 * b + i) continue;
+            const double da = d[(int64_t)(tv[i] - vb) * npt + x], db = d[(int64_t)(tv[i == 2 ? 0 : i + 1] - vb) * npt + x];
+            l[(int64_t)(3 * b + i) * npt + x] = sd_edge(da + db, tgeo[b * (int64_t)TGEO + 19 + i]);
+        }
+    }
+}
+
+// The pairs (triangle b, triangle a0 + ia of the batch): warp w of a CTA holds b, its lanes 32 triangles a.
+// S for a >= b only when `same`.
+template <bool WANT_S, bool WANT_D>
+__global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
+    int64_t tb, int nb, int64_t ta, int64_t a0, int na, int npt, int order, int same, double coeff,
+    const int32_t* __restrict__ T, int64_t vb, const double* __restrict__ tgeo, const int32_t* __restrict__ eown,
+    const double* __restrict__ qrec, const double* __restrict__ pts, const double* __restrict__ d,
+    const double* __restrict__ l, const int32_t* __restrict__ tpos, double* hm, int64_t ld, double* stmp, int64_t n2,
+    double* dtmp) {
+    const int b = blockIdx.y * (SD_THREADS / 32) + threadIdx.x / 32;
+    if (b >= nb) return;
+    const int lane_a = blockIdx.x * 32 + threadIdx.x % 32;
+    const bool live = lane_a < na;
+    const int ia = live ? lane_a : na - 1;
+    const int64_t a = a0 + ia;   // relative to ta
+    const bool wantS = WANT_S && (!same || a >= b);
+    if (!WANT_D && !__any_sync(0xffffffffu, wantS)) return;
+    const double* g = tgeo + (int64_t)b * TGEO;
+    const double p0x = g[0], p0y = g[1], p0z = g[2], nx = g[3], ny = g[4], nz = g[5];
+    const double m0x = g[6], m0y = g[7], m0z = g[8], m2x = g[9], m2y = g[10], m2z = g[11];
+    const double A2 = g[12], q0 = g[13], q1 = g[14], q2 = g[15], g01 = g[16], g12 = g[17], g20 = g[18];
+    const int32_t* tv = T + 3 * (tb + b);
+    const double* dr0 = d + (int64_t)(tv[0] - vb) * npt + ia;
+    const double* dr1 = d + (int64_t)(tv[1] - vb) * npt + ia;
+    const double* dr2 = d + (int64_t)(tv[2] - vb) * npt + ia;
+    const double* lr0 = l + (int64_t)eown[3 * b] * npt + ia;
+    const double* lr1 = l + (int64_t)eown[3 * b + 1] * npt + ia;
+    const double* lr2 = l + (int64_t)eown[3 * b + 2] * npt + ia;
+    const double* px = pts + ia;
+    const double* py = px + npt;
+    const double* pz = py + npt;
     const int np = c_nbpts[order];
-    for (int p = threadIdx.x; p < ni * nj; p += S_THREADS) {
-        const int i = p / nj, j = p % nj;
-        if (same && j0 + j < i0 + i) continue;
-        const double* s = sS + i * SREC;
-        const double* q = sQ + j * QREC;
-        double acc = 0.0;
-        for (int k = 0; k < np; ++k) acc += c_rules[order][k][3] * dev::operator_S(s, dev::ld3(q + 3 * k));
-        const double val = q[48] * acc;
-        const int64_t a = t1b + i0 + i, b = t2b + j0 + j;
+    double sS = 0.0, s0 = 0.0, s1 = 0.0, sw = 0.0;
+    for (int k = 0; k < np; ++k, dr0 += na, dr1 += na, dr2 += na, lr0 += na, lr1 += na, lr2 += na, px += na, py += na,
+             pz += na) {
+        const double d0 = *dr0, d1 = *dr1, d2 = *dr2, l0 = *lr0, l1 = *lr1, l2 = *lr2;
+        const double cx = *px - p0x, cy = *py - p0y, cz = *pz - p0z;
+        const double h = fma(nx, cx, fma(ny, cy, nz * cz));
+        const double E2 = fma(m0x, cx, fma(m0y, cy, m0z * cz));
+        const double E1 = fma(m2x, cx, fma(m2y, cy, m2z * cz));
+        const double E0 = (A2 - E1) - E2;
+        // 2 (d0 d1 d2 + sum d_i r_j.r_k), with 2 r_j.r_k = d_j^2 + d_k^2 - |edge|^2
+        const double s12 = d1 + d2, e0 = d0 * d0;
+        const double den = fma(d0, fma(s12, s12, -q1), fma(d1, fma(d2, d2, e0 - q2), d2 * fma(d1, d1, e0 - q0)));
+        const double dd = A2 * h;
+        const double W = sd_angle(dd + dd, den);
+        const double wr = c_rules[order][k][3];
+        if (WANT_S) {
+            const double el = fma(E2, l0, fma(E0, l1, E1 * l2));
+            sS = fma(wr, sd_flat(dd) ? el : fma(-h, W, el), sS);
+        }
+        if (WANT_D && !sd_flat(h)) {
+            const double f0 = fma(g01, l0, fma(q1, l1, g12 * l2));   // D1 . sum D_i l_i
+            const double f1 = fma(g20, l0, fma(g12, l1, q2 * l2));   // D2 . sum D_i l_i
+            s0 = fma(wr, fma(W, E0, h * f0), s0);
+            s1 = fma(wr, fma(W, E1, h * f1), s1);
+            sw = fma(wr, W, sw);
+        }
+    }
+    if (!live) return;
+    const double area = qrec[(ta + a) * QREC + 48];
+    if (wantS) {
+        const double val = area * sS;
         if (hm) {
-            hm[lower_at(tpos[a], tpos[b], ld)] = val * coeff;
+            hm[lower_at(tpos[tb + b], tpos[ta + a], ld)] = val * coeff;
         } else {
-            tmp[(i0 + i) * n2 + (j0 + j)] = val;
-            if (same) tmp[(j0 + j) * n2 + (i0 + i)] = val;
+            stmp[b * n2 + a] = val;
+            if (same) stmp[a * n2 + b] = val;
         }
     }
-}
-
-void launch_S_block(const DevGeom& g, int64_t t1b, int64_t t1e, int64_t t2b, int64_t t2e, bool same, double coeff,
-                    int order, double* hm, int64_t ld, double* tmp, int* err, cudaStream_t s) {
-    const int64_t n1 = t1e - t1b, n2 = t2e - t2b;
-    ProfScope prof_("s_block", s);
-    dim3 grid(nblocks(n2, S_TJ), nblocks(n1, S_TI));
-    const size_t sm = (size_t)(S_TI * SREC + S_TJ * QREC) * 8;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(s_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        attr = true;
-    }
-    s_block_kernel<<<grid, S_THREADS, sm, s>>>(g.srec, g.qrec, t1b, n1, t2b, n2, same ? 1 : 0, coeff, order, g.tpos,
-                                               hm, ld, tmp, err);
-    check_launch("S block");
-}
-
-// ---------------------------------------------------------------------------
-// D block (BlocksBase::D operators.h:83-115): for t1 in A, t2 in B the three
-// integrals over t1 of P1SingleLayerPotential(t2), stored per pair in a
-// scratch array; the gather kernel below adds them into (t1, vertex) entries
-// in a fixed order, so the result does not depend on thread timing.
-// ---------------------------------------------------------------------------
-constexpr int D_TI = 16, D_TJ = 32, D_THREADS = 256;
-
-__global__ void __launch_bounds__(D_THREADS) d_block_kernel(const double* __restrict__ qrec,
-                                                            const double* __restrict__ prec, int64_t tab, int64_t na,
-                                                            int64_t tbb, int64_t nb, int order, double* tmp,
-                                                            int* err) {
-    extern __shared__ __align__(16) double smem[];
-    __shared__ __align__(8) uint64_t bar;
-    const int64_t i0 = (int64_t)blockIdx.y * D_TI, j0 = (int64_t)blockIdx.x * D_TJ;
-    const int ni = (int)(na - i0 < (int64_t)D_TI ? na - i0 : (int64_t)D_TI), nj = (int)(nb - j0 < (int64_t)D_TJ ? nb - j0 : (int64_t)D_TJ);
-    double* sQ = smem;                 // ni x QREC (integration triangles t1)
-    double* sP = smem + D_TI * QREC;   // nj x PREC (analytic triangles t2)
-    if (!dev::stage_two(sQ, qrec + (tab + i0) * QREC, (uint32_t)(ni * QREC * 8), sP, prec + (tbb + j0) * PREC,
-                        (uint32_t)(nj * PREC * 8), &bar, err))
-        return;
-    const int np = c_nbpts[order];
-    for (int p = threadIdx.x; p < ni * nj; p += D_THREADS) {
-        const int i = p / nj, j = p % nj;
-        const double* q = sQ + i * QREC;
-        const double* P = sP + j * PREC;
-        double acc[3] = {0.0, 0.0, 0.0};
-        for (int k = 0; k < np; ++k) {
-            double v[3];
-            dev::p1_single_layer(P, dev::ld3(q + 3 * k), v);
-            const double w = c_rules[order][k][3];
-            acc[0] += w * v[0];
-            acc[1] += w * v[1];
-            acc[2] += w * v[2];
-        }
-        double* o = tmp + ((i0 + i) * nb + (j0 + j)) * 3;
-        o[0] = q[48] * acc[0];
-        o[1] = q[48] * acc[1];
-        o[2] = q[48] * acc[2];
+    if (WANT_D) {
+        double* o = dtmp + (a * nb + b) * 3;
+        const double i2A = 1.0 / A2;   // (W E_j + h f_j) / (2A) per component
+        s0 *= i2A;
+        s1 *= i2A;
+        o[0] = area * s0;
+        o[1] = area * s1;
+        o[2] = area * (sw - s0 - s1);
     }
 }
 
-void launch_D_block(const DevGeom& g, int64_t tab, int64_t tae, int64_t tbb, int64_t tbe, int order, double* tmp,
-                    int* err, cudaStream_t s) {
-    const int64_t na = tae - tab, nb = tbe - tbb;
-    ProfScope prof_("d_block", s);
-    dim3 grid(nblocks(nb, D_TJ), nblocks(na, D_TI));
-    const size_t sm = (size_t)(D_TI * QREC + D_TJ * PREC) * 8;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(d_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        attr = true;
+// The blocks of the analytic triangles [tbb, tbe) (vertices [vbb, vbe)) and the rule points of the triangles
+// [tab, tae).  wantS: S into hm (times coeff) or into the dense b-major stmp; `same`: one mesh against itself.
+// dtmp: D, [a][b][3], or null.
+void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, int64_t vbe, int64_t tab, int64_t tae,
+                     bool same, int order, bool wantS, double coeff, double* hm, int64_t ld, double* stmp,
+                     double* dtmp, cudaStream_t s) {
+    const int64_t nb = tbe - tbb, na = tae - tab, nv = vbe - vbb;
+    if (nb <= 0 || na <= 0 || (!wantS && !dtmp)) return;
+    ProfScope prof_("sd_block", s);
+    if (nb > (1 << 28)) throw Error(OMG_ERR_UNSUPPORTED, "S / D block too large");
+    constexpr int NPTS[4] = {3, 6, 7, 16};
+    const int np = NPTS[order];
+    // points per batch: tables of about 512 MB, a multiple of 32 triangles (full warps)
+    const int64_t per_tri = (nv + 3 * nb + 3) * 8 * np;
+    const int64_t batch = std::min(na, std::max<int64_t>(32, std::min<int64_t>((512ll << 20) / per_tri, 4096) / 32 * 32));
+    DevBuf geo((size_t)nb * (TGEO * 8 + 3 * 4), s), tab_((size_t)per_tri * batch, s);
+    double* tgeo = geo.as<double>();
+    int32_t* eown = reinterpret_cast<int32_t*>(tgeo + nb * TGEO);
+    sd_geometry_kernel<<<nblocks(nb, 64), 64, 0, s>>>(tbb, nb, g.V, g.T, g.v2t_beg, g.v2t_tri, tgeo, eown);
+    check_launch("S / D geometry");
+    for (int64_t a0 = 0; a0 < na; a0 += batch) {
+        const int n = (int)std::min(batch, na - a0), npt = n * np;
+        double* pts = tab_.as<double>();
+        double* d = pts + 3 * (int64_t)npt;
+        double* l = d + nv * npt;
+        const unsigned gx = nblocks(npt, SD_THREADS);
+        sd_distance_kernel<<<dim3(gx, nblocks(nv, SD_V)), SD_THREADS, 0, s>>>(g.qrec, tab + a0, n, npt, g.V, vbb, (int)nv,
+                                                                            pts, d);
+        check_launch("S / D distances");
+        sd_edge_kernel<<<dim3(gx, nblocks(nb, SD_E)), SD_THREADS, 0, s>>>(tbb, (int)nb, npt, g.T, vbb, tgeo, eown, d, l);
+        check_launch("S / D edges");
+        const dim3 grid(nblocks(n, 32), nblocks(nb, SD_THREADS / 32));
+        auto kern = wantS ? (dtmp ? sd_pair_kernel<true, true> : sd_pair_kernel<true, false>) : sd_pair_kernel<false, true>;
+        kern<<<grid, SD_THREADS, 0, s>>>(tbb, (int)nb, tab, a0, n, npt, order, same ? 1 : 0, coeff, g.T, vbb, tgeo, eown,
+                                         g.qrec, pts, d, l, g.tpos, hm, ld, stmp, na, dtmp);
+        check_launch("S / D pairs");
     }
-    d_block_kernel<<<grid, D_THREADS, sm, s>>>(g.qrec, g.prec, tab, na, tbb, nb, order, tmp, err);
-    check_launch("D block");
 }
 
 // HM(t1, v) += coeff * sum over triangles t2 of B containing v of tmp[t1][t2][local(v)]

@@ -149,13 +149,13 @@ struct Workspace;
 
 void launch_prepare_triangles(const DevGeom& g, cudaStream_t s);
 void launch_prepare_vertex_curls(const DevGeom& g, cudaStream_t s);
-// S block: out(t1, t2) for t1 in [t1b,t1e), t2 in [t2b,t2e); `same` restricts to t2>=t1.
-//   mode 0: write coeff*S into HM lower triangle at internal positions (ld)
-//   mode 1: write S into tmp (n1 x n2 row-major, both halves when same)
-void launch_S_block(const DevGeom& g, int64_t t1b, int64_t t1e, int64_t t2b, int64_t t2e, bool same, double coeff,
-                    int order, double* hm, int64_t ld, double* tmp, int* err, cudaStream_t s);
-void launch_D_block(const DevGeom& g, int64_t tab, int64_t tae, int64_t tbb, int64_t tbe, int order, double* tmp,
-                    int* err, cudaStream_t s);
+// The blocks of the analytic triangles [tbb, tbe) (vertices [vbb, vbe)) and the rule points of the triangles
+// [tab, tae).  wantS: S(b, a) times coeff into the head matrix's lower triangle at the internal positions (hm, ld),
+// or unscaled into the dense b-major stmp when hm is null; `same` (one mesh against itself): S for a >= b, both
+// halves of stmp.  dtmp: the three D integrals of every pair, [a][b][3], or null.
+void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, int64_t vbe, int64_t tab, int64_t tae,
+                     bool same, int order, bool wantS, double coeff, double* hm, int64_t ld, double* stmp,
+                     double* dtmp, cudaStream_t s);
 // rect: out(row = triangle unknown, col = vertex - vbb), column-major with ld, instead of the HM lower triangle
 void launch_D_gather(const DevGeom& g, int64_t tab, int64_t tae, int64_t tbb, int64_t tbe, int64_t vbb, int64_t vbe,
                      double coeff, const double* tmp, double* hm, int64_t ld, cudaStream_t s, bool rect = false);
