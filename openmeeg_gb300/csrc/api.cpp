@@ -101,10 +101,6 @@ void residual_df64(int64_t M, int64_t N, int64_t K, const float* Ahi, const floa
                    int64_t ldr, cudaStream_t s);
 void split_f64(int64_t m, int64_t n, const double* A, int64_t lda, float* H, float* L, int64_t ldo, cudaStream_t s);
 template <typename T>
-void potrf(T* A, int64_t lda, int n, int* err, int64_t* err_col, int64_t col_offset, cudaStream_t s);
-template <typename T>
-void trsm_rows(int64_t m, int n, const T* L, int64_t ldl, T* P, int64_t ldp, cudaStream_t s);
-template <typename T>
 void trsm_cols(int64_t nrhs, int n, const T* L, int64_t ldl, bool trans, T* B, int64_t ldb, cudaStream_t s,
                const T* Lr = nullptr);
 // tc_gemm.cu
@@ -142,6 +138,14 @@ void digits_columns(const double* M, int64_t n, int64_t ncol, int64_t ldm, int n
 void digit_gemm(int64_t n, int64_t k, int64_t kdim, const void* Ad, int nda, const int* rexp, const void* Xd, int ndx,
                 int64_t kpad, const int* cexp, int beta, int lmax, const double* B, int64_t ldb, double sgn, double* R,
                 int64_t ldr, int* err, cudaStream_t s, const char* prof_name);
+// f64_digits.cu
+void row_digits_f64(const double* A, int64_t lda, int64_t m, int k, int kpad, int64_t rows_per_plane, void* out, int* ex,
+                    cudaStream_t s);
+void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
+                      const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, bool lower,
+                      int* err, cudaStream_t s, const char* name);
+void potrf64(double* A, int64_t lda, int n, int* err, int64_t* err_col, int64_t col_offset, cudaStream_t s);
+void trsm64(int64_t m, const double* L, int64_t ldl, double* P, int64_t ldp, cudaStream_t s);
 // tc_solve.cu
 size_t sweep_scratch_bytes(int64_t nblocks, int64_t nrhs);
 void solve_sweep_tc(bool backward, int64_t N, int64_t nblocks, const float* W, int64_t w_rows, const float* A,
@@ -559,28 +563,56 @@ static void require_distinct_vertices(omg_geometry g, const char* what) {
 // ---------------------------------------------------------------------------
 // Factorization: HM = L diag(+I_P, -I_V) L^T, blocked right-looking.
 // ---------------------------------------------------------------------------
-template <typename T>
-static void factor_ldlt(omg_solver sv, T* A, int64_t ld, int nb) {
+// FP64, in place on the lower triangle: panels of 128 columns, each two sub-panels of 64 factored on the FP64 pipe
+// (potrf64, trsm64 and the second sub-panel's update: 64 columns of work per row, N^2 / 2 x 64 operations in all),
+// everything wider as FP64-accurate digit products on the tensor cores (f64_digits.cu).  Panels go in groups of
+// two (never across the start of the vertex part): the second takes the first one's update at K = 128, the trailing
+// block the group's at K = 256, which halves the FP64 passes over it.
+static void factor_ldlt_f64(omg_solver sv, double* A, int64_t ld) {
+    constexpr int64_t NB = 128, SB = 64;
     cudaStream_t s = sv->ctx->stream;
     const int64_t N = sv->N, nP = sv->nP;
+    int* err = sv->ctx->d_err;
     sv->bounds.clear();
     for (int64_t k = 0; k < N;) {
         sv->bounds.push_back(k);
-        int64_t e = std::min(N, k + nb);
+        int64_t e = std::min(N, k + NB);
         if (k < nP && e > nP) e = nP;
         k = e;
     }
     sv->bounds.push_back(N);
     const size_t nblocks = sv->bounds.size() - 1;
-    for (size_t b = 0; b < nblocks; ++b) {
-        const int64_t k0 = sv->bounds[b], k1 = sv->bounds[b + 1], nk = k1 - k0, m = N - k1;
-        if (k0 == nP) negate_lower<T>(A + k0 + k0 * ld, ld, N - k0, s);   // continue on -(vertex Schur complement)
-        potrf<T>(A + k0 + k0 * ld, ld, (int)nk, sv->ctx->d_err, sv->ctx->d_errcol, k0, s);
-        if (m > 0) {
-            trsm_rows<T>(m, (int)nk, A + k0 + k0 * ld, ld, A + k1 + k0 * ld, ld, s);          // L21 = A21 L11^-T
-            gemm<T>(m, m, nk, T(-1), A + k1 + k0 * ld, ld, false, A + k1 + k0 * ld, ld, true, T(1), A + k1 + k1 * ld,
-                    ld, s, true, 0, 0);                                                          // A22 -= L21 L21^T
+    const int64_t mmax = std::max<int64_t>(1, N - sv->bounds[1]);
+    DevBuf dig((size_t)7 * mmax * 2 * NB * 2, s), ex((size_t)mmax * sizeof(int), s);
+    auto at = [&](int64_t r, int64_t c) { return A + r + c * ld; };
+    // C(rows and columns from r0, ncol columns) -= (columns k0 .. k1 of the factor)
+    auto update = [&](int64_t k0, int64_t k1, int64_t r0, int64_t ncol, bool lower, const char* name) {
+        const int64_t m = N - r0;
+        const int kpad = k1 - k0 > NB ? 2 * NB : NB;
+        row_digits_f64(at(r0, k0), ld, m, (int)(k1 - k0), kpad, m, dig.p, ex.as<int>(), s);
+        digit_update_f64(m, ncol, kpad, dig.p, m, 0, ex.as<int>(), dig.p, m, 0, ex.as<int>(), at(r0, r0), ld, lower, err,
+                         s, name);
+    };
+    for (size_t b = 0; b < nblocks;) {
+        const size_t ge = b + (b + 1 < nblocks && sv->bounds[b + 1] != nP ? 2 : 1);
+        const int64_t g0 = sv->bounds[b];
+        if (g0 == nP) negate_lower<double>(at(nP, nP), ld, N - nP, s);   // continue on -(vertex Schur complement)
+        for (; b < ge; ++b) {
+            const int64_t k0 = sv->bounds[b], k1 = sv->bounds[b + 1], ks = std::min(k1, k0 + SB);
+            if (k0 > g0) update(g0, k0, k0, k1 - k0, false, "f64_next");
+            potrf64(at(k0, k0), ld, (int)(ks - k0), err, sv->ctx->d_errcol, k0, s);
+            if (ks == N) break;
+            trsm64(N - ks, at(k0, k0), ld, at(ks, k0), ld, s);
+            if (ks < k1) {
+                gemm<double>(N - ks, k1 - ks, SB, -1.0, at(ks, k0), ld, false, at(ks, k0), ld, true, 1.0, at(ks, ks), ld,
+                             s);
+                potrf64(at(ks, ks), ld, (int)(k1 - ks), err, sv->ctx->d_errcol, ks, s);
+                if (k1 < N) trsm64(N - k1, at(ks, ks), ld, at(k1, ks), ld, s);
+            }
         }
+        b = ge;
+        const int64_t r0 = sv->bounds[ge];
+        if (r0 < N) update(g0, r0, r0, N - r0, true, "f64_syrk");
     }
 }
 
@@ -923,9 +955,6 @@ static void solve_ldlt(omg_solver sv, const T* A, int64_t ld, T* B, int64_t ldb,
     }
 }
 
-constexpr int NB64 = 128;   // FP64 diagonal block (128 x 129 x 8 B of shared memory)
-constexpr int NB32 = 128;   // FP32 diagonal block
-
 // A current barrier that encloses a non-conductive hole (a barrier mesh that is
 // not outermost, geometry.cpp:424-461) leaves the constant potential on its
 // vertices in the head matrix's null space: the N block of a closed mesh and
@@ -956,7 +985,7 @@ void solver_factor(omg_solver sv, DevBuf&& hm, bool check) {
     deflate_enclosed_barriers(sv, hm.as<double>(), N);
     if (sv->precision == OMG_PREC_FP64) {
         sv->A64 = std::move(hm);
-        factor_ldlt<double>(sv, sv->A64.as<double>(), N, NB64);
+        factor_ldlt_f64(sv, sv->A64.as<double>(), N);
     } else {
         sv->ld32 = (N + 31) / 32 * 32;
         sv->A32 = DevBuf((size_t)sv->ld32 * N * sizeof(float), s, sv->persistent);

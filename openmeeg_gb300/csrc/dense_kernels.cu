@@ -407,102 +407,12 @@ void split_f64(int64_t m, int64_t n, const double* A, int64_t lda, float* H, flo
 }
 
 // ---------------------------------------------------------------------------
-// Diagonal block Cholesky (lower, right-looking) with the block resident in
-// shared memory; thread (r, c-chunk) mapping avoids integer division in the
-// update loop.
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(512) potrf_kernel(T* A, int64_t lda, int n, int* err, int64_t* err_col,
-                                                   int64_t col_offset) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T* L = reinterpret_cast<T*>(smraw);   // n x (n+1) column-major (padded)
-    const int ldl = n + 1;
-    const int tid = threadIdx.x;
-    for (int e = tid; e < n * n; e += 512) {
-        const int i = e % n, j = e / n;
-        L[i + j * ldl] = (i >= j) ? A[i + j * lda] : T(0);
-    }
-    __syncthreads();
-    const int lane_r = tid % 32, grp = tid / 32;   // 16 groups of 32 rows-threads
-    for (int j = 0; j < n; ++j) {
-        if (tid == 0) {
-            T d = L[j + j * ldl];
-            if (!(d > T(0))) {
-                if (atomicCAS(err, 0, -3 /* OMG_ERR_NOT_DEFINITE */) == 0) *err_col = col_offset + j;
-                d = T(1);
-            }
-            L[j + j * ldl] = sqrt(d);
-        }
-        __syncthreads();
-        const T inv = T(1) / L[j + j * ldl];
-        for (int i = j + 1 + tid; i < n; i += 512) L[i + j * ldl] *= inv;
-        __syncthreads();
-        // trailing update of columns c in (j, n): group g handles columns c = j+1+g, j+1+g+16, ...
-        for (int c = j + 1 + grp; c < n; c += 16) {
-            const T lc = L[c + j * ldl];
-            for (int r = c + lane_r; r < n; r += 32) L[r + c * ldl] -= L[r + j * ldl] * lc;
-        }
-        __syncthreads();
-    }
-    for (int e = tid; e < n * n; e += 512) {
-        const int i = e % n, j = e / n;
-        if (i >= j) A[i + j * lda] = L[i + j * ldl];
-    }
-}
-
-template <typename T>
-void potrf(T* A, int64_t lda, int n, int* err, int64_t* err_col, int64_t col_offset, cudaStream_t s) {
-    ProfScope prof_("potrf", s);
-    const size_t sm = (size_t)n * (n + 1) * sizeof(T);
-    if (sm > 227 * 1024) throw Error(OMG_ERR_INVALID, "diagonal block too large for shared memory");
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(potrf_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        attr = true;
-    }
-    potrf_kernel<T><<<1, 512, sm, s>>>(A, lda, n, err, err_col, col_offset);
-    check("potrf");
-}
-template void potrf<double>(double*, int64_t, int, int*, int64_t*, int64_t, cudaStream_t);
-template void potrf<float>(float*, int64_t, int, int*, int64_t*, int64_t, cudaStream_t);
-
-// ---------------------------------------------------------------------------
 // Triangular solves with a diagonal block L (n x n lower, staged in shared
 // memory).  Panel form (rows independent):  W = P L^-T  for P (m x n).
 // Column form (columns independent):       B <- L^-1 B  or  L^-T B.
 // Each row / column is one warp: the substitution runs serially over the
 // block, the inner products across the 32 lanes.
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256) trsm_rows_kernel(int64_t m, int n, const T* __restrict__ L, int64_t ldl,
-                                                        T* P, int64_t ldp) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T* sL = reinterpret_cast<T*>(smraw);          // n x n (row-major copy: sL[j*n + l] = L[j][l])
-    T* sx = sL + n * n;                           // 8 warps x n
-    for (int e = threadIdx.x; e < n * n; e += 256) {   // coalesced read down the columns of L
-        const int j = e % n, l = e / n;
-        sL[j * n + l] = (l <= j) ? L[j + l * ldl] : T(0);
-    }
-    __syncthreads();
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    T* x = sx + warp * n;
-    for (int64_t row = (int64_t)blockIdx.x * 8 + warp; row < m; row += (int64_t)gridDim.x * 8) {
-        for (int l = lane; l < n; l += 32) x[l] = P[row + (int64_t)l * ldp];
-        __syncwarp();
-        // x L^T = p  <=>  L x^T = p^T : forward substitution over j
-        for (int j = 0; j < n; ++j) {
-            T acc = T(0);
-            for (int l = lane; l < j; l += 32) acc += x[l] * sL[j * n + l];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) x[j] = (x[j] - acc) / sL[j * n + j];
-            __syncwarp();
-        }
-        for (int l = lane; l < n; l += 32) P[row + (int64_t)l * ldp] = x[l];
-        __syncwarp();
-    }
-}
-
 template <typename T>
 __global__ void __launch_bounds__(256) trsm_cols_kernel(int64_t nrhs, int n, const T* __restrict__ L, int64_t ldl,
                                                         const T* __restrict__ Lr, int trans, T* B, int64_t ldb) {
@@ -554,20 +464,6 @@ static void set_max_smem(const void* f) {
 }
 
 template <typename T>
-void trsm_rows(int64_t m, int n, const T* L, int64_t ldl, T* P, int64_t ldp, cudaStream_t s) {
-    if (m <= 0) return;
-    ProfScope prof_("trsm_rows", s);
-    static bool attr = false;
-    if (!attr) {
-        set_max_smem<T>((const void*)trsm_rows_kernel<T>);
-        attr = true;
-    }
-    const size_t sm = ((size_t)n * n + 8 * (size_t)n) * sizeof(T);
-    const unsigned grid = (unsigned)std::min<int64_t>((m + 7) / 8, 152 * 8);
-    trsm_rows_kernel<T><<<grid, 256, sm, s>>>(m, n, L, ldl, P, ldp);
-    check("trsm_rows");
-}
-template <typename T>
 void trsm_cols(int64_t nrhs, int n, const T* L, int64_t ldl, bool trans, T* B, int64_t ldb, cudaStream_t s,
                const T* Lr) {
     if (nrhs <= 0) return;
@@ -582,8 +478,6 @@ void trsm_cols(int64_t nrhs, int n, const T* L, int64_t ldl, bool trans, T* B, i
     trsm_cols_kernel<T><<<grid, 256, sm, s>>>(nrhs, n, L, ldl, Lr, trans ? 1 : 0, B, ldb);
     check("trsm_cols");
 }
-template void trsm_rows<double>(int64_t, int, const double*, int64_t, double*, int64_t, cudaStream_t);
-template void trsm_rows<float>(int64_t, int, const float*, int64_t, float*, int64_t, cudaStream_t);
 template void trsm_cols<double>(int64_t, int, const double*, int64_t, bool, double*, int64_t, cudaStream_t,
                                 const double*);
 template void trsm_cols<float>(int64_t, int, const float*, int64_t, bool, float*, int64_t, cudaStream_t, const float*);

@@ -1,0 +1,650 @@
+// FP64-accurate products on the bf16 tensor cores (sm_103a, tcgen05) for the FP64
+// factorization: C -= A B^T with the rows of A and B cut into exact fixed-point
+// digits (the scheme of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012):
+//
+//   A_ik = 2^(e_i) sum_{s=1..7} 2^(-8 s) a_s,ik,  |a_s| <= 128 integers (56 bits below the row's maximum),
+//   (A B^T)_ij = 2^(e_i + e_j) sum_l 2^(-8 l) v_l,  v_l = sum_{s+t=l} sum_k a_s,ik b_t,jk,  l = 2..9 (34 pairs).
+//
+// FP64's own pipe does 1.06 TFLOP/s here, the bf16 tensor cores 1.9 PFLOP/s, so 34
+// products are still ~50 times cheaper.  The seven digits hold more than FP64's 53
+// bits of the largest entry of a row, and the dropped pairs (l >= 10) are below 2^-58
+// of row maximum times row maximum each; with l = 9 left out (28 pairs) a solve
+// against a head matrix was three times further off than FP64 products, with it
+// it is level with them (N = 1126 and 4486, cond 4e3).
+//
+// Sums: a product of two digits is at most 2^14, K is at most 256, so the sums of the
+// levels 2..5 (1 to 4 pairs) stay within 2^24 and are exact in the FP32 accumulators.
+// The levels 6..9 weigh 2^-32 and less of the leading one; level 6 (5 pairs) is exact
+// up to the same limit, and 7, 8 and 9 share one accumulator (the digit planes carry
+// their power of two, so a product already has its level's scale): what FP32 rounds
+// there is below 2^-52 of the leading term's unit.
+//
+// One output tile of 128 x 128 is three units of work, each with two accumulators
+// (256 TMEM columns, the units alternate between the two halves of TMEM, so a unit's
+// products run while the one before is drained): levels {4, 5}, {2, 3}, {6, 7-9}.
+// Within a unit, the K chunks of 64 stream their digit tiles through a ring of 13
+// slots of 16 KB, each digit tile of A and of B loaded once per chunk: for s = 1..7
+// the tiles B_t with lmin <= s + t <= lmax slide from high to low t, so four B tiles
+// and one A tile are live (26 tile loads per chunk and output tile against 68 when
+// every pair streams its own).  The epilogue keeps levels 2..5 as one 64-bit integer
+// per entry and adds the rest as an FP32 value: three FP64 operations per entry and
+// K = 256, since the FP64 pipe would otherwise bound the kernel.
+// Output tiles run in super-columns of 12 tile columns, row by row, so the CTAs at
+// work at a time share their digit tiles in L2.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "digits.cuh"
+#include "handles.h"
+#include "tcgen05.cuh"
+
+namespace omg {
+namespace f64d {
+
+using tc::fence_after;
+using tc::fence_before;
+
+constexpr int ND = 7;                             // digits per entry, base 2^8
+constexpr int BT = 128;                           // tile rows and columns
+constexpr int BK = 64;                            // K per chunk: 128-byte swizzled rows
+constexpr int SLOT = BT * BK * 2;                 // 16 KB
+constexpr int STAGES = 13;
+constexpr int EPI_WARPS = 16;
+constexpr int THREADS = 64 + EPI_WARPS * 32;      // 576
+constexpr int SMEM_BYTES = STAGES * SLOT + 1024;
+constexpr uint32_t TMEM_COLS = 512;
+constexpr int SUPER = 12;                         // tile columns per super-column
+constexpr int EXP_ZERO = -(1 << 20);              // exponent of a zero row: its scale flushes to zero
+constexpr int EXP_NAN = 1 << 20;                  // a row with an infinity or a NaN: its outputs become NaN
+
+static inline void check(const char* what) {
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) throw Error(OMG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+    count_launch();
+}
+
+// Digits of PER consecutive entries of a row whose largest magnitude has the bits mb, at the entry's place in plane 0
+// (planes `plane` entries apart); the row's exponent to *ex.
+template <int PER>
+__device__ __forceinline__ void row_digits(const double (&x)[PER], unsigned long long mb, __nv_bfloat16* o, int64_t plane,
+                                           int* ex) {
+    // |x| < 2^e0 for every entry; the digits represent x 2^-(e0 + 1), below one half, so the first stays within 128
+    const int be = (int)(mb >> 52);
+    const bool finite = be < 0x7FF;
+    const int e = mb == 0 ? EXP_ZERO : (finite ? (be ? be : 1) - 1021 : EXP_NAN);
+    if (ex) *ex = e;
+    const int sh = mb == 0 || !finite ? 0 : 8 * ND - e;
+    constexpr long long BIAS = 0x0000808080808080ll;   // 128 sum_{j < 6} 2^(8 j): balanced digits without carries
+#pragma unroll
+    for (int i0 = 0; i0 < PER; i0 += 8) {
+        long long Z[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) Z[u] = (finite ? tcr::scaled_rn(x[i0 + u], sh) : 0ll) + BIAS;
+#pragma unroll
+        for (int s = 0; s < ND; ++s) {
+            const int bit = 8 * (ND - 1 - s);
+            const float scale = __int_as_float((127 - 8 * s) << 23);
+            unsigned f[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int d = s == 0 ? (int)(Z[u] >> bit) : (int)((unsigned)(Z[u] >> bit) & 255u) - 128;
+                f[u] = __float_as_uint((__int_as_float(0x4B400000 + d) - 12582912.0f) * scale);
+            }
+            *reinterpret_cast<uint4*>(o + (int64_t)s * plane + i0) =
+                make_uint4(__byte_perm(f[0], f[1], 0x7632), __byte_perm(f[2], f[3], 0x7632),
+                           __byte_perm(f[4], f[5], 0x7632), __byte_perm(f[6], f[7], 0x7632));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Digits of the rows of a column-major m x K block (K a multiple of 128, up to
+// 256): plane s - 1 holds a_s 2^(-8 (s - 1)) in bf16 (exact), rows of `ldk`
+// entries; ex[i]: the row's exponent.  A CTA takes 32 rows, lanes along them
+// (coalesced reads of the columns), eight groups of K / 8 consecutive columns.
+// ---------------------------------------------------------------------------
+template <int K>
+__global__ void __launch_bounds__(256) row_digits_kernel(const double* __restrict__ A, int64_t lda, int64_t m, int k,
+                                                         int64_t rows_per_plane, __nv_bfloat16* out, int* ex) {
+    constexpr int PER = K / 8;
+    __shared__ unsigned long long red[8][32];
+    const int lane = threadIdx.x % 32, grp = threadIdx.x / 32;
+    const int64_t row = (int64_t)blockIdx.x * 32 + lane;
+    double x[PER];
+    unsigned long long mb = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int c = grp * PER + i;
+        x[i] = row < m && c < k ? A[row + (int64_t)c * lda] : 0.0;
+        mb = max(mb, (unsigned long long)__double_as_longlong(x[i]) & 0x7FFFFFFFFFFFFFFFull);
+    }
+    red[grp][lane] = mb;
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < 8; ++g) mb = max(mb, red[g][lane]);
+    if (row >= m) return;
+    row_digits<PER>(x, mb, out + row * K + grp * PER, rows_per_plane * K, grp == 0 ? ex + row : nullptr);
+}
+
+// ---------------------------------------------------------------------------
+// The product kernel
+// ---------------------------------------------------------------------------
+// Instruction descriptor: D = F32, A = B = BF16, both K-major, M = N = 128.
+constexpr uint32_t IDESC =
+    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BT >> 3) << 17) | ((uint32_t)(BT >> 4) << 24);
+
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+            tmem),
+        "l"(a), "l"(b), "r"(IDESC), "r"(accumulate));
+}
+
+// The order of a unit's tiles (levels LMIN..LMAX): step s = 1..smax loads the B_t not yet loaded, then A_s, and
+// multiplies A_s by B_t for t = tlo(s)..thi(s).
+template <int LMIN, int LMAX>
+struct Unit {
+    __host__ __device__ static constexpr int least(int a, int b) { return a < b ? a : b; }
+    static constexpr int smax = LMAX - 1 < ND ? LMAX - 1 : ND;
+    __host__ __device__ static constexpr int tlo(int s) { return LMIN - s > 1 ? LMIN - s : 1; }
+    __host__ __device__ static constexpr int thi(int s) { return least(LMAX - s, ND); }
+    // the steps that use B_t first and last
+    __host__ __device__ static constexpr int first_use(int t) { return t >= tlo(1) ? 1 : LMIN - t; }
+    __host__ __device__ static constexpr int last_use(int t) { return least(LMAX - t, smax); }
+    // positions of B_t and A_s in the load order
+    __host__ __device__ static constexpr int pos_b(int t) { return first_use(t) - 1 + thi(1) - t; }
+    __host__ __device__ static constexpr int pos_a(int s) { return s - 1 + thi(1) - tlo(s) + 1; }
+    static constexpr int loads = smax + thi(1);
+};
+
+struct Ring {
+    uint32_t slot, phase;   // of the next load
+    __device__ __forceinline__ void at(int pos, uint32_t& s, uint32_t& ph) const {
+        s = slot + pos;
+        ph = phase;
+        if (s >= STAGES) {
+            s -= STAGES;
+            ph ^= 1u;
+        }
+        if (s >= STAGES) {   // (a unit's loads can pass the end twice)
+            s -= STAGES;
+            ph ^= 1u;
+        }
+    }
+    __device__ __forceinline__ void advance(int n) {
+        uint32_t s, p;
+        at(n, s, p);
+        slot = s;
+        phase = p;
+    }
+};
+
+struct Shared {
+    uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2], fin;
+    uint32_t tmem;
+    volatile int abort;
+    uint32_t issued[STAGES], consumed[STAGES];   // loads issued into / waited for in each slot
+};
+
+template <int LMIN, int LMAX>
+__device__ __forceinline__ bool load_chunk(Shared& sh, Ring& r, uint32_t sbase, const CUtensorMap* tA,
+                                           const CUtensorMap* tB, int x, int ya, int yb, int ra, int rb) {
+    using U = Unit<LMIN, LMAX>;
+    auto load = [&](const CUtensorMap* map, int pos, int y) -> bool {
+        uint32_t s, ph;
+        r.at(pos, s, ph);
+        if (!tc::wait_or_abort(&sh.empty[s], ph ^ 1u, &sh.abort)) return false;
+        dev::mbar_expect_tx(&sh.full[s], SLOT);
+        tc::tma_load_2d(sbase + s * SLOT, map, x, y, &sh.full[s]);
+        ++sh.issued[s];
+        return true;
+    };
+#pragma unroll
+    for (int s = 1; s <= U::smax; ++s) {
+#pragma unroll
+        for (int t = U::thi(s); t >= U::tlo(s); --t)
+            if (U::first_use(t) == s && !load(tB, U::pos_b(t), (t - 1) * rb + yb)) return false;
+        if (!load(tA, U::pos_a(s), (s - 1) * ra + ya)) return false;
+    }
+    r.advance(U::loads);
+    return true;
+}
+
+// The products of one chunk; levels LMIN into accumulator 0, the others into accumulator 1.
+template <int LMIN, int LMAX>
+__device__ __forceinline__ bool mma_chunk(Shared& sh, Ring& r, uint32_t sbase, uint32_t acc, bool first) {
+    using U = Unit<LMIN, LMAX>;
+    auto wait = [&](int pos, uint32_t& s) -> bool {
+        uint32_t ph;
+        r.at(pos, s, ph);
+        if (!tc::wait_or_abort(&sh.full[s], ph, &sh.abort)) return false;
+        ++sh.consumed[s];
+        return true;
+    };
+    uint32_t fresh = first ? 3u : 0u;   // accumulators not yet written in this unit
+#pragma unroll
+    for (int s = 1; s <= U::smax; ++s) {
+        uint32_t sa, sb, ph;
+#pragma unroll
+        for (int t = U::thi(s); t >= U::tlo(s); --t)
+            if (U::first_use(t) == s && !wait(U::pos_b(t), sb)) return false;
+        if (!wait(U::pos_a(s), sa)) return false;
+        fence_after();
+        const uint64_t dA = tc::sdesc_sw128(sbase + sa * SLOT);
+#pragma unroll
+        for (int t = U::thi(s); t >= U::tlo(s); --t) {
+            r.at(U::pos_b(t), sb, ph);
+            const uint64_t dB = tc::sdesc_sw128(sbase + sb * SLOT);
+            const int a = s + t == LMIN ? 0 : 1;
+#pragma unroll
+            for (int kk = 0; kk < BK / 16; ++kk) {
+                const uint64_t off = (uint64_t)(kk * 32) >> 4;   // 16 bf16 = 32 bytes
+                mma_bf16(acc + a * BT, dA + off, dB + off, (fresh >> a) & 1u ? 0u : 1u);
+                fresh &= ~(1u << a);
+            }
+        }
+        tc::mma_commit(&sh.empty[sa]);
+#pragma unroll
+        for (int t = U::thi(s); t >= U::tlo(s); --t)
+            if (U::last_use(t) == s) {
+                r.at(U::pos_b(t), sb, ph);
+                tc::mma_commit(&sh.empty[sb]);
+            }
+    }
+    r.advance(U::loads);
+    return true;
+}
+
+// Output tile number t of the walk: super-columns of SUPER tile columns, row by row inside.  `lower`: only tiles
+// with row >= column.
+struct Walk {
+    int mt, nt, lower;
+    int64_t base = 0;   // first tile number of super-column J
+    int J = 0;
+    __device__ __forceinline__ int width(int j) const { return min(SUPER, nt - j * SUPER); }
+    __device__ __forceinline__ int64_t count(int j) const {
+        const int w = width(j);
+        if (!lower) return (int64_t)mt * w;
+        return (int64_t)(mt - j * SUPER) * w - (int64_t)w * (w - 1) / 2;
+    }
+    __device__ __forceinline__ void tile(int64_t t, int& i, int& j) {
+        while (t >= base + count(J)) {
+            base += count(J);
+            ++J;
+        }
+        int64_t o = t - base;
+        const int w = width(J);
+        if (!lower) {
+            i = (int)(o / w);
+            j = J * SUPER + (int)(o % w);
+            return;
+        }
+        int r = 0;   // rows J SUPER + r with r + 1 < w tiles
+        while (r + 1 < w && o > r) {
+            o -= r + 1;
+            ++r;
+        }
+        if (r + 1 >= w) {
+            r += (int)(o / w);
+            o %= w;
+        }
+        i = J * SUPER + r;
+        j = J * SUPER + (int)o;
+    }
+};
+
+__global__ void __launch_bounds__(THREADS, 1)
+    digit_update_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, int64_t M,
+                        int64_t Nc, int nchunk, int ra, int rb, const int* __restrict__ exA,
+                        const int* __restrict__ exB, double* C, int64_t ldc, int lower, int64_t ntiles, int* err) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    __shared__ __align__(8) Shared sh;
+    const uint32_t sbase = (dev::smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            dev::mbar_init(&sh.full[s], 1);
+            dev::mbar_init(&sh.empty[s], 1);
+            sh.issued[s] = sh.consumed[s] = 0;
+        }
+        for (int a = 0; a < 2; ++a) {
+            dev::mbar_init(&sh.tfull[a], 1);
+            dev::mbar_init(&sh.tempty[a], EPI_WARPS);
+        }
+        dev::mbar_init(&sh.fin, 1);
+        sh.abort = 0;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dev::smem_u32(&sh.tmem)),
+                     "r"(TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = sh.tmem;
+    Walk walk{(int)((M + BT - 1) / BT), (int)((Nc + BT - 1) / BT), lower};
+
+    if (warp == 0) {
+        if (lane == 0) {   // ---- TMA producer
+            Ring r{0, 0};
+            bool ok = true;
+            for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+                int i, j;
+                walk.tile(t, i, j);
+                const int ya = i * BT, yb = j * BT;
+                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<4, 5>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<2, 3>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<6, 9>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+            }
+            if (!ok) sh.abort = 1;
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {   // ---- MMA issuer
+            Ring r{0, 0};
+            bool ok = true;
+            uint32_t lu = 0;
+            auto begin = [&](uint32_t& half) -> bool {
+                half = lu & 1u;
+                const bool go = tc::wait_or_abort(&sh.tempty[half], ((lu >> 1) & 1u) ^ 1u, &sh.abort);
+                fence_after();
+                return go;
+            };
+            for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+                uint32_t h;
+                ok = begin(h);
+                for (int c = 0; c < nchunk && ok; ++c) ok = mma_chunk<4, 5>(sh, r, sbase, tmem + h * 256, c == 0);
+                if (!ok) break;
+                tc::mma_commit(&sh.tfull[h]);
+                ++lu;
+                ok = begin(h);
+                for (int c = 0; c < nchunk && ok; ++c) ok = mma_chunk<2, 3>(sh, r, sbase, tmem + h * 256, c == 0);
+                if (!ok) break;
+                tc::mma_commit(&sh.tfull[h]);
+                ++lu;
+                ok = begin(h);
+                for (int c = 0; c < nchunk && ok; ++c) ok = mma_chunk<6, 9>(sh, r, sbase, tmem + h * 256, c == 0);
+                if (!ok) break;
+                tc::mma_commit(&sh.tfull[h]);
+                ++lu;
+            }
+            if (!ok) sh.abort = 1;
+            tc::mma_commit(&sh.fin);
+            if (!dev::mbar_wait_bounded(&sh.fin, 0)) sh.abort = 1;
+        }
+    } else {   // ---- epilogue: warp w owns TMEM lanes 32 (w % 4) .. +31 and columns 32 ((w - 2) / 4) .. +31
+        const int q = warp & 3, c0 = ((warp - 2) >> 2) * 32;
+        const uint32_t lanes = (uint32_t)(q * 32) << 16;
+        uint32_t lu = 0;
+        auto begin = [&]() -> bool {
+            bool ok = tc::wait_or_abort(&sh.tfull[lu & 1u], (lu >> 1) & 1u, &sh.abort);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok && lane == 0) sh.abort = 1;
+            fence_after();
+            return ok;
+        };
+        auto end = [&]() {
+            fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&sh.tempty[lu & 1u]);
+            ++lu;
+        };
+        for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+            int ti, tj;
+            walk.tile(t, ti, tj);
+            const int64_t row = (int64_t)ti * BT + q * 32 + lane, col0 = (int64_t)tj * BT + c0;
+            long long H[32];   // levels 2..5 in units of level 5
+            if (!begin()) break;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t a[16], b[16];
+                tc::tmem_ld16(tmem + lanes + (lu & 1u) * 256 + c0 + h * 16, a);
+                tc::tmem_ld16(tmem + lanes + (lu & 1u) * 256 + BT + c0 + h * 16, b);
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    H[h * 16 + j] = ((long long)__float2int_rn(__uint_as_float(a[j]) * 0x1p16f) << 8) +
+                                    __float2int_rn(__uint_as_float(b[j]) * 0x1p24f);
+            }
+            end();
+            if (!begin()) break;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t a[16], b[16];
+                tc::tmem_ld16(tmem + lanes + (lu & 1u) * 256 + c0 + h * 16, a);
+                tc::tmem_ld16(tmem + lanes + (lu & 1u) * 256 + BT + c0 + h * 16, b);
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    H[h * 16 + j] += ((long long)__float2int_rn(__uint_as_float(a[j])) << 24) +
+                                     ((long long)__float2int_rn(__uint_as_float(b[j]) * 0x1p8f) << 16);
+            }
+            end();
+            const int er = row < M ? exA[row] : EXP_ZERO;
+            if (!begin()) break;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                uint32_t a[8], b[8];
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + BT + c0 + h * 8, b);
+                double c[8];
+                bool in[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int64_t col = col0 + h * 8 + j;
+                    in[j] = row < M && col < Nc && !(lower && row < col);
+                    c[j] = in[j] ? C[row + col * ldc] : 0.0;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int64_t col = col0 + h * 8 + j;
+                    if (!in[j]) continue;
+                    // (levels 6..9) 2^24, an FP32 value, widened to FP64 by its bits
+                    const unsigned f = __float_as_uint(__uint_as_float(a[j]) + __uint_as_float(b[j]));
+                    const unsigned long long lo =
+                        (f << 1) == 0u ? 0ull
+                                       : ((unsigned long long)(f & 0x80000000u) << 32) |
+                                             (((unsigned long long)(f & 0x7FFFFFFFu) << 29) + ((896ull + 24ull) << 52));
+                    // levels 2..5: |H| < 2^51 placed in the mantissa of 1.5 2^52
+                    const double hi = __longlong_as_double(0x4338000000000000ll + H[h * 8 + j]) - 6755399441055744.0;
+                    const int e = 1023 + er + __ldg(exB + col) - 40;   // level 5 weighs 2^-40
+                    const long long sb = e > (1 << 19) ? 0x7FF8000000000000ll
+                                                       : (e <= 0 ? 0ll : (long long)min(e, 2047) << 52);
+                    C[row + col * ldc] = fma(-(hi + __longlong_as_double((long long)lo)), __longlong_as_double(sb), c[j]);
+                }
+            }
+            end();
+        }
+    }
+    __syncthreads();
+    if (sh.abort) {
+        if (threadIdx.x == 0) {
+            atomicExch(err, -8 /* OMG_ERR_TIMEOUT */);
+            // copies still in flight land before the shared memory is given up
+            for (int s = 0; s < STAGES; ++s)
+                if (sh.issued[s] != sh.consumed[s]) dev::mbar_wait_bounded(&sh.full[s], (sh.issued[s] - 1u) & 1u);
+        }
+        __syncthreads();
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Diagonal block (n <= 64) of the FP64 Cholesky in one CTA: the lower triangle packed by
+// columns in shared memory, so the trailing update of a step is one run of entries over all
+// lanes.  Warp 0 updates the next column first, takes its pivot's reciprocal square root and
+// scales it while the other warps finish the update: one barrier per column.
+// ---------------------------------------------------------------------------
+constexpr int NBD = 64;
+constexpr int POTRF_THREADS = 256;
+
+__global__ void __launch_bounds__(POTRF_THREADS) potrf64_kernel(double* A, int64_t lda, int n, int* err, int64_t* err_col,
+                                                                int64_t col_offset) {
+    constexpr int NE = NBD * (NBD + 1) / 2;
+    __shared__ double P[NE];
+    __shared__ double l[2][NBD];
+    __shared__ unsigned short ik[NE];
+    const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+    auto off = [](int j) { return j * NBD - j * (j - 1) / 2; };   // start of column j
+    for (int j = warp; j < NBD; j += POTRF_THREADS / 32)
+        for (int i = j + lane; i < NBD; i += 32) {
+            const int e = off(j) + i - j;
+            ik[e] = (unsigned short)(i | (j << 8));
+            P[e] = i < n && j < n ? A[i + (int64_t)j * lda] : (i == j ? 1.0 : 0.0);   // identity past n
+        }
+    __syncthreads();
+    auto pivot = [&](int j) {   // warp 0: column j final; l[j % 2] <- the scaled column
+        double d = P[off(j)];
+        if (!(d > 0.0)) {
+            if (lane == 0 && j < n && atomicCAS(err, 0, -3 /* OMG_ERR_NOT_DEFINITE */) == 0) *err_col = col_offset + j;
+            d = 1.0;
+        }
+        const double r = 1.0 / sqrt(d);
+        __syncwarp();
+        for (int i = j + lane; i < NBD; i += 32) {
+            const double v = i == j ? sqrt(d) : P[off(j) + i - j] * r;
+            P[off(j) + i - j] = v;
+            l[j & 1][i] = v;
+        }
+    };
+    if (warp == 0) pivot(0);
+    __syncthreads();
+    for (int j = 0; j + 1 < NBD; ++j) {
+        const double* lj = l[j & 1];
+        const int e1 = off(j + 1), e2 = off(j + 2);   // column j + 1, then the rest
+        if (warp == 0) {
+            const double lk = lj[j + 1];
+            for (int e = e1 + lane; e < e2; e += 32) P[e] = fma(-lj[j + 1 + e - e1], lk, P[e]);
+            __syncwarp();
+            pivot(j + 1);
+        } else {
+            for (int e = e2 + tid - 32; e < NE; e += POTRF_THREADS - 32) {
+                const int x = ik[e];
+                P[e] = fma(-lj[x & 255], lj[x >> 8], P[e]);
+            }
+        }
+        __syncthreads();
+    }
+    for (int j = warp; j < n; j += POTRF_THREADS / 32)
+        for (int i = j + lane; i < n; i += 32) A[i + (int64_t)j * lda] = P[off(j) + i - j];
+}
+
+// P <- P L^-T for an m x 64 panel P and a 64 x 64 lower L: one row per lane in 64 registers, each solved entry
+// removed from all later ones at once (independent FP64 operations; the pipe's rate bounds it), 32 rows per CTA.
+__global__ void __launch_bounds__(128) trsm64_kernel(int64_t m, const double* __restrict__ L, int64_t ldl, double* P,
+                                                     int64_t ldp) {
+    __shared__ __align__(16) double sL[NBD][NBD];   // sL[j][i] = L(i, j)
+    __shared__ double rd[NBD];
+    for (int e = threadIdx.x; e < NBD * NBD; e += 128) {
+        const int i = e % NBD, j = e / NBD;
+        sL[j][i] = i >= j ? L[i + (int64_t)j * ldl] : 0.0;
+    }
+    __syncthreads();
+    if (threadIdx.x < NBD) rd[threadIdx.x] = 1.0 / sL[threadIdx.x][threadIdx.x];
+    __syncthreads();
+    const int64_t row = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    if (threadIdx.x >= 32 || row >= m) return;
+    double x[NBD];
+#pragma unroll
+    for (int j = 0; j < NBD; ++j) x[j] = P[row + (int64_t)j * ldp];
+#pragma unroll
+    for (int j = 0; j < NBD; ++j) {
+        x[j] *= rd[j];
+#pragma unroll
+        for (int i = j + 1; i < NBD; ++i) x[i] = fma(-x[j], sL[j][i], x[i]);
+        P[row + (int64_t)j * ldp] = x[j];
+    }
+}
+
+}  // namespace f64d
+
+
+// Digit rows of a column-major m x k block (k <= kpad; kpad 128 or 256): 7 planes of rows_per_plane rows of kpad bf16.
+void row_digits_f64(const double* A, int64_t lda, int64_t m, int k, int kpad, int64_t rows_per_plane, void* out, int* ex,
+                    cudaStream_t s) {
+    if (m <= 0) return;
+    if ((kpad != 128 && kpad != 256) || k > kpad || rows_per_plane < m) throw Error(OMG_ERR_INVALID, "row digits: bad layout");
+    ProfScope prof_("f64_digits", s);
+    const unsigned grid = (unsigned)((m + 31) / 32);
+    auto kern = kpad == 128 ? f64d::row_digits_kernel<128> : f64d::row_digits_kernel<256>;
+    kern<<<grid, 256, 0, s>>>(A, lda, m, k, rows_per_plane, static_cast<__nv_bfloat16*>(out), ex);
+    f64d::check("FP64 row digits");
+}
+
+// C (M x Nc, column-major; `lower`: entries with row >= column only) -= A B^T from digit rows of kpad entries:
+// A's planes start at row a0 of buffers of ra rows per plane, B's at b0 of rb.
+void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
+                      const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, bool lower,
+                      int* err, cudaStream_t s, const char* name) {
+    if (M <= 0 || Nc <= 0) return;
+    if (kpad % f64d::BK || kpad > 256 || 7 * std::max(ra, rb) > (1ll << 30))
+        throw Error(OMG_ERR_UNSUPPORTED, "digit update: bad sizes");
+    ProfScope prof_(name, s);
+    static int n_sm = 0;
+    if (!n_sm) {
+        cudaFuncSetAttribute(f64d::digit_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f64d::SMEM_BYTES);
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        n_sm = n > 0 ? n : 1;
+    }
+    const CUtensorMap mA = tc::make_map_2d(static_cast<const uint16_t*>(A) + a0 * kpad, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                                           2, f64d::ND * ra - a0, kpad, kpad, f64d::BK, f64d::BT);
+    const CUtensorMap mB = tc::make_map_2d(static_cast<const uint16_t*>(B) + b0 * kpad, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                                           2, f64d::ND * rb - b0, kpad, kpad, f64d::BK, f64d::BT);
+    const int64_t mt = (M + f64d::BT - 1) / f64d::BT, nt = (Nc + f64d::BT - 1) / f64d::BT;
+    const int64_t ntiles = lower ? mt * nt - nt * (nt - 1) / 2 : mt * nt;
+    const unsigned grid = (unsigned)std::min<int64_t>(ntiles, n_sm);
+    f64d::digit_update_kernel<<<grid, f64d::THREADS, f64d::SMEM_BYTES, s>>>(
+        mA, mB, M, Nc, kpad / f64d::BK, (int)ra, (int)rb, exA + a0, exB + b0, C, ldc, lower ? 1 : 0, ntiles, err);
+    f64d::check(name);
+}
+
+// In place: the lower triangle of an n x n block (n <= 64) by its Cholesky factor.
+void potrf64(double* A, int64_t lda, int n, int* err, int64_t* err_col, int64_t col_offset, cudaStream_t s) {
+    ProfScope prof_("potrf64", s);
+    f64d::potrf64_kernel<<<1, f64d::POTRF_THREADS, 0, s>>>(A, lda, n, err, err_col, col_offset);
+    f64d::check("potrf64");
+}
+
+// P (m x 64) <- P L^-T.
+void trsm64(int64_t m, const double* L, int64_t ldl, double* P, int64_t ldp, cudaStream_t s) {
+    if (m <= 0) return;
+    ProfScope prof_("trsm64", s);
+    f64d::trsm64_kernel<<<(unsigned)((m + 31) / 32), 128, 0, s>>>(m, L, ldl, P, ldp);
+    f64d::check("trsm64");
+}
+
+}  // namespace omg
+
+// Test hook (not part of the public header): C -= A B^T through the digits and the tensor-core kernel; A M x k, B Nc x k,
+// C M x Nc (column-major FP64 device pointers, leading dimensions M, Nc, M), k <= 256.
+extern "C" int omg_internal_digit_update(int64_t M, int64_t Nc, int k, const double* A, const double* B, double* C,
+                                         int lower, int* err) {
+    try {
+        const int kpad = k <= 128 ? 128 : 256;
+        cudaStream_t s = 0;
+        DevBuf da((size_t)7 * M * kpad * 2, s), db((size_t)7 * Nc * kpad * 2, s), ea((size_t)M * 4, s), eb((size_t)Nc * 4, s);
+        omg::row_digits_f64(A, M, M, k, kpad, M, da.p, ea.as<int>(), s);
+        omg::row_digits_f64(B, Nc, Nc, k, kpad, Nc, db.p, eb.as<int>(), s);
+        omg::digit_update_f64(M, Nc, kpad, da.p, M, 0, ea.as<int>(), db.p, Nc, 0, eb.as<int>(), C, M, lower != 0, err, s,
+                              "digit_update");
+        return cudaDeviceSynchronize() == cudaSuccess ? 0 : -2;
+    } catch (const omg::Error& e) {
+        return e.code;
+    }
+}
+
+// Test hook: Cholesky of the n x n (n <= 64) A and P <- P L^-T for the m x 64 P (used when n is 64).
+extern "C" int omg_internal_potrf_trsm64(int n, double* A, int64_t m, double* P, int* err, int64_t* err_col) {
+    try {
+        omg::potrf64(A, n, n, err, err_col, 0, 0);
+        if (n == 64) omg::trsm64(m, A, n, P, m, 0);
+        return cudaDeviceSynchronize() == cudaSuccess ? 0 : -2;
+    } catch (const omg::Error& e) {
+        return e.code;
+    }
+}

@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "digits.cuh"
 #include "handles.h"
 #include "tcgen05.cuh"
 
@@ -303,31 +304,6 @@ __global__ void sum_groups_kernel(int64_t n, int64_t k, int ng, const double* __
 // balanced base-2^beta digits (first |d| <= 2^beta, others <= 2^(beta-1)), written as bf16
 // row c of digit plane d: out[(d * rows_per_plane + c) * ldo + j], zero for
 // n <= j < ldo.  Columns c >= ncol (up to rows_per_plane) are zero.
-// x 2^k rounded to the nearest integer (ties to even), exactly, by integer
-// arithmetic on the bits of x (|x 2^k| < 2^62): the same value as
-// __double2ll_rn(x * 2^k) without the FP64 pipe.
-__device__ __forceinline__ long long scaled_rn(double x, int k) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const int E = (int)((b >> 52) & 0x7FF);
-    const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (E ? (1ull << 52) : 0ull);
-    const int sh = (E ? E : 1) - 1075 + k;   // |x 2^k| = m 2^sh
-    unsigned long long q;
-    if (sh >= 0) {
-        q = m << sh;
-    } else if (sh < -63) {
-        q = 0;   // below 2^-11
-    } else {
-        // t = m >> (r - 1) keeps the half bit as its lowest bit; the bits below it are the sticky part:
-        // round up when the half bit is set and (anything below it is set, or q is odd)
-        const int r1 = -sh - 1;
-        const unsigned long long t = m >> r1;
-        const unsigned long long sticky = (m & ((1ull << r1) - 1ull)) != 0ull ? 1ull : 0ull;
-        q = t >> 1;
-        q += t & (sticky | q) & 1ull;
-    }
-    return (b >> 63) ? -(long long)q : (long long)q;
-}
-
 // bf16 bits of a small integer (|r| < 2^8, exact in bf16): 1.5 * 2^23 + r
 // has r in its low mantissa bits, the subtraction leaves float(r) exactly.
 __device__ __forceinline__ unsigned short small_int_bf16(long long r) {
