@@ -100,9 +100,6 @@ void residual_df64(int64_t M, int64_t N, int64_t K, const float* Ahi, const floa
                    const float* Xhi, const float* Xlo, int64_t ldx, const double* B, int64_t ldb, double* R,
                    int64_t ldr, cudaStream_t s);
 void split_f64(int64_t m, int64_t n, const double* A, int64_t lda, float* H, float* L, int64_t ldo, cudaStream_t s);
-template <typename T>
-void trsm_cols(int64_t nrhs, int n, const T* L, int64_t ldl, bool trans, T* B, int64_t ldb, cudaStream_t s,
-               const T* Lr = nullptr);
 // tc_gemm.cu
 void gemm_tf32x3(int64_t M, int64_t N, int64_t K, float alpha, const float* Ah, const float* Al, int64_t lda,
                  int64_t a_kext, int64_t a_k0, const float* Bh, const float* Bl, int64_t ldb, int64_t b_kext,
@@ -146,6 +143,9 @@ void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra
                       int* err, cudaStream_t s, const char* name);
 void potrf64(double* A, int64_t lda, int n, int* err, int64_t* err_col, int64_t col_offset, cudaStream_t s);
 void trsm64(int64_t m, const double* L, int64_t ldl, double* P, int64_t ldp, cudaStream_t s);
+void inverse_blocks_f64(int64_t n, const double* L, int64_t ld, double* Inv, double* InvT, cudaStream_t s);
+void solve_f64(int64_t n, int64_t nP, const double* L, int64_t ld, const double* Inv, const double* InvT, double* B,
+               int64_t ldb, int64_t nrhs, int* err, cudaStream_t s);
 // tc_solve.cu
 size_t sweep_scratch_bytes(int64_t nblocks, int64_t nrhs);
 void solve_sweep_tc(bool backward, int64_t N, int64_t nblocks, const float* W, int64_t w_rows, const float* A,
@@ -934,27 +934,6 @@ static void solve_ldlt_tc(omg_solver sv, float* B, int64_t ldb, int64_t nrhs) {
     apply_inv_blocks((int64_t)nblocks, nb, n_last, nrhs, sv->Linv32.as<float>(), true, B, ldb, s);
 }
 
-// In place: B <- HM^-1 B (internal numbering), HM = L diag(+I_P, -I_V) L^T.
-template <typename T>
-static void solve_ldlt(omg_solver sv, const T* A, int64_t ld, T* B, int64_t ldb, int64_t nrhs) {
-    cudaStream_t s = sv->ctx->stream;
-    const int64_t N = sv->N;
-    const size_t nblocks = sv->bounds.size() - 1;
-    for (size_t b = 0; b < nblocks; ++b) {   // L y = b
-        const int64_t k0 = sv->bounds[b], k1 = sv->bounds[b + 1], nk = k1 - k0;
-        trsm_cols<T>(nrhs, (int)nk, A + k0 + k0 * ld, ld, false, B + k0, ldb, s);
-        if (k1 < N) gemm<T>(N - k1, nrhs, nk, T(-1), A + k1 + k0 * ld, ld, false, B + k0, ldb, false, T(1), B + k1, ldb, s);
-    }
-    negate_rows<T>(B, ldb, sv->nP, N, nrhs, s);
-    // L^T x = y, right-looking: once block k is solved, remove its
-    // contribution from all earlier blocks (K = block size, M = k0).
-    for (size_t bb = nblocks; bb-- > 0;) {
-        const int64_t k0 = sv->bounds[bb], k1 = sv->bounds[bb + 1], nk = k1 - k0;
-        trsm_cols<T>(nrhs, (int)nk, A + k0 + k0 * ld, ld, true, B + k0, ldb, s);
-        if (k0 > 0) gemm<T>(k0, nrhs, nk, T(-1), A + k0, ld, true, B + k0, ldb, false, T(1), B, ldb, s);
-    }
-}
-
 // A current barrier that encloses a non-conductive hole (a barrier mesh that is
 // not outermost, geometry.cpp:424-461) leaves the constant potential on its
 // vertices in the head matrix's null space: the N block of a closed mesh and
@@ -986,6 +965,9 @@ void solver_factor(omg_solver sv, DevBuf&& hm, bool check) {
     if (sv->precision == OMG_PREC_FP64) {
         sv->A64 = std::move(hm);
         factor_ldlt_f64(sv, sv->A64.as<double>(), N);
+        const int64_t inv = (N + 127) / 128 * 128 * 128;
+        sv->Linv64 = DevBuf((size_t)2 * inv * 8, s, sv->persistent);
+        inverse_blocks_f64(N, sv->A64.as<double>(), N, sv->Linv64.as<double>(), sv->Linv64.as<double>() + inv, s);
     } else {
         sv->ld32 = (N + 31) / 32 * 32;
         sv->A32 = DevBuf((size_t)sv->ld32 * N * sizeof(float), s, sv->persistent);
@@ -1039,6 +1021,7 @@ void solver_factor_or_pivot(omg_solver sv, DevBuf&& hm, const std::function<DevB
     // a pivot of the wrong sign: the whole matrix, rebuilt, by LU with partial pivoting in FP64
     cudaStream_t s = sv->ctx->stream;
     sv->A64.release();
+    sv->Linv64.release();
     sv->A32.release();
     sv->A32r.release();
     sv->W.release();
@@ -1210,6 +1193,7 @@ static void solve_mixed_or_fp64(omg_solver sv, double* B, int64_t ldb, int64_t n
     sv->Adig.release();
     sv->rexp.release();
     sv->A64.release();
+    sv->Linv64.release();
     sv->w_off.clear();
     sv->precision = OMG_PREC_FP64;
     solver_factor_or_pivot(sv, sv->rebuild(), sv->rebuild);
@@ -1225,7 +1209,9 @@ void solver_solve_internal(omg_solver sv, double* B, int64_t ldb, int64_t nrhs) 
         sv->last_residual = 0.0;
         sv->last_correction = 0.0;
     } else if (sv->precision == OMG_PREC_FP64)
-        solve_ldlt<double>(sv, sv->A64.as<double>(), sv->N, B, ldb, nrhs);
+        solve_f64(sv->N, sv->nP, sv->A64.as<double>(), sv->N, sv->Linv64.as<double>(),
+                  sv->Linv64.as<double>() + (sv->N + 127) / 128 * 128 * 128, B, ldb, nrhs, sv->ctx->d_err,
+                  sv->ctx->stream);
     else
         solve_mixed_or_fp64(sv, B, ldb, nrhs);
 }
@@ -2217,15 +2203,15 @@ int omg_solver_solve_dev(omg_solver sv, double* b, int64_t ldb, int64_t nrhs) {
         DevBuf X((size_t)N * nrhs * 8, s);
         double* x = X.as<double>();
         OMG_CUDA(cudaMemsetAsync(x, 0, (size_t)N * nrhs * 8, s));
-        for (int64_t j = 0; j < nrhs; ++j) {
-            OMG_CUDA(cudaMemcpyAsync(x + j * N, b + j * ldb + nv, (size_t)nPt * 8, cudaMemcpyDeviceToDevice, s));
-            OMG_CUDA(cudaMemcpyAsync(x + j * N + nP, b + j * ldb, (size_t)nv * 8, cudaMemcpyDeviceToDevice, s));
-        }
+        auto rows = [&](double* dst, int64_t ldd, const double* src, int64_t lds, int64_t n) {
+            if (n > 0 && nrhs > 0)
+                OMG_CUDA(cudaMemcpy2DAsync(dst, ldd * 8, src, lds * 8, n * 8, nrhs, cudaMemcpyDeviceToDevice, s));
+        };
+        rows(x, N, b + nv, ldb, nPt);
+        rows(x + nP, N, b, ldb, nv);
         solver_solve_internal(sv, x, N, nrhs);
-        for (int64_t j = 0; j < nrhs; ++j) {
-            OMG_CUDA(cudaMemcpyAsync(b + j * ldb + nv, x + j * N, (size_t)nPt * 8, cudaMemcpyDeviceToDevice, s));
-            OMG_CUDA(cudaMemcpyAsync(b + j * ldb, x + j * N + nP, (size_t)nv * 8, cudaMemcpyDeviceToDevice, s));
-        }
+        rows(b + nv, ldb, x, N, nPt);
+        rows(b, ldb, x + nP, N, nv);
         OMG_CUDA(cudaStreamSynchronize(s));
     });
 }

@@ -1,6 +1,6 @@
 // Dense kernels for the head-matrix solve: a register-tiled GEMM (FP64 and
-// FP32 CUDA cores), the diagonal-block Cholesky + triangular inverse of the
-// quasi-definite LDL^T, and small matrix utilities.
+// FP32 CUDA cores), the diagonal-block Cholesky + triangular inverse of the FP32
+// quasi-definite LDL^T (the FP64 one is in f64_digits.cu), and small matrix utilities.
 //
 // The factorization replaces the reference's packed Bunch-Kaufman inverse
 // (SymMatrix::invert / solveLin -> DSPTRF/DSPTRI/DSPTRS,
@@ -405,82 +405,6 @@ void split_f64(int64_t m, int64_t n, const double* A, int64_t lda, float* H, flo
     split_f64_kernel<<<grid, 256, 0, s>>>(m, n, A, lda, H, L, ldo);
     check("split_f64");
 }
-
-// ---------------------------------------------------------------------------
-// Triangular solves with a diagonal block L (n x n lower, staged in shared
-// memory).  Panel form (rows independent):  W = P L^-T  for P (m x n).
-// Column form (columns independent):       B <- L^-1 B  or  L^-T B.
-// Each row / column is one warp: the substitution runs serially over the
-// block, the inner products across the 32 lanes.
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256) trsm_cols_kernel(int64_t nrhs, int n, const T* __restrict__ L, int64_t ldl,
-                                                        const T* __restrict__ Lr, int trans, T* B, int64_t ldb) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T* sL = reinterpret_cast<T*>(smraw);   // n x n, sL[j*n + l] = (trans ? L[l][j] : L[j][l]) for the used part
-    T* sx = sL + n * n;
-    for (int e = threadIdx.x; e < n * n; e += 256) {   // coalesced: r runs down column c of L
-        const int r = e % n, c = e / n;
-        const T v = (r >= c) ? (Lr ? L[r + c * ldl] + Lr[r + c * ldl] : L[r + c * ldl]) : T(0);
-        if (trans)
-            sL[c * n + r] = v;   // (L^T)[c][r]
-        else
-            sL[r * n + c] = v;   // L[r][c]
-    }
-    __syncthreads();
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    T* x = sx + warp * n;
-    for (int64_t col = (int64_t)blockIdx.x * 8 + warp; col < nrhs; col += (int64_t)gridDim.x * 8) {
-        T* b = B + col * ldb;
-        for (int l = lane; l < n; l += 32) x[l] = b[l];
-        __syncwarp();
-        if (!trans) {   // L x = b, forward
-            for (int j = 0; j < n; ++j) {
-                T acc = T(0);
-                for (int l = lane; l < j; l += 32) acc += sL[j * n + l] * x[l];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                if (lane == 0) x[j] = (x[j] - acc) / sL[j * n + j];
-                __syncwarp();
-            }
-        } else {        // L^T x = b, backward: row j of L^T is column j of L
-            for (int j = n - 1; j >= 0; --j) {
-                T acc = T(0);
-                for (int l = j + 1 + lane; l < n; l += 32) acc += sL[j * n + l] * x[l];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                if (lane == 0) x[j] = (x[j] - acc) / sL[j * n + j];
-                __syncwarp();
-            }
-        }
-        for (int l = lane; l < n; l += 32) b[l] = x[l];
-        __syncwarp();
-    }
-}
-
-template <typename T>
-static void set_max_smem(const void* f) {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-}
-
-template <typename T>
-void trsm_cols(int64_t nrhs, int n, const T* L, int64_t ldl, bool trans, T* B, int64_t ldb, cudaStream_t s,
-               const T* Lr) {
-    if (nrhs <= 0) return;
-    ProfScope prof_("trsm_cols", s);
-    static bool attr = false;
-    if (!attr) {
-        set_max_smem<T>((const void*)trsm_cols_kernel<T>);
-        attr = true;
-    }
-    const size_t sm = ((size_t)n * n + 8 * (size_t)n) * sizeof(T);
-    const unsigned grid = (unsigned)std::min<int64_t>((nrhs + 7) / 8, 152 * 8);
-    trsm_cols_kernel<T><<<grid, 256, sm, s>>>(nrhs, n, L, ldl, Lr, trans ? 1 : 0, B, ldb);
-    check("trsm_cols");
-}
-template void trsm_cols<double>(int64_t, int, const double*, int64_t, bool, double*, int64_t, cudaStream_t,
-                                const double*);
-template void trsm_cols<float>(int64_t, int, const float*, int64_t, bool, float*, int64_t, cudaStream_t, const float*);
 
 // Max-norm of each column of an m x n FP32 matrix scaled by colscale, and of
 // an FP64 matrix: one CTA per column (for the refinement stopping test).

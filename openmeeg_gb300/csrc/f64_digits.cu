@@ -40,6 +40,10 @@
 #include "tcgen05.cuh"
 
 namespace omg {
+
+template <typename T>
+void negate_rows(T* B, int64_t ldb, int64_t r0, int64_t r1, int64_t n, cudaStream_t s);
+
 namespace f64d {
 
 using tc::fence_after;
@@ -559,6 +563,172 @@ __global__ void __launch_bounds__(128) trsm64_kernel(int64_t m, const double* __
     }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 solves by 128-row blocks: the diagonal blocks' inverses, their products with the
+// right-hand sides, and the digits of everything the updates between blocks take.
+// ---------------------------------------------------------------------------
+constexpr int NBS = 128;
+
+// Digits of K = 128 consecutive entries held by a warp (lane: entries 4 lane .. 4 lane + 3), written to row `row` of
+// the planes.  mb: the largest magnitude's bits over the row.
+__device__ __forceinline__ void write_digits4(const double x[4], unsigned long long mb, __nv_bfloat16* out,
+                                              int64_t rows_per_plane, int64_t row, int* ex, int lane) {
+    const int be = (int)(mb >> 52);
+    const bool finite = be < 0x7FF;
+    const int e = mb == 0 ? EXP_ZERO : (finite ? (be ? be : 1) - 1021 : EXP_NAN);
+    if (lane == 0) ex[row] = e;
+    const int sh = mb == 0 || !finite ? 0 : 8 * ND - e;
+    long long Z[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) Z[u] = (finite ? tcr::scaled_rn(x[u], sh) : 0ll) + 0x0000808080808080ll;
+#pragma unroll
+    for (int s = 0; s < ND; ++s) {
+        const int bit = 8 * (ND - 1 - s);
+        const float scale = __int_as_float((127 - 8 * s) << 23);
+        unsigned f[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int d = s == 0 ? (int)(Z[u] >> bit) : (int)((unsigned)(Z[u] >> bit) & 255u) - 128;
+            f[u] = __float_as_uint((__int_as_float(0x4B400000 + d) - 12582912.0f) * scale);
+        }
+        *reinterpret_cast<uint2*>(out + ((int64_t)s * rows_per_plane + row) * NBS + 4 * lane) =
+            make_uint2(__byte_perm(f[0], f[1], 0x7632), __byte_perm(f[2], f[3], 0x7632));
+    }
+}
+
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long mb) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+    return mb;
+}
+
+// Block b of an n x n factor starts at row 128 b; rows below it (forward) or columns before it (backward).
+__device__ __host__ __forceinline__ int64_t below(int64_t n, int64_t b) { return n > (b + 1) * NBS ? n - (b + 1) * NBS : 0; }
+
+// Digit rows of the panels (columns 128 b .., rows below the diagonal block) of blocks b0 + blockIdx.y: block b's
+// planes (7 x below(b) rows of 128) follow those of the blocks before it.
+__global__ void __launch_bounds__(256) panel_rows_kernel(const double* __restrict__ A, int64_t lda, int64_t n, int b0,
+                                                         __nv_bfloat16* out, int* ex) {
+    constexpr int PER = NBS / 8;
+    __shared__ unsigned long long red[8][32];
+    const int64_t b = b0 + blockIdx.y, m = below(n, b);
+    if ((int64_t)blockIdx.x * 32 >= m) return;
+    int64_t before = 0;   // rows of the blocks before
+    for (int64_t i = b0; i < b; ++i) before += below(n, i);
+    const int lane = threadIdx.x % 32, grp = threadIdx.x / 32;
+    const int64_t row = (int64_t)blockIdx.x * 32 + lane;
+    const double* a = A + (b + 1) * NBS + b * NBS * lda;
+    double x[PER];
+    unsigned long long mb = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        x[i] = row < m ? a[row + (int64_t)(grp * PER + i) * lda] : 0.0;
+        mb = max(mb, (unsigned long long)__double_as_longlong(x[i]) & 0x7FFFFFFFFFFFFFFFull);
+    }
+    red[grp][lane] = mb;
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < 8; ++g) mb = max(mb, red[g][lane]);
+    if (row >= m) return;
+    row_digits<PER>(x, mb, out + (7 * before + row) * NBS + grp * PER, m * NBS, grp == 0 ? ex + before + row : nullptr);
+}
+
+// Digit rows of the block rows (rows 128 b .. , at most 128 of them, columns before) of blocks b0 + blockIdx.y: a warp per
+// column, the K direction contiguous in memory.
+__global__ void __launch_bounds__(256) block_cols_kernel(const double* __restrict__ A, int64_t lda, int64_t n, int b0,
+                                                         __nv_bfloat16* out, int* ex) {
+    const int64_t b = b0 + blockIdx.y, nc = b * NBS;
+    const int lane = threadIdx.x % 32;
+    const int64_t c = (int64_t)blockIdx.x * 8 + threadIdx.x / 32;
+    if (c >= nc) return;
+    int64_t before = 0;
+    for (int64_t i = b0; i < b; ++i) before += i * NBS;
+    const int nk = (int)(n - nc < NBS ? n - nc : NBS);
+    const double* a = A + nc + c * lda;
+    double x[4];
+    unsigned long long mb = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        x[u] = 4 * lane + u < nk ? a[4 * lane + u] : 0.0;
+        mb = max(mb, (unsigned long long)__double_as_longlong(x[u]) & 0x7FFFFFFFFFFFFFFFull);
+    }
+    write_digits4(x, warp_max(mb), out + 7 * before * NBS, nc, c, ex + before, lane);
+}
+
+// Inverses of the 128 x 128 lower diagonal blocks (identity past n): CTA (b, g) forms 32 columns by forward substitution,
+// lanes along the columns, the rows below the solved one shared by the warps.  Inv: column-major; InvT: its transpose.
+__global__ void __launch_bounds__(256) inverse128_kernel(const double* __restrict__ A, int64_t lda, int64_t n, double* Inv,
+                                                         double* InvT) {
+    extern __shared__ __align__(16) double sm[];   // X (row r, 32 columns), then the rows of L from c0 on
+    const int64_t b = blockIdx.x, k0 = b * NBS;
+    const int c0 = blockIdx.y * 32, nk = (int)(n - k0 < NBS ? n - k0 : NBS), rows = NBS - c0;
+    double* X = sm;
+    double* L = sm + NBS * 32;   // L[r * (rows + 1) + l], r, l relative to c0
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    const double* a = A + k0 + k0 * lda;
+    for (int e = threadIdx.x; e < rows * rows; e += 256) {
+        const int r = c0 + e % rows, l = c0 + e / rows;
+        L[(r - c0) * (rows + 1) + l - c0] = l > r ? 0.0 : (r < nk ? a[r + (int64_t)l * lda] : (r == l ? 1.0 : 0.0));
+    }
+    for (int r = warp; r < rows; r += 8) X[r * 32 + lane] = r == lane ? 1.0 : 0.0;
+    __syncthreads();
+    for (int r = threadIdx.x; r < rows; r += 256) L[r * (rows + 1) + r] = 1.0 / L[r * (rows + 1) + r];
+    __syncthreads();
+    for (int r = 0; r < rows; ++r) {
+        // every warp scales the row itself (the same value), warp r % 8 keeps it
+        const double x = X[r * 32 + lane] * L[r * (rows + 1) + r];
+        for (int i = r + 1 + ((warp - r - 1) & 7); i < rows; i += 8)
+            X[i * 32 + lane] = fma(-L[i * (rows + 1) + r], x, X[i * 32 + lane]);
+        __syncthreads();
+        if (warp == (r & 7)) X[r * 32 + lane] = x;
+    }
+    __syncthreads();
+    double* o = Inv + b * NBS * NBS;
+    double* ot = InvT + b * NBS * NBS;
+    for (int e = threadIdx.x; e < NBS * 32; e += 256) {
+        const int r = e % NBS, c = e / NBS;   // rows fastest: coalesced columns of Inv
+        o[r + (int64_t)(c0 + c) * NBS] = r < c0 ? 0.0 : X[(r - c0) * 32 + c];
+    }
+    for (int e = threadIdx.x; e < NBS * 32; e += 256) {
+        const int c = e % 32, r = e / 32;
+        ot[c0 + c + (int64_t)r * NBS] = r < c0 ? 0.0 : X[(r - c0) * 32 + c];
+    }
+}
+
+// x = M b for the rows of block k0 (nk <= 128 of them) of two right-hand sides per CTA, M lower (Inv) or upper (its
+// transpose) and 128 x 128, in place, with the digit rows of x^T (one row of 128 per right-hand side).
+__global__ void __launch_bounds__(256) diag_apply_kernel(const double* __restrict__ M, int upper, double* B, int64_t ldb,
+                                                         int nk, int64_t nrhs, __nv_bfloat16* out, int* ex) {
+    __shared__ double sb[2][NBS], sx[2][NBS];
+    const int r = threadIdx.x % NBS, g = threadIdx.x / NBS;
+    const int64_t col = 2 * (int64_t)blockIdx.x + g;
+    sb[g][r] = col < nrhs && r < nk ? B[r + col * ldb] : 0.0;
+    __syncthreads();
+    // l from 0 to the warp's last row (lower) or from its first row to the end (upper); the zeros of M do the rest
+    const int w0 = r & ~31;
+    const int l0 = upper ? w0 : 0, l1 = upper ? NBS : w0 + 32;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+    for (int l = l0; l < l1; l += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = fma(M[r + (l + u) * NBS], sb[g][l + u], acc[u]);
+    const double x = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    sx[g][r] = r < nk ? x : 0.0;
+    if (col < nrhs && r < nk) B[r + col * ldb] = x;
+    __syncthreads();
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (out && warp < 2 && 2 * (int64_t)blockIdx.x + warp < nrhs) {
+        double v[4];
+        unsigned long long mb = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            v[u] = sx[warp][4 * lane + u];
+            mb = max(mb, (unsigned long long)__double_as_longlong(v[u]) & 0x7FFFFFFFFFFFFFFFull);
+        }
+        write_digits4(v, warp_max(mb), out, nrhs, 2 * (int64_t)blockIdx.x + warp, ex, lane);
+    }
+}
+
 }  // namespace f64d
 
 
@@ -616,6 +786,71 @@ void trsm64(int64_t m, const double* L, int64_t ldl, double* P, int64_t ldp, cud
     ProfScope prof_("trsm64", s);
     f64d::trsm64_kernel<<<(unsigned)((m + 31) / 32), 128, 0, s>>>(m, L, ldl, P, ldp);
     f64d::check("trsm64");
+}
+
+// B (n x nrhs) <- (L D L^T)^-1 B with the FP64 factor's lower triangle L (128-row blocks) and D = diag(+I, -I) from row
+// nP on; Inv / InvT: the diagonal blocks' inverses (inverse_blocks_f64).  Each sweep is, per block, the product with the
+// inverse (FP64 pipe) and one FP64-accurate digit update of all rows still to come.  The factor's digits are formed per
+// call, for as many blocks at a time as 2 GB hold.
+void solve_f64(int64_t n, int64_t nP, const double* L, int64_t ld, const double* Inv, const double* InvT, double* B,
+               int64_t ldb, int64_t nrhs, int* err, cudaStream_t s) {
+    using namespace f64d;
+    if (n <= 0 || nrhs <= 0) return;
+    const int64_t nb = (n + NBS - 1) / NBS;
+    auto rows_of = [&](bool fwd, int64_t b) { return fwd ? below(n, b) : b * NBS; };
+    const int64_t budget = std::max<int64_t>(2ll << 30, 7 * n * NBS * 2);
+    DevBuf xd((size_t)7 * nrhs * NBS * 2, s), xe((size_t)nrhs * sizeof(int), s);
+    for (int back = 0; back < 2; ++back) {
+        const bool fwd = !back;
+        if (back) negate_rows<double>(B, ldb, nP, n, nrhs, s);
+        for (int64_t q0 = 0; q0 < nb;) {   // q: position in the sweep
+            int64_t q1 = q0, rows = 0;
+            auto block = [&](int64_t q) { return fwd ? q : nb - 1 - q; };
+            while (q1 < nb && (rows + rows_of(fwd, block(q1))) * 7 * NBS * 2 <= budget) rows += rows_of(fwd, block(q1++));
+            const int64_t lo = std::min(block(q0), block(q1 - 1)), cnt = q1 - q0;
+            DevBuf dig((size_t)7 * rows * NBS * 2, s), ex((size_t)rows * sizeof(int), s);
+            if (rows > 0) {
+                ProfScope prof_("f64_digits", s);
+                if (fwd)
+                    panel_rows_kernel<<<dim3((unsigned)((below(n, lo) + 31) / 32), (unsigned)cnt), 256, 0, s>>>(
+                        L, ld, n, (int)lo, dig.as<__nv_bfloat16>(), ex.as<int>());
+                else
+                    block_cols_kernel<<<dim3((unsigned)(((lo + cnt - 1) * NBS + 7) / 8), (unsigned)cnt), 256, 0, s>>>(
+                        L, ld, n, (int)lo, dig.as<__nv_bfloat16>(), ex.as<int>());
+                check("factor digits");
+            }
+            for (int64_t q = q0; q < q1; ++q) {
+                const int64_t b = block(q), k0 = b * NBS, m = rows_of(fwd, b);
+                const int nk = (int)std::min<int64_t>(NBS, n - k0);
+                {
+                    ProfScope prof_("f64_diag", s);
+                    diag_apply_kernel<<<(unsigned)((nrhs + 1) / 2), 256, 0, s>>>(
+                        (fwd ? Inv : InvT) + b * NBS * NBS, back, B + k0, ldb, nk, nrhs,
+                        m > 0 ? xd.as<__nv_bfloat16>() : nullptr, xe.as<int>());
+                    check("diagonal block");
+                }
+                if (m == 0) continue;
+                int64_t before = 0;
+                for (int64_t i = lo; i < b; ++i) before += rows_of(fwd, i);
+                digit_update_f64(m, nrhs, NBS, dig.as<uint16_t>() + 7 * before * NBS, m, 0, ex.as<int>() + before, xd.p,
+                                 nrhs, 0, xe.as<int>(), fwd ? B + k0 + NBS : B, ldb, false, err, s, "f64_solve");
+            }
+            q0 = q1;
+        }
+    }
+}
+
+// Inverses (and their transposes) of the 128 x 128 diagonal blocks of a lower factor, identity past n.
+void inverse_blocks_f64(int64_t n, const double* L, int64_t ld, double* Inv, double* InvT, cudaStream_t s) {
+    ProfScope prof_("f64_inverse", s);
+    constexpr int SM = (f64d::NBS * 32 + f64d::NBS * (f64d::NBS + 1)) * 8;
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(f64d::inverse128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
+        attr = true;
+    }
+    f64d::inverse128_kernel<<<dim3((unsigned)((n + f64d::NBS - 1) / f64d::NBS), 4), 256, SM, s>>>(L, ld, n, Inv, InvT);
+    f64d::check("diagonal inverses");
 }
 
 }  // namespace omg

@@ -19,6 +19,7 @@ struct omg_solver_s {
     std::vector<int64_t> bounds;            // block boundaries (include nP)
     DevBuf A64;                             // FP64: factor (lower).  Mixed: the head matrix as float pairs
                                             // (hi, lo; 2 x N x N floats) for the refinement residual
+    DevBuf Linv64;                          // FP64: inverses of the 128 x 128 diagonal blocks, then their transposes
     DevBuf A32;                             // mixed: FP32 factor (TF32 heads after the split), ld = ld32
     DevBuf A32r;                            // mixed: FP32 remainders of the factor
     DevBuf W;                               // mixed: K-major head/remainder copies of every panel
