@@ -1386,73 +1386,11 @@ constexpr int DSM_STACK = 3 * (DSM_MAX_LEVELS + 1) + 4;
 
 // Integrator::integrate with adaptive_integration (integrator.h:44-48,228-252)
 // as an explicit depth-first stack.  A node is its path of child indices from
-// the root (2 bits per level), so the stack holds no vertex coordinates.
-__device__ void dsm_adaptive(int kind, int order, int levels, double tol, const DsmTri& T, d3 r0, d3 q, d3 R0, d3 R1,
-                             d3 R2, double area, double result[3]) {
-    double coarse[3];
-    dsm_rule(kind, order, T, r0, q, R0, R1, R2, area, coarse);
-    if (levels == 0) {
-        result[0] = coarse[0]; result[1] = coarse[1]; result[2] = coarse[2];
-        return;
-    }
-    uint32_t st_path[DSM_STACK];
-    int8_t st_depth[DSM_STACK], st_level[DSM_STACK];
-    double st_c[DSM_STACK][3];
-    int sp = 0;
-    st_path[0] = 0; st_depth[0] = 0; st_level[0] = (int8_t)levels;
-    st_c[0][0] = coarse[0]; st_c[0][1] = coarse[1]; st_c[0][2] = coarse[2];
-    sp = 1;
-    double total[3] = {0.0, 0.0, 0.0};
-    const int dim = kind == 0 ? 3 : 1;
-    while (sp > 0) {
-        --sp;
-        const uint32_t path = st_path[sp];
-        const int depth = st_depth[sp], level = st_level[sp];
-        const double c0 = st_c[sp][0], c1 = st_c[sp][1], c2 = st_c[sp][2];
-        d3 P0 = R0, P1 = R1, P2 = R2;
-        double a = area;
-        for (int d = 0; d < depth; ++d) {
-            subtriangle(P0, P1, P2, (path >> (2 * d)) & 3);
-            a *= 0.25;
-        }
-        const double sub = 0.25 * a;
-        double integ[4][3];
-        double ref[3] = {0.0, 0.0, 0.0};
-        for (int c = 0; c < 4; ++c) {
-            d3 Q0 = P0, Q1 = P1, Q2 = P2;
-            subtriangle(Q0, Q1, Q2, c);
-            dsm_rule(kind, order, T, r0, q, Q0, Q1, Q2, sub, integ[c]);
-            for (int k = 0; k < dim; ++k) ref[k] += integ[c][k];
-        }
-        double dn, cn;
-        if (dim == 1) {
-            dn = fabs(c0 - ref[0]);
-            cn = fabs(c0);
-        } else {
-            const double e0 = c0 - ref[0], e1 = c1 - ref[1], e2 = c2 - ref[2];
-            dn = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
-            cn = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-        }
-        if (dn <= tol * cn || level == 0) {
-            for (int k = 0; k < dim; ++k) total[k] += ref[k];
-            continue;
-        }
-        for (int c = 3; c >= 0; --c) {
-            st_path[sp] = path | ((uint32_t)c << (2 * depth));
-            st_depth[sp] = (int8_t)(depth + 1);
-            st_level[sp] = (int8_t)(level - 1);
-            st_c[sp][0] = integ[c][0]; st_c[sp][1] = integ[c][1]; st_c[sp][2] = integ[c][2];
-            ++sp;
-        }
-    }
-    result[0] = total[0]; result[1] = total[1]; result[2] = total[2];
-}
-
-// The same integration by a group of four lanes (lanes 4 g .. 4 g + 3 of a
+// the root (2 bits per level), so the stack holds no vertex coordinates.  The
+// integration is done by a group of four lanes (lanes 4 g .. 4 g + 3 of a
 // warp, `mask` their bits): each node's four children are integrated one per
-// lane, each child's rule summed in the order of dsm_rule, and the values are
-// exchanged by shuffles, so every refinement decision and every sum is the
-// one of dsm_adaptive; the four lanes run the same control flow.
+// lane, each child's rule summed in order, and the values are exchanged by
+// shuffles; the four lanes run the same control flow.
 __device__ void dsm_adaptive_g4(int kind, int order, int levels, double tol, const DsmTri& T, d3 r0, d3 q, d3 R0,
                                 d3 R1, d3 R2, double area, double result[3], unsigned mask, int lane4) {
     double coarse[3];
@@ -1521,6 +1459,72 @@ __device__ void dsm_adaptive_g4(int kind, int order, int levels, double tol, con
     result[0] = total[0]; result[1] = total[1]; result[2] = total[2];
 }
 
+
+// FP64: the first adaptive level of both integrands of every (dipole, triangle)
+// pair, 80 points.  What depends on the triangle alone is tabled once per
+// launch, by rule point (the triangle's 16 and each child's 16), lanes along
+// the triangles: the point relative to the centroid c, -3 n.(point - c), and
+// the weight times the P1 values 1 and 2.  With X = c - r0 (r0, q: the dipole)
+// a point then takes 25 FP64 operations for the potential and its three
+// P1-weighted derivatives, with one reciprocal square root, against ~110 for
+// two separate adaptive integrations, on a pipe that bounds the DipSourceMat.
+// A pair is settled here when |coarse - refined| <= tol |coarse| holds with a
+// margin far above the rounding; the others (and those decided by rounding) are
+// listed for dsm_fallback_kernel.
+constexpr int DSM_FL = 6;   // table values per point
+
+__global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, int order, double* tab) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= nt) return;
+    const double* s = srec + t * SREC;
+    const d3 R0 = dev::ld3(s), R1 = dev::ld3(s + 3), R2 = dev::ld3(s + 6), n = dev::ld3(s + 9);
+    const d3 c = (R0 + R1 + R2) * (1.0 / 3.0);
+    const d3 e10 = R1 - R0, e20 = R2 - R0;
+    const double c11 = dev::dot(e10, e10), c12 = dev::dot(e10, e20), c22 = dev::dot(e20, e20);
+    const double inv_det = 1.0 / (c11 * c22 - c12 * c12);
+    const int np = c_nbpts[order];
+    d3 P0 = R0, P1 = R1, P2 = R2;
+    const int set = blockIdx.y;   // 0: the triangle; 1..4: its children
+    if (set > 0) subtriangle(P0, P1, P2, set - 1);
+    for (int k = 0; k < np; ++k) {
+        const double* r = c_rules[order][k];
+        const d3 x = bary_point(r, P0, P1, P2);
+        const d3 d = x - c, v = x - R0;
+        const double a1 = dev::dot(v, e10), a2 = dev::dot(v, e20);
+        double* o = tab + (int64_t)(set * np + k) * DSM_FL * nt + t;
+        o[0] = d.x;
+        o[nt] = d.y;
+        o[2 * nt] = d.z;
+        o[3 * nt] = -3.0 * dev::dot(n, d);
+        o[4 * nt] = r[3] * (inv_det * (c22 * a1 - c12 * a2));
+        o[5 * nt] = r[3] * (inv_det * (c11 * a2 - c12 * a1));
+    }
+}
+
+// One set of rule points: sums of w g (1, l1, l2) and w potential.
+__device__ __forceinline__ void dsm_set(const double* __restrict__ tab, int64_t nt, int order, d3 X, d3 q, double qn,
+                                        double h3, double acc[4]) {
+    acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
+    const int np = c_nbpts[order];
+#pragma unroll 2
+    for (int k = 0; k < np; ++k, tab += DSM_FL * nt) {
+        const double rx = X.x + tab[0], ry = X.y + tab[nt], rz = X.z + tab[2 * nt];
+        const double n2 = fma(rx, rx, fma(ry, ry, rz * rz));
+        const double qr = fma(q.x, rx, fma(q.y, ry, q.z * rz));
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n2));
+        const double e = fma(-(n2 * y), y, 1.0);   // one third-order Newton step
+        y = fma(y * e, fma(0.375, e, 0.5), y);
+        const double y2 = y * y, y3 = y2 * y;
+        const double w = c_rules[order][k][3];
+        acc[3] = fma(w, qr * y3, acc[3]);
+        const double g = fma(h3 + tab[3 * nt], qr * y2, qn) * y3;   // (q.n - 3 (q.r) (n.r) / r^2) / r^3
+        acc[0] = fma(w, g, acc[0]);
+        acc[1] = fma(tab[4 * nt], g, acc[1]);
+        acc[2] = fma(tab[5 * nt], g, acc[2]);
+    }
+    acc[0] -= acc[1] + acc[2];
+}
 
 // Mixed precision: the first adaptive level in FP32 with coordinates relative
 // to the triangle centroid.  The FP32 value is kept only when the acceptance
@@ -1703,10 +1707,10 @@ __device__ __forceinline__ bool dsm_pair(int64_t i, int64_t t, const double* __r
 // one thread per (dipole, triangle).  P0 rows are written directly (one
 // triangle per row); the three P1 contributions go to `p1tmp` for a
 // fixed-order vertex gather (the reference accumulates them atomically).
-// Mixed precision: a pair whose first adaptive level FP32 settles is written
-// here; the others are listed (with which of the two integrals is left) for
-// the FP64 adaptive integration in dsm_fallback_kernel, so the warps of that
-// deep recursion are not held up by pairs that need none.
+// A pair whose first adaptive level settles (FP64, or FP32 in mixed precision)
+// is written here; the others are listed (with which of the two integrals is
+// left) for the FP64 adaptive integration in dsm_fallback_kernel, so the warps
+// of that deep recursion are not held up by pairs that need none.
 constexpr int DSM_T_BITS = 29;   // triangle index bits of a list entry; the two top bits: integrals left
 
 __global__ void dsm_kernel(int64_t dip0, int64_t ndc, const double* __restrict__ dip, int64_t nt,
@@ -1715,8 +1719,74 @@ __global__ void dsm_kernel(int64_t dip0, int64_t ndc, const double* __restrict__
                            const int* __restrict__ orient, const int* __restrict__ dom, int maxb,
                            const int* __restrict__ dnb, const int* __restrict__ bmesh,
                            const int* __restrict__ binside, const double* __restrict__ dsigma, int order, int levels,
-                           double tol, int64_t nv, int64_t nP, int perm, double* out, int64_t ldo, double* p1tmp,
-                           int mixed, const DsmRecF* __restrict__ recf, int2* left, int* nleft) {
+                           double tol, int64_t nv, int perm, double* out, int64_t ldo, double* p1tmp,
+                           const double* __restrict__ tab, int2* left, int* nleft) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t il = blockIdx.y;
+    if (t >= nt || il >= ndc) return;
+    const int64_t i = dip0 + il;
+    double* o3 = p1tmp + (il * nt + t) * 3;
+    DsmPair P;
+    if (!dsm_pair_coeff(i, t, tmesh, orient, dom, maxb, dnb, bmesh, binside, dsigma, P)) {
+        o3[0] = o3[1] = o3[2] = 0.0;
+        return;
+    }
+    const bool p0row = !barrier[P.m];
+    const double* s = srec + t * SREC;
+    const d3 n = dev::ld3(s + 9), q = dev::ld3(dip + 6 * i + 3);
+    const d3 X = (dev::ld3(s) + dev::ld3(s + 3) + dev::ld3(s + 6)) * (1.0 / 3.0) - dev::ld3(dip + 6 * i);
+    const double qn = dev::dot(q, n), h3 = -3.0 * dev::dot(n, X), area = s[12];
+    const int64_t set = (int64_t)c_nbpts[order] * DSM_FL * nt;
+    double v[4];
+    dsm_set(tab + t, nt, order, X, q, qn, h3, v);
+    bool okv = true, okp = true;
+    if (levels == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] *= area;
+    } else {
+        double ref[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int c = 1; c <= 4; ++c) {
+            double a[4];
+            dsm_set(tab + c * set + t, nt, order, X, q, qn, h3, a);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ref[k] = fma(0.25 * area, a[k], ref[k]);
+        }
+        // settled with a margin of 1e-9 tol: rounding (1e-15) cannot turn the decision
+        const double lim = tol * (1.0 - 1e-9);
+        double d2 = 0.0, c2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] *= area;
+            const double e = v[k] - ref[k];
+            if (k < 3) {
+                d2 = fma(e, e, d2);
+                c2 = fma(v[k], v[k], c2);
+            } else {
+                okp = fabs(e) <= lim * fabs(v[k]);
+            }
+        }
+        okv = d2 <= lim * lim * c2;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = ref[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) o3[k] = okv ? v[k] * P.coeffD : 0.0;
+    if (p0row && okp) {
+        const int64_t ref = tidx_ref[t];
+        out[(perm ? ref - nv : ref) + i * ldo] = v[3] * (P.coeffD / P.sigma);
+    }
+    const int need = (okv ? 0 : 1) | (p0row && !okp ? 2 : 0);
+    if (need) left[atomicAdd(nleft, 1)] = make_int2((int)il, (int)t | (need << DSM_T_BITS));
+}
+
+// Mixed precision: the first level in FP32 (the 16-point rule, levels > 0).
+__global__ void dsm_mixed_kernel(int64_t dip0, int64_t ndc, const double* __restrict__ dip, int64_t nt,
+                                 const int32_t* __restrict__ tmesh, const int64_t* __restrict__ tidx_ref,
+                                 const int* __restrict__ barrier, const int* __restrict__ orient,
+                                 const int* __restrict__ dom, int maxb, const int* __restrict__ dnb,
+                                 const int* __restrict__ bmesh, const int* __restrict__ binside,
+                                 const double* __restrict__ dsigma, double tol, int64_t nv, int perm, double* out,
+                                 int64_t ldo, double* p1tmp, const DsmRecF* __restrict__ recf, int2* left, int* nleft) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t il = blockIdx.y;
     if (t >= nt || il >= ndc) return;
@@ -1726,46 +1796,31 @@ __global__ void dsm_kernel(int64_t dip0, int64_t ndc, const double* __restrict__
     DsmPair P;
     const int64_t ref = tidx_ref[t];
     const int64_t row = perm ? ref - nv : ref;
-    if (mixed && order == 3 && levels > 0) {
-        if (!dsm_pair_coeff(i, t, tmesh, orient, dom, maxb, dnb, bmesh, binside, dsigma, P)) return;
-        const bool p0row = !barrier[P.m];
-        const DsmRecF R = recf[t];
-        const double* dp = dip + 6 * i;
-        const float3 xc = make_float3((float)(R.cx - dp[0]), (float)(R.cy - dp[1]), (float)(R.cz - dp[2]));
-        const float3 qf = make_float3((float)dp[3], (float)dp[4], (float)dp[5]);
-        double v[3], pf[1];
-        bool f32v, f32p;
-        dsm_first_level2_f32(tol, R.T, xc, qf, R.T.p0, R.F1, R.F2, R.area, v, pf, f32v, f32p);
-        f32p = f32p && p0row;
-        // FP32-accurate values: scaled in FP32 (an FP64 division per pair costs more than the pair's
-        // FP32 work on GB300)
-        const float cf = (float)P.coeffD;
-        if (f32v) {
-            o3[0] = (double)((float)v[0] * cf);
-            o3[1] = (double)((float)v[1] * cf);
-            o3[2] = (double)((float)v[2] * cf);
-        }
-        if (f32p) out[row + i * ldo] = (double)((float)pf[0] * (cf / (float)P.sigma));
-        const int need = (f32v ? 0 : 1) | (p0row && !f32p ? 2 : 0);
-        if (need) left[atomicAdd(nleft, 1)] = make_int2((int)il, (int)t | (need << DSM_T_BITS));
-        return;
-    }
-    if (!dsm_pair(i, t, dip, srec, tmesh, orient, dom, maxb, dnb, bmesh, binside, dsigma, P)) return;
+    if (!dsm_pair_coeff(i, t, tmesh, orient, dom, maxb, dnb, bmesh, binside, dsigma, P)) return;
     const bool p0row = !barrier[P.m];
-    double v[3];
-    dsm_adaptive(0, order, levels, tol, P.T, P.r0, P.q, P.R0, P.R1, P.R2, P.area, v);
-    o3[0] = v[0] * P.coeffD;
-    o3[1] = v[1] * P.coeffD;
-    o3[2] = v[2] * P.coeffD;
-    if (p0row) {
-        double p[3];
-        dsm_adaptive(1, order, levels, tol, P.T, P.r0, P.q, P.R0, P.R1, P.R2, P.area, p);
-        out[row + i * ldo] = p[0] * (P.coeffD / P.sigma);
+    const DsmRecF R = recf[t];
+    const double* dp = dip + 6 * i;
+    const float3 xc = make_float3((float)(R.cx - dp[0]), (float)(R.cy - dp[1]), (float)(R.cz - dp[2]));
+    const float3 qf = make_float3((float)dp[3], (float)dp[4], (float)dp[5]);
+    double v[3], pf[1];
+    bool f32v, f32p;
+    dsm_first_level2_f32(tol, R.T, xc, qf, R.T.p0, R.F1, R.F2, R.area, v, pf, f32v, f32p);
+    f32p = f32p && p0row;
+    // FP32-accurate values: scaled in FP32 (an FP64 division per pair costs more than the pair's
+    // FP32 work on GB300)
+    const float cf = (float)P.coeffD;
+    if (f32v) {
+        o3[0] = (double)((float)v[0] * cf);
+        o3[1] = (double)((float)v[1] * cf);
+        o3[2] = (double)((float)v[2] * cf);
     }
+    if (f32p) out[row + i * ldo] = (double)((float)pf[0] * (cf / (float)P.sigma));
+    const int need = (f32v ? 0 : 1) | (p0row && !f32p ? 2 : 0);
+    if (need) left[atomicAdd(nleft, 1)] = make_int2((int)il, (int)t | (need << DSM_T_BITS));
 }
 
-// The listed pairs of the mixed first pass: FP64 adaptive integration of the
-// integrals FP32 did not settle (grid-stride over the device-side count, four
+// The listed pairs of the first pass: FP64 adaptive integration of the
+// integrals it did not settle (grid-stride over the device-side count, four
 // lanes per pair; block size a multiple of 32).
 __global__ void dsm_fallback_kernel(int64_t dip0, int64_t nt, const double* __restrict__ dip,
                                     const double* __restrict__ srec, const int32_t* __restrict__ tmesh,
@@ -2051,21 +2106,31 @@ void launch_dsm(const DevGeom& g, int64_t dip0, int64_t ndc, const double* dip, 
     ProfScope prof_("dsm", s);
     if (ndc == 0) return;
     if (g.nt >= ((int64_t)1 << DSM_T_BITS) || ndc > INT32_MAX) throw Error(OMG_ERR_UNSUPPORTED, "DSM: too many triangles");
-    const bool two_pass = mixed && order == 3 && levels > 0;
-    // the pairs FP32 does not settle (at most one entry per pair) and their count
-    DevBuf left(two_pass ? (size_t)ndc * g.nt * sizeof(int2) : 0, s), nleft(two_pass ? sizeof(int) : 0, s),
-        recf(two_pass ? (size_t)g.nt * sizeof(DsmRecF) : 0, s);
-    if (two_pass) {
-        OMG_CUDA(cudaMemsetAsync(nleft.p, 0, sizeof(int), s));
+    const bool fp32 = mixed && order == 3 && levels > 0;
+    // the pairs the first level does not settle (at most one entry per pair) and their count
+    DevBuf left(levels > 0 ? (size_t)ndc * g.nt * sizeof(int2) : 0, s), nleft(sizeof(int), s);
+    OMG_CUDA(cudaMemsetAsync(nleft.p, 0, sizeof(int), s));
+    const dim3 grid(nblocks(g.nt, 128), (unsigned)ndc);
+    if (fp32) {
+        DevBuf recf((size_t)g.nt * sizeof(DsmRecF), s);
         dsm_prepare_f_kernel<<<nblocks(g.nt, 128), 128, 0, s>>>(g.nt, g.srec, static_cast<DsmRecF*>(recf.p));
         check_launch("DSM records");
+        dsm_mixed_kernel<<<grid, 128, 0, s>>>(dip0, ndc, dip, g.nt, tmesh, tidx_ref, barrier, orient, dom, maxb, dnb, bmesh,
+                                              binside, dsigma, tol, g.nvg, perm, out, ldo, p1tmp,
+                                              static_cast<const DsmRecF*>(recf.p), left.as<int2>(), nleft.as<int>());
+        check_launch("DSM");
+    } else {
+        constexpr int NPTS[4] = {3, 6, 7, 16};
+        const int nsets = levels > 0 ? 5 : 1;
+        DevBuf tab((size_t)g.nt * nsets * NPTS[order] * DSM_FL * 8, s);
+        dsm_points_kernel<<<dim3(nblocks(g.nt, 128), nsets), 128, 0, s>>>(g.nt, g.srec, order, tab.as<double>());
+        check_launch("DSM points");
+        dsm_kernel<<<grid, 128, 0, s>>>(dip0, ndc, dip, g.nt, g.srec, tmesh, tidx_ref, barrier, orient, dom, maxb, dnb, bmesh,
+                                        binside, dsigma, order, levels, tol, g.nvg, perm, out, ldo, p1tmp,
+                                        tab.as<double>(), left.as<int2>(), nleft.as<int>());
+        check_launch("DSM");
     }
-    dim3 grid(nblocks(g.nt, 128), (unsigned)ndc);
-    dsm_kernel<<<grid, 128, 0, s>>>(dip0, ndc, dip, g.nt, g.srec, tmesh, tidx_ref, barrier, orient, dom, maxb, dnb,
-                                    bmesh, binside, dsigma, order, levels, tol, g.nvg, g.nP, perm, out, ldo, p1tmp, mixed,
-                                    static_cast<const DsmRecF*>(recf.p), left.as<int2>(), nleft.as<int>());
-    check_launch("DSM");
-    if (two_pass) {
+    if (levels > 0) {
         static int n_sm = 0;
         if (!n_sm) {
             int dev = 0;
