@@ -163,7 +163,16 @@ static thread_local std::string g_last_error;
 std::atomic<int64_t> g_dev_live{0}, g_dev_peak{0};
 void set_last_error(const char* msg) { g_last_error = msg; }
 
-void set_device(omg_context ctx) { OMG_CUDA(cudaSetDevice(ctx->device)); }
+// Start of a call: its work on the context's own stream (which does not synchronize with the default stream by itself)
+// comes after the work already queued on the device's default stream, so inputs that a program has just produced there
+// (a transposed copy, say) are complete.  A stream the caller has set is the caller's to order.
+void set_device(omg_context ctx) {
+    OMG_CUDA(cudaSetDevice(ctx->device));
+    if (ctx->stream != ctx->own) return;
+    if (!ctx->ev_in) OMG_CUDA(cudaEventCreateWithFlags(&ctx->ev_in, cudaEventDisableTiming));
+    OMG_CUDA(cudaEventRecord(ctx->ev_in, cudaStreamLegacy));
+    OMG_CUDA(cudaStreamWaitEvent(ctx->own, ctx->ev_in, 0));
+}
 
 // Handles are reference counted so that destroying them in any order is safe:
 // a context stays alive while a geometry or solver made from it lives, and a

@@ -27,6 +27,7 @@ struct omg_context_s {
     // second stream and the events of the factorization's look-ahead (created on first use)
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr, ev_d = nullptr, ev_e = nullptr;
+    cudaEvent_t ev_in = nullptr;   // work queued on the default stream before a call (created on first use)
     // highest-priority stream of the latency-bound solve chains (their CTAs go first onto SMs that free up
     // while other work runs on the second stream; created on first use)
     cudaStream_t hi = nullptr;
@@ -36,10 +37,10 @@ inline void release_aux(omg_context_s* c) {
     if (c->hi) cudaStreamDestroy(c->hi);
     c->hi = nullptr;
     if (c->aux) cudaStreamDestroy(c->aux);
-    for (cudaEvent_t e : {c->ev_a, c->ev_b, c->ev_c, c->ev_d, c->ev_e})
+    for (cudaEvent_t e : {c->ev_a, c->ev_b, c->ev_c, c->ev_d, c->ev_e, c->ev_in})
         if (e) cudaEventDestroy(e);
     c->aux = nullptr;
-    c->ev_a = c->ev_b = c->ev_c = c->ev_d = c->ev_e = nullptr;
+    c->ev_a = c->ev_b = c->ev_c = c->ev_d = c->ev_e = c->ev_in = nullptr;
 }
 
 // Live bytes of all device buffers of the library and their high-water mark
