@@ -141,8 +141,10 @@ void row_digits_f64(const double* A, int64_t lda, int64_t m, int k, int kpad, in
 void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
                       const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, bool lower,
                       int* err, cudaStream_t s, const char* name);
-void potrf64(double* A, int64_t lda, int n, int* err, int64_t* err_col, int64_t col_offset, cudaStream_t s);
-void trsm64(int64_t m, const double* L, int64_t ldl, double* P, int64_t ldp, cudaStream_t s);
+void panel32(double* A, int64_t lda, int w, int64_t m, double* Ld, int* err, int64_t* err_col, int64_t col_offset,
+             cudaStream_t s);
+void panel_update32(int64_t m, int nc, const double* X, double* C, int64_t ld, cudaStream_t s);
+void place_diagonal_f64(double* A, int64_t lda, int64_t n, const double* Ld, cudaStream_t s);
 void inverse_blocks_f64(int64_t n, const double* L, int64_t ld, double* Inv, double* InvT, cudaStream_t s);
 void solve_f64(int64_t n, int64_t nP, const double* L, int64_t ld, const double* Inv, const double* InvT, double* B,
                int64_t ldb, int64_t nrhs, int* err, cudaStream_t s);
@@ -572,13 +574,13 @@ static void require_distinct_vertices(omg_geometry g, const char* what) {
 // ---------------------------------------------------------------------------
 // Factorization: HM = L diag(+I_P, -I_V) L^T, blocked right-looking.
 // ---------------------------------------------------------------------------
-// FP64, in place on the lower triangle: panels of 128 columns, each two sub-panels of 64 factored on the FP64 pipe
-// (potrf64, trsm64 and the second sub-panel's update: 64 columns of work per row, N^2 / 2 x 64 operations in all),
-// everything wider as FP64-accurate digit products on the tensor cores (f64_digits.cu).  Panels go in groups of
+// FP64, in place on the lower triangle: panels of 128 columns, each four sub-panels of 32 factored on the FP64 pipe
+// (panel32) that update the panel's later columns there (panel_update32: 64 columns of work per row, N^2 / 2 x 64
+// operations in all), everything wider as FP64-accurate digit products on the tensor cores (f64_digits.cu).  Panels go in groups of
 // two (never across the start of the vertex part): the second takes the first one's update at K = 128, the trailing
 // block the group's at K = 256, which halves the FP64 passes over it.
 static void factor_ldlt_f64(omg_solver sv, double* A, int64_t ld) {
-    constexpr int64_t NB = 128, SB = 64;
+    constexpr int64_t NB = 128, SB = 32;
     cudaStream_t s = sv->ctx->stream;
     const int64_t N = sv->N, nP = sv->nP;
     int* err = sv->ctx->d_err;
@@ -593,6 +595,7 @@ static void factor_ldlt_f64(omg_solver sv, double* A, int64_t ld) {
     const size_t nblocks = sv->bounds.size() - 1;
     const int64_t mmax = std::max<int64_t>(1, N - sv->bounds[1]);
     DevBuf dig((size_t)7 * mmax * 2 * NB * 2, s), ex((size_t)mmax * sizeof(int), s);
+    DevBuf Ld((size_t)nblocks * NB * SB * 8, s);   // the factored 32 x 32 diagonal blocks
     auto at = [&](int64_t r, int64_t c) { return A + r + c * ld; };
     // C(rows and columns from r0, ncol columns) -= (columns k0 .. k1 of the factor)
     auto update = [&](int64_t k0, int64_t k1, int64_t r0, int64_t ncol, bool lower, const char* name) {
@@ -607,22 +610,19 @@ static void factor_ldlt_f64(omg_solver sv, double* A, int64_t ld) {
         const int64_t g0 = sv->bounds[b];
         if (g0 == nP) negate_lower<double>(at(nP, nP), ld, N - nP, s);   // continue on -(vertex Schur complement)
         for (; b < ge; ++b) {
-            const int64_t k0 = sv->bounds[b], k1 = sv->bounds[b + 1], ks = std::min(k1, k0 + SB);
+            const int64_t k0 = sv->bounds[b], k1 = sv->bounds[b + 1];
             if (k0 > g0) update(g0, k0, k0, k1 - k0, false, "f64_next");
-            potrf64(at(k0, k0), ld, (int)(ks - k0), err, sv->ctx->d_errcol, k0, s);
-            if (ks == N) break;
-            trsm64(N - ks, at(k0, k0), ld, at(ks, k0), ld, s);
-            if (ks < k1) {
-                gemm<double>(N - ks, k1 - ks, SB, -1.0, at(ks, k0), ld, false, at(ks, k0), ld, true, 1.0, at(ks, ks), ld,
-                             s);
-                potrf64(at(ks, ks), ld, (int)(k1 - ks), err, sv->ctx->d_errcol, ks, s);
-                if (k1 < N) trsm64(N - k1, at(ks, ks), ld, at(k1, ks), ld, s);
+            for (int64_t c = k0; c < k1; c += SB) {
+                const int64_t e = std::min(k1, c + SB);
+                panel32(at(c, c), ld, (int)(e - c), N - e, Ld.as<double>() + c * SB, err, sv->ctx->d_errcol, c, s);
+                panel_update32(N - e, (int)(k1 - e), at(e, c), at(e, e), ld, s);
             }
         }
         b = ge;
         const int64_t r0 = sv->bounds[ge];
         if (r0 < N) update(g0, r0, r0, N - r0, true, "f64_syrk");
     }
+    place_diagonal_f64(A, ld, N, Ld.as<double>(), s);
 }
 
 constexpr int NB32_TC = 128;   // tensor-core path: panel width = GEMM K = 4 x 32-element TMA chunks

@@ -19,16 +19,17 @@
 // their power of two, so a product already has its level's scale): what FP32 rounds
 // there is below 2^-52 of the leading term's unit.
 //
-// One output tile of 128 x 128 is three units of work, each with two accumulators
-// (256 TMEM columns, the units alternate between the two halves of TMEM, so a unit's
+// One output tile of 128 x TN is three units of work, each with two accumulators
+// (a half of TMEM's 512 columns, the units alternate between the halves, so a unit's
 // products run while the one before is drained): levels {4, 5}, {2, 3}, {6, 7-9}.
 // Within a unit, the K chunks of 64 stream their digit tiles through a ring of 13
 // slots of 16 KB, each digit tile of A and of B loaded once per chunk: for s = 1..7
 // the tiles B_t with lmin <= s + t <= lmax slide from high to low t, so four B tiles
 // and one A tile are live (26 tile loads per chunk and output tile against 68 when
 // every pair streams its own).  The epilogue keeps levels 2..5 as one 64-bit integer
-// per entry and adds the rest as an FP32 value: three FP64 operations per entry and
-// K = 256, since the FP64 pipe would otherwise bound the kernel.
+// per entry, adds the rest, and makes the FP64 value by integer operations: the FP64
+// pipe does one subtraction per entry (at three operations it took longer than the
+// products at K = 128).
 // Output tiles run in super-columns of 12 tile columns, row by row, so the CTAs at
 // work at a time share their digit tiles in L2.
 #include <cuda_bf16.h>
@@ -66,6 +67,29 @@ static inline void check(const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) throw Error(OMG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
     count_launch();
+}
+
+// Programmatic dependent launch (~2 us per launch of a chain): a kernel starts while its predecessor drains and waits for
+// it (pdl_wait) before it reads anything that or an earlier kernel wrote; pdl_next lets the successor start before the
+// end.  Kernels with several CTAs per SM are launched the ordinary way: launched early, their CTAs crowd onto the SMs that
+// are free at that moment (four panel32 + panel_update32 pairs took 296 instead of 150 us at 4400 rows).  What a kernel
+// reads after pdl_wait is never __restrict__ const or __ldg: the compiler may move those loads above the wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+static void launch(void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, (KArgs)args...);
 }
 
 // Digits of PER consecutive entries of a row whose largest magnitude has the bits mb, at the entry's place in plane 0
@@ -109,7 +133,7 @@ __device__ __forceinline__ void row_digits(const double (&x)[PER], unsigned long
 // (coalesced reads of the columns), eight groups of K / 8 consecutive columns.
 // ---------------------------------------------------------------------------
 template <int K>
-__global__ void __launch_bounds__(256) row_digits_kernel(const double* __restrict__ A, int64_t lda, int64_t m, int k,
+__global__ void __launch_bounds__(256) row_digits_kernel(const double* A, int64_t lda, int64_t m, int k,
                                                          int64_t rows_per_plane, __nv_bfloat16* out, int* ex) {
     constexpr int PER = K / 8;
     __shared__ unsigned long long red[8][32];
@@ -117,6 +141,7 @@ __global__ void __launch_bounds__(256) row_digits_kernel(const double* __restric
     const int64_t row = (int64_t)blockIdx.x * 32 + lane;
     double x[PER];
     unsigned long long mb = 0;
+    pdl_wait();
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int c = grp * PER + i;
@@ -134,15 +159,48 @@ __global__ void __launch_bounds__(256) row_digits_kernel(const double* __restric
 // ---------------------------------------------------------------------------
 // The product kernel
 // ---------------------------------------------------------------------------
-// Instruction descriptor: D = F32, A = B = BF16, both K-major, M = N = 128.
-constexpr uint32_t IDESC =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BT >> 3) << 17) | ((uint32_t)(BT >> 4) << 24);
+// Instruction descriptor: D = F32, A = B = BF16, both K-major, M = 128, N = n.
+__host__ __device__ constexpr uint32_t idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BT >> 4) << 24);
+}
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
+// The four K = 16 steps of a 64-wide chunk, issued by the lane that holds `lead` (the other lanes only keep the operands
+// uniform: in a one-lane branch every operand of every MMA went through a register-to-uniform move, ~100 cycles a step).
+__device__ __forceinline__ void mma_chunk4(uint32_t tmem, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate, uint32_t lead) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-            tmem),
-        "l"(a), "l"(b), "r"(IDESC), "r"(accumulate));
+        "{\n .reg .pred p, q, t;\n .reg .b64 a1, a2, a3, b1, b2, b3;\n"
+        " setp.ne.b32 q, %5, 0;\n setp.ne.b32 p, %4, 0;\n setp.eq.b32 t, 0, 0;\n"
+        " add.u64 a1, %1, 2;\n add.u64 b1, %2, 2;\n add.u64 a2, %1, 4;\n add.u64 b2, %2, 4;\n add.u64 a3, %1, 6;\n add.u64 b3, %2, 6;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n}\n" ::"r"(tmem),
+        "l"(a), "l"(b), "r"(id), "r"(accumulate), "r"(lead));
+}
+
+__device__ __forceinline__ void commit_by(uint64_t* bar, uint32_t lead) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(dev::smem_u32(bar)),
+        "r"(lead)
+        : "memory");
+}
+
+// T 2^e rounded to nearest even, by integer operations: the FP64 pipe (1/64 of the FP32 rate) is left one subtraction per
+// entry.  |T| < 2^62; an exponent past the range of normal numbers flushes to zero or infinity, EXP_NAN gives a NaN.
+__device__ __forceinline__ double scaled_double(long long T, int e) {
+    if (e > (1 << 19)) return __longlong_as_double(0x7FF8000000000000ll);
+    const unsigned long long u = (unsigned long long)(T < 0 ? -T : T);
+    const int lz = __clzll((long long)u);
+    const unsigned long long m = u << (lz & 63);
+    unsigned long long q = m >> 11;   // 53 bits with the leading one
+    const unsigned r = (unsigned)m & 0x7FFu;
+    q += (r > 0x400u || (r == 0x400u && (q & 1ull))) ? 1ull : 0ull;
+    const int ex = e + 1023 + 63 - lz;
+    unsigned long long bits = ((unsigned long long)(unsigned)(ex - 1) << 52) + q;   // (a carry moves to the exponent)
+    if (u == 0ull || ex <= 0) bits = 0ull;
+    else if (ex >= 2047) bits = 0x7FF0000000000000ull;
+    return __longlong_as_double((long long)(bits | ((unsigned long long)T & 0x8000000000000000ull)));
 }
 
 // The order of a unit's tiles (levels LMIN..LMAX): step s = 1..smax loads the B_t not yet loaded, then A_s, and
@@ -163,7 +221,7 @@ struct Unit {
 };
 
 struct Ring {
-    uint32_t slot, phase;   // of the next load
+    uint32_t slot, phase, count;   // of the next load; loads issued (producer)
     __device__ __forceinline__ void at(int pos, uint32_t& s, uint32_t& ph) const {
         s = slot + pos;
         ph = phase;
@@ -188,45 +246,44 @@ struct Shared {
     uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2], fin;
     uint32_t tmem;
     volatile int abort;
-    uint32_t issued[STAGES], consumed[STAGES];   // loads issued into / waited for in each slot
+    uint32_t issued;   // loads issued (load g goes to slot g % STAGES), written when the producer ends
 };
 
-template <int LMIN, int LMAX>
+template <int TN, int LMIN, int LMAX>
 __device__ __forceinline__ bool load_chunk(Shared& sh, Ring& r, uint32_t sbase, const CUtensorMap* tA,
                                            const CUtensorMap* tB, int x, int ya, int yb, int ra, int rb) {
     using U = Unit<LMIN, LMAX>;
-    auto load = [&](const CUtensorMap* map, int pos, int y) -> bool {
+    auto load = [&](const CUtensorMap* map, int pos, int y, int bytes) -> bool {
         uint32_t s, ph;
         r.at(pos, s, ph);
         if (!tc::wait_or_abort(&sh.empty[s], ph ^ 1u, &sh.abort)) return false;
-        dev::mbar_expect_tx(&sh.full[s], SLOT);
+        dev::mbar_expect_tx(&sh.full[s], bytes);
         tc::tma_load_2d(sbase + s * SLOT, map, x, y, &sh.full[s]);
-        ++sh.issued[s];
+        ++r.count;
         return true;
     };
 #pragma unroll
     for (int s = 1; s <= U::smax; ++s) {
 #pragma unroll
         for (int t = U::thi(s); t >= U::tlo(s); --t)
-            if (U::first_use(t) == s && !load(tB, U::pos_b(t), (t - 1) * rb + yb)) return false;
-        if (!load(tA, U::pos_a(s), (s - 1) * ra + ya)) return false;
+            if (U::first_use(t) == s && !load(tB, U::pos_b(t), (t - 1) * rb + yb, TN * BK * 2)) return false;
+        if (!load(tA, U::pos_a(s), (s - 1) * ra + ya, SLOT)) return false;
     }
     r.advance(U::loads);
     return true;
 }
 
-// The products of one chunk; levels LMIN into accumulator 0, the others into accumulator 1.
-template <int LMIN, int LMAX>
-__device__ __forceinline__ bool mma_chunk(Shared& sh, Ring& r, uint32_t sbase, uint32_t acc, bool first) {
+// The products of one chunk (called by the whole warp); levels LMIN into accumulator 0, the others into accumulator 1.
+// FIRST: the unit's first chunk, whose first product of each accumulator overwrites it.
+template <int TN, int LMIN, int LMAX, bool FIRST>
+__device__ __forceinline__ bool mma_chunk(Shared& sh, Ring& r, uint32_t sbase, uint32_t acc, uint32_t lead) {
     using U = Unit<LMIN, LMAX>;
     auto wait = [&](int pos, uint32_t& s) -> bool {
         uint32_t ph;
         r.at(pos, s, ph);
-        if (!tc::wait_or_abort(&sh.full[s], ph, &sh.abort)) return false;
-        ++sh.consumed[s];
-        return true;
+        return tc::wait_or_abort(&sh.full[s], ph, &sh.abort);
     };
-    uint32_t fresh = first ? 3u : 0u;   // accumulators not yet written in this unit
+    bool fresh0 = FIRST, fresh1 = FIRST;   // resolved at compile time after unrolling
 #pragma unroll
     for (int s = 1; s <= U::smax; ++s) {
         uint32_t sa, sb, ph;
@@ -240,23 +297,36 @@ __device__ __forceinline__ bool mma_chunk(Shared& sh, Ring& r, uint32_t sbase, u
         for (int t = U::thi(s); t >= U::tlo(s); --t) {
             r.at(U::pos_b(t), sb, ph);
             const uint64_t dB = tc::sdesc_sw128(sbase + sb * SLOT);
-            const int a = s + t == LMIN ? 0 : 1;
-#pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-                const uint64_t off = (uint64_t)(kk * 32) >> 4;   // 16 bf16 = 32 bytes
-                mma_bf16(acc + a * BT, dA + off, dB + off, (fresh >> a) & 1u ? 0u : 1u);
-                fresh &= ~(1u << a);
-            }
+            const bool hi = s + t == LMIN;
+            mma_chunk4(acc + (hi ? 0 : TN), dA, dB, idesc(TN), (hi ? fresh0 : fresh1) ? 0u : 1u, lead);
+            if (hi)
+                fresh0 = false;
+            else
+                fresh1 = false;
         }
-        tc::mma_commit(&sh.empty[sa]);
+        commit_by(&sh.empty[sa], lead);
 #pragma unroll
         for (int t = U::thi(s); t >= U::tlo(s); --t)
             if (U::last_use(t) == s) {
                 r.at(U::pos_b(t), sb, ph);
-                tc::mma_commit(&sh.empty[sb]);
+                commit_by(&sh.empty[sb], lead);
             }
     }
     r.advance(U::loads);
+    return true;
+}
+
+template <int TN, int LMIN, int LMAX>
+__device__ __forceinline__ bool mma_unit(Shared& sh, Ring& r, uint32_t sbase, uint32_t tmem, uint32_t& lu, int nchunk,
+                                         uint32_t lead) {
+    const uint32_t half = lu & 1u, acc = tmem + half * 256;
+    if (!tc::wait_or_abort(&sh.tempty[half], ((lu >> 1) & 1u) ^ 1u, &sh.abort)) return false;
+    fence_after();
+    if (!mma_chunk<TN, LMIN, LMAX, true>(sh, r, sbase, acc, lead)) return false;
+    for (int c = 1; c < nchunk; ++c)
+        if (!mma_chunk<TN, LMIN, LMAX, false>(sh, r, sbase, acc, lead)) return false;
+    commit_by(&sh.tfull[half], lead);
+    ++lu;
     return true;
 }
 
@@ -298,10 +368,11 @@ struct Walk {
     }
 };
 
+template <int TN>
 __global__ void __launch_bounds__(THREADS, 1)
     digit_update_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, int64_t M,
-                        int64_t Nc, int nchunk, int ra, int rb, const int* __restrict__ exA,
-                        const int* __restrict__ exB, double* C, int64_t ldc, int lower, int64_t ntiles, int* err) {
+                        int64_t Nc, int nchunk, int ra, int rb, const int* exA,
+                        const int* exB, double* C, int64_t ldc, int lower, int64_t ntiles, int* err) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ __align__(8) Shared sh;
     const uint32_t sbase = (dev::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -310,7 +381,6 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int s = 0; s < STAGES; ++s) {
             dev::mbar_init(&sh.full[s], 1);
             dev::mbar_init(&sh.empty[s], 1);
-            sh.issued[s] = sh.consumed[s] = 0;
         }
         for (int a = 0; a < 2; ++a) {
             dev::mbar_init(&sh.tfull[a], 1);
@@ -318,6 +388,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         dev::mbar_init(&sh.fin, 1);
         sh.abort = 0;
+        sh.issued = 0;
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dev::smem_u32(&sh.tmem)),
@@ -328,58 +399,44 @@ __global__ void __launch_bounds__(THREADS, 1)
     fence_before();
     __syncthreads();
     fence_after();
+    pdl_wait();
+    pdl_next();
     const uint32_t tmem = sh.tmem;
-    Walk walk{(int)((M + BT - 1) / BT), (int)((Nc + BT - 1) / BT), lower};
+    Walk walk{(int)((M + BT - 1) / BT), (int)((Nc + TN - 1) / TN), lower};
 
     if (warp == 0) {
         if (lane == 0) {   // ---- TMA producer
-            Ring r{0, 0};
+            Ring r{0, 0, 0};
             bool ok = true;
             for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 int i, j;
                 walk.tile(t, i, j);
-                const int ya = i * BT, yb = j * BT;
-                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<4, 5>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
-                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<2, 3>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
-                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<6, 9>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                const int ya = i * BT, yb = j * TN;
+                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 4, 5>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 2, 3>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 6, 9>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
             }
+            sh.issued = r.count;
             if (!ok) sh.abort = 1;
         }
     } else if (warp == 1) {
-        if (lane == 0) {   // ---- MMA issuer
-            Ring r{0, 0};
-            bool ok = true;
-            uint32_t lu = 0;
-            auto begin = [&](uint32_t& half) -> bool {
-                half = lu & 1u;
-                const bool go = tc::wait_or_abort(&sh.tempty[half], ((lu >> 1) & 1u) ^ 1u, &sh.abort);
-                fence_after();
-                return go;
-            };
-            for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-                uint32_t h;
-                ok = begin(h);
-                for (int c = 0; c < nchunk && ok; ++c) ok = mma_chunk<4, 5>(sh, r, sbase, tmem + h * 256, c == 0);
-                if (!ok) break;
-                tc::mma_commit(&sh.tfull[h]);
-                ++lu;
-                ok = begin(h);
-                for (int c = 0; c < nchunk && ok; ++c) ok = mma_chunk<2, 3>(sh, r, sbase, tmem + h * 256, c == 0);
-                if (!ok) break;
-                tc::mma_commit(&sh.tfull[h]);
-                ++lu;
-                ok = begin(h);
-                for (int c = 0; c < nchunk && ok; ++c) ok = mma_chunk<6, 9>(sh, r, sbase, tmem + h * 256, c == 0);
-                if (!ok) break;
-                tc::mma_commit(&sh.tfull[h]);
-                ++lu;
-            }
-            if (!ok) sh.abort = 1;
-            tc::mma_commit(&sh.fin);
-            if (!dev::mbar_wait_bounded(&sh.fin, 0)) sh.abort = 1;
-        }
-    } else {   // ---- epilogue: warp w owns TMEM lanes 32 (w % 4) .. +31 and columns 32 ((w - 2) / 4) .. +31
-        const int q = warp & 3, c0 = ((warp - 2) >> 2) * 32;
+        // ---- MMA issuer: the warp stays together, one lane issues
+        Ring r{0, 0, 0};
+        bool ok = true;
+        uint32_t lu = 0;
+        const uint32_t lead = lane == 0 ? 1u : 0u;
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x)
+            ok = mma_unit<TN, 4, 5>(sh, r, sbase, tm, lu, nchunk, lead) &&
+                 mma_unit<TN, 2, 3>(sh, r, sbase, tm, lu, nchunk, lead) &&
+                 mma_unit<TN, 6, 9>(sh, r, sbase, tm, lu, nchunk, lead);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) sh.abort = 1;
+        commit_by(&sh.fin, lead);
+        if (!dev::mbar_wait_bounded(&sh.fin, 0)) sh.abort = 1;
+    } else {   // ---- epilogue: warp w owns TMEM lanes 32 (w % 4) .. +31 and columns NCW ((w - 2) / 4) .. + NCW - 1
+        constexpr int NCW = TN / 4;
+        const int q = warp & 3, c0 = ((warp - 2) >> 2) * NCW;
         const uint32_t lanes = (uint32_t)(q * 32) << 16;
         uint32_t lu = 0;
         auto begin = [&]() -> bool {
@@ -398,75 +455,69 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
             int ti, tj;
             walk.tile(t, ti, tj);
-            const int64_t row = (int64_t)ti * BT + q * 32 + lane, col0 = (int64_t)tj * BT + c0;
-            long long H[32];   // levels 2..5 in units of level 5
+            const int64_t row = (int64_t)ti * BT + q * 32 + lane, col0 = (int64_t)tj * TN + c0;
+            long long H[NCW];   // levels 2..5 in units of level 5, |H| < 2^47
             if (!begin()) break;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t a[16], b[16];
-                tc::tmem_ld16(tmem + lanes + (lu & 1u) * 256 + c0 + h * 16, a);
-                tc::tmem_ld16(tmem + lanes + (lu & 1u) * 256 + BT + c0 + h * 16, b);
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    H[h * 16 + j] = ((long long)__float2int_rn(__uint_as_float(a[j]) * 0x1p16f) << 8) +
-                                    __float2int_rn(__uint_as_float(b[j]) * 0x1p24f);
-            }
-            end();
-            if (!begin()) break;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t a[16], b[16];
-                tc::tmem_ld16(tmem + lanes + (lu & 1u) * 256 + c0 + h * 16, a);
-                tc::tmem_ld16(tmem + lanes + (lu & 1u) * 256 + BT + c0 + h * 16, b);
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    H[h * 16 + j] += ((long long)__float2int_rn(__uint_as_float(a[j])) << 24) +
-                                     ((long long)__float2int_rn(__uint_as_float(b[j]) * 0x1p8f) << 16);
-            }
-            end();
-            const int er = row < M ? exA[row] : EXP_ZERO;
-            if (!begin()) break;
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
+            for (int h = 0; h < NCW / 8; ++h) {
                 uint32_t a[8], b[8];
                 tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
-                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + BT + c0 + h * 8, b);
-                double c[8];
-                bool in[8];
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + TN + c0 + h * 8, b);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int64_t col = col0 + h * 8 + j;
-                    in[j] = row < M && col < Nc && !(lower && row < col);
-                    c[j] = in[j] ? C[row + col * ldc] : 0.0;
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int64_t col = col0 + h * 8 + j;
-                    if (!in[j]) continue;
-                    // (levels 6..9) 2^24, an FP32 value, widened to FP64 by its bits
-                    const unsigned f = __float_as_uint(__uint_as_float(a[j]) + __uint_as_float(b[j]));
-                    const unsigned long long lo =
-                        (f << 1) == 0u ? 0ull
-                                       : ((unsigned long long)(f & 0x80000000u) << 32) |
-                                             (((unsigned long long)(f & 0x7FFFFFFFu) << 29) + ((896ull + 24ull) << 52));
-                    // levels 2..5: |H| < 2^51 placed in the mantissa of 1.5 2^52
-                    const double hi = __longlong_as_double(0x4338000000000000ll + H[h * 8 + j]) - 6755399441055744.0;
-                    const int e = 1023 + er + __ldg(exB + col) - 40;   // level 5 weighs 2^-40
-                    const long long sb = e > (1 << 19) ? 0x7FF8000000000000ll
-                                                       : (e <= 0 ? 0ll : (long long)min(e, 2047) << 52);
-                    C[row + col * ldc] = fma(-(hi + __longlong_as_double((long long)lo)), __longlong_as_double(sb), c[j]);
-                }
+                for (int j = 0; j < 8; ++j)
+                    H[h * 8 + j] = ((long long)__float2int_rn(__uint_as_float(a[j]) * 0x1p16f) << 8) +
+                                   __float2int_rn(__uint_as_float(b[j]) * 0x1p24f);
             }
             end();
+            if (!begin()) break;
+#pragma unroll
+            for (int h = 0; h < NCW / 8; ++h) {
+                uint32_t a[8], b[8];
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + TN + c0 + h * 8, b);
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    H[h * 8 + j] += ((long long)__float2int_rn(__uint_as_float(a[j])) << 24) +
+                                    ((long long)__float2int_rn(__uint_as_float(b[j]) * 0x1p8f) << 16);
+            }
+            end();
+            if (!begin()) break;
+#pragma unroll
+            for (int h = 0; h < NCW / 8; ++h) {
+                uint32_t a[8], b[8];
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + TN + c0 + h * 8, b);
+#pragma unroll
+                for (int j = 0; j < 8; ++j)   // in units of 2^-13 of level 5 (levels 6..9 are below 2^30 of them)
+                    H[h * 8 + j] = (H[h * 8 + j] << 13) +
+                                   __float2int_rn((__uint_as_float(a[j]) + __uint_as_float(b[j])) * 0x1p37f);
+            }
+            end();
+            const int er = (row < M ? exA[row] : EXP_ZERO) - 53;   // those units, 2^-53 of the exponents' product
+            double* const Cr = C + row + col0 * ldc;
+            const int64_t j1 = min((int64_t)NCW, Nc - col0), jl = lower ? min(j1, row - col0 + 1) : j1;
+            if (row >= M) continue;
+#pragma unroll
+            for (int h = 0; h < NCW / 8; ++h) {
+                double c[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) c[j] = h * 8 + j < jl ? Cr[(h * 8 + j) * ldc] : 0.0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (h * 8 + j < jl)
+                        Cr[(h * 8 + j) * ldc] = c[j] - scaled_double(H[h * 8 + j], er + exB[col0 + h * 8 + j]);
+            }
         }
     }
     __syncthreads();
     if (sh.abort) {
         if (threadIdx.x == 0) {
             atomicExch(err, -8 /* OMG_ERR_TIMEOUT */);
-            // copies still in flight land before the shared memory is given up
-            for (int s = 0; s < STAGES; ++s)
-                if (sh.issued[s] != sh.consumed[s]) dev::mbar_wait_bounded(&sh.full[s], (sh.issued[s] - 1u) & 1u);
+            // copies still in flight land before the shared memory is given up (the last one into each slot)
+            for (uint32_t k = 0; k < STAGES && k < sh.issued; ++k) {
+                const uint32_t g = sh.issued - 1u - k;
+                dev::mbar_wait_bounded(&sh.full[g % STAGES], (g / STAGES) & 1u);
+            }
         }
         __syncthreads();
     }
@@ -477,90 +528,150 @@ __global__ void __launch_bounds__(THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Diagonal block (n <= 64) of the FP64 Cholesky in one CTA: the lower triangle packed by
-// columns in shared memory, so the trailing update of a step is one run of entries over all
-// lanes.  Warp 0 updates the next column first, takes its pivot's reciprocal square root and
-// scales it while the other warps finish the update: one barrier per column.
+// Sub-panel of 32 columns: Cholesky of the 32 x 32 diagonal block and P <- P L^-T for the m rows below it, 32 rows per
+// CTA.  A warp's FP64 instruction takes its quarter of the SM 64 cycles, however few lanes take part, so both halves are
+// laid out for few instructions per warp:
+//  * every CTA factors the diagonal block itself (cheaper than a launch that only one SM works on).  Warp 0 runs the
+//    serial chain, five FP64 instructions per column (update of the next column, its pivot's reciprocal, the column
+//    times it): a_ik <- a_ik - u_i t_k with u the column as it stands and t = u / a_jj; the other warps update the rest
+//    of the triangle beside it (packed by columns: one run of entries over all lanes).  The square roots come last;
+//  * a warp then solves 8 rows, four lanes per row with every fourth column: the entry solved last goes to the row's
+//    lanes by a shuffle and is removed from the later ones with the same t; the results are scaled at the end.
+// A 64-column version in two launches took 39 + 28 us for 64 columns, this one ~2 x 14 us.
+// The factored block goes to Ld (other CTAs still read it in A); place_diagonal_kernel puts the blocks into A at the end.
 // ---------------------------------------------------------------------------
-constexpr int NBD = 64;
-constexpr int POTRF_THREADS = 256;
+constexpr int NBD = 32;
 
-__global__ void __launch_bounds__(POTRF_THREADS) potrf64_kernel(double* A, int64_t lda, int n, int* err, int64_t* err_col,
-                                                                int64_t col_offset) {
+__global__ void __launch_bounds__(128) panel32_kernel(const double* A, int64_t lda, int n, int64_t m, double* P, double* Ld,
+                                                      int* err, int64_t* err_col, int64_t col_offset) {
     constexpr int NE = NBD * (NBD + 1) / 2;
-    __shared__ double P[NE];
-    __shared__ double l[2][NBD];
+    __shared__ double U[NE];                     // the triangle, packed by columns
+    __shared__ __align__(16) double T[NBD][NBD];   // T[j][i]: t of column j, 0 up to row j
+    __shared__ double rs[NBD];
     __shared__ unsigned short ik[NE];
     const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
-    auto off = [](int j) { return j * NBD - j * (j - 1) / 2; };   // start of column j
-    for (int j = warp; j < NBD; j += POTRF_THREADS / 32)
-        for (int i = j + lane; i < NBD; i += 32) {
+    auto off = [](int j) { return j * NBD - j * (j - 1) / 2; };
+    pdl_wait();
+    pdl_next();
+    for (int j = warp; j < NBD; j += 4) {
+        const int i = lane;
+        if (i >= j) {
             const int e = off(j) + i - j;
             ik[e] = (unsigned short)(i | (j << 8));
-            P[e] = i < n && j < n ? A[i + (int64_t)j * lda] : (i == j ? 1.0 : 0.0);   // identity past n
+            U[e] = i < n && j < n ? A[i + (int64_t)j * lda] : (i == j ? 1.0 : 0.0);   // identity past n
         }
+        T[j][i] = 0.0;
+    }
+    // this CTA's rows, on their way while the block is factored
+    const int g = lane & 3;
+    const int64_t row = (int64_t)blockIdx.x * 32 + warp * 8 + lane / 4;
+    const bool live = row < m;
+    double* p = P + (live ? row : 0) + (int64_t)g * lda;
+    double x[NBD / 4];
+#pragma unroll
+    for (int i = 0; i < NBD / 4; ++i) x[i] = live ? p[(int64_t)(4 * i) * lda] : 0.0;
     __syncthreads();
-    auto pivot = [&](int j) {   // warp 0: column j final; l[j % 2] <- the scaled column
-        double d = P[off(j)];
-        if (!(d > 0.0)) {
-            if (lane == 0 && j < n && atomicCAS(err, 0, -3 /* OMG_ERR_NOT_DEFINITE */) == 0) *err_col = col_offset + j;
-            d = 1.0;
-        }
-        const double r = 1.0 / sqrt(d);
-        __syncwarp();
-        for (int i = j + lane; i < NBD; i += 32) {
-            const double v = i == j ? sqrt(d) : P[off(j) + i - j] * r;
-            P[off(j) + i - j] = v;
-            l[j & 1][i] = v;
-        }
+    int bad = NBD;   // warp 0: the first column with a pivot of the wrong sign
+    auto pivot = [&](int j, double v) {   // warp 0: column j is final, v its entry of row j + lane
+        const long long bits = __double_as_longlong(__shfl_sync(0xffffffffu, v, 0));
+        const bool good = bits > 0 && bits <= 0x7FF0000000000000ll;   // d > 0, off the FP64 pipe
+        bad = good ? bad : min(bad, j);
+        const double d = __longlong_as_double(good ? bits : 0x3FF0000000000000ll);
+        double y;   // 1 / d: the hardware approximation and one third-order Newton step
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+        const double e = fma(-d, y, 1.0);
+        y = fma(fma(e, e, e), y, y);
+        const double t = v * y;
+        if (lane > 0 && j + lane < NBD) T[j][j + lane] = t;
     };
-    if (warp == 0) pivot(0);
+    if (warp == 0) pivot(0, U[lane]);
     __syncthreads();
     for (int j = 0; j + 1 < NBD; ++j) {
-        const double* lj = l[j & 1];
-        const int e1 = off(j + 1), e2 = off(j + 2);   // column j + 1, then the rest
+        const double* t = T[j];
+        const double* u = U + off(j) - j;              // u[i]: column j
+        const int e1 = off(j + 1), e2 = off(j + 2);    // column j + 1, then the rest
         if (warp == 0) {
-            const double lk = lj[j + 1];
-            for (int e = e1 + lane; e < e2; e += 32) P[e] = fma(-lj[j + 1 + e - e1], lk, P[e]);
-            __syncwarp();
-            pivot(j + 1);
+            const int r = j + 1 + lane;
+            const double v = fma(-u[min(r, NBD - 1)], t[j + 1], U[min(e1 + lane, NE - 1)]);
+            if (r < NBD) U[e1 + lane] = v;
+            pivot(j + 1, v);
         } else {
-            for (int e = e2 + tid - 32; e < NE; e += POTRF_THREADS - 32) {
-                const int x = ik[e];
-                P[e] = fma(-lj[x & 255], lj[x >> 8], P[e]);
+#pragma unroll 2
+            for (int e = e2 + tid - 32; e < NE; e += 96) {
+                const int q = ik[e];
+                U[e] = fma(-u[q & 255], t[q >> 8], U[e]);
             }
         }
         __syncthreads();
     }
-    for (int j = warp; j < n; j += POTRF_THREADS / 32)
-        for (int i = j + lane; i < n; i += 32) A[i + (int64_t)j * lda] = P[off(j) + i - j];
-}
-
-// P <- P L^-T for an m x 64 panel P and a 64 x 64 lower L: one row per lane in 64 registers, each solved entry
-// removed from all later ones at once (independent FP64 operations; the pipe's rate bounds it), 32 rows per CTA.
-__global__ void __launch_bounds__(128) trsm64_kernel(int64_t m, const double* __restrict__ L, int64_t ldl, double* P,
-                                                     int64_t ldp) {
-    __shared__ __align__(16) double sL[NBD][NBD];   // sL[j][i] = L(i, j)
-    __shared__ double rd[NBD];
-    for (int e = threadIdx.x; e < NBD * NBD; e += 128) {
-        const int i = e % NBD, j = e / NBD;
-        sL[j][i] = i >= j ? L[i + (int64_t)j * ldl] : 0.0;
+    if (warp == 0) {   // rs = 1 / sqrt(d): the approximation and one third-order Newton step
+        const double d0 = U[off(lane)];
+        const double d = __double_as_longlong(d0) > 0 ? d0 : 1.0;
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+        const double e = fma(-(d * y), y, 1.0);
+        rs[lane] = fma(y * e, fma(0.375, e, 0.5), y);
+        if (blockIdx.x == 0 && lane == 0 && bad < n && atomicCAS(err, 0, -3 /* OMG_ERR_NOT_DEFINITE */) == 0)
+            *err_col = col_offset + bad;
     }
     __syncthreads();
-    if (threadIdx.x < NBD) rd[threadIdx.x] = 1.0 / sL[threadIdx.x][threadIdx.x];
-    __syncthreads();
-    const int64_t row = (int64_t)blockIdx.x * 32 + threadIdx.x;
-    if (threadIdx.x >= 32 || row >= m) return;
-    double x[NBD];
-#pragma unroll
-    for (int j = 0; j < NBD; ++j) x[j] = P[row + (int64_t)j * ldp];
+    if (blockIdx.x == 0)
+        for (int j = warp; j < NBD; j += 4) Ld[lane + j * NBD] = lane >= j ? U[off(j) + lane - j] * rs[j] : 0.0;
+    if (!__any_sync(0xffffffffu, live)) return;
 #pragma unroll
     for (int j = 0; j < NBD; ++j) {
-        x[j] *= rd[j];
+        const double xj = __shfl_sync(0xffffffffu, x[j / 4], (lane & ~3) | (j & 3));
 #pragma unroll
-        for (int i = j + 1; i < NBD; ++i) x[i] = fma(-x[j], sL[j][i], x[i]);
-        P[row + (int64_t)j * ldp] = x[j];
+        for (int i = j / 4 + (j % 4 == 3 ? 1 : 0); i < NBD / 4; ++i) x[i] = fma(-xj, T[j][4 * i + g], x[i]);
     }
+    if (!live) return;
+#pragma unroll
+    for (int i = 0; i < NBD / 4; ++i) p[(int64_t)(4 * i) * lda] = x[i] * rs[4 * i + g];
+}
+
+// C (m x nc) -= X Y^T, X the m x 32 sub-panel at the rows of C and Y its first nc rows (C starts at row and column
+// 32 (b + 1) of a panel, X at the same row): tiles of 16 rows x 32 columns (4.7 us of FP64 work on an SM; at 32 x 32 the
+// short updates left SMs idle and the last wave was longer), the whole K staged at once.
+__global__ void __launch_bounds__(128) panel_update32_kernel(int64_t m, int nc, const double* X, double* C,
+                                                             int64_t ld) {
+    __shared__ double sX[NBD][16], sY[NBD][NBD];   // [k][row]
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    const int64_t r0 = (int64_t)blockIdx.x * 16;
+    const int c0 = blockIdx.y * 32;
+    const int nj = nc - c0 < 32 ? nc - c0 : 32;
+    if (r0 + 15 < c0) return;   // above the diagonal
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const int k = warp * 8 + u;
+        if (lane < 16) sX[k][lane] = r0 + lane < m ? X[r0 + lane + (int64_t)k * ld] : 0.0;
+        sY[k][lane] = lane < nj ? X[c0 + lane + (int64_t)k * ld] : 0.0;
+    }
+    const int r = lane % 16, j0 = warp * 8 + lane / 16 * 4;   // the thread's row and four columns
+    const bool live = r0 + r < m;
+    double acc[4];
+    double* c = C + r0 + r + (int64_t)(c0 + j0) * ld;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[u] = live && j0 + u < nj ? c[(int64_t)u * ld] : 0.0;
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < NBD; ++k) {
+        const double x = sX[k][r];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = fma(-x, sY[k][j0 + u], acc[u]);
+    }
+    if (!live) return;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (j0 + u < nj) c[(int64_t)u * ld] = acc[u];
+}
+
+// The factored diagonal blocks (32 x 32, one after the other) into the lower triangle of A.  Block b covers the columns
+// from 32 b on: the panels start on multiples of 128.
+__global__ void place_diagonal_kernel(double* A, int64_t lda, int64_t n, const double* __restrict__ Ld) {
+    const int64_t k0 = (int64_t)blockIdx.x * NBD;
+    const int i = threadIdx.x % 32;
+    for (int j = threadIdx.x / 32; j <= i; j += blockDim.x / 32)
+        if (k0 + i < n && k0 + j < n) A[k0 + i + (k0 + j) * lda] = Ld[blockIdx.x * (int64_t)(NBD * NBD) + i + j * NBD];
 }
 
 // ---------------------------------------------------------------------------
@@ -695,38 +806,38 @@ __global__ void __launch_bounds__(256) inverse128_kernel(const double* __restric
     }
 }
 
-// x = M b for the rows of block k0 (nk <= 128 of them) of two right-hand sides per CTA, M lower (Inv) or upper (its
-// transpose) and 128 x 128, in place, with the digit rows of x^T (one row of 128 per right-hand side).
-__global__ void __launch_bounds__(256) diag_apply_kernel(const double* __restrict__ M, int upper, double* B, int64_t ldb,
+// x = M b for the rows of a block (nk <= 128 of them) of one right-hand side per CTA, M lower (Inv) or upper (its
+// transpose) and 128 x 128, in place, with the digit row of x^T.  Each row group's dot products are halved between two
+// warps, paired so that the four FP64 quarters get the same number of operations (16 (g + 1) and 16 (4 - g)).
+__global__ void __launch_bounds__(256) diag_apply_kernel(const double* M, int upper, double* B, int64_t ldb,
                                                          int nk, int64_t nrhs, __nv_bfloat16* out, int* ex) {
-    __shared__ double sb[2][NBS], sx[2][NBS];
-    const int r = threadIdx.x % NBS, g = threadIdx.x / NBS;
-    const int64_t col = 2 * (int64_t)blockIdx.x + g;
-    sb[g][r] = col < nrhs && r < nk ? B[r + col * ldb] : 0.0;
-    __syncthreads();
-    // l from 0 to the warp's last row (lower) or from its first row to the end (upper); the zeros of M do the rest
-    const int w0 = r & ~31;
-    const int l0 = upper ? w0 : 0, l1 = upper ? NBS : w0 + 32;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 2
-    for (int l = l0; l < l1; l += 4)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] = fma(M[r + (l + u) * NBS], sb[g][l + u], acc[u]);
-    const double x = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-    sx[g][r] = r < nk ? x : 0.0;
-    if (col < nrhs && r < nk) B[r + col * ldb] = x;
-    __syncthreads();
+    __shared__ double sb[NBS], part[2][NBS];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    if (out && warp < 2 && 2 * (int64_t)blockIdx.x + warp < nrhs) {
-        double v[4];
-        unsigned long long mb = 0;
+    double* b = B + (int64_t)blockIdx.x * ldb;
+    pdl_wait();
+    pdl_next();
+    if (threadIdx.x < NBS) sb[threadIdx.x] = threadIdx.x < nk ? b[threadIdx.x] : 0.0;
+    const int half = warp >> 2, g = half ? 3 - (warp & 3) : warp & 3;   // rows 32 g + lane
+    const int len = upper ? 4 - g : g + 1, r = 32 * g + lane;             // 32 len entries of the row, 16 len per half
+    const int l0 = (upper ? 32 * g : 0) + half * 16 * len;
+    __syncthreads();
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int l = l0; l < l0 + 16 * len; l += 16)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            v[u] = sx[warp][4 * lane + u];
-            mb = max(mb, (unsigned long long)__double_as_longlong(v[u]) & 0x7FFFFFFFFFFFFFFFull);
-        }
-        write_digits4(v, warp_max(mb), out, nrhs, 2 * (int64_t)blockIdx.x + warp, ex, lane);
+        for (int u = 0; u < 16; ++u) acc[u & 3] = fma(M[r + (l + u) * NBS], sb[l + u], acc[u & 3]);
+    part[half][r] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    __syncthreads();
+    if (warp != 0) return;
+    double v[4];
+    unsigned long long mb = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = 4 * lane + u;
+        v[u] = i < nk ? part[0][i] + part[1][i] : 0.0;
+        if (i < nk) b[i] = v[u];
+        mb = max(mb, (unsigned long long)__double_as_longlong(v[u]) & 0x7FFFFFFFFFFFFFFFull);
     }
+    if (out) write_digits4(v, warp_max(mb), out, nrhs, blockIdx.x, ex, lane);
 }
 
 }  // namespace f64d
@@ -740,7 +851,7 @@ void row_digits_f64(const double* A, int64_t lda, int64_t m, int k, int kpad, in
     ProfScope prof_("f64_digits", s);
     const unsigned grid = (unsigned)((m + 31) / 32);
     auto kern = kpad == 128 ? f64d::row_digits_kernel<128> : f64d::row_digits_kernel<256>;
-    kern<<<grid, 256, 0, s>>>(A, lda, m, k, rows_per_plane, static_cast<__nv_bfloat16*>(out), ex);
+    f64d::launch(kern, grid, 256, 0, s, A, lda, m, k, rows_per_plane, static_cast<__nv_bfloat16*>(out), ex);
     f64d::check("FP64 row digits");
 }
 
@@ -755,37 +866,64 @@ void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra
     ProfScope prof_(name, s);
     static int n_sm = 0;
     if (!n_sm) {
-        cudaFuncSetAttribute(f64d::digit_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f64d::SMEM_BYTES);
+        for (auto k : {f64d::digit_update_kernel<128>, f64d::digit_update_kernel<64>, f64d::digit_update_kernel<32>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, f64d::SMEM_BYTES);
         int dev = 0, n = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         n_sm = n > 0 ? n : 1;
     }
+    // Tile width: narrow tiles put a short product (a solve's right-hand sides, the next panel) on more SMs and leave a
+    // shorter last epilogue, wide ones feed the tensor cores better.  Cycles of a tile's products (a K = 16 step takes
+    // 64 / 48 / 40 cycles at 128 / 64 / 32 columns: shared memory feeds 128 bytes a cycle) by the number of waves, plus
+    // one epilogue of ~100 cycles a column.
+    const int64_t mt = (M + f64d::BT - 1) / f64d::BT;
+    int tn = 128;
+    if (!lower) {
+        int64_t best = INT64_MAX;
+        for (int w : {128, 64, 32}) {
+            const int64_t waves = (mt * ((Nc + w - 1) / w) + n_sm - 1) / n_sm;
+            const int64_t t = waves * 34 * (kpad / 16) * (w == 128 ? 64 : w == 64 ? 48 : 40) + 100 * w;
+            if (t < best) {
+                best = t;
+                tn = w;
+            }
+        }
+    }
     const CUtensorMap mA = tc::make_map_2d(static_cast<const uint16_t*>(A) + a0 * kpad, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
                                            2, f64d::ND * ra - a0, kpad, kpad, f64d::BK, f64d::BT);
     const CUtensorMap mB = tc::make_map_2d(static_cast<const uint16_t*>(B) + b0 * kpad, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                                           2, f64d::ND * rb - b0, kpad, kpad, f64d::BK, f64d::BT);
-    const int64_t mt = (M + f64d::BT - 1) / f64d::BT, nt = (Nc + f64d::BT - 1) / f64d::BT;
+                                           2, f64d::ND * rb - b0, kpad, kpad, f64d::BK, tn);
+    const int64_t nt = (Nc + tn - 1) / tn;
     const int64_t ntiles = lower ? mt * nt - nt * (nt - 1) / 2 : mt * nt;
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, n_sm);
-    f64d::digit_update_kernel<<<grid, f64d::THREADS, f64d::SMEM_BYTES, s>>>(
-        mA, mB, M, Nc, kpad / f64d::BK, (int)ra, (int)rb, exA + a0, exB + b0, C, ldc, lower ? 1 : 0, ntiles, err);
+    auto kern = tn == 128 ? f64d::digit_update_kernel<128> : tn == 64 ? f64d::digit_update_kernel<64> : f64d::digit_update_kernel<32>;
+    f64d::launch(kern, grid, f64d::THREADS, f64d::SMEM_BYTES, s, mA, mB, M, Nc, kpad / f64d::BK, (int)ra, (int)rb, exA + a0,
+                 exB + b0, C, ldc, lower ? 1 : 0, ntiles, err);
     f64d::check(name);
 }
 
-// In place: the lower triangle of an n x n block (n <= 64) by its Cholesky factor.
-void potrf64(double* A, int64_t lda, int n, int* err, int64_t* err_col, int64_t col_offset, cudaStream_t s) {
-    ProfScope prof_("potrf64", s);
-    f64d::potrf64_kernel<<<1, f64d::POTRF_THREADS, 0, s>>>(A, lda, n, err, err_col, col_offset);
-    f64d::check("potrf64");
+// Sub-panel at (k0, k0) of the matrix, w <= 32 columns: the diagonal block's factor to Ld, the rows below solved in place.
+void panel32(double* A, int64_t lda, int w, int64_t m, double* Ld, int* err, int64_t* err_col, int64_t col_offset,
+             cudaStream_t s) {
+    ProfScope prof_("f64_panel", s);
+    f64d::launch(f64d::panel32_kernel, dim3((unsigned)std::max<int64_t>(1, (m + 31) / 32)), 128, 0, s, (const double*)A, lda,
+                 w, m, A + w, Ld, err, err_col, col_offset);
+    f64d::check("FP64 panel");
 }
 
-// P (m x 64) <- P L^-T.
-void trsm64(int64_t m, const double* L, int64_t ldl, double* P, int64_t ldp, cudaStream_t s) {
-    if (m <= 0) return;
-    ProfScope prof_("trsm64", s);
-    f64d::trsm64_kernel<<<(unsigned)((m + 31) / 32), 128, 0, s>>>(m, L, ldl, P, ldp);
-    f64d::check("trsm64");
+// C (m x nc, its first nc rows lower) -= X (m x 32) (first nc rows of X)^T.
+void panel_update32(int64_t m, int nc, const double* X, double* C, int64_t ld, cudaStream_t s) {
+    if (m <= 0 || nc <= 0) return;
+    ProfScope prof_("f64_panel_update", s);
+    f64d::panel_update32_kernel<<<dim3((unsigned)((m + 15) / 16), (unsigned)((nc + 31) / 32)), 128, 0, s>>>(m, nc, X, C, ld);
+    f64d::check("FP64 panel update");
+}
+
+void place_diagonal_f64(double* A, int64_t lda, int64_t n, const double* Ld, cudaStream_t s) {
+    if (n <= 0) return;
+    f64d::place_diagonal_kernel<<<(unsigned)((n + 31) / 32), 256, 0, s>>>(A, lda, n, Ld);
+    f64d::check("FP64 diagonal blocks");
 }
 
 // B (n x nrhs) <- (L D L^T)^-1 B with the FP64 factor's lower triangle L (128-row blocks) and D = diag(+I, -I) from row
@@ -824,9 +962,8 @@ void solve_f64(int64_t n, int64_t nP, const double* L, int64_t ld, const double*
                 const int nk = (int)std::min<int64_t>(NBS, n - k0);
                 {
                     ProfScope prof_("f64_diag", s);
-                    diag_apply_kernel<<<(unsigned)((nrhs + 1) / 2), 256, 0, s>>>(
-                        (fwd ? Inv : InvT) + b * NBS * NBS, back, B + k0, ldb, nk, nrhs,
-                        m > 0 ? xd.as<__nv_bfloat16>() : nullptr, xe.as<int>());
+                    launch(diag_apply_kernel, dim3((unsigned)nrhs), 256, 0, s, (fwd ? Inv : InvT) + b * NBS * NBS, back,
+                           B + k0, ldb, nk, nrhs, m > 0 ? xd.as<__nv_bfloat16>() : nullptr, xe.as<int>());
                     check("diagonal block");
                 }
                 if (m == 0) continue;
@@ -873,11 +1010,14 @@ extern "C" int omg_internal_digit_update(int64_t M, int64_t Nc, int k, const dou
     }
 }
 
-// Test hook: Cholesky of the n x n (n <= 64) A and P <- P L^-T for the m x 64 P (used when n is 64).
-extern "C" int omg_internal_potrf_trsm64(int n, double* A, int64_t m, double* P, int* err, int64_t* err_col) {
+// Test hook: Cholesky of the w x w (w <= 32) block at the top of the (w + m) x w matrix A (column-major) and the rows below
+// it <- rows L^-T, in place.
+extern "C" int omg_internal_panel32(int w, int64_t m, double* A, int* err, int64_t* err_col) {
     try {
-        omg::potrf64(A, n, n, err, err_col, 0, 0);
-        if (n == 64) omg::trsm64(m, A, n, P, m, 0);
+        cudaStream_t s = 0;
+        DevBuf Ld(32 * 32 * 8, s);
+        omg::panel32(A, w + m, w, m, Ld.as<double>(), err, err_col, 0, s);
+        omg::place_diagonal_f64(A, w + m, w, Ld.as<double>(), s);
         return cudaDeviceSynchronize() == cudaSuccess ? 0 : -2;
     } catch (const omg::Error& e) {
         return e.code;

@@ -1,4 +1,4 @@
-"""FP64-accurate digit products and the 64-column kernels of the FP64 factorization.
+"""FP64-accurate digit products and the 32-column panel kernel of the FP64 factorization.
 
 The digits keep 56 bits below each row's maximum and all digit pairs down to 2^-58 of
 the product of the row maxima, so an entry of C - A B^T is off by at most
@@ -18,7 +18,7 @@ def _lib():
     lib = _lib.load()
     lib.omg_internal_digit_update.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int] + [ctypes.c_void_p] * 3 + [
         ctypes.c_int, ctypes.c_void_p]
-    lib.omg_internal_potrf_trsm64.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_int64] + [ctypes.c_void_p] * 3
+    lib.omg_internal_panel32.argtypes = [ctypes.c_int, ctypes.c_int64] + [ctypes.c_void_p] * 3
     return lib
 
 
@@ -82,33 +82,32 @@ def test_digit_update_not_finite_rows(cuda):
     _check(out[np.ix_(*ok)], A[ok[0]], B[ok[1]], C[np.ix_(*ok)], 0)
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 63, 64])
-def test_potrf_and_panel_solve(cuda, n):
+def _panel(cuda, A, P):
+    """The factor of A and the rows P L^-T by the kernel (w x w, m x w numpy), its status and column."""
     import torch
-    rng = np.random.default_rng(n)
-    X = rng.standard_normal((n, n))
-    A = X @ X.T + n * np.eye(n)
-    P = rng.standard_normal((77, 64))
-    a, p = torch.as_tensor(A).to(cuda), torch.as_tensor(np.ascontiguousarray(P.T)).to(cuda)
+    w, m = A.shape[0], P.shape[0]
+    a = torch.as_tensor(np.ascontiguousarray(np.vstack([A, P]).T)).to(cuda)
     err, col = torch.zeros(4, dtype=torch.int32, device=cuda), torch.zeros(1, dtype=torch.int64, device=cuda)
     torch.cuda.synchronize()
-    assert _lib().omg_internal_potrf_trsm64(n, _p(a), 77, _p(p), _p(err), _p(col)) == 0
-    assert int(err[0]) == 0
-    L = np.tril(a.cpu().numpy().T)
-    # Cholesky's and the substitution's backward error, n eps
-    assert np.linalg.norm(L @ L.T - A) <= 2.0**-52 * n * np.linalg.norm(A)
-    if n == 64:
-        W = p.cpu().numpy().T
-        assert np.linalg.norm(W @ L.T - P) <= 2.0**-52 * n * np.linalg.norm(W) * np.linalg.norm(L)
+    assert _lib().omg_internal_panel32(w, m, _p(a), _p(err), _p(col)) == 0
+    out = a.cpu().numpy().T
+    return np.tril(out[:w]), out[w:], int(err[0]), int(col[0])
 
 
-def test_potrf_reports_the_wrong_sign(cuda):
-    import torch
-    A = np.eye(64)
+@pytest.mark.parametrize("w,m", [(1, 0), (2, 0), (31, 0), (32, 0), (32, 1), (32, 33), (32, 300)])
+def test_panel(cuda, w, m):
+    rng = np.random.default_rng(w + m)
+    X = rng.standard_normal((w, w))
+    A, P = X @ X.T + w * np.eye(w), rng.standard_normal((m, w))
+    L, W, status, _ = _panel(cuda, A, P)
+    assert status == 0
+    # Cholesky's and the substitution's backward error, w eps
+    assert np.linalg.norm(L @ L.T - A) <= 2.0**-52 * w * np.linalg.norm(A)
+    assert np.linalg.norm(W @ L.T - P) <= 2.0**-52 * w * np.linalg.norm(W) * np.linalg.norm(L)
+
+
+def test_panel_reports_the_wrong_sign(cuda):
+    A = np.eye(32)
     A[9, 9] = -1.0
-    a = torch.as_tensor(A).to(cuda)
-    p = torch.zeros((64, 1), dtype=torch.float64, device=cuda)
-    err, col = torch.zeros(4, dtype=torch.int32, device=cuda), torch.zeros(1, dtype=torch.int64, device=cuda)
-    torch.cuda.synchronize()
-    assert _lib().omg_internal_potrf_trsm64(64, _p(a), 1, _p(p), _p(err), _p(col)) == 0
-    assert int(err[0]) == -3 and int(col[0]) == 9
+    A[20, 20] = np.nan
+    assert _panel(cuda, A, np.zeros((1, 32)))[2:] == (-3, 9)
