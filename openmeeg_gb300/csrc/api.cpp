@@ -136,6 +136,9 @@ void digit_gemm(int64_t n, int64_t k, int64_t kdim, const void* Ad, int nda, con
                 int64_t kpad, const int* cexp, int beta, int lmax, const double* B, int64_t ldb, double sgn, double* R,
                 int64_t ldr, int* err, cudaStream_t s, const char* prof_name);
 // f64_digits.cu
+void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t lda, bool ta, const double* B,
+              int64_t ldb, bool tb, double beta, double* C, int64_t ldc, int* err, cudaStream_t s,
+              const std::vector<std::pair<int64_t, int64_t>>* ranges = nullptr);
 void row_digits_f64(const double* A, int64_t lda, int64_t m, int k, int kpad, int64_t rows_per_plane, void* out, int* ex,
                     cudaStream_t s);
 void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
@@ -1344,17 +1347,25 @@ void gain_contract(const std::vector<std::pair<int64_t, int64_t>>& merged, const
         if (nm > 0) OMG_CUDA(cudaMemcpy2DAsync(gmeg, nm * 8, g + ne, k * 8, nm * 8, nd, cudaMemcpyDeviceToDevice, s));
         return;
     }
-    if (ne > 0 && nd > 0) {
-        if (merged.empty()) OMG_CUDA(cudaMemsetAsync(geeg, 0, (size_t)ne * nd * 8, s));
-        for (size_t q = 0; q < merged.size(); ++q) {
-            const int64_t r0 = merged[q].first, kk = merged[q].second - merged[q].first;
-            gemm<double>(ne, nd, kk, 1.0, Y + r0, N, true, DSM + r0, N, false, q == 0 ? 0.0 : 1.0, geeg, ne, s);
-        }
+    if (nd <= 0 || k <= 0) return;
+    if (kdim == 0) {
+        if (ne > 0) OMG_CUDA(cudaMemsetAsync(geeg, 0, (size_t)ne * nd * 8, s));
+        return;
     }
-    if (nm > 0 && nd > 0)
-        for (const auto& r : merged)
-            gemm<double>(nm, nd, r.second - r.first, 1.0, Y + ne * N + r.first, N, true, DSM + r.first, N, false, 1.0,
-                         gmeg, nm, s);
+    // FP64: one product for both sensor kinds (the sources' digits are formed once)
+    if (ne == 0) {
+        gemm_f64(nm, nd, 0, 1.0, Y, N, true, DSM, N, false, 1.0, gmeg, nm, err, s, &merged);
+    } else if (nm == 0) {
+        gemm_f64(ne, nd, 0, 1.0, Y, N, true, DSM, N, false, 0.0, geeg, ne, err, s, &merged);
+    } else {
+        DevBuf G((size_t)k * nd * 8, s);
+        double* g = G.as<double>();
+        OMG_CUDA(cudaMemsetAsync(g, 0, (size_t)k * nd * 8, s));
+        OMG_CUDA(cudaMemcpy2DAsync(g + ne, k * 8, gmeg, nm * 8, nm * 8, nd, cudaMemcpyDeviceToDevice, s));
+        gemm_f64(k, nd, 0, 1.0, Y, N, true, DSM, N, false, 1.0, g, k, err, s, &merged);
+        OMG_CUDA(cudaMemcpy2DAsync(geeg, ne * 8, g, k * 8, ne * 8, nd, cudaMemcpyDeviceToDevice, s));
+        OMG_CUDA(cudaMemcpy2DAsync(gmeg, nm * 8, g + ne, k * 8, nm * 8, nd, cudaMemcpyDeviceToDevice, s));
+    }
 }
 
 // A geometry's meshes plus one source surface (SurfSourceMat, SurfSource2MEGMat) as
@@ -2143,7 +2154,10 @@ int omg_gemm_f64_dev(omg_context ctx, int32_t trans_a, int32_t trans_b, int64_t 
             if (beta == 0.0)
                 for (int64_t j = 0; j < n; ++j) OMG_CUDA(cudaMemsetAsync(C + j * ldc, 0, (size_t)m * 8, ctx->stream));
         } else {
-            gemm<double>(m, n, k, alpha, A, lda, trans_a != 0, B, ldb, trans_b != 0, beta, C, ldc, ctx->stream);
+            reset_err(ctx);
+            gemm_f64(m, n, k, alpha, A, lda, trans_a != 0, B, ldb, trans_b != 0, beta, C, ldc, ctx->d_err, ctx->stream);
+            check_err(ctx, "GEMM");
+            return;
         }
         OMG_CUDA(cudaStreamSynchronize(ctx->stream));
     });

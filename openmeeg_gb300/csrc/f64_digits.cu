@@ -35,6 +35,8 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <cmath>
+#include <vector>
 
 #include "digits.cuh"
 #include "handles.h"
@@ -44,6 +46,9 @@ namespace omg {
 
 template <typename T>
 void negate_rows(T* B, int64_t ldb, int64_t r0, int64_t r1, int64_t n, cudaStream_t s);
+template <typename T>
+void gemm(int64_t M, int64_t N, int64_t K, T alpha, const T* A, int64_t lda, bool ta, const T* B, int64_t ldb, bool tb,
+          T beta, T* C, int64_t ldc, cudaStream_t s, bool lower = false, int64_t row0 = 0, int64_t col0 = 0);
 
 namespace f64d {
 
@@ -127,25 +132,27 @@ __device__ __forceinline__ void row_digits(const double (&x)[PER], unsigned long
 }
 
 // ---------------------------------------------------------------------------
-// Digits of the rows of a column-major m x K block (K a multiple of 128, up to
-// 256): plane s - 1 holds a_s 2^(-8 (s - 1)) in bf16 (exact), rows of `ldk`
+// Digits of the rows of a column-major m x k matrix in segments of K columns
+// (blockIdx.y; 128 or 256, zero-padded): plane s - 1 holds a_s 2^(-8 (s - 1)) in bf16 (exact), rows of `ldk`
 // entries; ex[i]: the row's exponent.  A CTA takes 32 rows, lanes along them
 // (coalesced reads of the columns), eight groups of K / 8 consecutive columns.
 // ---------------------------------------------------------------------------
 template <int K>
-__global__ void __launch_bounds__(256) row_digits_kernel(const double* A, int64_t lda, int64_t m, int k,
+__global__ void __launch_bounds__(256) row_digits_kernel(const double* A, int64_t lda, int64_t m, int64_t k,
                                                          int64_t rows_per_plane, __nv_bfloat16* out, int* ex) {
     constexpr int PER = K / 8;
     __shared__ unsigned long long red[8][32];
     const int lane = threadIdx.x % 32, grp = threadIdx.x / 32;
-    const int64_t row = (int64_t)blockIdx.x * 32 + lane;
+    const int64_t row = (int64_t)blockIdx.x * 32 + lane, c0 = (int64_t)blockIdx.y * K;
+    out += (int64_t)blockIdx.y * ND * rows_per_plane * K;
+    ex += (int64_t)blockIdx.y * rows_per_plane;
     double x[PER];
     unsigned long long mb = 0;
     pdl_wait();
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-        const int c = grp * PER + i;
-        x[i] = row < m && c < k ? A[row + (int64_t)c * lda] : 0.0;
+        const int64_t c = c0 + grp * PER + i;
+        x[i] = row < m && c < k ? A[row + c * lda] : 0.0;
         mb = max(mb, (unsigned long long)__double_as_longlong(x[i]) & 0x7FFFFFFFFFFFFFFFull);
     }
     red[grp][lane] = mb;
@@ -368,7 +375,9 @@ struct Walk {
     }
 };
 
-template <int TN>
+// UPDATE: C -= A B^T; otherwise segment s of the products, C_s = A_s B_s^T, to the s-th of the M x Nc slices of C (operands:
+// ND planes per segment, exponents per segment; tile numbers run over the segments).
+template <int TN, bool UPDATE>
 __global__ void __launch_bounds__(THREADS, 1)
     digit_update_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, int64_t M,
                         int64_t Nc, int nchunk, int ra, int rb, const int* exA,
@@ -402,7 +411,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     pdl_wait();
     pdl_next();
     const uint32_t tmem = sh.tmem;
-    Walk walk{(int)((M + BT - 1) / BT), (int)((Nc + TN - 1) / TN), lower};
+    const int64_t per_seg = UPDATE ? ntiles : ((M + BT - 1) / BT) * ((Nc + TN - 1) / TN);
+    const Walk walk0{(int)((M + BT - 1) / BT), (int)((Nc + TN - 1) / TN), lower};
+    Walk walk = walk0;
 
     if (warp == 0) {
         if (lane == 0) {   // ---- TMA producer
@@ -410,8 +421,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             bool ok = true;
             for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 int i, j;
-                walk.tile(t, i, j);
-                const int ya = i * BT, yb = j * TN;
+                const int seg = UPDATE ? 0 : (int)(t / per_seg);
+                if (!UPDATE) walk = walk0;
+                walk.tile(t - seg * per_seg, i, j);
+                const int ya = i * BT + seg * ND * ra, yb = j * TN + seg * ND * rb;
                 for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 4, 5>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
                 for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 2, 3>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
                 for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 6, 9>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
@@ -454,7 +467,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         };
         for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
             int ti, tj;
-            walk.tile(t, ti, tj);
+            const int seg = UPDATE ? 0 : (int)(t / per_seg);
+            if (!UPDATE) walk = walk0;
+            walk.tile(t - seg * per_seg, ti, tj);
             const int64_t row = (int64_t)ti * BT + q * 32 + lane, col0 = (int64_t)tj * TN + c0;
             long long H[NCW];   // levels 2..5 in units of level 5, |H| < 2^47
             if (!begin()) break;
@@ -493,19 +508,23 @@ __global__ void __launch_bounds__(THREADS, 1)
                                    __float2int_rn((__uint_as_float(a[j]) + __uint_as_float(b[j])) * 0x1p37f);
             }
             end();
-            const int er = (row < M ? exA[row] : EXP_ZERO) - 53;   // those units, 2^-53 of the exponents' product
-            double* const Cr = C + row + col0 * ldc;
+            // (the integers' unit is 2^-53 of the exponents' product)
+            const int er = (row < M ? exA[row + (int64_t)seg * ra] : EXP_ZERO) - 53;
+            const int* const eb = exB + (int64_t)seg * rb + col0;
+            double* const Cr = C + (int64_t)seg * M * Nc + row + col0 * ldc;
             const int64_t j1 = min((int64_t)NCW, Nc - col0), jl = lower ? min(j1, row - col0 + 1) : j1;
             if (row >= M) continue;
 #pragma unroll
             for (int h = 0; h < NCW / 8; ++h) {
                 double c[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) c[j] = h * 8 + j < jl ? Cr[(h * 8 + j) * ldc] : 0.0;
+                for (int j = 0; j < 8; ++j) c[j] = UPDATE && h * 8 + j < jl ? Cr[(h * 8 + j) * ldc] : 0.0;
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    if (h * 8 + j < jl)
-                        Cr[(h * 8 + j) * ldc] = c[j] - scaled_double(H[h * 8 + j], er + exB[col0 + h * 8 + j]);
+                    if (h * 8 + j < jl) {
+                        const double v = scaled_double(H[h * 8 + j], er + eb[h * 8 + j]);
+                        Cr[(h * 8 + j) * ldc] = UPDATE ? c[j] - v : v;
+                    }
             }
         }
     }
@@ -840,6 +859,74 @@ __global__ void __launch_bounds__(256) diag_apply_kernel(const double* M, int up
     if (out) write_digits4(v, warp_max(mb), out, nrhs, blockIdx.x, ex, lane);
 }
 
+// ---------------------------------------------------------------------------
+// General products, K in segments of 256
+// ---------------------------------------------------------------------------
+constexpr int KS = 256;
+constexpr int MAXRANGES = 8;
+struct RowRanges {   // the K index runs over rows [beg[q], beg[q] + len[q]) one after the other; n = 0: all rows in order
+    int n;
+    int64_t beg[MAXRANGES], len[MAXRANGES];
+    __device__ __forceinline__ int64_t row(int64_t k) const {
+        for (int q = 0; q < n; ++q) {
+            if (k < len[q]) return beg[q] + k;
+            k -= len[q];
+        }
+        return k;
+    }
+};
+
+// Digit rows of the n columns of a column-major matrix, K (kdim of its rows) contiguous in memory: a warp per column and
+// segment (blockIdx.y), eight entries per lane.
+__global__ void __launch_bounds__(256) col_segments_kernel(const double* __restrict__ A, int64_t lda, int64_t n, int64_t kdim,
+                                                           const __grid_constant__ RowRanges rr, __nv_bfloat16* out,
+                                                           int* ex) {
+    const int lane = threadIdx.x % 32;
+    const int64_t c = (int64_t)blockIdx.x * 8 + threadIdx.x / 32, seg = blockIdx.y;
+    if (c >= n) return;
+    const double* a = A + c * lda;
+    double x[8];
+    unsigned long long mb = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const int64_t k = seg * KS + 8 * lane + u;
+        x[u] = k < kdim ? a[rr.row(k)] : 0.0;
+        mb = max(mb, (unsigned long long)__double_as_longlong(x[u]) & 0x7FFFFFFFFFFFFFFFull);
+    }
+    row_digits<8>(x, warp_max(mb), out + (seg * ND * n + c) * KS + 8 * lane, n * KS, lane == 0 ? ex + seg * n + c : nullptr);
+}
+
+// C = alpha sum of the segments' products + beta C, in segment order.  An entry whose row of A or of B^T holds an infinity
+// or a NaN is summed directly, with IEEE arithmetic's result.
+struct Operand {   // element (i, k) of op(A): p[i * si + row(k) * sk]
+    const double* p;
+    int64_t si, sk;
+};
+__global__ void sum_segments_kernel(int64_t M, int64_t N, int64_t kdim, int nseg, const double* __restrict__ P,
+                                    const int* __restrict__ exA, const int* __restrict__ exB, Operand A, Operand B,
+                                    const __grid_constant__ RowRanges rr, int64_t k0, double alpha, double beta, double* C,
+                                    int64_t ldc) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= M) return;
+    for (int64_t j = blockIdx.y; j < N; j += gridDim.y) {
+        double v = 0.0;
+        bool special = false;
+        for (int g = 0; g < nseg; ++g) {
+            v += P[((int64_t)g * N + j) * M + i];
+            special |= exA[(int64_t)g * M + i] == EXP_NAN || exB[(int64_t)g * N + j] == EXP_NAN;
+        }
+        if (special) {
+            v = 0.0;
+            for (int64_t k = 0; k < kdim; ++k) {
+                const int64_t r = rr.row(k0 + k);
+                v = fma(A.p[i * A.si + r * A.sk], B.p[j * B.si + r * B.sk], v);
+            }
+        }
+        double* c = C + i + j * ldc;
+        *c = beta == 0.0 ? alpha * v : fma(alpha, v, beta * *c);
+    }
+}
+
 }  // namespace f64d
 
 
@@ -851,22 +938,24 @@ void row_digits_f64(const double* A, int64_t lda, int64_t m, int k, int kpad, in
     ProfScope prof_("f64_digits", s);
     const unsigned grid = (unsigned)((m + 31) / 32);
     auto kern = kpad == 128 ? f64d::row_digits_kernel<128> : f64d::row_digits_kernel<256>;
-    f64d::launch(kern, grid, 256, 0, s, A, lda, m, k, rows_per_plane, static_cast<__nv_bfloat16*>(out), ex);
+    f64d::launch(kern, grid, 256, 0, s, A, lda, m, (int64_t)k, rows_per_plane, static_cast<__nv_bfloat16*>(out), ex);
     f64d::check("FP64 row digits");
 }
 
-// C (M x Nc, column-major; `lower`: entries with row >= column only) -= A B^T from digit rows of kpad entries:
-// A's planes start at row a0 of buffers of ra rows per plane, B's at b0 of rb.
-void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
-                      const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, bool lower,
-                      int* err, cudaStream_t s, const char* name) {
+// nseg > 0: the products of nseg segments, to slices of C; otherwise the update.
+static void digit_product(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
+                          const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, bool lower,
+                          int nseg, int* err, cudaStream_t s, const char* name) {
     if (M <= 0 || Nc <= 0) return;
-    if (kpad % f64d::BK || kpad > 256 || 7 * std::max(ra, rb) > (1ll << 30))
+    const int64_t segs = std::max(1, nseg);
+    if (kpad % f64d::BK || kpad > 256 || segs * f64d::ND * std::max(ra, rb) > (1ll << 30))
         throw Error(OMG_ERR_UNSUPPORTED, "digit update: bad sizes");
     ProfScope prof_(name, s);
     static int n_sm = 0;
     if (!n_sm) {
-        for (auto k : {f64d::digit_update_kernel<128>, f64d::digit_update_kernel<64>, f64d::digit_update_kernel<32>})
+        for (auto k : {f64d::digit_update_kernel<128, true>, f64d::digit_update_kernel<64, true>, f64d::digit_update_kernel<32, true>,
+                       f64d::digit_update_kernel<128, false>, f64d::digit_update_kernel<64, false>,
+                       f64d::digit_update_kernel<32, false>})
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, f64d::SMEM_BYTES);
         int dev = 0, n = 0;
         cudaGetDevice(&dev);
@@ -882,7 +971,7 @@ void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra
     if (!lower) {
         int64_t best = INT64_MAX;
         for (int w : {128, 64, 32}) {
-            const int64_t waves = (mt * ((Nc + w - 1) / w) + n_sm - 1) / n_sm;
+            const int64_t waves = (segs * mt * ((Nc + w - 1) / w) + n_sm - 1) / n_sm;
             const int64_t t = waves * 34 * (kpad / 16) * (w == 128 ? 64 : w == 64 ? 48 : 40) + 100 * w;
             if (t < best) {
                 best = t;
@@ -891,16 +980,104 @@ void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra
         }
     }
     const CUtensorMap mA = tc::make_map_2d(static_cast<const uint16_t*>(A) + a0 * kpad, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                                           2, f64d::ND * ra - a0, kpad, kpad, f64d::BK, f64d::BT);
+                                           2, segs * f64d::ND * ra - a0, kpad, kpad, f64d::BK, f64d::BT);
     const CUtensorMap mB = tc::make_map_2d(static_cast<const uint16_t*>(B) + b0 * kpad, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                                           2, f64d::ND * rb - b0, kpad, kpad, f64d::BK, tn);
+                                           2, segs * f64d::ND * rb - b0, kpad, kpad, f64d::BK, tn);
     const int64_t nt = (Nc + tn - 1) / tn;
-    const int64_t ntiles = lower ? mt * nt - nt * (nt - 1) / 2 : mt * nt;
+    const int64_t ntiles = segs * (lower ? mt * nt - nt * (nt - 1) / 2 : mt * nt);
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, n_sm);
-    auto kern = tn == 128 ? f64d::digit_update_kernel<128> : tn == 64 ? f64d::digit_update_kernel<64> : f64d::digit_update_kernel<32>;
+    auto kern = nseg > 0 ? (tn == 128  ? f64d::digit_update_kernel<128, false>
+                            : tn == 64 ? f64d::digit_update_kernel<64, false>
+                                       : f64d::digit_update_kernel<32, false>)
+                         : (tn == 128  ? f64d::digit_update_kernel<128, true>
+                            : tn == 64 ? f64d::digit_update_kernel<64, true>
+                                       : f64d::digit_update_kernel<32, true>);
     f64d::launch(kern, grid, f64d::THREADS, f64d::SMEM_BYTES, s, mA, mB, M, Nc, kpad / f64d::BK, (int)ra, (int)rb, exA + a0,
                  exB + b0, C, ldc, lower ? 1 : 0, ntiles, err);
     f64d::check(name);
+}
+
+// C (M x Nc, column-major; `lower`: entries with row >= column only) -= A B^T from digit rows of kpad entries:
+// A's planes start at row a0 of buffers of ra rows per plane, B's at b0 of rb.
+void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
+                      const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, bool lower,
+                      int* err, cudaStream_t s, const char* name) {
+    digit_product(M, Nc, kpad, A, ra, a0, exA, B, rb, b0, exB, C, ldc, lower, 0, err, s, name);
+}
+
+// C (M x N) = alpha op(A) op(B) + beta C over the K rows (columns) the ranges list (null: all K), FP64, column-major.
+// From about 60 us of FP64-pipe time on by FP64-accurate digit products, segment by segment of K (partial products of up to
+// 512 MB at a time); below that the operands' digits and the launches cost more than the FP64 kernel.
+void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t lda, bool ta, const double* B,
+              int64_t ldb, bool tb, double beta, double* C, int64_t ldc, int* err, cudaStream_t s,
+              const std::vector<std::pair<int64_t, int64_t>>* ranges) {
+    using namespace f64d;
+    if (M <= 0 || N <= 0) return;
+    RowRanges rr{};
+    if (ranges) {
+        if (ranges->size() > (size_t)MAXRANGES) throw Error(OMG_ERR_UNSUPPORTED, "GEMM: too many row ranges");
+        K = 0;
+        for (const auto& r : *ranges) {
+            rr.beg[rr.n] = r.first;
+            rr.len[rr.n] = r.second - r.first;
+            K += rr.len[rr.n++];
+        }
+        if (rr.n > 0 && (!ta || tb)) throw Error(OMG_ERR_INVALID, "GEMM: row ranges need both operands K-contiguous");
+    }
+    // the FP64 kernel: waves of 32 x 32 tiles, 0.29 us per K on an SM
+    const double us = std::ceil((double)((M + 31) / 32) * ((N + 31) / 32) / 152.0) * 0.29 * (double)K;
+    if (us < 60.0 || K <= 0) {
+        if (K <= 0 || rr.n == 0) {
+            gemm<double>(M, N, K, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, s);
+            return;
+        }
+        for (int q = 0; q < rr.n; ++q)
+            gemm<double>(M, N, rr.len[q], alpha, A + rr.beg[q], lda, true, B + rr.beg[q], ldb, false, q == 0 ? beta : 1.0, C,
+                         ldc, s);
+        return;
+    }
+    // segments at a time: the partial products, and the operands' digits (14 bytes an entry), within 512 MB each
+    const int64_t nseg = (K + KS - 1) / KS;
+    const int64_t at_once = std::max<int64_t>(
+        1, std::min<int64_t>({nseg, (512ll << 20) / (M * N * 8), (512ll << 20) / (std::max(M, N) * KS * 14)}));
+    DevBuf P((size_t)at_once * M * N * 8, s), dA((size_t)at_once * ND * M * KS * 2, s),
+        dB((size_t)at_once * ND * N * KS * 2, s), ex((size_t)at_once * (M + N) * sizeof(int), s);
+    int* exA = ex.as<int>();
+    int* exB = exA + at_once * M;
+    for (int64_t g0 = 0; g0 < nseg; g0 += at_once) {
+        const int64_t ns = std::min(at_once, nseg - g0), k0 = g0 * KS, kk = std::min(K - k0, ns * KS);
+        RowRanges part = rr;   // the rows from k0 on
+        for (int64_t skip = k0; part.n > 0 && skip > 0;) {
+            const int64_t d = std::min(skip, part.len[0]);
+            part.beg[0] += d;
+            part.len[0] -= d;
+            skip -= d;
+            if (part.len[0] == 0 && part.n > 1) {
+                for (int q = 1; q < part.n; ++q) {
+                    part.beg[q - 1] = part.beg[q];
+                    part.len[q - 1] = part.len[q];
+                }
+                --part.n;
+            }
+        }
+        auto digits = [&](const double* X, int64_t ldx, bool k_contiguous, int64_t n, void* out, int* e) {
+            ProfScope prof_("f64_digits", s);
+            if (k_contiguous)
+                col_segments_kernel<<<dim3((unsigned)((n + 7) / 8), (unsigned)ns), 256, 0, s>>>(
+                    X + (part.n ? 0 : k0), ldx, n, kk, part, static_cast<__nv_bfloat16*>(out), e);
+            else
+                launch(row_digits_kernel<KS>, dim3((unsigned)((n + 31) / 32), (unsigned)ns), 256, 0, s, X + k0 * ldx, ldx, n,
+                       kk, n, static_cast<__nv_bfloat16*>(out), e);
+            check("GEMM digits");
+        };
+        digits(A, lda, ta, M, dA.p, exA);
+        digits(B, ldb, !tb, N, dB.p, exB);
+        digit_product(M, N, KS, dA.p, M, 0, exA, dB.p, N, 0, exB, P.as<double>(), M, false, (int)ns, err, s, "f64_product");
+        const Operand oa{A, ta ? lda : 1, ta ? 1 : lda}, ob{B, tb ? 1 : ldb, tb ? ldb : 1};
+        sum_segments_kernel<<<dim3((unsigned)((M + 127) / 128), (unsigned)std::min<int64_t>(N, 65535)), 128, 0, s>>>(
+            M, N, kk, (int)ns, P.as<double>(), exA, exB, oa, ob, rr, k0, alpha, g0 == 0 ? beta : 1.0, C, ldc);
+        check("GEMM segments");
+    }
 }
 
 // Sub-panel at (k0, k0) of the matrix, w <= 32 columns: the diagonal block's factor to Ld, the rows below solved in place.

@@ -11,9 +11,9 @@
 //    is the weighted sum of the inverse's columns at the electrode's vertices,
 //    gathered by one kernel (HBM-bound, 3 N reads per electrode).
 //  - MEG: V = Head2MEGMat is dense; Q is an N x N x n_squids product.
-// then gain = Q^T DSM (+ DS2MM).  FP64: CUDA-core FP64 GEMMs.  Mixed: the
-// FP64-accurate fixed-point digit GEMM on the bf16 tensor cores (the one the
-// refinement residual uses; error below 5e-13 of |Q||DSM| normwise).
+// then gain = Q^T DSM (+ DS2MM).  FP64: FP64-accurate digit products (gemm_f64).
+// Mixed: the shorter digits of the refinement residual (error below 5e-13 of
+// |Q||DSM| normwise).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -22,9 +22,9 @@
 #include "pipeline.h"
 
 namespace omg {
-template <typename T>
-void gemm(int64_t M, int64_t N, int64_t K, T alpha, const T* A, int64_t lda, bool ta, const T* B, int64_t ldb, bool tb,
-          T beta, T* C, int64_t ldc, cudaStream_t s, bool lower = false, int64_t row0 = 0, int64_t col0 = 0);
+void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t lda, bool ta, const double* B,
+              int64_t ldb, bool tb, double beta, double* C, int64_t ldc, int* err, cudaStream_t s,
+              const std::vector<std::pair<int64_t, int64_t>>* ranges = nullptr);
 int64_t digits_ld(int64_t n);
 void digits_columns(const double* M, int64_t n, int64_t ncol, int64_t ldm, int nd, int beta, int64_t rows_per_plane,
                     int64_t ldo, void* out, int* ex, cudaStream_t s,
@@ -104,7 +104,7 @@ void contract(int64_t N, int64_t k, const double* Q, const double* DSM, int64_t 
         return;
     }
     if (init) OMG_CUDA(cudaMemcpyAsync(gain, init, (size_t)k * nd * 8, cudaMemcpyDeviceToDevice, s));
-    gemm<double>(k, nd, N, 1.0, Q, N, true, DSM, N, false, init ? 1.0 : 0.0, gain, k, s);
+    gemm_f64(k, nd, N, 1.0, Q, N, true, DSM, N, false, init ? 1.0 : 0.0, gain, k, err, s);
 }
 
 void check_common(omg_context ctx, int64_t N, const double* hminv, int64_t ld, int32_t packed, const double* dsm,
@@ -215,7 +215,7 @@ extern "C" int omg_gain_meg_dev(omg_context ctx, int64_t N, const double* hminv,
             digit_gemm(N, n_squids, N, Ad.p, ndg, rexp, Xd.p, ndg, kpad, rexp + N, beta, lmax, Q.as<double>(), N, 1.0,
                        Q.as<double>(), N, ctx->d_err, s, "gain_direct_tc");
         } else {
-            gemm<double>(N, n_squids, N, 1.0, H, ldh, false, Vt.as<double>(), N, false, 0.0, Q.as<double>(), N, s);
+            gemm_f64(N, n_squids, N, 1.0, H, ldh, false, Vt.as<double>(), N, false, 0.0, Q.as<double>(), N, ctx->d_err, s);
         }
         contract(N, n_squids, Q.as<double>(), dsm, n_dipoles, ds2mm, gain, precision, ctx->d_err, s);
         check_err(ctx, "GainMEG");
