@@ -212,26 +212,22 @@ __device__ __forceinline__ int64_t lower_at(int64_t a, int64_t b, int64_t ld) {
 //   2. l[e][x] = (integral over the edge of 1/|x - y|) / length
 //      = 2 atanh(len / (d_a + d_b)) / len for every edge (1.5 per triangle instead
 //      of three logarithms each in S and in D: D's log((d_b + r_b.u)/(d_a + r_a.u))
-//      is the same integral);
-//   3. per (triangle, point): the heights h = n.(p0 - x), E_j = n.(r_j+1 x r_j+2)
-//      (linear in x; E_0 + E_1 + E_2 = 2A), the solid angle
-//      W = 2 atan(2 A h / (d0 d1 d2 + sum d_i r_j.r_k)) with r_j.r_k from the tabled
-//      distances and the edge lengths, then
-//        S = sum_i E_opp(i) l_i - h W,
-//        D_j = (W E_j + h sum_i (D_j+1 . D_i) l_i) / 2A, D_0 + D_1 + D_2 = W.
-// About 80 FP64 operations per (triangle, point) for S and D together.  The
-// arctangent and the logarithm take their series where the argument is small
-// (|x| <= 1/16 or 1/4, by the far terms' size against 2^-55) and the library
-// functions elsewhere; square roots and reciprocals are the hardware
+//      is the same integral), and (d_a + d_b)^2 - len^2 = 2 (d_a d_b + r_a.r_b);
+//   3. per (triangle, point): h = n.(p0 - x) and E_j = n.(r_j+1 x r_j+2) (linear in
+//      x; E_0 + E_1 + E_2 = 2A), half the solid angle
+//      w = atan(2 A h / (d0 d1 d2 + sum d_i r_j.r_k)), then
+//        S = sum_i E_opp(i) l_i - 2 h w,
+//        D_j = (w E_j + h/2 D_j+1.(sum_i D_i l_i)) / A, D_0 + D_1 + D_2 = 2 w,
+//      in 46 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
+// About 75 FP64 operations per (triangle, point) for S and D together.  The
+// arctangent and the logarithm take polynomials where the argument is small and the
+// library functions elsewhere; square roots and reciprocals are the hardware
 // approximations refined by one third-order Newton step.
-// Measured: 27.4 ms for the blocks of a 4486-unknown head (131 M values; 20 ms at the
-// 529 G FMA/s of the FP64 pipe) against 121 ms for one thread per pair without
-// tables; the 4-layer head of 7 / 9 / 10 / 11-frequency spheres 73 ms against 320 ms.
 // Lanes run over the triangles a at the same rule point, so every table read is
 // coalesced, the triangle b is uniform in a warp, and the sum over the rule stays
 // in registers (no shuffles, which cost FP64 additions).
 // ---------------------------------------------------------------------------
-constexpr int TGEO = 22;   // p0, -n, m0 = n x D0, m2 = n x D2 (3 each), 2A, |D_i|^2 (3), D0.D1 D1.D2 D2.D0, |D_i| (3)
+constexpr int TGEO = 22;   // p0, -2 n, m0 = n x D0, m2 = n x D2 (3 each), 2A, |D_i|^2 (3), (|D0|^2 |D2|^2 D0.D2) / 4, |D_i| (3)
 
 __global__ void sd_geometry_kernel(int64_t t0, int64_t nt, const double* __restrict__ V,
                                    const int32_t* __restrict__ T, const int32_t* __restrict__ v2t_beg,
@@ -248,12 +244,12 @@ __global__ void sd_geometry_kernel(int64_t t0, int64_t nt, const double* __restr
     const d3 m0 = dev::cross(n, D0), m2 = dev::cross(n, D2);
     double* g = tgeo + it * TGEO;
     g[0] = p0.x; g[1] = p0.y; g[2] = p0.z;
-    g[3] = -n.x; g[4] = -n.y; g[5] = -n.z;
+    g[3] = -2.0 * n.x; g[4] = -2.0 * n.y; g[5] = -2.0 * n.z;
     g[6] = m0.x; g[7] = m0.y; g[8] = m0.z;
     g[9] = m2.x; g[10] = m2.y; g[11] = m2.z;
     g[12] = nrm;
     g[13] = dev::dot(D0, D0); g[14] = dev::dot(D1, D1); g[15] = dev::dot(D2, D2);
-    g[16] = dev::dot(D0, D1); g[17] = dev::dot(D1, D2); g[18] = dev::dot(D2, D0);
+    g[16] = 0.25 * g[13]; g[17] = 0.25 * g[15]; g[18] = 0.25 * dev::dot(D2, D0);
     g[19] = sqrt(g[13]); g[20] = sqrt(g[14]); g[21] = sqrt(g[15]);
     // table row of edge i (corners i, i + 1): the slot 3 t + i of the first triangle of the range that has it
     for (int i = 0; i < 3; ++i) {
@@ -290,9 +286,9 @@ __device__ __forceinline__ double sd_sqrt(double x) {
     const double e = fma(-g, y, 1.0);
     return fma(g * e, fma(0.375, e, 0.5), g);
 }
-// |x| < 1e-10 on the integer pipe.
-__device__ __forceinline__ bool sd_flat(double x) {
-    return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) < __double_as_longlong(1e-10);
+// |x| / 2 < 1e-10 on the integer pipe.
+__device__ __forceinline__ bool sd_flat2(double x) {
+    return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) < __double_as_longlong(2e-10);
 }
 // |x| < 2^k by the exponent field (integer pipe; NaN and infinity compare false).
 __device__ __forceinline__ bool sd_below(double x, int k) {
@@ -328,60 +324,61 @@ __global__ void __launch_bounds__(SD_THREADS) sd_distance_kernel(const double* _
     }
 }
 
-// 2 atanh(len / R) / len, R = d_a + d_b.  With y = 1/R and z = len y: 2 y (1 + z^2/3 + z^4/5 + ...); the last
-// term kept is above 2^-55 at each limit.
+// 2 atanh(len / R) / len, R = d_a + d_b.  With y = 1/R, z = len y and w = z^2: 2 y (1 + w f(w)), f(w) = (atanh(z)/z - 1)/w by
+// the polynomial that interpolates it at the Chebyshev nodes of [0, limit^2] (relative error of the result 2^-56.8 for
+// z < 1/8 and 2^-58.8 for z < 1/4; the Taylor series takes three terms more).
 __device__ __forceinline__ double sd_edge(double R, double len) {
     const double y = sd_rcp(R);
     const double z = len * y, w = z * z;
-    double p;
-    if (sd_below(z, -4)) {          // z < 1/16
-        p = fma(w, 1.0 / 13, 1.0 / 11);
-    } else if (sd_below(z, -3)) {   // z < 1/8
-        p = fma(w, 1.0 / 17, 1.0 / 15);
-        p = fma(w, p, 1.0 / 13);
-        p = fma(w, p, 1.0 / 11);
-    } else if (sd_below(z, -2)) {   // z < 1/4
-        p = fma(w, 1.0 / 27, 1.0 / 25);
-        p = fma(w, p, 1.0 / 23);
-        p = fma(w, p, 1.0 / 21);
-        p = fma(w, p, 1.0 / 19);
-        p = fma(w, p, 1.0 / 17);
-        p = fma(w, p, 1.0 / 15);
-        p = fma(w, p, 1.0 / 13);
-        p = fma(w, p, 1.0 / 11);
+    double f;
+    if (__all_sync(__activemask(), sd_below(z, -3))) {   // (one of the two for the whole warp: mixed warps would run both)
+        f = fma(w, 0.08013059813075277, 0.09085223469123827);
+        f = fma(w, f, 0.11111157356123932);
+        f = fma(w, f, 0.14285714116012183);
+        f = fma(w, f, 0.20000000000227505);
+        f = fma(w, f, 0.3333333333333328);
+    } else if (sd_below(z, -2)) {
+        f = fma(w, 0.06828732233627811, 0.05689643661793962);
+        f = fma(w, f, 0.066791397041253);
+        f = fma(w, f, 0.07691841912131238);
+        f = fma(w, f, 0.09090919255417686);
+        f = fma(w, f, 0.1111111098689728);
+        f = fma(w, f, 0.14285714286473053);
+        f = fma(w, f, 0.1999999999999822);
+        f = fma(w, f, 0.3333333333333333);
     } else {
-        return 2.0 * atanh(len / R) / len;
+        return log((R + len) * sd_rcp(R - len)) * sd_rcp(len);
     }
-    p = fma(w, p, 1.0 / 9);
-    p = fma(w, p, 1.0 / 7);
-    p = fma(w, p, 1.0 / 5);
-    p = fma(w, p, 1.0 / 3);
-    return 2.0 * fma(w * p, y, y);
+    const double y2 = y + y;
+    return fma(w * f, y2, y2);
 }
 
-// The solid angle, 2 atan2(num, den): its series where num / den < 1/16 (den > 0).
-__device__ __forceinline__ double sd_angle(double num, double den) {
+// Half the solid angle, atan2(num, den): where t = num / den < 1/16 (den > 0) by t (1 + w f(w)), w = t^2, f interpolated as
+// above (relative error 2^-60.7; 2^-64.2 below 2^-7).
+__device__ __forceinline__ double sd_half_angle(double num, double den) {
     const double t = num * sd_rcp(den);
-    if (__double2hiint(den) < 0 || !sd_below(t, -4)) return 2.0 * atan2(num, den);
+    if (__double2hiint(den) < 0 || !sd_below(t, -4)) return atan2(num, den);
     const double w = t * t;
-    double p;
-    if (sd_below(t, -7)) {
-        p = fma(w, -1.0 / 7, 1.0 / 5);
+    double f;
+    if (__all_sync(__activemask(), sd_below(t, -7))) {
+        f = fma(w, -0.14284697090256454, 0.19999999976718616);
+        f = fma(w, f, -0.33333333333333254);
     } else {
-        p = fma(w, 1.0 / 13, -1.0 / 11);
-        p = fma(w, p, 1.0 / 9);
-        p = fma(w, p, -1.0 / 7);
-        p = fma(w, p, 1.0 / 5);
+        f = fma(w, -0.09016200248147936, 0.11110856205699567);
+        f = fma(w, f, -0.1428571393037775);
+        f = fma(w, f, 0.19999999999826557);
+        f = fma(w, f, -0.3333333333333332);
     }
-    p = fma(w, p, -1.0 / 3);
-    return fma(w * p, t + t, t + t);
+    return fma(w * f, t, t);
 }
 
-// l[3 b + i]: edge i (corners i, i + 1) of triangle b, in the rows that own their edge.
+// Row 3 b + i, edge i (corners i, i + 1) of triangle b, of the rows that own their edge: l, and in prod
+// (d_a + d_b)^2 - len^2 = 2 (d_a d_b + r_a.r_b).
 __global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb, int npt, const int32_t* __restrict__ T,
                                                              int64_t vb, const double* __restrict__ tgeo,
                                                              const int32_t* __restrict__ eown,
-                                                             const double* __restrict__ d, double* __restrict__ l) {
+                                                             const double* __restrict__ d, double* __restrict__ l,
+                                                             double* __restrict__ prod) {
     const int x = blockIdx.x * SD_THREADS + threadIdx.x;
     if (x >= npt) return;
     const int b1 = min(nb, (int)(blockIdx.y + 1) * SD_E);
@@ -391,7 +388,9 @@ __global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb,
         for (int i = 0; i < 3; ++i) {
             if (eown[3 * b + i] != 3 * b + i) continue;
             const double da = d[(int64_t)(tv[i] - vb) * npt + x], db = d[(int64_t)(tv[i == 2 ? 0 : i + 1] - vb) * npt + x];
-            l[(int64_t)(3 * b + i) * npt + x] = sd_edge(da + db, tgeo[b * (int64_t)TGEO + 19 + i]);
+            const double R = da + db;
+            l[(int64_t)(3 * b + i) * npt + x] = sd_edge(R, tgeo[b * (int64_t)TGEO + 19 + i]);
+            prod[(int64_t)(3 * b + i) * npt + x] = fma(R, R, -tgeo[b * (int64_t)TGEO + 13 + i]);
         }
     }
 }
@@ -403,7 +402,7 @@ __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     int64_t tb, int nb, int64_t ta, int64_t a0, int na, int npt, int order, int same, double coeff,
     const int32_t* __restrict__ T, int64_t vb, const double* __restrict__ tgeo, const int32_t* __restrict__ eown,
     const double* __restrict__ qrec, const double* __restrict__ pts, const double* __restrict__ d,
-    const double* __restrict__ l, const int32_t* __restrict__ tpos, double* hm, int64_t ld, double* stmp, int64_t n2,
+    const double* __restrict__ l, const double* __restrict__ prod, const int32_t* __restrict__ tpos, double* hm, int64_t ld, double* stmp, int64_t n2,
     double* dtmp) {
     const int b = blockIdx.y * (SD_THREADS / 32) + threadIdx.x / 32;
     if (b >= nb) return;
@@ -416,43 +415,40 @@ __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     const double* g = tgeo + (int64_t)b * TGEO;
     const double p0x = g[0], p0y = g[1], p0z = g[2], nx = g[3], ny = g[4], nz = g[5];
     const double m0x = g[6], m0y = g[7], m0z = g[8], m2x = g[9], m2y = g[10], m2z = g[11];
-    const double A2 = g[12], q0 = g[13], q1 = g[14], q2 = g[15], g01 = g[16], g12 = g[17], g20 = g[18];
+    const double A2 = g[12], g00 = g[16], g22 = g[17], g02 = g[18];
     const int32_t* tv = T + 3 * (tb + b);
     const double* dr0 = d + (int64_t)(tv[0] - vb) * npt + ia;
     const double* dr1 = d + (int64_t)(tv[1] - vb) * npt + ia;
     const double* dr2 = d + (int64_t)(tv[2] - vb) * npt + ia;
-    const double* lr0 = l + (int64_t)eown[3 * b] * npt + ia;
-    const double* lr1 = l + (int64_t)eown[3 * b + 1] * npt + ia;
-    const double* lr2 = l + (int64_t)eown[3 * b + 2] * npt + ia;
+    const int64_t x0 = (int64_t)eown[3 * b] * npt + ia, x1 = (int64_t)eown[3 * b + 1] * npt + ia,
+                  x2 = (int64_t)eown[3 * b + 2] * npt + ia;
     const double* px = pts + ia;
     const double* py = px + npt;
     const double* pz = py + npt;
     const int np = c_nbpts[order];
-    double sS = 0.0, s0 = 0.0, s1 = 0.0, sw = 0.0;
-    for (int k = 0; k < np; ++k, dr0 += na, dr1 += na, dr2 += na, lr0 += na, lr1 += na, lr2 += na, px += na, py += na,
-             pz += na) {
-        const double d0 = *dr0, d1 = *dr1, d2 = *dr2, l0 = *lr0, l1 = *lr1, l2 = *lr2;
-        const double cx = *px - p0x, cy = *py - p0y, cz = *pz - p0z;
-        const double h = fma(nx, cx, fma(ny, cy, nz * cz));
+    const bool anyS = WANT_S && __any_sync(0xffffffffu, wantS);
+    double sS = 0.0, s1 = 0.0, s2 = 0.0, sw = 0.0;
+    for (int k = 0, o = 0; k < np; ++k, o += na) {
+        const double d0 = dr0[o], d1 = dr1[o], d2 = dr2[o], l1 = l[x1 + o];
+        const double m0 = l[x0 + o] - l1, m2 = l[x2 + o] - l1;
+        const double cx = px[o] - p0x, cy = py[o] - p0y, cz = pz[o] - p0z;
+        const double hh = fma(nx, cx, fma(ny, cy, nz * cz));   // 2 h
         const double E2 = fma(m0x, cx, fma(m0y, cy, m0z * cz));
         const double E1 = fma(m2x, cx, fma(m2y, cy, m2z * cz));
-        const double E0 = (A2 - E1) - E2;
-        // 2 (d0 d1 d2 + sum d_i r_j.r_k), with 2 r_j.r_k = d_j^2 + d_k^2 - |edge|^2
-        const double s12 = d1 + d2, e0 = d0 * d0;
-        const double den = fma(d0, fma(s12, s12, -q1), fma(d1, fma(d2, d2, e0 - q2), d2 * fma(d1, d1, e0 - q0)));
-        const double dd = A2 * h;
-        const double W = sd_angle(dd + dd, den);
+        // 2 (d0 d1 d2 + sum d_i r_j.r_k) by the tabled 2 (d_j d_k + r_j.r_k)
+        const double den = fma(-4.0, d0 * d1 * d2, fma(d0, prod[x1 + o], fma(d1, prod[x2 + o], d2 * prod[x0 + o])));
+        const double num = A2 * hh;
+        const double w = sd_half_angle(num, den);
         const double wr = c_rules[order][k][3];
-        if (WANT_S) {
-            const double el = fma(E2, l0, fma(E0, l1, E1 * l2));
-            sS = fma(wr, sd_flat(dd) ? el : fma(-h, W, el), sS);
+        if (anyS) {   // E0 = 2A - E1 - E2
+            const double el = fma(A2, l1, fma(E2, m0, E1 * m2));
+            sS = fma(wr, sd_flat2(num) ? el : fma(-hh, w, el), sS);
         }
-        if (WANT_D && !sd_flat(h)) {
-            const double f0 = fma(g01, l0, fma(q1, l1, g12 * l2));   // D1 . sum D_i l_i
-            const double f1 = fma(g20, l0, fma(g12, l1, q2 * l2));   // D2 . sum D_i l_i
-            s0 = fma(wr, fma(W, E0, h * f0), s0);
-            s1 = fma(wr, fma(W, E1, h * f1), s1);
-            sw = fma(wr, W, sw);
+        if (WANT_D && !sd_flat2(hh)) {   // sum D_i l_i = D0 m0 + D2 m2
+            const double f1 = fma(g02, m0, g22 * m2), f2 = fma(g00, m0, g02 * m2);
+            s1 = fma(wr, fma(w, E1, hh * f1), s1);
+            s2 = fma(wr, fma(w, E2, hh * f2), s2);
+            sw = fma(wr, w, sw);
         }
     }
     if (!live) return;
@@ -468,12 +464,12 @@ __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     }
     if (WANT_D) {
         double* o = dtmp + (a * nb + b) * 3;
-        const double i2A = 1.0 / A2;   // (W E_j + h f_j) / (2A) per component
-        s0 *= i2A;
-        s1 *= i2A;
-        o[0] = area * s0;
+        const double iA = 2.0 / A2;   // (w E_j + 2h f_j / 4) / A per component; their sum is 2 w
+        s1 *= iA;
+        s2 *= iA;
+        o[0] = area * (2.0 * sw - s1 - s2);
         o[1] = area * s1;
-        o[2] = area * (sw - s0 - s1);
+        o[2] = area * s2;
     }
 }
 
@@ -490,7 +486,7 @@ void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, in
     constexpr int NPTS[4] = {3, 6, 7, 16};
     const int np = NPTS[order];
     // points per batch: tables of about 512 MB, a multiple of 32 triangles (full warps)
-    const int64_t per_tri = (nv + 3 * nb + 3) * 8 * np;
+    const int64_t per_tri = (nv + 6 * nb + 3) * 8 * np;
     const int64_t batch = std::min(na, std::max<int64_t>(32, std::min<int64_t>((512ll << 20) / per_tri, 4096) / 32 * 32));
     DevBuf geo((size_t)nb * (TGEO * 8 + 3 * 4), s), tab_((size_t)per_tri * batch, s);
     double* tgeo = geo.as<double>();
@@ -502,16 +498,18 @@ void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, in
         double* pts = tab_.as<double>();
         double* d = pts + 3 * (int64_t)npt;
         double* l = d + nv * npt;
+        double* prod = l + 3 * nb * npt;
         const unsigned gx = nblocks(npt, SD_THREADS);
         sd_distance_kernel<<<dim3(gx, nblocks(nv, SD_V)), SD_THREADS, 0, s>>>(g.qrec, tab + a0, n, npt, g.V, vbb, (int)nv,
                                                                             pts, d);
         check_launch("S / D distances");
-        sd_edge_kernel<<<dim3(gx, nblocks(nb, SD_E)), SD_THREADS, 0, s>>>(tbb, (int)nb, npt, g.T, vbb, tgeo, eown, d, l);
+        sd_edge_kernel<<<dim3(gx, nblocks(nb, SD_E)), SD_THREADS, 0, s>>>(tbb, (int)nb, npt, g.T, vbb, tgeo, eown, d, l,
+                                                                              prod);
         check_launch("S / D edges");
         const dim3 grid(nblocks(n, 32), nblocks(nb, SD_THREADS / 32));
         auto kern = wantS ? (dtmp ? sd_pair_kernel<true, true> : sd_pair_kernel<true, false>) : sd_pair_kernel<false, true>;
         kern<<<grid, SD_THREADS, 0, s>>>(tbb, (int)nb, tab, a0, n, npt, order, same ? 1 : 0, coeff, g.T, vbb, tgeo, eown,
-                                         g.qrec, pts, d, l, g.tpos, hm, ld, stmp, na, dtmp);
+                                         g.qrec, pts, d, l, prod, g.tpos, hm, ld, stmp, na, dtmp);
         check_launch("S / D pairs");
     }
 }
