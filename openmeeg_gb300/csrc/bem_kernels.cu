@@ -1093,17 +1093,47 @@ __global__ void __launch_bounds__(FF_TI, 3) ff_block_kernel(const float* __restr
     }
 }
 
+// OperatorS and, in out, the three P1 double-layer integrals of one triangle (OperatorS record p) at one point by the shared
+// forms of the S / D tables: one logarithm per edge and one arctangent for both, h = r0.n, E_j = n.(r_j+1 x r_j+2).
+template <bool WANT_S, bool WANT_D>
+__device__ __forceinline__ double near_eval(const double* __restrict__ p, d3 x, double* out) {
+    const d3 r0 = dev::ld3(p) - x, r1 = dev::ld3(p + 3) - x, r2 = dev::ld3(p + 6) - x, n = dev::ld3(p + 9);
+    const double A2 = 2.0 * p[12], e0 = p[13], e1 = p[14], e2 = p[15];
+    const double q0 = e0 * e0, q1 = e1 * e1, q2 = e2 * e2;
+    const double d0 = sd_sqrt(dev::dot(r0, r0)), d1 = sd_sqrt(dev::dot(r1, r1)), d2 = sd_sqrt(dev::dot(r2, r2));
+    const double R0 = d0 + d1, R1 = d1 + d2, R2 = d2 + d0;
+    const double l0 = sd_edge(R0, e0), l1 = sd_edge(R1, e1), l2 = sd_edge(R2, e2);
+    const double m0 = l0 - l1, m2 = l2 - l1;
+    const d3 nr = dev::cross(n, r0);
+    const double E2 = dev::dot(nr, r1), E1 = -dev::dot(nr, r2);
+    const double hh = 2.0 * dev::dot(r0, n), num = A2 * hh;
+    const double den = fma(-4.0, d0 * d1 * d2, fma(d0, fma(R1, R1, -q1), fma(d1, fma(R2, R2, -q2), d2 * fma(R0, R0, -q0))));
+    const double w = sd_half_angle(num, den);
+    if (WANT_D) {
+        out[0] = out[1] = out[2] = 0.0;
+        if (!sd_flat2(hh)) {
+            const double h4 = 0.25 * hh, iA = 2.0 * sd_rcp(A2), g02 = 0.5 * (q1 - q0 - q2);   // D0.D2
+            out[1] = iA * fma(w, E1, h4 * fma(g02, m0, q2 * m2));
+            out[2] = iA * fma(w, E2, h4 * fma(q0, m0, g02 * m2));
+            out[0] = 2.0 * w - out[1] - out[2];
+        }
+    }
+    if (!WANT_S) return 0.0;
+    const double el = fma(A2, l1, fma(E2, m0, E1 * m2));
+    return sd_flat2(num) ? el : fma(-hh, w, el);
+}
+
 // Near pairs: the FP64 analytic kernels of the reference (same outer rule).
 // One lane per (pair, point of the rule): 16 lanes hold a pair, each lane
 // evaluates the analytic integrals at its point (S and D21 over t1 at the
-// points of t2, with shared distances and solid angle; D12 over t2 at the
-// points of t1) and the weighted values are summed across the 16 lanes by
+// points of t2, D12 over t2 at the points of t1, near_eval: about 500 FP64
+// operations against 930 with separate logarithms) and the weighted values are summed across the 16 lanes by
 // shuffles.  Short per-thread chains and many warps hide the latency of the
 // FP64 transcendentals.
 constexpr int NP_LANES = 16;
 
 __global__ void __launch_bounds__(128) near_pairs_kernel(
-    const int2* __restrict__ near, int count, const double* __restrict__ srec, const double* __restrict__ prec,
+    const int2* __restrict__ near, int count, const double* __restrict__ srec,
     const double* __restrict__ qrec, int64_t t1b, int64_t n1, int64_t t2b, int64_t n2, int same, int wantS,
     int wantD12, int wantD21, double cS, int order, const int32_t* __restrict__ tpos, double* hm, int64_t ld,
     double* stmp, double* d12, double* d21) {
@@ -1124,16 +1154,16 @@ __global__ void __launch_bounds__(128) near_pairs_kernel(
             const d3 x2 = dev::ld3(qrec + b * QREC + 3 * m);
             double v[3] = {0, 0, 0};
             if (wantS && wantP)
-                sv = w * dev::operator_S_p1(srec + a * SREC, prec + a * PREC, x2, v);
+                sv = w * near_eval<true, true>(srec + a * SREC, x2, v);
             else if (wantS)
-                sv = w * dev::operator_S(srec + a * SREC, x2);
+                sv = w * near_eval<true, false>(srec + a * SREC, x2, v);
             else
-                dev::p1_single_layer(prec + a * PREC, x2, v);
+                near_eval<false, true>(srec + a * SREC, x2, v);
             p[0] = w * v[0]; p[1] = w * v[1]; p[2] = w * v[2];
         }
         if (wantD12) {   // integral over t1 of P1SLP(t2)
             double v[3];
-            dev::p1_single_layer(prec + b * PREC, dev::ld3(qrec + a * QREC + 3 * m), v);
+            near_eval<false, true>(srec + b * SREC, dev::ld3(qrec + a * QREC + 3 * m), v);
             e[0] = w * v[0]; e[1] = w * v[1]; e[2] = w * v[2];
         }
     }
@@ -1187,7 +1217,7 @@ void launch_near_pairs(const DevGeom& g, const int2* near, int count, int64_t t1
     if (count <= 0) return;
     if (order < 0 || order > 3) throw Error(OMG_ERR_INVALID, "near pairs: rule of more than 16 points");
     ProfScope prof_("near_pairs", s);
-    near_pairs_kernel<<<nblocks((int64_t)count * NP_LANES, 128), 128, 0, s>>>(near, count, g.srec, g.prec, g.qrec,
+    near_pairs_kernel<<<nblocks((int64_t)count * NP_LANES, 128), 128, 0, s>>>(near, count, g.srec, g.qrec,
                                                                               t1b, t1e - t1b, t2b,
                                                           t2e - t2b, same ? 1 : 0, wantS ? 1 : 0, wantD12 ? 1 : 0,
                                                           wantD21 ? 1 : 0, cS, order, g.tpos, hm, ld, stmp, d12, d21);
@@ -2013,8 +2043,8 @@ __global__ void ferguson_s_kernel(const double* __restrict__ sq, int64_t np, int
                                   const double* __restrict__ srec, double* F) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= nt) return;
-    for (int64_t i = blockIdx.y; i < np; i += gridDim.y)
-        F[i * nt + t] = dev::operator_S(srec + t * SREC, dev::ld3(sq + 6 * i));
+    for (int64_t i = blockIdx.y; i < np; i += gridDim.y)   // (about 110 FP64 operations; 270 with three atanh and atan2)
+        F[i * nt + t] = near_eval<true, false>(srec + t * SREC, dev::ld3(sq + 6 * i), nullptr);
 }
 
 __global__ void ferguson_gather_kernel(const double* __restrict__ sq, int64_t np, int64_t nv, int64_t nt,
