@@ -1361,46 +1361,6 @@ struct DsmTri {
     d3 p0, e10, e20, n;
     double d11, d12, d22;
 };
-__device__ __forceinline__ void dsm_eval(int kind, const DsmTri& T, d3 r0, d3 q, d3 r, double out[3]) {
-    const d3 x = r - r0;
-    if (kind == 1) {
-        const double nrm2 = dev::dot(x, x);
-        out[0] = dev::dot(q, x) / (nrm2 * sqrt(nrm2));
-        return;
-    }
-    const double inv = 1.0 / dev::dot(x, x);
-    const d3 grad = q - x * (3 * dev::dot(q, x) * inv);
-    const double g = dev::dot(grad, T.n) * (inv * sqrt(inv));
-    const d3 v = r - T.p0;
-    const double a1 = dev::dot(v, T.e10), a2 = dev::dot(v, T.e20);
-    const double l1 = T.d11 * a1 + T.d12 * a2;
-    const double l2 = T.d12 * a1 + T.d22 * a2;
-    const double l0 = 1.0 - l1 - l2;
-    out[0] = g * l0;
-    out[1] = g * l1;
-    out[2] = g * l2;
-}
-
-__device__ __forceinline__ void dsm_rule(int kind, int order, const DsmTri& T, d3 r0, d3 q, d3 P0, d3 P1, d3 P2,
-                                         double area, double res[3]) {
-    double acc[3] = {0.0, 0.0, 0.0};
-    const int np = c_nbpts[order];
-    for (int k = 0; k < np; ++k) {
-        const d3 x = bary_point(c_rules[order][k], P0, P1, P2);
-        double v[3];
-        dsm_eval(kind, T, r0, q, x, v);
-        const double w = c_rules[order][k][3];
-        acc[0] += w * v[0];
-        if (kind == 0) {
-            acc[1] += w * v[1];
-            acc[2] += w * v[2];
-        }
-    }
-    res[0] = area * acc[0];
-    res[1] = area * acc[1];
-    res[2] = area * acc[2];
-}
-
 __device__ __forceinline__ void subtriangle(d3& P0, d3& P1, d3& P2, int c) {
     const d3 m0 = (P1 + P2) * 0.5, m1 = (P2 + P0) * 0.5, m2 = (P0 + P1) * 0.5;
     if (c == 0) { P1 = m1; P2 = m2; }
@@ -1411,58 +1371,88 @@ __device__ __forceinline__ void subtriangle(d3& P0, d3& P1, d3& P2, int c) {
 
 constexpr int DSM_MAX_LEVELS = 12;
 constexpr int DSM_STACK = 3 * (DSM_MAX_LEVELS + 1) + 4;
+struct DsmNode {   // a triangle to refine: its corners, its own rule's values, the levels left
+    double p[9], coarse[3], area;
+    int level;
+};
 
-// Integrator::integrate with adaptive_integration (integrator.h:44-48,228-252)
-// as an explicit depth-first stack.  A node is its path of child indices from
-// the root (2 bits per level), so the stack holds no vertex coordinates.  The
-// integration is done by a group of four lanes (lanes 4 g .. 4 g + 3 of a
-// warp, `mask` their bits): each node's four children are integrated one per
-// lane, each child's rule summed in order, and the values are exchanged by
-// shuffles; the four lanes run the same control flow.
-__device__ void dsm_adaptive_g4(int kind, int order, int levels, double tol, const DsmTri& T, d3 r0, d3 q, d3 R0,
-                                d3 R1, d3 R2, double area, double result[3], unsigned mask, int lane4) {
-    double coarse[3];
-    dsm_rule(kind, order, T, r0, q, R0, R1, R2, area, coarse);
-    if (levels == 0) {
-        result[0] = coarse[0]; result[1] = coarse[1]; result[2] = coarse[2];
+// Rule-weighted integrand values at one point (zero for k past the rule).
+__device__ __forceinline__ void dsm_point(int kind, int order, const DsmTri& T, d3 r0, d3 q, double qn, const d3 P[3], int k,
+                                          double acc[3]) {
+    if (k >= c_nbpts[order]) return;
+    const d3 r = bary_point(c_rules[order][k], P[0], P[1], P[2]);
+    const double w = c_rules[order][k][3];
+    const d3 x = r - r0;
+    const double n2 = dev::dot(x, x), qx = dev::dot(q, x);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n2));
+    const double e = fma(-(n2 * y), y, 1.0);   // one third-order Newton step
+    y = fma(y * e, fma(0.375, e, 0.5), y);
+    const double y2 = y * y, wy3 = w * (y2 * y);
+    if (kind == 1) {
+        acc[0] = fma(qx, wy3, acc[0]);
         return;
     }
-    const int base = (threadIdx.x & 31) & ~3;
-    uint32_t st_path[DSM_STACK];
-    int8_t st_depth[DSM_STACK], st_level[DSM_STACK];
-    double st_c[DSM_STACK][3];
-    int sp = 0;
-    st_path[0] = 0; st_depth[0] = 0; st_level[0] = (int8_t)levels;
-    st_c[0][0] = coarse[0]; st_c[0][1] = coarse[1]; st_c[0][2] = coarse[2];
-    sp = 1;
-    double total[3] = {0.0, 0.0, 0.0};
+    const double g = fma(-3.0 * dev::dot(T.n, x), qx * y2, qn) * wy3;
+    const d3 v = r - T.p0;
+    const double a1 = dev::dot(v, T.e10), a2 = dev::dot(v, T.e20);
+    const double l1 = fma(T.d11, a1, T.d12 * a2), l2 = fma(T.d12, a1, T.d22 * a2);
+    acc[0] = fma(g, 1.0 - l1 - l2, acc[0]);
+    acc[1] = fma(g, l1, acc[1]);
+    acc[2] = fma(g, l2, acc[2]);
+}
+
+// Integrator::integrate with adaptive_integration (integrator.h:44-48,228-252)
+// by a warp, depth first with a stack in shared memory: eight lanes integrate
+// each of a node's four children, two points a lane, so a node is about 150
+// FP64 instructions deep (four lanes with 16 points each: 1800, which set the
+// length of the deepest pairs' chains).  leaf(P, sub, ref) is called by every
+// lane for each accepted node: its child P (corners), a child's area, the
+// node's refined values.  levels > 0.
+template <typename Leaf>
+__device__ __forceinline__ void dsm_adaptive_warp(int kind, int order, int levels, double tol, const DsmTri& T, d3 r0,
+                                                  d3 q, d3 R0, d3 R1, d3 R2, double area, DsmNode* st, int lane,
+                                                  Leaf leaf) {
+    const double qn = dev::dot(q, T.n);
     const int dim = kind == 0 ? 3 : 1;
-    while (sp > 0) {
+    auto reduce = [&](double v[3], int width) {   // sum over groups of `width` lanes
+        for (int o = width / 2; o > 0; o >>= 1)
+            for (int k = 0; k < dim; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    };
+    {
+        double c[3] = {0.0, 0.0, 0.0};
+        const d3 P[3] = {R0, R1, R2};
+        dsm_point(kind, order, T, r0, q, qn, P, lane, c);
+        reduce(c, 32);
+        if (lane == 0) {
+            for (int k = 0; k < 3; ++k) {
+                st[0].p[3 * k] = P[k].x;
+                st[0].p[3 * k + 1] = P[k].y;
+                st[0].p[3 * k + 2] = P[k].z;
+                st[0].coarse[k] = area * c[k];
+            }
+            st[0].area = area;
+            st[0].level = levels;
+        }
+        __syncwarp();
+    }
+    const int child = lane >> 3, l8 = lane & 7;
+    for (int sp = 1; sp > 0;) {
         --sp;
-        const uint32_t path = st_path[sp];
-        const int depth = st_depth[sp], level = st_level[sp];
-        const double c0 = st_c[sp][0], c1 = st_c[sp][1], c2 = st_c[sp][2];
-        d3 P0 = R0, P1 = R1, P2 = R2;
-        double a = area;
-        for (int d = 0; d < depth; ++d) {
-            subtriangle(P0, P1, P2, (path >> (2 * d)) & 3);
-            a *= 0.25;
-        }
-        const double sub = 0.25 * a;
-        double mine[3];
-        {
-            d3 Q0 = P0, Q1 = P1, Q2 = P2;
-            subtriangle(Q0, Q1, Q2, lane4);
-            dsm_rule(kind, order, T, r0, q, Q0, Q1, Q2, sub, mine);
-        }
-        double integ[4][3];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) integ[c][k] = __shfl_sync(mask, mine[k], base + c);
+        d3 P[3] = {dev::ld3(st[sp].p), dev::ld3(st[sp].p + 3), dev::ld3(st[sp].p + 6)};
+        const double c0 = st[sp].coarse[0], c1 = st[sp].coarse[1], c2 = st[sp].coarse[2], sub = 0.25 * st[sp].area;
+        const int level = st[sp].level;
+        __syncwarp();
+        subtriangle(P[0], P[1], P[2], child);
+        double mine[3] = {0.0, 0.0, 0.0};
+        dsm_point(kind, order, T, r0, q, qn, P, l8, mine);
+        dsm_point(kind, order, T, r0, q, qn, P, l8 + 8, mine);
+        reduce(mine, 8);
         double ref[3] = {0.0, 0.0, 0.0};
-        for (int c = 0; c < 4; ++c)
-            for (int k = 0; k < dim; ++k) ref[k] += integ[c][k];
+        for (int k = 0; k < dim; ++k) {
+            mine[k] *= sub;
+            for (int c = 0; c < 4; ++c) ref[k] += __shfl_sync(0xffffffffu, mine[k], 8 * c);
+        }
         double dn, cn;
         if (dim == 1) {
             dn = fabs(c0 - ref[0]);
@@ -1472,21 +1462,25 @@ __device__ void dsm_adaptive_g4(int kind, int order, int levels, double tol, con
             dn = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
             cn = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
         }
-        if (dn <= tol * cn || level == 0) {
-            for (int k = 0; k < dim; ++k) total[k] += ref[k];
+        if (dn <= tol * cn || level == 0) {   // (the same on every lane)
+            leaf(P, sub, ref);
             continue;
         }
-        for (int c = 3; c >= 0; --c) {
-            st_path[sp] = path | ((uint32_t)c << (2 * depth));
-            st_depth[sp] = (int8_t)(depth + 1);
-            st_level[sp] = (int8_t)(level - 1);
-            st_c[sp][0] = integ[c][0]; st_c[sp][1] = integ[c][1]; st_c[sp][2] = integ[c][2];
-            ++sp;
+        if (l8 == 0) {   // child 0 on top
+            DsmNode& n = st[sp + 3 - child];
+            for (int k = 0; k < 3; ++k) {
+                n.p[3 * k] = P[k].x;
+                n.p[3 * k + 1] = P[k].y;
+                n.p[3 * k + 2] = P[k].z;
+                n.coarse[k] = mine[k];
+            }
+            n.area = sub;
+            n.level = level - 1;
         }
+        sp += 4;
+        __syncwarp();
     }
-    result[0] = total[0]; result[1] = total[1]; result[2] = total[2];
 }
-
 
 // FP64: the first adaptive level of both integrands of every (dipole, triangle)
 // pair, 80 points.  What depends on the triangle alone is tabled once per
@@ -1848,32 +1842,35 @@ __global__ void dsm_mixed_kernel(int64_t dip0, int64_t ndc, const double* __rest
 }
 
 // The listed pairs of the first pass: FP64 adaptive integration of the
-// integrals it did not settle (grid-stride over the device-side count, four
-// lanes per pair; block size a multiple of 32).
-__global__ void dsm_fallback_kernel(int64_t dip0, int64_t nt, const double* __restrict__ dip,
-                                    const double* __restrict__ srec, const int32_t* __restrict__ tmesh,
-                                    const int64_t* __restrict__ tidx_ref, const int* __restrict__ orient,
-                                    const int* __restrict__ dom, int maxb, const int* __restrict__ dnb,
-                                    const int* __restrict__ bmesh, const int* __restrict__ binside,
-                                    const double* __restrict__ dsigma, int order, int levels, double tol, int64_t nv,
-                                    int perm, double* out, int64_t ldo, double* p1tmp, const int2* __restrict__ left,
-                                    const int* __restrict__ nleft) {
-    // one group of four lanes per listed pair (the children of every node are integrated in parallel)
+// integrals it did not settle (a warp per pair, grid-stride over the
+// device-side count).  A walk is a serial chain of nodes, so what bounds it is
+// the latency of one node: eight lanes per child and two points a lane (of 16)
+// instead of a lane per child.  The FP64 source matrix of 8 dipoles on 960
+// triangles took 0.21 ms after 0.58 with four lanes a pair.
+constexpr int DSM_WARPS = 4;
+__global__ void __launch_bounds__(32 * DSM_WARPS) dsm_fallback_kernel(
+    int64_t dip0, int64_t nt, const double* __restrict__ dip, const double* __restrict__ srec,
+    const int32_t* __restrict__ tmesh, const int64_t* __restrict__ tidx_ref, const int* __restrict__ orient,
+    const int* __restrict__ dom, int maxb, const int* __restrict__ dnb, const int* __restrict__ bmesh,
+    const int* __restrict__ binside, const double* __restrict__ dsigma, int order, int levels, double tol, int64_t nv,
+    int perm, double* out, int64_t ldo, double* p1tmp, const int2* __restrict__ left, const int* __restrict__ nleft) {
+    __shared__ DsmNode stack[DSM_WARPS][DSM_STACK];
     const int n = *nleft;
-    const int lane = threadIdx.x & 31, lane4 = lane & 3;
-    const unsigned mask = 0xFu << (lane & ~3);
-    const int groups = (int)(gridDim.x * blockDim.x / 4);
-    for (int idx = (int)((blockIdx.x * blockDim.x + threadIdx.x) / 4); idx < n; idx += groups) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int idx = blockIdx.x * DSM_WARPS + warp; idx < n; idx += gridDim.x * DSM_WARPS) {
         const int2 e = left[idx];
         const int64_t il = e.x, t = e.y & ((1 << DSM_T_BITS) - 1);
         const int need = (int)((unsigned)e.y >> DSM_T_BITS);
         const int64_t i = dip0 + il;
         DsmPair P;
         if (!dsm_pair(i, t, dip, srec, tmesh, orient, dom, maxb, dnb, bmesh, binside, dsigma, P)) continue;
+        double v[3] = {0.0, 0.0, 0.0};
+        auto add = [&](const d3*, double, const double* ref) {
+            for (int k = 0; k < 3; ++k) v[k] += ref[k];
+        };
         if (need & 1) {
-            double v[3];
-            dsm_adaptive_g4(0, order, levels, tol, P.T, P.r0, P.q, P.R0, P.R1, P.R2, P.area, v, mask, lane4);
-            if (lane4 == 0) {
+            dsm_adaptive_warp(0, order, levels, tol, P.T, P.r0, P.q, P.R0, P.R1, P.R2, P.area, stack[warp], lane, add);
+            if (lane == 0) {
                 double* o3 = p1tmp + (il * nt + t) * 3;
                 o3[0] = v[0] * P.coeffD;
                 o3[1] = v[1] * P.coeffD;
@@ -1881,10 +1878,10 @@ __global__ void dsm_fallback_kernel(int64_t dip0, int64_t nt, const double* __re
             }
         }
         if (need & 2) {
-            double p[3];
-            dsm_adaptive_g4(1, order, levels, tol, P.T, P.r0, P.q, P.R0, P.R1, P.R2, P.area, p, mask, lane4);
+            v[0] = 0.0;
+            dsm_adaptive_warp(1, order, levels, tol, P.T, P.r0, P.q, P.R0, P.R1, P.R2, P.area, stack[warp], lane, add);
             const int64_t ref = tidx_ref[t];
-            if (lane4 == 0) out[(perm ? ref - nv : ref) + i * ldo] = p[0] * (P.coeffD / P.sigma);
+            if (lane == 0) out[(perm ? ref - nv : ref) + i * ldo] = v[0] * (P.coeffD / P.sigma);
         }
     }
 }
@@ -2127,6 +2124,17 @@ void launch_domain_check(int64_t n, const int* dom, uint64_t allowed, int* err, 
     check_launch("domain check");
 }
 
+static int dsm_sms() {
+    static int n = 0;
+    if (!n) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 1;
+    }
+    return n;
+}
+
 void launch_dsm(const DevGeom& g, int64_t dip0, int64_t ndc, const double* dip, const int32_t* tmesh,
                 const int64_t* tidx_ref, const int* barrier, const int* orient, const int* dom, int maxb,
                 const int* dnb, const int* bmesh, const int* binside, const double* dsigma, int order, int levels,
@@ -2159,14 +2167,7 @@ void launch_dsm(const DevGeom& g, int64_t dip0, int64_t ndc, const double* dip, 
         check_launch("DSM");
     }
     if (levels > 0) {
-        static int n_sm = 0;
-        if (!n_sm) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-            if (n_sm <= 0) n_sm = 1;
-        }
-        dsm_fallback_kernel<<<(unsigned)(n_sm * 8), 128, 0, s>>>(dip0, g.nt, dip, g.srec, tmesh, tidx_ref, orient, dom,
+        dsm_fallback_kernel<<<(unsigned)(8 * dsm_sms()), 32 * DSM_WARPS, 0, s>>>(dip0, g.nt, dip, g.srec, tmesh, tidx_ref, orient, dom,
                                                                   maxb, dnb, bmesh, binside, dsigma, order, levels,
                                                                   tol, g.nvg, perm, out, ldo, p1tmp, left.as<int2>(),
                                                                   nleft.as<int>());
@@ -2252,84 +2253,30 @@ __device__ __forceinline__ void dsm_vjp_point(int kind, const DsmTri& T, d3 r0, 
     out[3] = w1 * dq.x; out[4] = w1 * dq.y; out[5] = w1 * dq.z;
 }
 
-__device__ __forceinline__ void dsm_vjp_rule(int kind, int order, const DsmTri& T, d3 r0, d3 q, const VjpW& w,
-                                             d3 P0, d3 P1, d3 P2, double area, double acc[6]) {
-    double s[6] = {0, 0, 0, 0, 0, 0};
-    const int np = c_nbpts[order];
-    for (int k = 0; k < np; ++k) {
-        const d3 xk = bary_point(c_rules[order][k], P0, P1, P2);
-        double e[6];
-        dsm_vjp_point(kind, T, r0, q, xk, w, e);
-        const double wk = c_rules[order][k][3];
-        for (int c = 0; c < 6; ++c) s[c] += wk * e[c];
-    }
-    for (int c = 0; c < 6; ++c) acc[c] += area * s[c];
+// The weights of a pair.
+__device__ __forceinline__ VjpW dsm_vjp_weights(const DsmPair& P, int64_t i, int64_t t, const int32_t* __restrict__ T32,
+                                                const int64_t* __restrict__ tidx_ref, const int* __restrict__ barrier,
+                                                const double* __restrict__ U, int64_t ldu) {
+    const double* Uj = U + i * ldu;
+    VjpW w;
+    for (int k = 0; k < 3; ++k) w.W[k] = Uj[T32[3 * t + k]] * P.coeffD;
+    w.w0 = barrier[P.m] ? 0.0 : Uj[tidx_ref[t]] * (P.coeffD / P.sigma);
+    return w;
 }
 
-// Same traversal as dsm_adaptive; accepted nodes contribute the derivative
-// rule over their four children (the values the forward sums).
-__device__ void dsm_vjp_adaptive(int kind, int order, int levels, double tol, const DsmTri& T, d3 r0, d3 q,
-                                 const VjpW& w, d3 R0, d3 R1, d3 R2, double area, double grad[6]) {
-    if (levels == 0) {
-        dsm_vjp_rule(kind, order, T, r0, q, w, R0, R1, R2, area, grad);
-        return;
-    }
-    double coarse[3];
-    dsm_rule(kind, order, T, r0, q, R0, R1, R2, area, coarse);
-    uint32_t st_path[DSM_STACK];
-    int8_t st_depth[DSM_STACK], st_level[DSM_STACK];
-    double st_c[DSM_STACK][3];
-    int sp = 1;
-    st_path[0] = 0; st_depth[0] = 0; st_level[0] = (int8_t)levels;
-    st_c[0][0] = coarse[0]; st_c[0][1] = coarse[1]; st_c[0][2] = coarse[2];
-    const int dim = kind == 0 ? 3 : 1;
-    while (sp > 0) {
-        --sp;
-        const uint32_t path = st_path[sp];
-        const int depth = st_depth[sp], level = st_level[sp];
-        const double c0 = st_c[sp][0], c1 = st_c[sp][1], c2 = st_c[sp][2];
-        d3 P0 = R0, P1 = R1, P2 = R2;
-        double a = area;
-        for (int d = 0; d < depth; ++d) {
-            subtriangle(P0, P1, P2, (path >> (2 * d)) & 3);
-            a *= 0.25;
-        }
-        const double sub = 0.25 * a;
-        double integ[4][3];
-        double ref[3] = {0.0, 0.0, 0.0};
-        for (int c = 0; c < 4; ++c) {
-            d3 Q0 = P0, Q1 = P1, Q2 = P2;
-            subtriangle(Q0, Q1, Q2, c);
-            dsm_rule(kind, order, T, r0, q, Q0, Q1, Q2, sub, integ[c]);
-            for (int k = 0; k < dim; ++k) ref[k] += integ[c][k];
-        }
-        double dn, cn;
-        if (dim == 1) {
-            dn = fabs(c0 - ref[0]);
-            cn = fabs(c0);
-        } else {
-            const double e0 = c0 - ref[0], e1 = c1 - ref[1], e2 = c2 - ref[2];
-            dn = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
-            cn = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-        }
-        if (dn <= tol * cn || level == 0) {
-            for (int c = 0; c < 4; ++c) {
-                d3 Q0 = P0, Q1 = P1, Q2 = P2;
-                subtriangle(Q0, Q1, Q2, c);
-                dsm_vjp_rule(kind, order, T, r0, q, w, Q0, Q1, Q2, sub, grad);
-            }
-            continue;
-        }
-        for (int c = 3; c >= 0; --c) {
-            st_path[sp] = path | ((uint32_t)c << (2 * depth));
-            st_depth[sp] = (int8_t)(depth + 1);
-            st_level[sp] = (int8_t)(level - 1);
-            st_c[sp][0] = integ[c][0]; st_c[sp][1] = integ[c][1]; st_c[sp][2] = integ[c][2];
-            ++sp;
-        }
-    }
-}
-
+// One thread per (dipole, triangle): the first adaptive level of both
+// integrals from the tabled points, as dsm_kernel forms it, and in the same
+// pass the derivatives over the points the accepted values sum (54 FP64
+// operations per point for both, with one reciprocal square root; the separate
+// recursions took ~330); bound by FP64 issue.  100 dipoles on 3840 triangles
+// took 1.05 ms after 5.85 with a recursion per pair and integral.  With x = r - r0, y = 1/|x|:
+//   g = (q.n) y^3 - 3 (q.x)(n.x) y^5, weighted c1 = w (W0 l0 + W1 l1 + W2 l2):
+//     d/dq  = c1 (n y^3 - 3 (n.x) y^5 x),
+//     d/dr0 = -c1 ((-3 (q.n) y^5 + 15 (q.x)(n.x) y^7) x - 3 (n.x) y^5 q - 3 (q.x) y^5 n);
+//   p = (q.x) y^3, weighted c0 = w w0:
+//     d/dq  = c0 y^3 x,   d/dr0 = -c0 (y^3 q - 3 (q.x) y^5 x).
+// Pairs not settled are listed as in dsm_kernel; their integral's part is left
+// to dsm_vjp_fallback_kernel.
 __global__ void dsm_vjp_kernel(int64_t dip0, int64_t ndc, const double* __restrict__ dip, int64_t nt,
                                const double* __restrict__ srec, const int32_t* __restrict__ T32,
                                const int32_t* __restrict__ tmesh, const int64_t* __restrict__ tidx_ref,
@@ -2337,47 +2284,144 @@ __global__ void dsm_vjp_kernel(int64_t dip0, int64_t ndc, const double* __restri
                                const int* __restrict__ dom, int maxb, const int* __restrict__ dnb,
                                const int* __restrict__ bmesh, const int* __restrict__ binside,
                                const double* __restrict__ dsigma, int order, int levels, double tol,
-                               const double* __restrict__ U, int64_t ldu, double* part) {
+                               const double* __restrict__ U, int64_t ldu, double* part, const double* __restrict__ tab,
+                               int2* left, int* nleft) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t il = blockIdx.y;
     if (t >= nt || il >= ndc) return;
     const int64_t i = dip0 + il;
     double* o = part + (il * nt + t) * 6;
-    for (int c = 0; c < 6; ++c) o[c] = 0.0;
-    const int d = dom[i];
-    if (d < 0) return;
-    const double sigma = dsigma[d];
-    if (sigma == 0.0) return;
-    const int m = tmesh[t];
-    double coeffD = 0.0;
-    bool on = false;
-    for (int k = 0; k < dnb[d]; ++k)
-        if (bmesh[d * maxb + k] == m) {
-            coeffD = (binside[d * maxb + k] ? -kK : kK) * orient[d * maxb + k];
-            on = true;
-        }
-    if (!on) return;
+    DsmPair P;
+    if (!dsm_pair_coeff(i, t, tmesh, orient, dom, maxb, dnb, bmesh, binside, dsigma, P)) {
+        for (int c = 0; c < 6; ++c) o[c] = 0.0;
+        return;
+    }
+    const bool p0row = !barrier[P.m];
+    const VjpW w = dsm_vjp_weights(P, i, t, T32, tidx_ref, barrier, U, ldu);
     const double* s = srec + t * SREC;
-    const d3 R0 = dev::ld3(s), R1 = dev::ld3(s + 3), R2 = dev::ld3(s + 6);
-    DsmTri T;
-    T.p0 = R0;
-    T.n = dev::ld3(s + 9);
-    T.e10 = R1 - R0;
-    T.e20 = R2 - R0;
-    const double c11 = dev::dot(T.e10, T.e10), c12 = dev::dot(T.e10, T.e20), c22 = dev::dot(T.e20, T.e20);
-    const double inv_det = 1.0 / (c11 * c22 - c12 * c12);
-    T.d11 = c22 * inv_det;
-    T.d12 = -c12 * inv_det;
-    T.d22 = c11 * inv_det;
-    const d3 r0 = dev::ld3(dip + 6 * i), q = dev::ld3(dip + 6 * i + 3);
-    const double* Uj = U + i * ldu;
-    VjpW w;
-    for (int k = 0; k < 3; ++k) w.W[k] = Uj[T32[3 * t + k]] * coeffD;
-    w.w0 = barrier[m] ? 0.0 : Uj[tidx_ref[t]] * (coeffD / sigma);
+    const d3 n = dev::ld3(s + 9), q = dev::ld3(dip + 6 * i + 3);
+    const d3 X = (dev::ld3(s) + dev::ld3(s + 3) + dev::ld3(s + 6)) * (1.0 / 3.0) - dev::ld3(dip + 6 * i);
+    const double qn = dev::dot(q, n), h3 = -3.0 * dev::dot(n, X), area = s[12], qn3 = -3.0 * qn;
+    const double W1 = w.W[1] - w.W[0], W2 = w.W[2] - w.W[0];
+    const int np = c_nbpts[order];
+    const int64_t set = (int64_t)np * DSM_FL * nt;
+    double coarse[4];
+    if (levels > 0) dsm_set(tab + t, nt, order, X, q, qn, h3, coarse);
+    double f[4] = {0, 0, 0, 0};                                    // forward sums over the children
+    double An = 0, Sq = 0, Sn = 0, Sy = 0;
+    d3 Bx = dev::mk(0, 0, 0), Ax = Bx, Cx = Bx, Dx = Bx;
+    const double* tb = tab + t + (levels > 0 ? set : 0);
+    const int points = (levels > 0 ? 4 : 1) * np;
+    for (int j = 0, k = 0; j < points; ++j, k = k + 1 == np ? 0 : k + 1, tb += DSM_FL * nt) {
+        const d3 x = dev::mk(X.x + tb[0], X.y + tb[nt], X.z + tb[2 * nt]);
+        const double t3 = h3 + tb[3 * nt];                         // -3 n.x
+        const double wl1 = tb[4 * nt], wl2 = tb[5 * nt], wk = c_rules[order][k][3];
+        const double n2 = fma(x.x, x.x, fma(x.y, x.y, x.z * x.z));
+        const double qx = fma(q.x, x.x, fma(q.y, x.y, q.z * x.z));
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n2));
+        const double e = fma(-(n2 * y), y, 1.0);
+        y = fma(y * e, fma(0.375, e, 0.5), y);
+        const double y2 = y * y, y3 = y2 * y, y5 = y3 * y2, u = qx * y2, tu = t3 * u;
+        const double g = (qn + tu) * y3, wy3 = wk * y3;
+        f[0] = fma(wk, g, f[0]);
+        f[1] = fma(wl1, g, f[1]);
+        f[2] = fma(wl2, g, f[2]);
+        f[3] = fma(qx, wy3, f[3]);
+        const double c1 = fma(W1, wl1, fma(W2, wl2, w.W[0] * wk)), m = c1 * y5, mt = m * t3;
+        An = fma(c1, y3, An);
+        Sq += mt;
+        Sn = fma(qx, m, Sn);
+        const double ma = m * fma(-5.0, tu, qn3);
+        Bx = dev::mk(fma(mt, x.x, Bx.x), fma(mt, x.y, Bx.y), fma(mt, x.z, Bx.z));
+        Ax = dev::mk(fma(ma, x.x, Ax.x), fma(ma, x.y, Ax.y), fma(ma, x.z, Ax.z));
+        Sy += wy3;
+        const double d = wy3 * u;
+        Cx = dev::mk(fma(wy3, x.x, Cx.x), fma(wy3, x.y, Cx.y), fma(wy3, x.z, Cx.z));
+        Dx = dev::mk(fma(d, x.x, Dx.x), fma(d, x.y, Dx.y), fma(d, x.z, Dx.z));
+    }
+    bool okv = true, okp = true;
+    const double sub = levels > 0 ? 0.25 * area : area;
+    if (levels > 0) {   // the test of dsm_kernel
+        f[0] -= f[1] + f[2];
+        const double lim = tol * (1.0 - 1e-9);
+        double d2 = 0.0, c2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const double c = coarse[k] * area, e = c - sub * f[k];
+            if (k < 3) {
+                d2 = fma(e, e, d2);
+                c2 = fma(c, c, c2);
+            } else {
+                okp = fabs(e) <= lim * fabs(c);
+            }
+        }
+        okv = d2 <= lim * lim * c2;
+    }
     double g[6] = {0, 0, 0, 0, 0, 0};
-    dsm_vjp_adaptive(0, order, levels, tol, T, r0, q, w, R0, R1, R2, s[12], g);
-    if (!barrier[m]) dsm_vjp_adaptive(1, order, levels, tol, T, r0, q, w, R0, R1, R2, s[12], g);
+    if (okv) {
+        const double sn = -3.0 * Sn;
+        g[0] = -sub * (Ax.x + q.x * Sq + n.x * sn);
+        g[1] = -sub * (Ax.y + q.y * Sq + n.y * sn);
+        g[2] = -sub * (Ax.z + q.z * Sq + n.z * sn);
+        g[3] = sub * (n.x * An + Bx.x);
+        g[4] = sub * (n.y * An + Bx.y);
+        g[5] = sub * (n.z * An + Bx.z);
+    }
+    if (p0row && okp) {
+        const double a = sub * w.w0;
+        g[0] -= a * (q.x * Sy - 3.0 * Dx.x);
+        g[1] -= a * (q.y * Sy - 3.0 * Dx.y);
+        g[2] -= a * (q.z * Sy - 3.0 * Dx.z);
+        g[3] += a * Cx.x;
+        g[4] += a * Cx.y;
+        g[5] += a * Cx.z;
+    }
     for (int c = 0; c < 6; ++c) o[c] = g[c];
+    const int need = (okv ? 0 : 1) | (p0row && !okp ? 2 : 0);
+    if (need) left[atomicAdd(nleft, 1)] = make_int2((int)il, (int)t | (need << DSM_T_BITS));
+}
+
+// The listed pairs: a warp walks the forward's adaptive tree and adds the
+// derivative rule over the children of every accepted node, two points a lane.
+__global__ void __launch_bounds__(32 * DSM_WARPS) dsm_vjp_fallback_kernel(
+    int64_t dip0, int64_t nt, const double* __restrict__ dip, const double* __restrict__ srec,
+    const int32_t* __restrict__ T32, const int32_t* __restrict__ tmesh, const int64_t* __restrict__ tidx_ref,
+    const int* __restrict__ barrier, const int* __restrict__ orient, const int* __restrict__ dom, int maxb,
+    const int* __restrict__ dnb, const int* __restrict__ bmesh, const int* __restrict__ binside,
+    const double* __restrict__ dsigma, int order, int levels, double tol, const double* __restrict__ U, int64_t ldu,
+    double* part, const int2* __restrict__ left, const int* __restrict__ nleft) {
+    __shared__ DsmNode stack[DSM_WARPS][DSM_STACK];
+    const int count = *nleft;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int idx = blockIdx.x * DSM_WARPS + warp; idx < count; idx += gridDim.x * DSM_WARPS) {
+        const int2 e = left[idx];
+        const int64_t il = e.x, t = e.y & ((1 << DSM_T_BITS) - 1);
+        const int need = (int)((unsigned)e.y >> DSM_T_BITS);
+        const int64_t i = dip0 + il;
+        DsmPair P;
+        if (!dsm_pair(i, t, dip, srec, tmesh, orient, dom, maxb, dnb, bmesh, binside, dsigma, P)) continue;
+        const VjpW w = dsm_vjp_weights(P, i, t, T32, tidx_ref, barrier, U, ldu);
+        double acc[6] = {0, 0, 0, 0, 0, 0};
+        for (int kind = 0; kind < 2; ++kind) {
+            if (!(need & (1 << kind))) continue;
+            dsm_adaptive_warp(kind, order, levels, tol, P.T, P.r0, P.q, P.R0, P.R1, P.R2, P.area, stack[warp], lane,
+                              [&](const d3* C, double sub, const double*) {
+                                  for (int k = lane & 7; k < c_nbpts[order]; k += 8) {
+                                      double d[6];
+                                      dsm_vjp_point(kind, P.T, P.r0, P.q, bary_point(c_rules[order][k], C[0], C[1], C[2]),
+                                                    w, d);
+                                      const double wk = sub * c_rules[order][k][3];
+                                      for (int c = 0; c < 6; ++c) acc[c] = fma(wk, d[c], acc[c]);
+                                  }
+                              });
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            for (int c = 0; c < 6; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        if (lane == 0)
+            for (int c = 0; c < 6; ++c) part[(il * nt + t) * 6 + c] += acc[c];
+    }
 }
 
 // Fixed-order sum over triangles: one CTA per dipole.
@@ -2404,10 +2448,25 @@ void launch_dsm_vjp(const DevGeom& g, int64_t dip0, int64_t ndc, const double* d
                     double tol, const double* U, int64_t ldu, double* part, double* out, cudaStream_t s) {
     if (ndc == 0) return;
     ProfScope prof_("dsm_vjp", s);
+    if (g.nt >= ((int64_t)1 << DSM_T_BITS) || ndc > INT32_MAX) throw Error(OMG_ERR_UNSUPPORTED, "DSM: too many triangles");
+    constexpr int NPTS[4] = {3, 6, 7, 16};
+    const int nsets = levels > 0 ? 5 : 1;
+    DevBuf tab((size_t)g.nt * nsets * NPTS[order] * DSM_FL * 8, s), nleft(sizeof(int), s),
+        left(levels > 0 ? (size_t)ndc * g.nt * sizeof(int2) : 0, s);
+    OMG_CUDA(cudaMemsetAsync(nleft.p, 0, sizeof(int), s));
+    dsm_points_kernel<<<dim3(nblocks(g.nt, 128), nsets), 128, 0, s>>>(g.nt, g.srec, order, tab.as<double>());
+    check_launch("DSM points");
     dim3 grid(nblocks(g.nt, 128), (unsigned)ndc);
     dsm_vjp_kernel<<<grid, 128, 0, s>>>(dip0, ndc, dip, g.nt, g.srec, g.T, tmesh, tidx_ref, barrier, orient, dom, maxb,
-                                        dnb, bmesh, binside, dsigma, order, levels, tol, U, ldu, part);
+                                        dnb, bmesh, binside, dsigma, order, levels, tol, U, ldu, part, tab.as<double>(),
+                                        left.as<int2>(), nleft.as<int>());
     check_launch("DSM vjp");
+    if (levels > 0) {
+        dsm_vjp_fallback_kernel<<<(unsigned)(8 * dsm_sms()), 32 * DSM_WARPS, 0, s>>>(
+            dip0, g.nt, dip, g.srec, g.T, tmesh, tidx_ref, barrier, orient, dom, maxb, dnb, bmesh, binside, dsigma, order,
+            levels, tol, U, ldu, part, left.as<int2>(), nleft.as<int>());
+        check_launch("DSM vjp (listed pairs)");
+    }
     dsm_vjp_reduce_kernel<<<(unsigned)ndc, 128, 0, s>>>(dip0, ndc, g.nt, part, out);
     check_launch("DSM vjp reduce");
 }
