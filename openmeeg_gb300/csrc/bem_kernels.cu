@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "device_common.cuh"
+#include "fixed64.cuh"
 #include "handles.h"
 #include "omg_internal.h"
 
@@ -218,16 +219,19 @@ __device__ __forceinline__ int64_t lower_at(int64_t a, int64_t b, int64_t ld) {
 //      w = atan(2 A h / (d0 d1 d2 + sum d_i r_j.r_k)), then
 //        S = sum_i E_opp(i) l_i - 2 h w,
 //        D_j = (w E_j + h/2 D_j+1.(sum_i D_i l_i)) / A, D_0 + D_1 + D_2 = 2 w,
-//      in 46 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
-// About 75 FP64 operations per (triangle, point) for S and D together.  The
-// arctangent and the logarithm take polynomials where the argument is small and the
-// library functions elsewhere; square roots and reciprocals are the hardware
-// approximations refined by one third-order Newton step.
+//      in 29 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
+// About 35 FP64 operations per (triangle, point) for S and D together: the square
+// roots, logarithms and arctangents and the weights of the rule run on the integer
+// pipe (fixed64.cuh), which issues beside the FP64 operations.  With all of it in FP64
+// (75 operations, 88% of the pipe's rate) the blocks of a head of 7080 triangles in
+// four layers took 67 ms, now 34.1.
 // Lanes run over the triangles a at the same rule point, so every table read is
 // coalesced, the triangle b is uniform in a warp, and the sum over the rule stays
 // in registers (no shuffles, which cost FP64 additions).
 // ---------------------------------------------------------------------------
-constexpr int TGEO = 22;   // p0, -2 n, m0 = n x D0, m2 = n x D2 (3 each), 2A, |D_i|^2 (3), (|D0|^2 |D2|^2 D0.D2) / 4, |D_i| (3)
+// Record of an analytic triangle: -2 N, N x D0, N x D2 (N = D0 x (p2 - p0), |N| = 2A; 3 each), 4A^2, |D0|^2 / 4, |D2|^2 / 4,
+// D0.D2 / 4, the bits of 2e-10 * 2A, 1 / 2A, 2 / 4A^2, |D_i|^2 (3), |D_i| (3)
+constexpr int TGEO = 22;
 
 __global__ void sd_geometry_kernel(int64_t t0, int64_t nt, const double* __restrict__ V,
                                    const int32_t* __restrict__ T, const int32_t* __restrict__ v2t_beg,
@@ -238,19 +242,19 @@ __global__ void sd_geometry_kernel(int64_t t0, int64_t nt, const double* __restr
     const d3 p0 = dev::ld3(V + 3 * (int64_t)tv[0]), p1 = dev::ld3(V + 3 * (int64_t)tv[1]),
              p2 = dev::ld3(V + 3 * (int64_t)tv[2]);
     const d3 D0 = p1 - p0, D1 = p2 - p1, D2 = p0 - p2;
-    d3 nn = dev::cross(D0, p2 - p0);
-    const double nrm = dev::norm(nn);
-    const d3 n = nn * (1.0 / nrm);
-    const d3 m0 = dev::cross(n, D0), m2 = dev::cross(n, D2);
+    const d3 nn = dev::cross(D0, p2 - p0);
+    const d3 m0 = dev::cross(nn, D0), m2 = dev::cross(nn, D2);
+    const double a22 = dev::dot(nn, nn), a2 = sqrt(a22);
     double* g = tgeo + it * TGEO;
-    g[0] = p0.x; g[1] = p0.y; g[2] = p0.z;
-    g[3] = -2.0 * n.x; g[4] = -2.0 * n.y; g[5] = -2.0 * n.z;
-    g[6] = m0.x; g[7] = m0.y; g[8] = m0.z;
-    g[9] = m2.x; g[10] = m2.y; g[11] = m2.z;
-    g[12] = nrm;
-    g[13] = dev::dot(D0, D0); g[14] = dev::dot(D1, D1); g[15] = dev::dot(D2, D2);
-    g[16] = 0.25 * g[13]; g[17] = 0.25 * g[15]; g[18] = 0.25 * dev::dot(D2, D0);
-    g[19] = sqrt(g[13]); g[20] = sqrt(g[14]); g[21] = sqrt(g[15]);
+    g[0] = -2.0 * nn.x; g[1] = -2.0 * nn.y; g[2] = -2.0 * nn.z;
+    g[3] = m0.x; g[4] = m0.y; g[5] = m0.z;
+    g[6] = m2.x; g[7] = m2.y; g[8] = m2.z;
+    g[9] = a22;
+    g[16] = dev::dot(D0, D0); g[17] = dev::dot(D1, D1); g[18] = dev::dot(D2, D2);
+    g[10] = 0.25 * g[16]; g[11] = 0.25 * g[18]; g[12] = 0.25 * dev::dot(D2, D0);
+    g[13] = 2e-10 * a2;
+    g[14] = 1.0 / a2; g[15] = 2.0 / a22;
+    g[19] = sqrt(g[16]); g[20] = sqrt(g[17]); g[21] = sqrt(g[18]);
     // table row of edge i (corners i, i + 1): the slot 3 t + i of the first triangle of the range that has it
     for (int i = 0; i < 3; ++i) {
         const int32_t a = tv[i], b = tv[(i + 1) % 3];
@@ -278,109 +282,52 @@ __device__ __forceinline__ double sd_rcp(double x) {
     const double e = fma(-x, y, 1.0);
     return fma(fma(e, e, e), y, y);
 }
-// sqrt(x) to about an ulp (x > 0), likewise from the approximate reciprocal square root.
-__device__ __forceinline__ double sd_sqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double g = x * y;
-    const double e = fma(-g, y, 1.0);
-    return fma(g * e, fma(0.375, e, 0.5), g);
-}
 // |x| / 2 < 1e-10 on the integer pipe.
 __device__ __forceinline__ bool sd_flat2(double x) {
     return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) < __double_as_longlong(2e-10);
 }
-// |x| < 2^k by the exponent field (integer pipe; NaN and infinity compare false).
-__device__ __forceinline__ bool sd_below(double x, int k) {
-    return ((__double2hiint(x) >> 20) & 0x7FF) < 1023 + k;
-}
-
 constexpr int SD_V = 16;      // vertices per CTA of the distance table
 constexpr int SD_E = 8;       // triangles per CTA of the edge table
 constexpr int SD_THREADS = 256;
 
-// Point x = q na + ia of a batch of na triangles from a0: point q of triangle a0 + ia.  Row 0..2 of pts:
-// coordinates; d[v * npt + x]: distance to vertex vb + v.
+// Point x = q na + ia of a batch of na triangles from a0: point q of triangle a0 + ia.  For vertex vb + v: the distance
+// d[v * npt + x] and, in the rows 3 v .. 3 v + 2 of cv, the point minus the vertex.
 __global__ void __launch_bounds__(SD_THREADS) sd_distance_kernel(const double* __restrict__ qrec, int64_t a0, int na,
                                                                  int npt, const double* __restrict__ V, int64_t vb,
-                                                                 int nv, double* __restrict__ pts,
+                                                                 int nv, double* __restrict__ cv,
                                                                  double* __restrict__ d) {
     const int x = blockIdx.x * SD_THREADS + threadIdx.x;
     if (x >= npt) return;
     const int q = x / na, ia = x - q * na;
     const double* src = qrec + (a0 + ia) * QREC + 3 * q;
     const double px = src[0], py = src[1], pz = src[2];
-    if (blockIdx.y == 0) {
-        pts[x] = px;
-        pts[(int64_t)npt + x] = py;
-        pts[2 * (int64_t)npt + x] = pz;
-    }
     const int v1 = min(nv, (int)(blockIdx.y + 1) * SD_V);
 #pragma unroll 4
     for (int v = blockIdx.y * SD_V; v < v1; ++v) {
         const double* p = V + 3 * (vb + v);
-        const double rx = p[0] - px, ry = p[1] - py, rz = p[2] - pz;
-        d[(int64_t)v * npt + x] = sd_sqrt(fma(rx, rx, fma(ry, ry, rz * rz)));
+        const double rx = px - p[0], ry = py - p[1], rz = pz - p[2];
+        const int64_t o = (int64_t)v * npt + x;
+        d[o] = fx::sqrt64(fma(rx, rx, fma(ry, ry, rz * rz)));
+        double* c = cv + o + 2 * (int64_t)v * npt;
+        c[0] = rx;
+        c[npt] = ry;
+        c[2 * (int64_t)npt] = rz;
     }
 }
 
-// 2 atanh(len / R) / len, R = d_a + d_b.  With y = 1/R, z = len y and w = z^2: 2 y (1 + w f(w)), f(w) = (atanh(z)/z - 1)/w by
-// the polynomial that interpolates it at the Chebyshev nodes of [0, limit^2] (relative error of the result 2^-56.8 for
-// z < 1/8 and 2^-58.8 for z < 1/4; the Taylor series takes three terms more).
-__device__ __forceinline__ double sd_edge(double R, double len) {
-    const double y = sd_rcp(R);
-    const double z = len * y, w = z * z;
-    double f;
-    if (__all_sync(__activemask(), sd_below(z, -3))) {   // (one of the two for the whole warp: mixed warps would run both)
-        f = fma(w, 0.08013059813075277, 0.09085223469123827);
-        f = fma(w, f, 0.11111157356123932);
-        f = fma(w, f, 0.14285714116012183);
-        f = fma(w, f, 0.20000000000227505);
-        f = fma(w, f, 0.3333333333333328);
-    } else if (sd_below(z, -2)) {
-        f = fma(w, 0.06828732233627811, 0.05689643661793962);
-        f = fma(w, f, 0.066791397041253);
-        f = fma(w, f, 0.07691841912131238);
-        f = fma(w, f, 0.09090919255417686);
-        f = fma(w, f, 0.1111111098689728);
-        f = fma(w, f, 0.14285714286473053);
-        f = fma(w, f, 0.1999999999999822);
-        f = fma(w, f, 0.3333333333333333);
-    } else {
-        return log((R + len) * sd_rcp(R - len)) * sd_rcp(len);
-    }
-    const double y2 = y + y;
-    return fma(w * f, y2, y2);
-}
-
-// Half the solid angle, atan2(num, den): where t = num / den < 1/16 (den > 0) by t (1 + w f(w)), w = t^2, f interpolated as
-// above (relative error 2^-60.7; 2^-64.2 below 2^-7).
-__device__ __forceinline__ double sd_half_angle(double num, double den) {
-    const double t = num * sd_rcp(den);
-    if (__double2hiint(den) < 0 || !sd_below(t, -4)) return atan2(num, den);
-    const double w = t * t;
-    double f;
-    if (__all_sync(__activemask(), sd_below(t, -7))) {
-        f = fma(w, -0.14284697090256454, 0.19999999976718616);
-        f = fma(w, f, -0.33333333333333254);
-    } else {
-        f = fma(w, -0.09016200248147936, 0.11110856205699567);
-        f = fma(w, f, -0.1428571393037775);
-        f = fma(w, f, 0.19999999999826557);
-        f = fma(w, f, -0.3333333333333332);
-    }
-    return fma(w * f, t, t);
-}
-
-// Row 3 b + i, edge i (corners i, i + 1) of triangle b, of the rows that own their edge: l, and in prod
-// (d_a + d_b)^2 - len^2 = 2 (d_a d_b + r_a.r_b).
-__global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb, int npt, const int32_t* __restrict__ T,
-                                                             int64_t vb, const double* __restrict__ tgeo,
+// Row 3 b + i, edge i (corners i, i + 1) of triangle b, of the rows that own their edge: l times the point's weight, and in
+// prod (d_a + d_b)^2 - len^2 = 2 (d_a d_b + r_a.r_b).
+__global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb, int na, int npt, int order,
+                                                             const int32_t* __restrict__ T, int64_t vb,
+                                                             const double* __restrict__ tgeo,
                                                              const int32_t* __restrict__ eown,
                                                              const double* __restrict__ d, double* __restrict__ l,
                                                              double* __restrict__ prod) {
     const int x = blockIdx.x * SD_THREADS + threadIdx.x;
     if (x >= npt) return;
+    const double wr = c_rules[order][x / na][3];
+    const uint64_t wm = fx::mant(wr);
+    const int we = (int)fx::expo(wr);
     const int b1 = min(nb, (int)(blockIdx.y + 1) * SD_E);
     for (int b = blockIdx.y * SD_E; b < b1; ++b) {
         const int32_t* tv = T + 3 * (tb + b);
@@ -389,8 +336,8 @@ __global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb,
             if (eown[3 * b + i] != 3 * b + i) continue;
             const double da = d[(int64_t)(tv[i] - vb) * npt + x], db = d[(int64_t)(tv[i == 2 ? 0 : i + 1] - vb) * npt + x];
             const double R = da + db;
-            l[(int64_t)(3 * b + i) * npt + x] = sd_edge(R, tgeo[b * (int64_t)TGEO + 19 + i]);
-            prod[(int64_t)(3 * b + i) * npt + x] = fma(R, R, -tgeo[b * (int64_t)TGEO + 13 + i]);
+            l[(int64_t)(3 * b + i) * npt + x] = fx::edge<true>(R, tgeo[b * (int64_t)TGEO + 19 + i], wm, we, wr);
+            prod[(int64_t)(3 * b + i) * npt + x] = fma(R, R, -tgeo[b * (int64_t)TGEO + 16 + i]);
         }
     }
 }
@@ -401,9 +348,9 @@ template <bool WANT_S, bool WANT_D>
 __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     int64_t tb, int nb, int64_t ta, int64_t a0, int na, int npt, int order, int same, double coeff,
     const int32_t* __restrict__ T, int64_t vb, const double* __restrict__ tgeo, const int32_t* __restrict__ eown,
-    const double* __restrict__ qrec, const double* __restrict__ pts, const double* __restrict__ d,
-    const double* __restrict__ l, const double* __restrict__ prod, const int32_t* __restrict__ tpos, double* hm, int64_t ld, double* stmp, int64_t n2,
-    double* dtmp) {
+    const double* __restrict__ qrec, const double* __restrict__ cv, const double* __restrict__ d,
+    const double* __restrict__ l, const double* __restrict__ prod, const int32_t* __restrict__ tpos, double* hm,
+    int64_t ld, double* stmp, int64_t n2, double* dtmp) {
     const int b = blockIdx.y * (SD_THREADS / 32) + threadIdx.x / 32;
     if (b >= nb) return;
     const int lane_a = blockIdx.x * 32 + threadIdx.x % 32;
@@ -413,48 +360,49 @@ __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     const bool wantS = WANT_S && (!same || a >= b);
     if (!WANT_D && !__any_sync(0xffffffffu, wantS)) return;
     const double* g = tgeo + (int64_t)b * TGEO;
-    const double p0x = g[0], p0y = g[1], p0z = g[2], nx = g[3], ny = g[4], nz = g[5];
-    const double m0x = g[6], m0y = g[7], m0z = g[8], m2x = g[9], m2y = g[10], m2z = g[11];
-    const double A2 = g[12], g00 = g[16], g22 = g[17], g02 = g[18];
+    const double nx = g[0], ny = g[1], nz = g[2], m0x = g[3], m0y = g[4], m0z = g[5], m2x = g[6], m2y = g[7], m2z = g[8];
+    const double A4 = g[9];
+    const long long flat = __double_as_longlong(g[13]);
     const int32_t* tv = T + 3 * (tb + b);
     const double* dr0 = d + (int64_t)(tv[0] - vb) * npt + ia;
     const double* dr1 = d + (int64_t)(tv[1] - vb) * npt + ia;
     const double* dr2 = d + (int64_t)(tv[2] - vb) * npt + ia;
     const int64_t x0 = (int64_t)eown[3 * b] * npt + ia, x1 = (int64_t)eown[3 * b + 1] * npt + ia,
                   x2 = (int64_t)eown[3 * b + 2] * npt + ia;
-    const double* px = pts + ia;
-    const double* py = px + npt;
-    const double* pz = py + npt;
+    const double* cx = cv + 3 * (int64_t)(tv[0] - vb) * npt + ia;
+    const double* cy = cx + npt;
+    const double* cz = cy + npt;
     const int np = c_nbpts[order];
     const bool anyS = WANT_S && __any_sync(0xffffffffu, wantS);
-    double sS = 0.0, s1 = 0.0, s2 = 0.0, sw = 0.0;
+    // times 2A: S; s_j of D without the terms h sum D_i l_i, whose sums over the rule are f0 (of l_0 - l_1) and f2 (l_2 - l_1)
+    double sS = 0.0, s1 = 0.0, s2 = 0.0, sw = 0.0, f0 = 0.0, f2 = 0.0;
     for (int k = 0, o = 0; k < np; ++k, o += na) {
         const double d0 = dr0[o], d1 = dr1[o], d2 = dr2[o], l1 = l[x1 + o];
         const double m0 = l[x0 + o] - l1, m2 = l[x2 + o] - l1;
-        const double cx = px[o] - p0x, cy = py[o] - p0y, cz = pz[o] - p0z;
-        const double hh = fma(nx, cx, fma(ny, cy, nz * cz));   // 2 h
-        const double E2 = fma(m0x, cx, fma(m0y, cy, m0z * cz));
-        const double E1 = fma(m2x, cx, fma(m2y, cy, m2z * cz));
+        const double x = cx[o], y = cy[o], z = cz[o];
+        const double num = fma(nx, x, fma(ny, y, nz * z));   // 2A 2h
+        const double E2 = fma(m0x, x, fma(m0y, y, m0z * z));
+        const double E1 = fma(m2x, x, fma(m2y, y, m2z * z));
         // 2 (d0 d1 d2 + sum d_i r_j.r_k) by the tabled 2 (d_j d_k + r_j.r_k)
-        const double den = fma(-4.0, d0 * d1 * d2, fma(d0, prod[x1 + o], fma(d1, prod[x2 + o], d2 * prod[x0 + o])));
-        const double num = A2 * hh;
-        const double w = sd_half_angle(num, den);
+        const double den = fma(d0, fma(-4.0, d1 * d2, prod[x1 + o]), fma(d1, prod[x2 + o], d2 * prod[x0 + o]));
         const double wr = c_rules[order][k][3];
+        const double w = fx::half_angle<true>(num, den, fx::mant(wr), (int)fx::expo(wr), wr);
         if (anyS) {   // E0 = 2A - E1 - E2
-            const double el = fma(A2, l1, fma(E2, m0, E1 * m2));
-            sS = fma(wr, sd_flat2(num) ? el : fma(-hh, w, el), sS);
+            const double el = fma(A4, l1, fma(E2, m0, E1 * m2));   // (summed before sS: one rounding of the sum per point)
+            sS += fma(-num, sd_flat2(num) ? 0.0 : w, el);
         }
-        if (WANT_D && !sd_flat2(hh)) {   // sum D_i l_i = D0 m0 + D2 m2
-            const double f1 = fma(g02, m0, g22 * m2), f2 = fma(g00, m0, g02 * m2);
-            s1 = fma(wr, fma(w, E1, hh * f1), s1);
-            s2 = fma(wr, fma(w, E2, hh * f2), s2);
-            sw = fma(wr, w, sw);
+        if (WANT_D && (__double_as_longlong(num) & 0x7FFFFFFFFFFFFFFFll) >= flat) {   // |2h| >= 2e-10
+            s1 = fma(w, E1, s1);
+            s2 = fma(w, E2, s2);
+            sw += w;
+            f0 = fma(num, m0, f0);
+            f2 = fma(num, m2, f2);
         }
     }
     if (!live) return;
     const double area = qrec[(ta + a) * QREC + 48];
     if (wantS) {
-        const double val = area * sS;
+        const double val = area * (g[14] * sS);
         if (hm) {
             hm[lower_at(tpos[tb + b], tpos[ta + a], ld)] = val * coeff;
         } else {
@@ -464,9 +412,9 @@ __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     }
     if (WANT_D) {
         double* o = dtmp + (a * nb + b) * 3;
-        const double iA = 2.0 / A2;   // (w E_j + 2h f_j / 4) / A per component; their sum is 2 w
-        s1 *= iA;
-        s2 *= iA;
+        const double iA = g[15];   // sum D_i l_i = D0 m0 + D2 m2; the components' sum is 2 w
+        s1 = iA * fma(g[12], f0, fma(g[11], f2, s1));
+        s2 = iA * fma(g[10], f0, fma(g[12], f2, s2));
         o[0] = area * (2.0 * sw - s1 - s2);
         o[1] = area * s1;
         o[2] = area * s2;
@@ -486,7 +434,7 @@ void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, in
     constexpr int NPTS[4] = {3, 6, 7, 16};
     const int np = NPTS[order];
     // points per batch: tables of about 512 MB, a multiple of 32 triangles (full warps)
-    const int64_t per_tri = (nv + 6 * nb + 3) * 8 * np;
+    const int64_t per_tri = (4 * nv + 6 * nb) * 8 * np;
     const int64_t batch = std::min(na, std::max<int64_t>(32, std::min<int64_t>((512ll << 20) / per_tri, 4096) / 32 * 32));
     DevBuf geo((size_t)nb * (TGEO * 8 + 3 * 4), s), tab_((size_t)per_tri * batch, s);
     double* tgeo = geo.as<double>();
@@ -495,21 +443,21 @@ void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, in
     check_launch("S / D geometry");
     for (int64_t a0 = 0; a0 < na; a0 += batch) {
         const int n = (int)std::min(batch, na - a0), npt = n * np;
-        double* pts = tab_.as<double>();
-        double* d = pts + 3 * (int64_t)npt;
+        double* cv = tab_.as<double>();
+        double* d = cv + 3 * nv * npt;
         double* l = d + nv * npt;
         double* prod = l + 3 * nb * npt;
         const unsigned gx = nblocks(npt, SD_THREADS);
         sd_distance_kernel<<<dim3(gx, nblocks(nv, SD_V)), SD_THREADS, 0, s>>>(g.qrec, tab + a0, n, npt, g.V, vbb, (int)nv,
-                                                                            pts, d);
+                                                                            cv, d);
         check_launch("S / D distances");
-        sd_edge_kernel<<<dim3(gx, nblocks(nb, SD_E)), SD_THREADS, 0, s>>>(tbb, (int)nb, npt, g.T, vbb, tgeo, eown, d, l,
-                                                                              prod);
+        sd_edge_kernel<<<dim3(gx, nblocks(nb, SD_E)), SD_THREADS, 0, s>>>(tbb, (int)nb, n, npt, order, g.T, vbb, tgeo,
+                                                                          eown, d, l, prod);
         check_launch("S / D edges");
         const dim3 grid(nblocks(n, 32), nblocks(nb, SD_THREADS / 32));
         auto kern = wantS ? (dtmp ? sd_pair_kernel<true, true> : sd_pair_kernel<true, false>) : sd_pair_kernel<false, true>;
         kern<<<grid, SD_THREADS, 0, s>>>(tbb, (int)nb, tab, a0, n, npt, order, same ? 1 : 0, coeff, g.T, vbb, tgeo, eown,
-                                         g.qrec, pts, d, l, prod, g.tpos, hm, ld, stmp, na, dtmp);
+                                         g.qrec, cv, d, l, prod, g.tpos, hm, ld, stmp, na, dtmp);
         check_launch("S / D pairs");
     }
 }
@@ -1100,15 +1048,15 @@ __device__ __forceinline__ double near_eval(const double* __restrict__ p, d3 x, 
     const d3 r0 = dev::ld3(p) - x, r1 = dev::ld3(p + 3) - x, r2 = dev::ld3(p + 6) - x, n = dev::ld3(p + 9);
     const double A2 = 2.0 * p[12], e0 = p[13], e1 = p[14], e2 = p[15];
     const double q0 = e0 * e0, q1 = e1 * e1, q2 = e2 * e2;
-    const double d0 = sd_sqrt(dev::dot(r0, r0)), d1 = sd_sqrt(dev::dot(r1, r1)), d2 = sd_sqrt(dev::dot(r2, r2));
+    const double d0 = fx::sqrt64(dev::dot(r0, r0)), d1 = fx::sqrt64(dev::dot(r1, r1)), d2 = fx::sqrt64(dev::dot(r2, r2));
     const double R0 = d0 + d1, R1 = d1 + d2, R2 = d2 + d0;
-    const double l0 = sd_edge(R0, e0), l1 = sd_edge(R1, e1), l2 = sd_edge(R2, e2);
+    const double l0 = fx::edge<false>(R0, e0, 0, 0, 0.0), l1 = fx::edge<false>(R1, e1, 0, 0, 0.0), l2 = fx::edge<false>(R2, e2, 0, 0, 0.0);
     const double m0 = l0 - l1, m2 = l2 - l1;
     const d3 nr = dev::cross(n, r0);
     const double E2 = dev::dot(nr, r1), E1 = -dev::dot(nr, r2);
     const double hh = 2.0 * dev::dot(r0, n), num = A2 * hh;
     const double den = fma(-4.0, d0 * d1 * d2, fma(d0, fma(R1, R1, -q1), fma(d1, fma(R2, R2, -q2), d2 * fma(R0, R0, -q0))));
-    const double w = sd_half_angle(num, den);
+    const double w = fx::half_angle<false>(num, den, 0, 0, 0.0);
     if (WANT_D) {
         out[0] = out[1] = out[2] = 0.0;
         if (!sd_flat2(hh)) {
@@ -1126,9 +1074,11 @@ __device__ __forceinline__ double near_eval(const double* __restrict__ p, d3 x, 
 // Near pairs: the FP64 analytic kernels of the reference (same outer rule).
 // One lane per (pair, point of the rule): 16 lanes hold a pair, each lane
 // evaluates the analytic integrals at its point (S and D21 over t1 at the
-// points of t2, D12 over t2 at the points of t1, near_eval: about 500 FP64
-// operations against 930 with separate logarithms) and the weighted values are summed across the 16 lanes by
-// shuffles.  Short per-thread chains and many warps hide the latency of the
+// points of t2, D12 over t2 at the points of t1, near_eval: one logarithm per
+// edge, and it, the square roots and the arctangent on the integer pipe where
+// their polynomials reach) and the weighted values are summed across the 16
+// lanes by shuffles.  The 17926-unknown head's near pairs take 3.6 ms, with
+// FP64 polynomials 3.9, with separate logarithms for S and D 5.2.  Short per-thread chains and many warps hide the latency of the
 // FP64 transcendentals.
 constexpr int NP_LANES = 16;
 
@@ -2892,3 +2842,25 @@ void launch_fold_to_reference(int64_t Nref, int64_t nvg, int64_t nP, const int64
 }
 
 }  // namespace omg
+
+// Test hook (not part of the public header): the functions of fixed64.cuh on device arrays; which = 0 sqrt(a),
+// 1 2 atanh(b / a) / b, 2 atan2(b, a), with the weight wr where it is not 0.
+namespace omg {
+__global__ void fixed64_eval_kernel(int which, int64_t n, const double* a, const double* b, double wr, double* out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint64_t wm = fx::mant(wr);
+    const int we = (int)fx::expo(wr);
+    if (which == 0)
+        out[i] = fx::sqrt64(a[i]);
+    else if (which == 1)
+        out[i] = wr != 0.0 ? fx::edge<true>(a[i], b[i], wm, we, wr) : fx::edge<false>(a[i], b[i], 0, 0, 0.0);
+    else
+        out[i] = wr != 0.0 ? fx::half_angle<true>(b[i], a[i], wm, we, wr) : fx::half_angle<false>(b[i], a[i], 0, 0, 0.0);
+}
+}  // namespace omg
+extern "C" int omg_internal_fixed64(int which, int64_t n, const double* a, const double* b, double wr, double* out) {
+    if (n <= 0 || which < 0 || which > 2) return OMG_ERR_INVALID;
+    omg::fixed64_eval_kernel<<<omg::nblocks(n, 128), 128>>>(which, n, a, b, wr, out);
+    return cudaDeviceSynchronize() == cudaSuccess ? OMG_OK : OMG_ERR_CUDA;
+}
