@@ -223,7 +223,7 @@ __device__ __forceinline__ int64_t lower_at(int64_t a, int64_t b, int64_t ld) {
 // About 35 FP64 operations per (triangle, point) for S and D together: the square
 // roots, logarithms and arctangents and the weights of the rule run on the integer
 // pipe (fixed64.cuh), which issues beside the FP64 operations.  With all of it in FP64
-// (75 operations, 88% of the pipe's rate) the blocks of a head of 7080 triangles in
+// (75 operations, 88% of the pipe's rate) the blocks of a head of 7020 triangles in
 // four layers took 67 ms, now 34.1.
 // Lanes run over the triangles a at the same rule point, so every table read is
 // coalesced, the triangle b is uniform in a warp, and the sum over the rule stays
@@ -1077,7 +1077,7 @@ __device__ __forceinline__ double near_eval(const double* __restrict__ p, d3 x, 
 // points of t2, D12 over t2 at the points of t1, near_eval: one logarithm per
 // edge, and it, the square roots and the arctangent on the integer pipe where
 // their polynomials reach) and the weighted values are summed across the 16
-// lanes by shuffles.  The 17926-unknown head's near pairs take 3.6 ms, with
+// lanes by shuffles.  The 17926-unknown head's near pairs take 2.9 ms, with
 // FP64 polynomials 3.9, with separate logarithms for S and D 5.2.  Short per-thread chains and many warps hide the latency of the
 // FP64 transcendentals.
 constexpr int NP_LANES = 16;

@@ -80,9 +80,31 @@ __device__ __forceinline__ double sqrt64(double x) {
     return pack(mulh(m, g), xe + ye - 1023 + 2);
 }
 
-// 2 atanh(len / R) / len (times the weight of mantissa wm and biased exponent we where WEIGHT), 0 < len < R: with z = len / R
-// and w = z^2, 2 / R (1 + u), u = w f(w) = atanh(z) / z - 1 by the polynomials that interpolate f at the Chebyshev nodes of
-// [0, 2^-6] and [0, 1/4] (relative error of the result 2^-65 and 2^-62.8), the library's logarithm beyond z = 1/2.
+// atanh(z) / z - 1 of z in Q64 below 1/2, Q64: w f(w), w = z^2, f by the polynomial that interpolates it at the Chebyshev
+// nodes of [0, 1/4] (2^-62.8).
+__device__ __forceinline__ uint64_t atanh_half(uint64_t z) {
+    const int64_t v = (int64_t)(mulh(z, z) << 1);   // w / (1/4) in Q63
+    int64_t a = -0x2f3bcdad3ll + (__mul64hi(v, 0xe7f9933cll) << 1);
+    a = 0xa798b13acll + (__mul64hi(v, a) << 1);
+    a = -0x17b097a15ll + (__mul64hi(v, a) << 1);
+    a = 0x37febab086ll + (__mul64hi(v, a) << 1);
+    a = 0xbb2926705bll + (__mul64hi(v, a) << 1);
+    a = 0x3622dd23e5cll + (__mul64hi(v, a) << 1);
+    a = 0xf0db60f9e55ll + (__mul64hi(v, a) << 1);
+    a = 0x444498cb9d98ll + (__mul64hi(v, a) << 1);
+    a = 0x13b13a3184d91ll + (__mul64hi(v, a) << 1);
+    a = 0x5d1745ea0cee5ll + (__mul64hi(v, a) << 1);
+    a = 0x1c71c71c58156bll + (__mul64hi(v, a) << 1);
+    a = 0x924924924a04e3ll + (__mul64hi(v, a) << 1);
+    a = 0x333333333333030ll + (__mul64hi(v, a) << 1);
+    a = 0x1555555555555557ll + (__mul64hi(v, a) << 1);
+    return (uint64_t)(__mul64hi(v, a) << 1);
+}
+
+// 2 atanh(len / R) / len = log((R + len) / (R - len)) / len (times the weight of mantissa wm and biased exponent we where
+// WEIGHT), 0 < len < R.  With z = len / R: 2 / R (1 + u), u = atanh(z) / z - 1, by a polynomial on [0, 1/8] (2^-65) or
+// atanh_half.  From z = 1/2 on, with a = R + len and b = R - len (exact): (k log 2 + 2 atanh((a - 2^k b) / (a + 2^k b))) / len,
+// k the difference of their exponents, so that the quotient is below 1/3.
 template <bool WEIGHT>
 __device__ __forceinline__ double edge(double R, double len, uint64_t wm, int we, double wr) {
     uint32_t ym;
@@ -90,10 +112,11 @@ __device__ __forceinline__ double edge(double R, double len, uint64_t wm, int we
     uint64_t c;
     const bool ok = rcp21(R, ym, ye, c);
     const int sh = 2044 - (int)expo(len) - ye;
-    const uint64_t z = (mulh(mul21(mant(len), ym), c) << 1) >> min(max(sh, 0), 63);   // Q64
-    uint64_t w = mulh(z, z), u;
-    if (__all_sync(__activemask(), ok && sh >= 0 && z < (1ull << 61))) {   // (one polynomial for the whole warp)
-        w <<= 6;
+    uint64_t z = (mulh(mul21(mant(len), ym), c) << 1) >> min(max(sh, 0), 63);   // Q64
+    const bool direct = ok && sh >= 0 && z < (1ull << 63);
+    uint64_t u;
+    if (__all_sync(__activemask(), direct && z < (1ull << 61))) {   // (one polynomial for the whole warp)
+        const uint64_t w = mulh(z, z) << 6;
         const uint32_t wh = hi32(w);
         uint32_t t = __umulhi(wh, 0x47a94u) + 0x13ac84au;
         t = __umulhi(wh, t) + 0x5d177978u;
@@ -102,46 +125,59 @@ __device__ __forceinline__ double edge(double R, double len, uint64_t wm, int we
         u = 0x3333333333303ull + mulh(u, w);
         u = 0x155555555555556ull + mulh(u, w);
         u = mulh(u, w);
-    } else if (ok && sh >= 0 && z < (1ull << 63)) {
-        const int64_t v = (int64_t)(w << 1);   // w / (1/4) in Q63
-        int64_t a = -0x2f3bcdad3ll + (__mul64hi(v, 0xe7f9933cll) << 1);
-        a = 0xa798b13acll + (__mul64hi(v, a) << 1);
-        a = -0x17b097a15ll + (__mul64hi(v, a) << 1);
-        a = 0x37febab086ll + (__mul64hi(v, a) << 1);
-        a = 0xbb2926705bll + (__mul64hi(v, a) << 1);
-        a = 0x3622dd23e5cll + (__mul64hi(v, a) << 1);
-        a = 0xf0db60f9e55ll + (__mul64hi(v, a) << 1);
-        a = 0x444498cb9d98ll + (__mul64hi(v, a) << 1);
-        a = 0x13b13a3184d91ll + (__mul64hi(v, a) << 1);
-        a = 0x5d1745ea0cee5ll + (__mul64hi(v, a) << 1);
-        a = 0x1c71c71c58156bll + (__mul64hi(v, a) << 1);
-        a = 0x924924924a04e3ll + (__mul64hi(v, a) << 1);
-        a = 0x333333333333030ll + (__mul64hi(v, a) << 1);
-        a = 0x1555555555555557ll + (__mul64hi(v, a) << 1);
-        u = (uint64_t)(__mul64hi(v, a) << 1);
     } else {
-        const double l = log((R + len) / (R - len)) / len;
-        return WEIGHT ? l * wr : l;
+        int k = 0;
+        uint32_t minus = 0;
+        if (!direct) {
+            const double a = R + len, b = R - len;
+            k = (int)expo(a) - (int)expo(b);
+            const double bk = __hiloint2double(__double2hiint(b) + (k << 20), __double2loint(b));
+            const double n = a - bk, d = a + bk;
+            uint32_t dm;
+            int de;
+            uint64_t dc;
+            if (!(__double2hiint(b) > 0x100000 && expo(a) < 0x7FE && (unsigned)k < 64u && rcp21(d, dm, de, dc) && expo(len) != 0))
+                return (WEIGHT ? wr : 1.0) * (log((R + len) / (R - len)) / len);
+            minus = (uint32_t)__double2hiint(n) >> 31;
+            const int s = 2044 - (int)expo(n) - de;
+            z = expo(n) ? (mulh(mul21(mant(n), dm), dc) << 1) >> min(max(s, 0), 63) : 0;
+        }
+        u = atanh_half(z);
+        if (!direct) {
+            const uint64_t t = mulh(z, 0x8000000000000000ull + (u >> 1)) >> 5;   // 2 atanh in Q57
+            const uint64_t base = 0x162E42FEFA39EF3ull * (uint64_t)k;            // k log 2 in Q57
+            const uint64_t sum = minus ? base - t : base + t;
+            const int zs = __clzll((long long)sum);
+            rcp21(len, ym, ye, c);
+            uint64_t m = mulh(sum << zs, c);
+            if (WEIGHT) m = mulh(m, wm);
+            // sum 2^-57 / len: m = sum 2^zs / 2 (/ 2), mul21 another 2^-21 of ym 2^20
+            return pack(mul21(m, ym), (WEIGHT ? we - 1023 + 1 : 0) + ye + 8 - zs);
+        }
     }
     uint64_t m = mulh(0x8000000000000000ull + (u >> 1), c);
     if (WEIGHT) m = mulh(m, wm);
     return pack(mul21(m, ym), (WEIGHT ? we - 1023 + 1 : 0) + ye + 3);
 }
 
-// atan2(num, den), half a solid angle (times the weight where WEIGHT): where t = num / den < 1/2 and den > 0 by
-// t (1 - w g(w)), w = t^2, g interpolated on [0, 2^-8] and [0, 1/4] (relative error of the result 2^-70 and 2^-64).
+// atan2(num, den), half a solid angle (times the weight where WEIGHT).  Where t = num / den < 1/2 and den > 0:
+// t (1 - w g(w)), w = t^2, g interpolated on [0, 2^-8] and [0, 1/4] (2^-70 and 2^-64).  Elsewhere the angle from the nearest of
+// pi/4, pi/2, 3 pi/4 and pi, whose tangent is below 1/2.
 template <bool WEIGHT>
 __device__ __forceinline__ double half_angle(double num, double den, uint64_t wm, int we, double wr) {
     uint32_t ym;
     int ye;
     uint64_t c;
-    const bool ok = rcp21(den, ym, ye, c);
-    const int ne = (int)expo(num), sh = 2044 - ne - ye;
-    const uint64_t q = mulh(mul21(mant(num), ym), c) << 1;   // the quotient's mantissa in Q62
-    const uint64_t t = q >> min(max(sh, 0), 63);
-    uint64_t w = mulh(t, t), u;
-    if (__all_sync(__activemask(), ok && sh >= 0 && t < (1ull << 60))) {
-        w <<= 8;
+    bool ok = rcp21(den, ym, ye, c);
+    int ne = (int)expo(num), sh = 2044 - ne - ye;
+    uint64_t q = mulh(mul21(mant(num), ym), c) << 1;   // the quotient's mantissa in Q62
+    uint64_t t = q >> min(max(sh, 0), 63);
+    const bool direct = ok && sh >= 0 && t < (1ull << 63);
+    uint32_t sign = (uint32_t)__double2hiint(num) >> 31;
+    double base = 0.0;
+    uint64_t u;
+    if (__all_sync(__activemask(), direct && t < (1ull << 60))) {
+        const uint64_t w = mulh(t, t) << 8;
         const uint32_t wh = hi32(w);
         uint32_t a = 0x174598u - __umulhi(wh, 0x137eu);
         a = 0x1c71c6ffu - __umulhi(wh, a);
@@ -149,8 +185,37 @@ __device__ __forceinline__ double half_angle(double num, double den, uint64_t wm
         u = 0x333333333333ull - mulh(u, w);
         u = 0x55555555555555ull - mulh(u, w);
         u = mulh(u, w);
-    } else if (ok && sh >= 0 && t < (1ull << 63)) {
-        w <<= 2;
+    } else {
+        if (!direct) {
+            const double an = fabs(num), ad = fabs(den);
+            const long long in = __double_as_longlong(an), id = __double_as_longlong(ad), one = 1ll << 52;
+            const bool left = __double2hiint(den) < 0;
+            double n, d;
+            if (in > id + one) {   // |num| > 2 |den|: from pi/2
+                base = 1.5707963267948966;
+                n = -den;
+                d = an;
+            } else if (in + one > id) {   // from pi/4 or 3 pi/4
+                base = left ? 2.356194490192345 : 0.7853981633974483;
+                n = an - ad;
+                d = an + ad;
+                n = left ? -n : n;
+            } else {   // from pi (num < den / 2 with den > 0 is direct, or not finite)
+                base = 3.141592653589793;
+                n = -an;
+                d = ad;
+            }
+            const long long big = in > id ? in : id;
+            ok = rcp21(d, ym, ye, c) && big >= (one << 1) && big < 0x7FD0000000000000ll && (left || in + one > id);
+            if (!ok) return (WEIGHT ? wr : 1.0) * atan2(num, den);
+            base = sign ? -base : base;
+            sign ^= (uint32_t)__double2hiint(n) >> 31;
+            ne = (int)expo(n);
+            sh = 2044 - ne - ye;
+            q = mulh(mul21(mant(n), ym), c) << 1;
+            t = q >> min(max(sh, 0), 63);
+        }
+        const uint64_t w = mulh(t, t) << 2;
         uint64_t a = 0x1633de284ull - mulh(w, 0x1f5c3523ull);
         a = 0x8b3543996ull - mulh(w, a);
         a = 0x2ad65f05c0ull - mulh(w, a);
@@ -165,13 +230,11 @@ __device__ __forceinline__ double half_angle(double num, double den, uint64_t wm
         a = 0x3333333333331ceull - mulh(w, a);
         a = 0x1555555555555554ull - mulh(w, a);
         u = mulh(w, a);
-    } else {
-        const double v = atan2(num, den);
-        return WEIGHT ? v * wr : v;
     }
     uint64_t m = mulh(0x8000000000000000ull - (u >> 1), q);
-    if (WEIGHT) m = mulh(m, wm);
-    return pack(m, ne ? (WEIGHT ? we - 1023 + 1 : 0) + ne + ye - 1023 + 2 : 0, (uint32_t)__double2hiint(num) >> 31);
+    if (WEIGHT && direct) m = mulh(m, wm);
+    const double v = pack(m, ne ? (WEIGHT && direct ? we - 1023 + 1 : 0) + ne + ye - 1023 + 2 : 0, sign);
+    return direct ? v : (WEIGHT ? wr : 1.0) * (base + v);
 }
 
 }  // namespace fx

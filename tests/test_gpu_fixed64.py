@@ -4,8 +4,8 @@ Arguments on both sides of every polynomial's limit, powers of two and their
 neighbours (where the residual of the approximate reciprocal changes scale),
 mantissas of all ones, and what no polynomial takes.  Error bound: the rounding,
 2^-53, and at most four products of 60 bits, 2 units each, and the residual's
-third order, 2^-58.8: under 2^-56 together.  The library's functions (beyond
-1/2): a few roundings, 2^-50.
+third order, 2^-58.8: under 2^-56 together.  Beyond 1/2 a few roundings of the
+sums that the argument is reduced by: 2^-50.
 """
 import ctypes
 
@@ -13,7 +13,7 @@ import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
-TIGHT, LIBRARY = 2.0 ** -53 * 1.125, 2.0 ** -50
+TIGHT, REDUCED = 2.0 ** -53 * 1.125, 2.0 ** -50
 
 
 def _eval(which, a, b, wr=0.0):
@@ -59,8 +59,35 @@ def test_edge_and_angle(cuda, which, wr, lo, hi):
     for x, z, y in zip(a, b, _eval(which, a, b, wr)):
         X, Z = mp.mpf(float(x)), mp.mpf(float(z))
         r = (2 * mp.atanh(Z / X) / Z if which == 1 else mp.atan2(Z, X)) * mp.mpf(wr if wr else 1.0)
-        tol = TIGHT if abs(z) < 0.4999999 * x else LIBRARY
+        tol = TIGHT if abs(z) < 0.4999999 * x else REDUCED
         assert abs(mp.mpf(float(y)) / r - 1) <= tol, (float(x), float(z))
+
+
+@pytest.mark.parametrize("wr", [0.0, 0.027230314174434])
+def test_every_quadrant(cuda, wr):
+    mp = pytest.importorskip("mpmath").mp
+    mp.dps = 60
+    rng = np.random.default_rng(4)
+    t = np.concatenate([np.tan(np.arange(-16, 17) * np.pi / 16 + 1e-9), [2.0, 0.5, 1.0, -1.0, -2.0, -0.5],
+                        np.ldexp(rng.uniform(-1, 1, 300), rng.integers(-8, 9, 300))])
+    a = _values(len(t), rng) * rng.choice([-1.0, 1.0], len(t))
+    b = a * t
+    for x, z, y in zip(a, b, _eval(2, a, b, wr)):
+        r = mp.atan2(mp.mpf(float(z)), mp.mpf(float(x))) * mp.mpf(wr if wr else 1.0)
+        assert abs(mp.mpf(float(y)) / r - 1) <= REDUCED, (float(x), float(z))
+
+
+@pytest.mark.parametrize("wr", [0.0, 0.027230314174434])
+def test_points_close_to_an_edge(cuda, wr):
+    mp = pytest.importorskip("mpmath").mp
+    mp.dps = 60
+    rng = np.random.default_rng(5)
+    b = _values(300, rng)
+    a = b * (1 + np.ldexp(rng.uniform(0.5, 1, 300), rng.integers(-50, 1, 300)))
+    for x, z, y in zip(a, b, _eval(1, a, b, wr)):
+        X, Z = mp.mpf(float(x)), mp.mpf(float(z))
+        r = mp.log((X + Z) / (X - Z)) / Z * mp.mpf(wr if wr else 1.0)
+        assert abs(mp.mpf(float(y)) / r - 1) <= REDUCED, (float(x), float(z))
 
 
 def test_values_no_polynomial_takes(cuda):
