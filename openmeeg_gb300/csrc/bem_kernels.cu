@@ -219,23 +219,36 @@ __device__ __forceinline__ int64_t lower_at(int64_t a, int64_t b, int64_t ld) {
 //      w = atan(2 A h / (d0 d1 d2 + sum d_i r_j.r_k)), then
 //        S = sum_i E_opp(i) l_i - 2 h w,
 //        D_j = (w E_j + h/2 D_j+1.(sum_i D_i l_i)) / A, D_0 + D_1 + D_2 = 2 w,
-//      in 29 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
-// About 35 FP64 operations per (triangle, point) for S and D together: the square
-// roots, logarithms and arctangents and the weights of the rule run on the integer
-// pipe (fixed64.cuh), which issues beside the FP64 operations.  With all of it in FP64
-// (75 operations, 88% of the pipe's rate) the blocks of a head of 7020 triangles in
-// four layers took 67 ms, now 34.1.
+//      in 19 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
+// About 26 FP64 operations per (triangle, point) for S and D together.  The square
+// roots, logarithms, arctangents, the weights of the rule and the linear forms h, E_j
+// run on the integer pipe (fixed64.cuh), which issues beside the FP64 operations: the
+// forms as inner products of 60-bit vectors, of the triangle and of x - p0 from the
+// table.  A head matrix of four layers (7020 triangles) took 67 ms in these kernels
+// with all of it in FP64 (75 operations), 34 with the linear forms in FP64 (35), now
+// 23.7: the pair kernel holds the FP64 pipe 84% busy, the distances likewise, and the
+// edges (285 instructions each, 29% of the time) issue 66% of what the SM can.
 // Lanes run over the triangles a at the same rule point, so every table read is
 // coalesced, the triangle b is uniform in a warp, and the sum over the rule stays
 // in registers (no shuffles, which cost FP64 additions).
 // ---------------------------------------------------------------------------
-// Record of an analytic triangle: -2 N, N x D0, N x D2 (N = D0 x (p2 - p0), |N| = 2A; 3 each), 4A^2, |D0|^2 / 4, |D2|^2 / 4,
+// Record of an analytic triangle: -2 N, N x D0, N x D2 (N = D0 x (p2 - p0), |N| = 2A; in block fixed point, 3 each; their
+// exponents in an int4 of their own table), 4A^2, |D0|^2 / 4, |D2|^2 / 4,
 // D0.D2 / 4, the bits of 2e-10 * 2A, 1 / 2A, 2 / 4A^2, |D_i|^2 (3), |D_i| (3)
 constexpr int TGEO = 22;
 
+// v in block fixed point; returns its exponent.
+__device__ __forceinline__ int sd_fix(d3 v, int2* out) {
+    const int ex = (int)fx::expo(v.x), ey = (int)fx::expo(v.y), ez = (int)fx::expo(v.z), em = max(ex, max(ey, ez));
+    out[0] = fx::limbs(fx::fix60(v.x, em - ex));
+    out[1] = fx::limbs(fx::fix60(v.y, em - ey));
+    out[2] = fx::limbs(fx::fix60(v.z, em - ez));
+    return em - 1022;
+}
+
 __global__ void sd_geometry_kernel(int64_t t0, int64_t nt, const double* __restrict__ V,
                                    const int32_t* __restrict__ T, const int32_t* __restrict__ v2t_beg,
-                                   const int32_t* __restrict__ v2t_tri, double* tgeo, int32_t* eown) {
+                                   const int32_t* __restrict__ v2t_tri, double* tgeo, int4* gexp, int32_t* eown) {
     const int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (it >= nt) return;
     const int32_t* tv = T + 3 * (t0 + it);
@@ -246,9 +259,8 @@ __global__ void sd_geometry_kernel(int64_t t0, int64_t nt, const double* __restr
     const d3 m0 = dev::cross(nn, D0), m2 = dev::cross(nn, D2);
     const double a22 = dev::dot(nn, nn), a2 = sqrt(a22);
     double* g = tgeo + it * TGEO;
-    g[0] = -2.0 * nn.x; g[1] = -2.0 * nn.y; g[2] = -2.0 * nn.z;
-    g[3] = m0.x; g[4] = m0.y; g[5] = m0.z;
-    g[6] = m2.x; g[7] = m2.y; g[8] = m2.z;
+    int2* gf = reinterpret_cast<int2*>(g);
+    gexp[it] = make_int4(sd_fix(nn * -2.0, gf), sd_fix(m0, gf + 3), sd_fix(m2, gf + 6), 0);
     g[9] = a22;
     g[16] = dev::dot(D0, D0); g[17] = dev::dot(D1, D1); g[18] = dev::dot(D2, D2);
     g[10] = 0.25 * g[16]; g[11] = 0.25 * g[18]; g[12] = 0.25 * dev::dot(D2, D0);
@@ -286,15 +298,16 @@ __device__ __forceinline__ double sd_rcp(double x) {
 __device__ __forceinline__ bool sd_flat2(double x) {
     return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) < __double_as_longlong(2e-10);
 }
-constexpr int SD_V = 16;      // vertices per CTA of the distance table
-constexpr int SD_E = 8;       // triangles per CTA of the edge table
+constexpr int SD_V = 8;      // vertices per CTA of the distance table
+constexpr int SD_E = 4;       // triangles per CTA of the edge table
 constexpr int SD_THREADS = 256;
 
 // Point x = q na + ia of a batch of na triangles from a0: point q of triangle a0 + ia.  For vertex vb + v: the distance
-// d[v * npt + x] and, in the rows 3 v .. 3 v + 2 of cv, the point minus the vertex.
+// d[v * npt + x] and, in the rows 3 v .. 3 v + 2 of cv, the point minus the vertex in block fixed point with E = the exponent
+// of the distance + 1.
 __global__ void __launch_bounds__(SD_THREADS) sd_distance_kernel(const double* __restrict__ qrec, int64_t a0, int na,
                                                                  int npt, const double* __restrict__ V, int64_t vb,
-                                                                 int nv, double* __restrict__ cv,
+                                                                 int nv, int2* __restrict__ cv,
                                                                  double* __restrict__ d) {
     const int x = blockIdx.x * SD_THREADS + threadIdx.x;
     if (x >= npt) return;
@@ -307,11 +320,13 @@ __global__ void __launch_bounds__(SD_THREADS) sd_distance_kernel(const double* _
         const double* p = V + 3 * (vb + v);
         const double rx = px - p[0], ry = py - p[1], rz = pz - p[2];
         const int64_t o = (int64_t)v * npt + x;
-        d[o] = fx::sqrt64(fma(rx, rx, fma(ry, ry, rz * rz)));
-        double* c = cv + o + 2 * (int64_t)v * npt;
-        c[0] = rx;
-        c[npt] = ry;
-        c[2 * (int64_t)npt] = rz;
+        const double dist = fx::sqrt64(fma(rx, rx, fma(ry, ry, rz * rz)));
+        const int e = (int)fx::expo(dist);
+        d[o] = dist;
+        int2* c = cv + o + 2 * (int64_t)v * npt;
+        c[0] = fx::limbs(fx::fix60(rx, e - (int)fx::expo(rx)));
+        c[npt] = fx::limbs(fx::fix60(ry, e - (int)fx::expo(ry)));
+        c[2 * (int64_t)npt] = fx::limbs(fx::fix60(rz, e - (int)fx::expo(rz)));
     }
 }
 
@@ -344,14 +359,19 @@ __global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb,
 
 // The pairs (triangle b, triangle a0 + ia of the batch): warp w of a CTA holds b, its lanes 32 triangles a.
 // S for a >= b only when `same`.
+// CTAs of two warps: a small head fills more SMs evenly (the smallest gain's blocks 1.26 ms, 1.5 with four warps, 1.6 with
+// eight); 8 CTAs of 105 registers (more, with fewer registers, were no faster).
+constexpr int SD_WARPS = 2, SD_CTAS = 8;
 template <bool WANT_S, bool WANT_D>
-__global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
-    int64_t tb, int nb, int64_t ta, int64_t a0, int na, int npt, int order, int same, double coeff,
-    const int32_t* __restrict__ T, int64_t vb, const double* __restrict__ tgeo, const int32_t* __restrict__ eown,
-    const double* __restrict__ qrec, const double* __restrict__ cv, const double* __restrict__ d,
+__global__ void __launch_bounds__(32 * SD_WARPS, SD_CTAS) sd_pair_kernel(
+    int64_t tb, int nb, unsigned first, int64_t ta, int64_t a0, int na, int npt, int order, int same, double coeff,
+    const int32_t* __restrict__ T, int64_t vb, const double* __restrict__ tgeo, const int4* __restrict__ gexp,
+    const int32_t* __restrict__ eown, const double* __restrict__ qrec, const int2* __restrict__ cv,
+    const double* __restrict__ d,
     const double* __restrict__ l, const double* __restrict__ prod, const int32_t* __restrict__ tpos, double* hm,
     int64_t ld, double* stmp, int64_t n2, double* dtmp) {
-    const int b = blockIdx.y * (SD_THREADS / 32) + threadIdx.x / 32;
+    const unsigned by = blockIdx.y + first;
+    const int b = (by < gridDim.y ? by : by - gridDim.y) * SD_WARPS + threadIdx.x / 32;
     if (b >= nb) return;
     const int lane_a = blockIdx.x * 32 + threadIdx.x % 32;
     const bool live = lane_a < na;
@@ -360,7 +380,10 @@ __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     const bool wantS = WANT_S && (!same || a >= b);
     if (!WANT_D && !__any_sync(0xffffffffu, wantS)) return;
     const double* g = tgeo + (int64_t)b * TGEO;
-    const double nx = g[0], ny = g[1], nz = g[2], m0x = g[3], m0y = g[4], m0z = g[5], m2x = g[6], m2y = g[7], m2z = g[8];
+    const int2* gf = reinterpret_cast<const int2*>(g);
+    const int2 nx = gf[0], ny = gf[1], nz = gf[2], m0x = gf[3], m0y = gf[4], m0z = gf[5], m2x = gf[6], m2y = gf[7],
+               m2z = gf[8];
+    const int4 ge = gexp[b];
     const double A4 = g[9];
     const long long flat = __double_as_longlong(g[13]);
     const int32_t* tv = T + 3 * (tb + b);
@@ -369,9 +392,9 @@ __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     const double* dr2 = d + (int64_t)(tv[2] - vb) * npt + ia;
     const int64_t x0 = (int64_t)eown[3 * b] * npt + ia, x1 = (int64_t)eown[3 * b + 1] * npt + ia,
                   x2 = (int64_t)eown[3 * b + 2] * npt + ia;
-    const double* cx = cv + 3 * (int64_t)(tv[0] - vb) * npt + ia;
-    const double* cy = cx + npt;
-    const double* cz = cy + npt;
+    const int2* cx = cv + 3 * (int64_t)(tv[0] - vb) * npt + ia;
+    const int2* cy = cx + npt;
+    const int2* cz = cy + npt;
     const int np = c_nbpts[order];
     const bool anyS = WANT_S && __any_sync(0xffffffffu, wantS);
     // times 2A: S; s_j of D without the terms h sum D_i l_i, whose sums over the rule are f0 (of l_0 - l_1) and f2 (l_2 - l_1)
@@ -379,10 +402,11 @@ __global__ void __launch_bounds__(SD_THREADS) sd_pair_kernel(
     for (int k = 0, o = 0; k < np; ++k, o += na) {
         const double d0 = dr0[o], d1 = dr1[o], d2 = dr2[o], l1 = l[x1 + o];
         const double m0 = l[x0 + o] - l1, m2 = l[x2 + o] - l1;
-        const double x = cx[o], y = cy[o], z = cz[o];
-        const double num = fma(nx, x, fma(ny, y, nz * z));   // 2A 2h
-        const double E2 = fma(m0x, x, fma(m0y, y, m0z * z));
-        const double E1 = fma(m2x, x, fma(m2y, y, m2z * z));
+        const int2 x = cx[o], y = cy[o], z = cz[o];
+        const int ce = (int)fx::expo(d0) - 1022;
+        const double num = fx::value60(fx::dot60(nx, ny, nz, x, y, z), ge.x + ce);   // 2A 2h
+        const double E2 = fx::value60(fx::dot60(m0x, m0y, m0z, x, y, z), ge.y + ce);
+        const double E1 = fx::value60(fx::dot60(m2x, m2y, m2z, x, y, z), ge.z + ce);
         // 2 (d0 d1 d2 + sum d_i r_j.r_k) by the tabled 2 (d_j d_k + r_j.r_k)
         const double den = fma(d0, fma(-4.0, d1 * d2, prod[x1 + o]), fma(d1, prod[x2 + o], d2 * prod[x0 + o]));
         const double wr = c_rules[order][k][3];
@@ -433,18 +457,22 @@ void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, in
     if (nb > (1 << 28)) throw Error(OMG_ERR_UNSUPPORTED, "S / D block too large");
     constexpr int NPTS[4] = {3, 6, 7, 16};
     const int np = NPTS[order];
-    // points per batch: tables of about 512 MB, a multiple of 32 triangles (full warps)
+    // Points per batch: tables of about 1 GB, batches of equal size in multiples of 32 triangles (full warps).  A batch's
+    // kernels each end with a part-empty last wave, which costs more than tables that stay in L2 would save: the four-layer
+    // head takes 36.5 ms at 128 MB, 28.1 at 256, 25.4 at 512, 24.1 here, 23.5 at 2 GB.
     const int64_t per_tri = (4 * nv + 6 * nb) * 8 * np;
-    const int64_t batch = std::min(na, std::max<int64_t>(32, std::min<int64_t>((512ll << 20) / per_tri, 4096) / 32 * 32));
-    DevBuf geo((size_t)nb * (TGEO * 8 + 3 * 4), s), tab_((size_t)per_tri * batch, s);
-    double* tgeo = geo.as<double>();
+    const int64_t most = std::max<int64_t>(32, std::min<int64_t>((1024ll << 20) / per_tri, 4096) / 32 * 32);
+    const int64_t nbatch = (na + most - 1) / most, batch = std::min(na, ((na + nbatch - 1) / nbatch + 31) / 32 * 32);
+    DevBuf geo((size_t)nb * (TGEO * 8 + 16 + 3 * 4), s), tab_((size_t)per_tri * batch, s);
+    int4* gexp = geo.as<int4>();
+    double* tgeo = reinterpret_cast<double*>(gexp + nb);
     int32_t* eown = reinterpret_cast<int32_t*>(tgeo + nb * TGEO);
-    sd_geometry_kernel<<<nblocks(nb, 64), 64, 0, s>>>(tbb, nb, g.V, g.T, g.v2t_beg, g.v2t_tri, tgeo, eown);
+    sd_geometry_kernel<<<nblocks(nb, 64), 64, 0, s>>>(tbb, nb, g.V, g.T, g.v2t_beg, g.v2t_tri, tgeo, gexp, eown);
     check_launch("S / D geometry");
     for (int64_t a0 = 0; a0 < na; a0 += batch) {
         const int n = (int)std::min(batch, na - a0), npt = n * np;
-        double* cv = tab_.as<double>();
-        double* d = cv + 3 * nv * npt;
+        int2* cv = tab_.as<int2>();
+        double* d = reinterpret_cast<double*>(cv + 3 * nv * npt);
         double* l = d + nv * npt;
         double* prod = l + 3 * nb * npt;
         const unsigned gx = nblocks(npt, SD_THREADS);
@@ -454,10 +482,13 @@ void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, in
         sd_edge_kernel<<<dim3(gx, nblocks(nb, SD_E)), SD_THREADS, 0, s>>>(tbb, (int)nb, n, npt, order, g.T, vbb, tgeo,
                                                                           eown, d, l, prod);
         check_launch("S / D edges");
-        const dim3 grid(nblocks(n, 32), nblocks(nb, SD_THREADS / 32));
+        const dim3 grid(nblocks(n, 32), nblocks(nb, SD_WARPS));
+        // Triangles close to the batch's (the same part of the other mesh's numbering) take up to three times as long:
+        // their CTAs are started first.
+        const unsigned first = (unsigned)(a0 * grid.y / na);
         auto kern = wantS ? (dtmp ? sd_pair_kernel<true, true> : sd_pair_kernel<true, false>) : sd_pair_kernel<false, true>;
-        kern<<<grid, SD_THREADS, 0, s>>>(tbb, (int)nb, tab, a0, n, npt, order, same ? 1 : 0, coeff, g.T, vbb, tgeo, eown,
-                                         g.qrec, cv, d, l, prod, g.tpos, hm, ld, stmp, na, dtmp);
+        kern<<<grid, 32 * SD_WARPS, 0, s>>>(tbb, (int)nb, first, tab, a0, n, npt, order, same ? 1 : 0, coeff, g.T, vbb, tgeo, gexp,
+                                         eown, g.qrec, cv, d, l, prod, g.tpos, hm, ld, stmp, na, dtmp);
         check_launch("S / D pairs");
     }
 }
