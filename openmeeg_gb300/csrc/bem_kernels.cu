@@ -213,20 +213,20 @@ __device__ __forceinline__ int64_t lower_at(int64_t a, int64_t b, int64_t ld) {
 //   2. l[e][x] = (integral over the edge of 1/|x - y|) / length
 //      = 2 atanh(len / (d_a + d_b)) / len for every edge (1.5 per triangle instead
 //      of three logarithms each in S and in D: D's log((d_b + r_b.u)/(d_a + r_a.u))
-//      is the same integral), and (d_a + d_b)^2 - len^2 = 2 (d_a d_b + r_a.r_b);
+//      is the same integral), and (d_a +- d_b)^2 - len^2 = 2 (r_a.r_b +- d_a d_b);
 //   3. per (triangle, point): h = n.(p0 - x) and E_j = n.(r_j+1 x r_j+2) (linear in
 //      x; E_0 + E_1 + E_2 = 2A), half the solid angle
 //      w = atan(2 A h / (d0 d1 d2 + sum d_i r_j.r_k)), then
 //        S = sum_i E_opp(i) l_i - 2 h w,
 //        D_j = (w E_j + h/2 D_j+1.(sum_i D_i l_i)) / A, D_0 + D_1 + D_2 = 2 w,
-//      in 19 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
+//      in 18 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
 // About 26 FP64 operations per (triangle, point) for S and D together.  The square
 // roots, logarithms, arctangents, the weights of the rule and the linear forms h, E_j
 // run on the integer pipe (fixed64.cuh), which issues beside the FP64 operations: the
 // forms as inner products of 60-bit vectors, of the triangle and of x - p0 from the
 // table.  A head matrix of four layers (7020 triangles) took 67 ms in these kernels
 // with all of it in FP64 (75 operations), 34 with the linear forms in FP64 (35), now
-// 23.7: the pair kernel holds the FP64 pipe 84% busy, the distances likewise, and the
+// 22.5: the pair kernel holds the FP64 pipe 84% busy, the distances likewise, and the
 // edges (285 instructions each, 29% of the time) issue 66% of what the SM can.
 // Lanes run over the triangles a at the same rule point, so every table read is
 // coalesced, the triangle b is uniform in a warp, and the sum over the rule stays
@@ -331,13 +331,13 @@ __global__ void __launch_bounds__(SD_THREADS) sd_distance_kernel(const double* _
 }
 
 // Row 3 b + i, edge i (corners i, i + 1) of triangle b, of the rows that own their edge: l times the point's weight, and in
-// prod (d_a + d_b)^2 - len^2 = 2 (d_a d_b + r_a.r_b).
+// prod (d_a + d_b)^2 - len^2 = 2 (d_a d_b + r_a.r_b) and (d_a - d_b)^2 - len^2 = 2 (r_a.r_b - d_a d_b).
 __global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb, int na, int npt, int order,
                                                              const int32_t* __restrict__ T, int64_t vb,
                                                              const double* __restrict__ tgeo,
                                                              const int32_t* __restrict__ eown,
                                                              const double* __restrict__ d, double* __restrict__ l,
-                                                             double* __restrict__ prod) {
+                                                             double2* __restrict__ prod) {
     const int x = blockIdx.x * SD_THREADS + threadIdx.x;
     if (x >= npt) return;
     const double wr = c_rules[order][x / na][3];
@@ -352,7 +352,8 @@ __global__ void __launch_bounds__(SD_THREADS) sd_edge_kernel(int64_t tb, int nb,
             const double da = d[(int64_t)(tv[i] - vb) * npt + x], db = d[(int64_t)(tv[i == 2 ? 0 : i + 1] - vb) * npt + x];
             const double R = da + db;
             l[(int64_t)(3 * b + i) * npt + x] = fx::edge<true>(R, tgeo[b * (int64_t)TGEO + 19 + i], wm, we, wr);
-            prod[(int64_t)(3 * b + i) * npt + x] = fma(R, R, -tgeo[b * (int64_t)TGEO + 16 + i]);
+            const double q = tgeo[b * (int64_t)TGEO + 16 + i], D = da - db;
+            prod[(int64_t)(3 * b + i) * npt + x] = make_double2(fma(R, R, -q), fma(D, D, -q));
         }
     }
 }
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(32 * SD_WARPS, SD_CTAS) sd_pair_kernel(
     const int32_t* __restrict__ T, int64_t vb, const double* __restrict__ tgeo, const int4* __restrict__ gexp,
     const int32_t* __restrict__ eown, const double* __restrict__ qrec, const int2* __restrict__ cv,
     const double* __restrict__ d,
-    const double* __restrict__ l, const double* __restrict__ prod, const int32_t* __restrict__ tpos, double* hm,
+    const double* __restrict__ l, const double2* __restrict__ prod, const int32_t* __restrict__ tpos, double* hm,
     int64_t ld, double* stmp, int64_t n2, double* dtmp) {
     const unsigned by = blockIdx.y + first;
     const int b = (by < gridDim.y ? by : by - gridDim.y) * SD_WARPS + threadIdx.x / 32;
@@ -407,8 +408,8 @@ __global__ void __launch_bounds__(32 * SD_WARPS, SD_CTAS) sd_pair_kernel(
         const double num = fx::value60(fx::dot60(nx, ny, nz, x, y, z), ge.x + ce);   // 2A 2h
         const double E2 = fx::value60(fx::dot60(m0x, m0y, m0z, x, y, z), ge.y + ce);
         const double E1 = fx::value60(fx::dot60(m2x, m2y, m2z, x, y, z), ge.z + ce);
-        // 2 (d0 d1 d2 + sum d_i r_j.r_k) by the tabled 2 (d_j d_k + r_j.r_k)
-        const double den = fma(d0, fma(-4.0, d1 * d2, prod[x1 + o]), fma(d1, prod[x2 + o], d2 * prod[x0 + o]));
+        // 2 (d0 d1 d2 + sum d_i r_j.r_k) by the tabled 2 (r_j.r_k +- d_j d_k)
+        const double den = fma(d0, prod[x1 + o].y, fma(d1, prod[x2 + o].x, d2 * prod[x0 + o].x));
         const double wr = c_rules[order][k][3];
         const double w = fx::half_angle<true>(num, den, fx::mant(wr), (int)fx::expo(wr), wr);
         if (anyS) {   // E0 = 2A - E1 - E2
@@ -457,11 +458,11 @@ void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, in
     if (nb > (1 << 28)) throw Error(OMG_ERR_UNSUPPORTED, "S / D block too large");
     constexpr int NPTS[4] = {3, 6, 7, 16};
     const int np = NPTS[order];
-    // Points per batch: tables of about 1 GB, batches of equal size in multiples of 32 triangles (full warps).  A batch's
+    // Points per batch: tables of about 2 GB, batches of equal size in multiples of 32 triangles (full warps).  A batch's
     // kernels each end with a part-empty last wave, which costs more than tables that stay in L2 would save: the four-layer
-    // head takes 36.5 ms at 128 MB, 28.1 at 256, 25.4 at 512, 24.1 here, 23.5 at 2 GB.
-    const int64_t per_tri = (4 * nv + 6 * nb) * 8 * np;
-    const int64_t most = std::max<int64_t>(32, std::min<int64_t>((1024ll << 20) / per_tri, 4096) / 32 * 32);
+    // head takes 23.3 ms at 1 GB, 22.7 at 1.5, 22.5 here (with smaller tables 36.5 at 128 MB, 28.1 at 256, 25.4 at 512).
+    const int64_t per_tri = (4 * nv + 9 * nb) * 8 * np;
+    const int64_t most = std::max<int64_t>(32, std::min<int64_t>((2048ll << 20) / per_tri, 4096) / 32 * 32);
     const int64_t nbatch = (na + most - 1) / most, batch = std::min(na, ((na + nbatch - 1) / nbatch + 31) / 32 * 32);
     DevBuf geo((size_t)nb * (TGEO * 8 + 16 + 3 * 4), s), tab_((size_t)per_tri * batch, s);
     int4* gexp = geo.as<int4>();
@@ -471,10 +472,10 @@ void launch_SD_block(const DevGeom& g, int64_t tbb, int64_t tbe, int64_t vbb, in
     check_launch("S / D geometry");
     for (int64_t a0 = 0; a0 < na; a0 += batch) {
         const int n = (int)std::min(batch, na - a0), npt = n * np;
-        int2* cv = tab_.as<int2>();
+        double2* prod = tab_.as<double2>();
+        int2* cv = reinterpret_cast<int2*>(prod + 3 * nb * npt);
         double* d = reinterpret_cast<double*>(cv + 3 * nv * npt);
         double* l = d + nv * npt;
-        double* prod = l + 3 * nb * npt;
         const unsigned gx = nblocks(npt, SD_THREADS);
         sd_distance_kernel<<<dim3(gx, nblocks(nv, SD_V)), SD_THREADS, 0, s>>>(g.qrec, tab + a0, n, npt, g.V, vbb, (int)nv,
                                                                             cv, d);
