@@ -1467,11 +1467,13 @@ __device__ __forceinline__ void dsm_adaptive_warp(int kind, int order, int level
 // FP64: the first adaptive level of both integrands of every (dipole, triangle)
 // pair, 80 points.  What depends on the triangle alone is tabled once per
 // launch, by rule point (the triangle's 16 and each child's 16), lanes along
-// the triangles: the point relative to the centroid c, -3 n.(point - c), and
-// the weight times the P1 values 1 and 2.  With X = c - r0 (r0, q: the dipole)
-// a point then takes 25 FP64 operations for the potential and its three
-// P1-weighted derivatives, with one reciprocal square root, against ~110 for
-// two separate adaptive integrations, on a pipe that bounds the DipSourceMat.
+// the triangles: the point relative to the centroid c, the P1 values 1 and 2 and
+// -3 n.(point - c).  With X = c - r0 (r0, q: the dipole) a point then takes 19
+// FP64 operations for the potential and its three P1-weighted derivatives, with
+// the reciprocal square root and its product with the weight on the integer pipe
+// (fixed64.cuh), against ~110 for two separate adaptive integrations, on a pipe
+// that bounds the DipSourceMat: 500 dipoles on 12960 triangles take 7.5 ms,
+// with the root in FP64 (25 operations) 9.8.
 // A pair is settled here when |coarse - refined| <= tol |coarse| holds with a
 // margin far above the rounding; the others (and those decided by rounding) are
 // listed for dsm_fallback_kernel.
@@ -1499,9 +1501,9 @@ __global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, i
         o[0] = d.x;
         o[nt] = d.y;
         o[2 * nt] = d.z;
-        o[3 * nt] = -3.0 * dev::dot(n, d);
-        o[4 * nt] = r[3] * (inv_det * (c22 * a1 - c12 * a2));
-        o[5 * nt] = r[3] * (inv_det * (c11 * a2 - c12 * a1));
+        o[3 * nt] = inv_det * (c22 * a1 - c12 * a2);
+        o[4 * nt] = inv_det * (c11 * a2 - c12 * a1);
+        o[5 * nt] = -3.0 * dev::dot(n, d);   // (not 0: the rules' truncated digits do not sum to 1)
     }
 }
 
@@ -1515,17 +1517,14 @@ __device__ __forceinline__ void dsm_set(const double* __restrict__ tab, int64_t 
         const double rx = X.x + tab[0], ry = X.y + tab[nt], rz = X.z + tab[2 * nt];
         const double n2 = fma(rx, rx, fma(ry, ry, rz * rz));
         const double qr = fma(q.x, rx, fma(q.y, ry, q.z * rz));
-        double y;
-        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n2));
-        const double e = fma(-(n2 * y), y, 1.0);   // one third-order Newton step
-        y = fma(y * e, fma(0.375, e, 0.5), y);
-        const double y2 = y * y, y3 = y2 * y;
         const double w = c_rules[order][k][3];
-        acc[3] = fma(w, qr * y3, acc[3]);
-        const double g = fma(h3 + tab[3 * nt], qr * y2, qn) * y3;   // (q.n - 3 (q.r) (n.r) / r^2) / r^3
-        acc[0] = fma(w, g, acc[0]);
-        acc[1] = fma(tab[4 * nt], g, acc[1]);
-        acc[2] = fma(tab[5 * nt], g, acc[2]);
+        double wy;
+        const double y = fx::rsqrt64(n2, fx::mant(w), (int)fx::expo(w), w, wy), y2 = y * y, wy3 = y2 * wy;
+        acc[3] = fma(qr, wy3, acc[3]);
+        const double g = fma(h3 + tab[5 * nt], qr * y2, qn) * wy3;   // w (q.n - 3 (q.r) (n.r) / r^2) / r^3
+        acc[0] += g;
+        acc[1] = fma(tab[3 * nt], g, acc[1]);
+        acc[2] = fma(tab[4 * nt], g, acc[2]);
     }
     acc[0] -= acc[1] + acc[2];
 }
@@ -2296,22 +2295,19 @@ __global__ void dsm_vjp_kernel(int64_t dip0, int64_t ndc, const double* __restri
     const int points = (levels > 0 ? 4 : 1) * np;
     for (int j = 0, k = 0; j < points; ++j, k = k + 1 == np ? 0 : k + 1, tb += DSM_FL * nt) {
         const d3 x = dev::mk(X.x + tb[0], X.y + tb[nt], X.z + tb[2 * nt]);
-        const double t3 = h3 + tb[3 * nt];                         // -3 n.x
-        const double wl1 = tb[4 * nt], wl2 = tb[5 * nt], wk = c_rules[order][k][3];
+        const double l1 = tb[3 * nt], l2 = tb[4 * nt], t3 = h3 + tb[5 * nt], wk = c_rules[order][k][3];   // t3 = -3 n.x
         const double n2 = fma(x.x, x.x, fma(x.y, x.y, x.z * x.z));
         const double qx = fma(q.x, x.x, fma(q.y, x.y, q.z * x.z));
-        double y;
-        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n2));
-        const double e = fma(-(n2 * y), y, 1.0);
-        y = fma(y * e, fma(0.375, e, 0.5), y);
-        const double y2 = y * y, y3 = y2 * y, y5 = y3 * y2, u = qx * y2, tu = t3 * u;
-        const double g = (qn + tu) * y3, wy3 = wk * y3;
-        f[0] = fma(wk, g, f[0]);
-        f[1] = fma(wl1, g, f[1]);
-        f[2] = fma(wl2, g, f[2]);
+        double wy;
+        const double y = fx::rsqrt64(n2, fx::mant(wk), (int)fx::expo(wk), wk, wy);
+        const double y2 = y * y, wy3 = y2 * wy, u = qx * y2, tu = t3 * u;
+        const double g = (qn + tu) * wy3;
+        f[0] += g;
+        f[1] = fma(l1, g, f[1]);
+        f[2] = fma(l2, g, f[2]);
         f[3] = fma(qx, wy3, f[3]);
-        const double c1 = fma(W1, wl1, fma(W2, wl2, w.W[0] * wk)), m = c1 * y5, mt = m * t3;
-        An = fma(c1, y3, An);
+        const double c1 = fma(W1, l1, fma(W2, l2, w.W[0])) * wy3, m = c1 * y2, mt = m * t3;
+        An += c1;
         Sq += mt;
         Sn = fma(qx, m, Sn);
         const double ma = m * fma(-5.0, tu, qn3);
@@ -2876,7 +2872,7 @@ void launch_fold_to_reference(int64_t Nref, int64_t nvg, int64_t nP, const int64
 }  // namespace omg
 
 // Test hook (not part of the public header): the functions of fixed64.cuh on device arrays; which = 0 sqrt(a),
-// 1 2 atanh(b / a) / b, 2 atan2(b, a), with the weight wr where it is not 0.
+// 1 2 atanh(b / a) / b, 2 atan2(b, a), with the weight wr where it is not 0; 3 1 / sqrt(a), 4 the weight times it.
 namespace omg {
 __global__ void fixed64_eval_kernel(int which, int64_t n, const double* a, const double* b, double wr, double* out) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -2887,12 +2883,17 @@ __global__ void fixed64_eval_kernel(int which, int64_t n, const double* a, const
         out[i] = fx::sqrt64(a[i]);
     else if (which == 1)
         out[i] = wr != 0.0 ? fx::edge<true>(a[i], b[i], wm, we, wr) : fx::edge<false>(a[i], b[i], 0, 0, 0.0);
-    else
+    else if (which == 2)
         out[i] = wr != 0.0 ? fx::half_angle<true>(b[i], a[i], wm, we, wr) : fx::half_angle<false>(b[i], a[i], 0, 0, 0.0);
+    else {
+        double wy;
+        const double y = fx::rsqrt64(a[i], wm, we, wr, wy);
+        out[i] = which == 3 ? y : wy;
+    }
 }
 }  // namespace omg
 extern "C" int omg_internal_fixed64(int which, int64_t n, const double* a, const double* b, double wr, double* out) {
-    if (n <= 0 || which < 0 || which > 2) return OMG_ERR_INVALID;
+    if (n <= 0 || which < 0 || which > 4) return OMG_ERR_INVALID;
     omg::fixed64_eval_kernel<<<omg::nblocks(n, 128), 128>>>(which, n, a, b, wr, out);
     return cudaDeviceSynchronize() == cudaSuccess ? OMG_OK : OMG_ERR_CUDA;
 }

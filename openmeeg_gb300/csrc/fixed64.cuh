@@ -63,28 +63,47 @@ __device__ __forceinline__ bool rcp21(double x, uint32_t& ym, int& ye, uint64_t&
     return (unsigned)(s + 1) <= 1u;
 }
 
-// x y = sqrt(x) for y the hardware approximation of 1/sqrt(x), corrected by 1 + e / 2 + 3 e^2 / 8 from the residual
-// e = 1 - x y^2: sqrt(x) = (returned) 2^(xe + ye - 2046 - 61) of x = xm 2^(xe - 1023 - 63).  False where x is not normal.
-__device__ __forceinline__ bool sqrt_mant(double x, uint64_t xm, uint64_t& m, int& e) {
+// y = the hardware approximation of 1/sqrt(x) (21 bits, 2^-19) and c = 1 / (y sqrt(x)) in Q63: 1 + e / 2 + 3 e^2 / 8 from the
+// residual e = 1 - x y^2, x = xm 2^(xe - 1023 - 63).  False where x is not positive and normal.
+__device__ __forceinline__ bool rsqrt21(double x, uint64_t xm, uint32_t& ym, int& xe, int& ye, uint64_t& c) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const uint32_t xh = (uint32_t)__double2hiint(x), yh = (uint32_t)__double2hiint(y);
-    const uint32_t ym = (yh & 0xFFFFF) | 0x100000;
-    const int xe = (int)(xh >> 20), ye = (int)(yh >> 20);
+    ym = (yh & 0xFFFFF) | 0x100000;
+    xe = (int)(xh >> 20);
+    ye = (int)(yh >> 20);
     const int s = xe + 2 * ye - 3069 + 2;   // 0 .. 2: x y^2 = product / 2^(63 - s)
     const int64_t r = (int64_t)(0x8000000000000000ull - (mulh(xm, ((uint64_t)ym * ym) << 22) << (s & 3)));   // e in Q63
     const int e49 = (int)(r >> 14);
     const uint64_t q = (uint64_t)((int64_t)e49 * e49) >> 35;   // e^2 in Q63
-    m = mulh(0x8000000000000000ull + (uint64_t)(r >> 1) + ((3 * q) >> 3), mul21(xm, ym));
-    e = xe + ye - 1023 + 2;
+    c = 0x8000000000000000ull + (uint64_t)(r >> 1) + ((3 * q) >> 3);
     return (unsigned)s <= 2u;
 }
 
 // sqrt(x) (x > 0), to nearest up to 2^-59.
 __device__ __forceinline__ double sqrt64(double x) {
-    uint64_t m;
-    int e;
-    return sqrt_mant(x, mant(x), m, e) ? pack<false>(m, e) : sqrt(x);
+    uint32_t ym;
+    int xe, ye;
+    uint64_t c;
+    const uint64_t xm = mant(x);
+    return rsqrt21(x, xm, ym, xe, ye, c) ? pack<false>(mulh(c, mul21(xm, ym)), xe + ye - 1023 + 2) : sqrt(x);
+}
+
+// 1 / sqrt(x) (x > 0), to nearest up to 2^-58, and in wy w times it, w of mantissa wm and biased exponent we.
+__device__ __forceinline__ double rsqrt64(double x, uint64_t wm, int we, double w, double& wy) {
+    uint32_t ym;
+    int xe, ye;
+    uint64_t c;
+    const bool ok = rsqrt21(x, mant(x), ym, xe, ye, c);
+    const uint64_t m = mul21(c, ym);
+    double y = pack<false>(m, ye + 1);
+    wy = pack<false>(mulh(m, wm), ye + 1 + we - 1023 + 1);
+    if (__any_sync(__activemask(), !ok)) {
+        const double l = 1.0 / sqrt(x);
+        y = ok ? y : l;
+        wy = ok ? wy : w * l;
+    }
+    return y;
 }
 
 // Vectors in block fixed point: component = (h 2^30 + l) 2^(E - 60), |h| <= 2^30, |l| <= 2^29, one E per vector.

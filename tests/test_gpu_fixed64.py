@@ -44,6 +44,21 @@ def test_square_root(cuda, n):
         assert abs(mp.mpf(float(y)) / r - 1) <= TIGHT, float(x)
 
 
+@pytest.mark.parametrize("n", [1, 31, 400])
+@pytest.mark.parametrize("which", [3, 4])
+def test_reciprocal_square_root(cuda, n, which):
+    mp = pytest.importorskip("mpmath").mp
+    mp.dps = 60
+    wr = 0.027230314174434
+    a = _values(max(n, 8), np.random.default_rng(n))[:n]
+    for x, y in zip(a, _eval(which, a, a, wr)):
+        r = (mp.mpf(wr) if which == 4 else 1) / mp.sqrt(mp.mpf(float(x)))
+        assert abs(mp.mpf(float(y)) / r - 1) <= TIGHT, float(x)
+    with np.errstate(all="ignore"):
+        end = _eval(which, [0.0, np.inf, np.nan, -1.0], [0.0] * 4, wr)
+    assert np.isinf(end[0]) and end[1] == 0.0 and np.isnan(end[2:]).all()
+
+
 @pytest.mark.parametrize("which", [1, 2])
 @pytest.mark.parametrize("wr", [0.0, 0.027230314174434, 0.333333333333334])
 @pytest.mark.parametrize("lo,hi", [(1e-9, 2.0 ** -7), (0.99 / 16, 1.01 / 16), (0.99 / 8, 1.01 / 8), (0.2, 0.3),
