@@ -1468,18 +1468,21 @@ __device__ __forceinline__ void dsm_adaptive_warp(int kind, int order, int level
 // pair, 80 points.  What depends on the triangle alone is tabled once per
 // launch, by rule point (the triangle's 16 and each child's 16), lanes along
 // the triangles: the point relative to the centroid c, the P1 values 1 and 2 and
-// -3 n.(point - c).  With X = c - r0 (r0, q: the dipole) a point then takes 19
-// FP64 operations for the potential and its three P1-weighted derivatives, with
-// the reciprocal square root and its product with the weight on the integer pipe
-// (fixed64.cuh), against ~110 for two separate adaptive integrations, on a pipe
-// that bounds the DipSourceMat: 500 dipoles on 12960 triangles take 7.5 ms,
-// with the root in FP64 (25 operations) 9.8.
+// -3 n.(point - c).  With X = c - r0 (r0, q: the dipole) a point then takes 10
+// FP64 operations for the potential and its three P1-weighted derivatives:
+// r = X + (point - c), |r|^2, q.r, the reciprocal square root and its product with
+// the weight run on the integer pipe beside them (fixed64.cuh), in 60-bit vectors
+// with one exponent per pair.  Two separate adaptive integrations took ~110, on a
+// pipe that bounds the DipSourceMat: 500 dipoles on 12960 triangles take 4.3 ms,
+// with r and the products in FP64 (19 operations) 7.5, with the root as well (25) 9.8.
 // A pair is settled here when |coarse - refined| <= tol |coarse| holds with a
 // margin far above the rounding; the others (and those decided by rounding) are
 // listed for dsm_fallback_kernel.
 constexpr int DSM_FL = 6;   // table values per point
 
-__global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, int order, double* tab) {
+// FIXED: the point relative to c in block fixed point, its exponent per triangle in te.
+template <bool FIXED>
+__global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, int order, double* tab, int32_t* te) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= nt) return;
     const double* s = srec + t * SREC;
@@ -1491,6 +1494,10 @@ __global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, i
     const int np = c_nbpts[order];
     d3 P0 = R0, P1 = R1, P2 = R2;
     const int set = blockIdx.y;   // 0: the triangle; 1..4: its children
+    int em = 0;
+    for (const d3& R : {R0 - c, R1 - c, R2 - c})
+        em = max(em, max((int)fx::expo(R.x), max((int)fx::expo(R.y), (int)fx::expo(R.z))));
+    if (FIXED && set == 0) te[t] = em - 1022;
     if (set > 0) subtriangle(P0, P1, P2, set - 1);
     for (int k = 0; k < np; ++k) {
         const double* r = c_rules[order][k];
@@ -1498,28 +1505,94 @@ __global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, i
         const d3 d = x - c, v = x - R0;
         const double a1 = dev::dot(v, e10), a2 = dev::dot(v, e20);
         double* o = tab + (int64_t)(set * np + k) * DSM_FL * nt + t;
-        o[0] = d.x;
-        o[nt] = d.y;
-        o[2 * nt] = d.z;
+        if (FIXED) {   // (a rule's point is in the triangle, up to the digits of its barycentric coordinates)
+            int64_t* f = reinterpret_cast<int64_t*>(o);
+            f[0] = fx::fix60(d.x, max(em - (int)fx::expo(d.x), 0));
+            f[nt] = fx::fix60(d.y, max(em - (int)fx::expo(d.y), 0));
+            f[2 * nt] = fx::fix60(d.z, max(em - (int)fx::expo(d.z), 0));
+        } else {
+            o[0] = d.x;
+            o[nt] = d.y;
+            o[2 * nt] = d.z;
+        }
         o[3 * nt] = inv_det * (c22 * a1 - c12 * a2);
         o[4 * nt] = inv_det * (c11 * a2 - c12 * a1);
         o[5 * nt] = -3.0 * dev::dot(n, d);   // (not 0: the rules' truncated digits do not sum to 1)
     }
 }
 
-// One set of rule points: sums of w g (1, l1, l2) and w potential.
+// The dipole's part in block fixed point: X and q (limbs with 0 <= l < 2^30), the exponent E of X + (point - c), that of q,
+// and how far the table's points shift.
+struct DsmFix {
+    int64_t X[3];
+    int2 q[3];
+    int E, qe, down;
+    bool use;   // (finite, and far from the ends of the range)
+};
+__device__ __forceinline__ int2 dsm_limbs(int64_t i) { return make_int2((int)(i >> 30), (int)(i & 0x3FFFFFFF)); }
+__device__ __forceinline__ DsmFix dsm_fix(d3 X, d3 q, int te) {
+    DsmFix f;
+    const int ex = (int)fx::expo(X.x), ey = (int)fx::expo(X.y), ez = (int)fx::expo(X.z);
+    const int em = max(max(ex, max(ey, ez)), te + 1022) + 1;
+    f.E = em - 1022;
+    f.down = f.E - te;
+    f.X[0] = fx::fix60(X.x, em - ex);
+    f.X[1] = fx::fix60(X.y, em - ey);
+    f.X[2] = fx::fix60(X.z, em - ez);
+    const int qx = (int)fx::expo(q.x), qy = (int)fx::expo(q.y), qz = (int)fx::expo(q.z), qm = max(qx, max(qy, qz));
+    f.q[0] = dsm_limbs(fx::fix60(q.x, qm - qx));
+    f.q[1] = dsm_limbs(fx::fix60(q.y, qm - qy));
+    f.q[2] = dsm_limbs(fx::fix60(q.z, qm - qz));
+    f.qe = qm - 1022;
+    f.use = abs(f.E) < 400 && qm < 1900;
+    return f;
+}
+
+// One set of rule points: sums of w g (1, l1, l2) and w potential.  FIXED: r = X + (point - c), |r|^2 and q.r on the integer
+// pipe; a point closer than 2^-6 of the pair's scale (and X or q that are not finite) in FP64.
+template <bool FIXED>
 __device__ __forceinline__ void dsm_set(const double* __restrict__ tab, int64_t nt, int order, d3 X, d3 q, double qn,
-                                        double h3, double acc[4]) {
+                                        double h3, const DsmFix& F, double acc[4]) {
     acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
     const int np = c_nbpts[order];
 #pragma unroll 2
     for (int k = 0; k < np; ++k, tab += DSM_FL * nt) {
-        const double rx = X.x + tab[0], ry = X.y + tab[nt], rz = X.z + tab[2 * nt];
-        const double n2 = fma(rx, rx, fma(ry, ry, rz * rz));
-        const double qr = fma(q.x, rx, fma(q.y, ry, q.z * rz));
         const double w = c_rules[order][k][3];
-        double wy;
-        const double y = fx::rsqrt64(n2, fx::mant(w), (int)fx::expo(w), w, wy), y2 = y * y, wy3 = y2 * wy;
+        const uint64_t wm = fx::mant(w);
+        const int we = (int)fx::expo(w);
+        double qr, y, wy;
+        bool exact = true;
+        if (FIXED) {
+            const int64_t* d = reinterpret_cast<const int64_t*>(tab);
+            const int down = min(F.down, 63);
+            const int2 r[3] = {dsm_limbs(F.X[0] + (d[0] >> down)), dsm_limbs(F.X[1] + (d[nt] >> down)),
+                               dsm_limbs(F.X[2] + (d[2 * nt] >> down))};
+            exact = !fx::rnorm60(r, F.E, wm, we, y, wy) || !F.use;
+            const int64_t mid = (int64_t)F.q[0].x * r[0].y + (int64_t)F.q[0].y * r[0].x + (int64_t)F.q[1].x * r[1].y +
+                                (int64_t)F.q[1].y * r[1].x + (int64_t)F.q[2].x * r[2].y + (int64_t)F.q[2].y * r[2].x;
+            const int64_t hi = (int64_t)F.q[0].x * r[0].x + (int64_t)F.q[1].x * r[1].x + (int64_t)F.q[2].x * r[2].x;
+            qr = fx::value60(hi + (mid >> 30), F.qe + F.E);
+        }
+        if (!FIXED || __any_sync(__activemask(), exact)) {
+            double dx = tab[0], dy = tab[nt], dz = tab[2 * nt];
+            if (FIXED) {
+                const int te = F.E - F.down;
+                dx = fx::value60(__double_as_longlong(dx), te);
+                dy = fx::value60(__double_as_longlong(dy), te);
+                dz = fx::value60(__double_as_longlong(dz), te);
+            }
+            const double rx = X.x + dx, ry = X.y + dy, rz = X.z + dz;
+            const double n2 = fma(rx, rx, fma(ry, ry, rz * rz));
+            const double qr1 = fma(q.x, rx, fma(q.y, ry, q.z * rz));
+            double wy1;
+            const double y1 = fx::rsqrt64(n2, wm, we, w, wy1);
+            if (exact) {
+                qr = qr1;
+                y = y1;
+                wy = wy1;
+            }
+        }
+        const double y2 = y * y, wy3 = y2 * wy;
         acc[3] = fma(qr, wy3, acc[3]);
         const double g = fma(h3 + tab[5 * nt], qr * y2, qn) * wy3;   // w (q.n - 3 (q.r) (n.r) / r^2) / r^3
         acc[0] += g;
@@ -1723,7 +1796,7 @@ __global__ void dsm_kernel(int64_t dip0, int64_t ndc, const double* __restrict__
                            const int* __restrict__ dnb, const int* __restrict__ bmesh,
                            const int* __restrict__ binside, const double* __restrict__ dsigma, int order, int levels,
                            double tol, int64_t nv, int perm, double* out, int64_t ldo, double* p1tmp,
-                           const double* __restrict__ tab, int2* left, int* nleft) {
+                           const double* __restrict__ tab, const int32_t* __restrict__ te, int2* left, int* nleft) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t il = blockIdx.y;
     if (t >= nt || il >= ndc) return;
@@ -1741,7 +1814,8 @@ __global__ void dsm_kernel(int64_t dip0, int64_t ndc, const double* __restrict__
     const double qn = dev::dot(q, n), h3 = -3.0 * dev::dot(n, X), area = s[12];
     const int64_t set = (int64_t)c_nbpts[order] * DSM_FL * nt;
     double v[4];
-    dsm_set(tab + t, nt, order, X, q, qn, h3, v);
+    const DsmFix F = dsm_fix(X, q, te[t]);
+    dsm_set<true>(tab + t, nt, order, X, q, qn, h3, F, v);
     bool okv = true, okp = true;
     if (levels == 0) {
 #pragma unroll
@@ -1750,7 +1824,7 @@ __global__ void dsm_kernel(int64_t dip0, int64_t ndc, const double* __restrict__
         double ref[4] = {0.0, 0.0, 0.0, 0.0};
         for (int c = 1; c <= 4; ++c) {
             double a[4];
-            dsm_set(tab + c * set + t, nt, order, X, q, qn, h3, a);
+            dsm_set<true>(tab + c * set + t, nt, order, X, q, qn, h3, F, a);
 #pragma unroll
             for (int k = 0; k < 4; ++k) ref[k] = fma(0.25 * area, a[k], ref[k]);
         }
@@ -2140,11 +2214,13 @@ void launch_dsm(const DevGeom& g, int64_t dip0, int64_t ndc, const double* dip, 
         constexpr int NPTS[4] = {3, 6, 7, 16};
         const int nsets = levels > 0 ? 5 : 1;
         DevBuf tab((size_t)g.nt * nsets * NPTS[order] * DSM_FL * 8, s);
-        dsm_points_kernel<<<dim3(nblocks(g.nt, 128), nsets), 128, 0, s>>>(g.nt, g.srec, order, tab.as<double>());
+        DevBuf te((size_t)g.nt * sizeof(int32_t), s);
+        dsm_points_kernel<true><<<dim3(nblocks(g.nt, 128), nsets), 128, 0, s>>>(g.nt, g.srec, order, tab.as<double>(),
+                                                                                te.as<int32_t>());
         check_launch("DSM points");
         dsm_kernel<<<grid, 128, 0, s>>>(dip0, ndc, dip, g.nt, g.srec, tmesh, tidx_ref, barrier, orient, dom, maxb, dnb, bmesh,
                                         binside, dsigma, order, levels, tol, g.nvg, perm, out, ldo, p1tmp,
-                                        tab.as<double>(), left.as<int2>(), nleft.as<int>());
+                                        tab.as<double>(), te.as<int32_t>(), left.as<int2>(), nleft.as<int>());
         check_launch("DSM");
     }
     if (levels > 0) {
@@ -2287,7 +2363,7 @@ __global__ void dsm_vjp_kernel(int64_t dip0, int64_t ndc, const double* __restri
     const int np = c_nbpts[order];
     const int64_t set = (int64_t)np * DSM_FL * nt;
     double coarse[4];
-    if (levels > 0) dsm_set(tab + t, nt, order, X, q, qn, h3, coarse);
+    if (levels > 0) dsm_set<false>(tab + t, nt, order, X, q, qn, h3, DsmFix(), coarse);
     double f[4] = {0, 0, 0, 0};                                    // forward sums over the children
     double An = 0, Sq = 0, Sn = 0, Sy = 0;
     d3 Bx = dev::mk(0, 0, 0), Ax = Bx, Cx = Bx, Dx = Bx;
@@ -2432,7 +2508,7 @@ void launch_dsm_vjp(const DevGeom& g, int64_t dip0, int64_t ndc, const double* d
     DevBuf tab((size_t)g.nt * nsets * NPTS[order] * DSM_FL * 8, s), nleft(sizeof(int), s),
         left(levels > 0 ? (size_t)ndc * g.nt * sizeof(int2) : 0, s);
     OMG_CUDA(cudaMemsetAsync(nleft.p, 0, sizeof(int), s));
-    dsm_points_kernel<<<dim3(nblocks(g.nt, 128), nsets), 128, 0, s>>>(g.nt, g.srec, order, tab.as<double>());
+    dsm_points_kernel<false><<<dim3(nblocks(g.nt, 128), nsets), 128, 0, s>>>(g.nt, g.srec, order, tab.as<double>(), nullptr);
     check_launch("DSM points");
     dim3 grid(nblocks(g.nt, 128), (unsigned)ndc);
     dsm_vjp_kernel<<<grid, 128, 0, s>>>(dip0, ndc, dip, g.nt, g.srec, g.T, tmesh, tidx_ref, barrier, orient, dom, maxb,

@@ -129,6 +129,29 @@ __device__ __forceinline__ double value60(int64_t r, int e) {
     return pack<true>(m | 1, m ? e + 1026 : 0, (uint32_t)((uint64_t)r >> 63));
 }
 
+// 1 / sqrt(n) and w / sqrt(n), n = |r|^2 of r in block fixed point (h 2^30 + l with 0 <= l < 2^30, below 2^60; exponent E).
+// False where |r| < 2^(E - 6), for which 60 bits of r are too few, or |r| = 0.
+__device__ __forceinline__ bool rnorm60(const int2 r[3], int E, uint64_t wm, int we, double& y, double& wy) {
+    const int64_t hh = (int64_t)r[0].x * r[0].x + (int64_t)r[1].x * r[1].x + (int64_t)r[2].x * r[2].x;
+    const int64_t hl = (int64_t)r[0].x * r[0].y + (int64_t)r[1].x * r[1].y + (int64_t)r[2].x * r[2].y;
+    const int64_t ll = (int64_t)r[0].y * r[0].y + (int64_t)r[1].y * r[1].y + (int64_t)r[2].y * r[2].y;
+    const int z = max(__clz((int)hi32((uint64_t)hh)) - 2, 0);   // n 2^60 2^(-2 E) in Q(z): s < 2^63
+    const uint64_t s = ((uint64_t)hh << z) + (uint64_t)(hl >> (29 - min(z, 29))) + (uint64_t)(ll >> (60 - z));
+    const int up = __clz((int)hi32(s));
+    const uint64_t m = s << up;
+    // n = m 2^-63 2^x, x = 2 E + 3 - z - up
+    const int odd = (z + up + 1) & 1, xh = 2 * E + 3 - z - up - odd;
+    uint32_t ym;
+    int xe, ye;
+    uint64_t c;
+    rsqrt21(__hiloint2double((int)(((1022 + odd) << 20) + (int)(m >> 43)), (int)(m >> 11)), m, ym, xe, ye, c);
+    const uint64_t q = mul21(c, ym);
+    const int e = ye + 1 - xh / 2;
+    y = pack<false>(q, e);
+    wy = pack<false>(mulh(q, wm), e + we - 1022);
+    return z <= 10;
+}
+
 // atanh(z) / z - 1 of z in Q64 below 1/2, Q64: w f(w), w = z^2, f by the polynomial that interpolates it at the Chebyshev
 // nodes of [0, 1/4] (2^-66.7), in v = 1 - 4 w, where its terms alternate and every partial sum is positive.
 __device__ __forceinline__ uint64_t atanh_half(uint64_t z) {
