@@ -225,9 +225,9 @@ def run_reference(args):
 # ---------------------------------------------------------------------------
 # GPU arm
 # ---------------------------------------------------------------------------
-# executed FP64 flops per near pair (DADD + DMUL + 2 DFMA thread instructions) of near_pairs_kernel, ncu at config1
-# (launch 3: 93,224 pairs, 1.735 GFLOP)
-FP64_FLOPS_PER_NEAR_PAIR = 1.735e9 / 93224
+# executed FP64 flops per near pair (DADD + DMUL + 2 DFMA thread instructions) of near_pairs_kernel, ncu at config0
+# (its five launches: 84,550 pairs, 0.287 GFLOP)
+FP64_FLOPS_PER_NEAR_PAIR = 0.287e9 / 84550
 
 # DRAM bytes per launch measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum)
 # on a smaller head, per unit of the kernel's size (the summaries in profiles/ give
@@ -391,8 +391,8 @@ def roofline_entry(name, launches, ms, steps, N, k, nd, stats, peaks_, pipes):
                      "note": "FP32-pipe bound (rsqrt + FMA); peak: measured FP32 FMA instruction rate of this GPU"})
     elif name == "near_pairs":
         # FP64 analytic near-pair integrals (OperatorS, P1 single layer both ways at the 16 points of the rule):
-        # FP64 operations executed per near pair from an ncu capture (thread-level DADD + DMUL + 2 DFMA, the
-        # library's log/atan2/sqrt/division sequences included) against the nominal FP64 rate
+        # FP64 operations executed per near pair from an ncu capture (thread-level DADD + DMUL + 2 DFMA; the
+        # square roots, logarithms and angles run on the integer pipe) against the measured FP64 rate
         pairs = stats.get("_near_pairs", 0)
         flops = FP64_FLOPS_PER_NEAR_PAIR * pairs / per_step
         achieved = flops / t_launch
