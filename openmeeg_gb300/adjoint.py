@@ -175,10 +175,12 @@ class _Gain(torch.autograd.Function):
             (r0, r1), (c0, c1) = r, c
             P = torch.empty((k, r1 - r0), dtype=torch.float64, device=dev)
             _gemm(lib_ctx, 0, 0, r1 - r0, k, c1 - c0, 1.0, HM, r0 + c0 * N, N, Zc, c0, N, 0.0, P, 0, r1 - r0)
-            return float((P * Yc[:, r0:r1]).sum())
+            return (P * Yc[:, r0:r1]).sum()
 
         ndom = len(domains)
-        grad_sigma = np.zeros(ndom)
+        # terms (domain, factor, device scalar), read by the host in one copy at the end: a read per trace left the GPU
+        # idle for about 50 us each
+        terms = []
         for pr in pairs:
             common = _common(domains, orient, pr.m1, pr.m2)
             blocks = []
@@ -188,40 +190,44 @@ class _Gain(torch.autograd.Function):
                 blocks.append(("S", s1, s2, pr.cS))
             blocks.append(("N", rows_of(pr.m1, "V"), rows_of(pr.m2, "V"), pr.cN))
             for kind, r, c, coef in blocks:
-                t = trace(r, c) + (trace(c, r) if pr.m1 != pr.m2 else 0.0)
+                t = trace(r, c)
+                if pr.m1 != pr.m2:
+                    t = t + trace(c, r)
                 for dk in common:
                     if kind == "S":
                         dc = -pr.orientation * K / sig[dk] ** 2
                     else:
                         dc = pr.orientation * K
-                    grad_sigma[dk] -= (dc / coef) * t
+                    terms.append((dk, -(dc / coef), t))
         # P0 rows of D scale with 1/sigma of the dipole's domain
         dom = torch.empty(nd, dtype=torch.int32, device=dev)
         check(lib_ctx.lib.omg_dipole_domains_dev(lib_ctx.handle, geo.handle, _p(dip), nd, ctypes.c_void_p(dom.data_ptr())))
-        domh = dom.cpu().numpy()
+        sums = {}   # per interface: the products of each dipole
         for dk in range(ndom):
-            js = np.nonzero(domh == dk)[0]
-            if len(js) == 0 or sig[dk] == 0.0:
+            if sig[dk] == 0.0:
                 continue
-            acc = 0.0
             for b in domains[dk][1]:
                 rr = rows_of(abs(b) - 1, "T")
                 if rr is None:
                     continue
-                jj = torch.as_tensor(js, device=dev)
-                acc += float((U[jj, rr[0]:rr[1]] * Dc[jj, rr[0]:rr[1]]).sum())
-            grad_sigma[dk] -= acc / sig[dk]
+                if rr not in sums:
+                    sums[rr] = (U[:, rr[0]:rr[1]] * Dc[:, rr[0]:rr[1]]).sum(1)
+                terms.append((dk, -1.0 / sig[dk], torch.where(dom == dk, sums[rr], 0.0).sum()))
         # MEG rows carry the conductivity jumps: H2MM = sum_m jump_m F_m
         if nm:
             sq = st["squids"]
             for m in range(len(layout)):
                 F = torch.empty((N, nm), dtype=torch.float64, device=dev)         # column-major nm x N
                 check(lib_ctx.lib.omg_head2megmat_mesh_dev(lib_ctx.handle, geo.handle, _p(sq), nm, m, _p(F)))
-                t = float((F * Zc[ne:, :].T).sum())                               # sum_i F[i,:] . Z[:, ne+i]
+                t = (F * Zc[ne:, :].T).sum()                                      # sum_i F[i,:] . Z[:, ne+i]
                 for dk in range(ndom):
                     o = _mesh_orientation(domains, orient, dk, m)
                     if o:
-                        grad_sigma[dk] += o * t
+                        terms.append((dk, o, t))
+        grad_sigma = np.zeros(ndom)
+        if terms:
+            for (dk, factor, _), t in zip(terms, torch.stack([t for _, _, t in terms]).cpu().numpy()):
+                grad_sigma[dk] += factor * t
         # a zero conductivity (air) fixes the structure of the system (no
         # potential-jump unknowns outside); it is not a parameter
         grad_sigma[np.asarray(sig) == 0.0] = 0.0

@@ -219,8 +219,8 @@ __device__ __forceinline__ int64_t lower_at(int64_t a, int64_t b, int64_t ld) {
 //      w = atan(2 A h / (d0 d1 d2 + sum d_i r_j.r_k)), then
 //        S = sum_i E_opp(i) l_i - 2 h w,
 //        D_j = (w E_j + h/2 D_j+1.(sum_i D_i l_i)) / A, D_0 + D_1 + D_2 = 2 w,
-//      in 18 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
-// About 26 FP64 operations per (triangle, point) for S and D together.  The square
+//      in 16 operations with l_0 - l_1 and l_2 - l_1 (the D_i sum to zero).
+// About 25 FP64 operations per (triangle, point) for S and D together.  The square
 // roots, logarithms, arctangents, the weights of the rule and the linear forms h, E_j
 // run on the integer pipe (fixed64.cuh), which issues beside the FP64 operations: the
 // forms as inner products of 60-bit vectors, of the triangle and of x - p0 from the
