@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "digits.cuh"
+#include "fixed64.cuh"
 #include "handles.h"
 #include "tcgen05.cuh"
 
@@ -551,17 +552,20 @@ __global__ void __launch_bounds__(THREADS, 1)
 // CTA.  A warp's FP64 instruction takes its quarter of the SM 64 cycles, however few lanes take part, so both halves are
 // laid out for few instructions per warp:
 //  * every CTA factors the diagonal block itself (cheaper than a launch that only one SM works on).  Warp 0 runs the
-//    serial chain, five FP64 instructions per column (update of the next column, its pivot's reciprocal, the column
-//    times it): a_ik <- a_ik - u_i t_k with u the column as it stands and t = u / a_jj; the other warps update the rest
-//    of the triangle beside it (packed by columns: one run of entries over all lanes).  The square roots come last;
-//  * a warp then solves 8 rows, four lanes per row with every fourth column: the entry solved last goes to the row's
-//    lanes by a shuffle and is removed from the later ones with the same t; the results are scaled at the end.
-// A 64-column version in two launches took 39 + 28 us for 64 columns, this one ~2 x 14 us.
+//    serial chain, one FP64 instruction per column (the update of the next column) and the column over its pivot on the
+//    integer pipe: a_ik <- a_ik - u_i t_k with u the column as it stands and t = u / a_jj; the other seven warps update
+//    the rest of the triangle beside it (packed by columns: one run of entries over all lanes; with three warps the first
+//    columns waited for them).  The square roots come last;
+//  * four of the warps then solve 8 rows each, four lanes per row with every fourth column: the entry solved last goes to
+//    the row's lanes by a shuffle and is removed from the later ones with the same t; the results are scaled at the end.
+// A 64-column version in two launches took 39 + 28 us for 64 columns, four warps with the reciprocals in FP64 27 us for 32
+// (between events), this one 24.
 // The factored block goes to Ld (other CTAs still read it in A); place_diagonal_kernel puts the blocks into A at the end.
 // ---------------------------------------------------------------------------
 constexpr int NBD = 32;
+constexpr int PANEL_WARPS = 8;   // 4: solver of N = 6646 19.4 ms, 6: 18.8, 8: 18.5, 12: 18.4
 
-__global__ void __launch_bounds__(128) panel32_kernel(const double* A, int64_t lda, int n, int64_t m, double* P, double* Ld,
+__global__ void __launch_bounds__(32 * PANEL_WARPS) panel32_kernel(const double* A, int64_t lda, int n, int64_t m, double* P, double* Ld,
                                                       int* err, int64_t* err_col, int64_t col_offset) {
     constexpr int NE = NBD * (NBD + 1) / 2;
     __shared__ double U[NE];                     // the triangle, packed by columns
@@ -572,7 +576,7 @@ __global__ void __launch_bounds__(128) panel32_kernel(const double* A, int64_t l
     auto off = [](int j) { return j * NBD - j * (j - 1) / 2; };
     pdl_wait();
     pdl_next();
-    for (int j = warp; j < NBD; j += 4) {
+    for (int j = warp; j < NBD; j += PANEL_WARPS) {
         const int i = lane;
         if (i >= j) {
             const int e = off(j) + i - j;
@@ -584,7 +588,7 @@ __global__ void __launch_bounds__(128) panel32_kernel(const double* A, int64_t l
     // this CTA's rows, on their way while the block is factored
     const int g = lane & 3;
     const int64_t row = (int64_t)blockIdx.x * 32 + warp * 8 + lane / 4;
-    const bool live = row < m;
+    const bool live = warp < 4 && row < m;
     double* p = P + (live ? row : 0) + (int64_t)g * lda;
     double x[NBD / 4];
 #pragma unroll
@@ -596,11 +600,16 @@ __global__ void __launch_bounds__(128) panel32_kernel(const double* A, int64_t l
         const bool good = bits > 0 && bits <= 0x7FF0000000000000ll;   // d > 0, off the FP64 pipe
         bad = good ? bad : min(bad, j);
         const double d = __longlong_as_double(good ? bits : 0x3FF0000000000000ll);
-        double y;   // 1 / d: the hardware approximation and one third-order Newton step
-        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-        const double e = fma(-d, y, 1.0);
-        y = fma(fma(e, e, e), y, y);
-        const double t = v * y;
+        // v / d on the integer pipe (rounded once): the chain of dependent FP64 operations it takes there, three for the
+        // reciprocal's Newton step and the product, is twice as long
+        uint32_t ym;
+        int ye;
+        uint64_t c;
+        const bool ok = fx::rcp21(d, ym, ye, c);
+        const int ve = (int)fx::expo(v);
+        double t = fx::pack<true>(fx::mulh(fx::mul21(fx::mant(v), ym), c) | 1, ve ? ve + ye - 1023 + 2 : 0,
+                                  (uint32_t)__double2hiint(v) >> 31);
+        t = ve == 0x7FF || !ok ? __longlong_as_double(0x7FF8000000000000ll) : t;
         if (lane > 0 && j + lane < NBD) T[j][j + lane] = t;
     };
     if (warp == 0) pivot(0, U[lane]);
@@ -616,7 +625,7 @@ __global__ void __launch_bounds__(128) panel32_kernel(const double* A, int64_t l
             pivot(j + 1, v);
         } else {
 #pragma unroll 2
-            for (int e = e2 + tid - 32; e < NE; e += 96) {
+            for (int e = e2 + tid - 32; e < NE; e += 32 * (PANEL_WARPS - 1)) {
                 const int q = ik[e];
                 U[e] = fma(-u[q & 255], t[q >> 8], U[e]);
             }
@@ -635,7 +644,7 @@ __global__ void __launch_bounds__(128) panel32_kernel(const double* A, int64_t l
     }
     __syncthreads();
     if (blockIdx.x == 0)
-        for (int j = warp; j < NBD; j += 4) Ld[lane + j * NBD] = lane >= j ? U[off(j) + lane - j] * rs[j] : 0.0;
+        for (int j = warp; j < NBD; j += PANEL_WARPS) Ld[lane + j * NBD] = lane >= j ? U[off(j) + lane - j] * rs[j] : 0.0;
     if (!__any_sync(0xffffffffu, live)) return;
 #pragma unroll
     for (int j = 0; j < NBD; ++j) {
@@ -1084,7 +1093,7 @@ void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, in
 void panel32(double* A, int64_t lda, int w, int64_t m, double* Ld, int* err, int64_t* err_col, int64_t col_offset,
              cudaStream_t s) {
     ProfScope prof_("f64_panel", s);
-    f64d::launch(f64d::panel32_kernel, dim3((unsigned)std::max<int64_t>(1, (m + 31) / 32)), 128, 0, s, (const double*)A, lda,
+    f64d::launch(f64d::panel32_kernel, dim3((unsigned)std::max<int64_t>(1, (m + 31) / 32)), 32 * f64d::PANEL_WARPS, 0, s, (const double*)A, lda,
                  w, m, A + w, Ld, err, err_col, col_offset);
     f64d::check("FP64 panel");
 }
