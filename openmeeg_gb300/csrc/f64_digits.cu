@@ -556,7 +556,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 //    integer pipe: a_ik <- a_ik - u_i t_k with u the column as it stands and t = u / a_jj; the other seven warps update
 //    the rest of the triangle beside it (packed by columns: one run of entries over all lanes; with three warps the first
 //    columns waited for them).  The square roots come last;
-//  * four of the warps then solve 8 rows each, four lanes per row with every fourth column: the entry solved last goes to
+//  * four of the warps then solve 8 rows each (4 or 2 where m is small), four lanes per row with every fourth column (8 or
+//    16, with every 8th or 16th): the entry solved last goes to
 //    the row's lanes by a shuffle and is removed from the later ones with the same t; the results are scaled at the end.
 // A 64-column version in two launches took 39 + 28 us for 64 columns, four warps with the reciprocals in FP64 27 us for 32
 // (between events), this one 24.
@@ -565,6 +566,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 constexpr int NBD = 32;
 constexpr int PANEL_WARPS = 8;   // 4: solver of N = 6646 19.4 ms, 6: 18.8, 8: 18.5, 12: 18.4
 
+template <int LPR>   // lanes per row
 __global__ void __launch_bounds__(32 * PANEL_WARPS) panel32_kernel(const double* A, int64_t lda, int n, int64_t m, double* P, double* Ld,
                                                       int* err, int64_t* err_col, int64_t col_offset) {
     constexpr int NE = NBD * (NBD + 1) / 2;
@@ -586,13 +588,13 @@ __global__ void __launch_bounds__(32 * PANEL_WARPS) panel32_kernel(const double*
         T[j][i] = 0.0;
     }
     // this CTA's rows, on their way while the block is factored
-    const int g = lane & 3;
-    const int64_t row = (int64_t)blockIdx.x * 32 + warp * 8 + lane / 4;
+    const int g = lane % LPR;
+    const int64_t row = (int64_t)blockIdx.x * (128 / LPR) + warp * (32 / LPR) + lane / LPR;
     const bool live = warp < 4 && row < m;
     double* p = P + (live ? row : 0) + (int64_t)g * lda;
-    double x[NBD / 4];
+    double x[NBD / LPR];
 #pragma unroll
-    for (int i = 0; i < NBD / 4; ++i) x[i] = live ? p[(int64_t)(4 * i) * lda] : 0.0;
+    for (int i = 0; i < NBD / LPR; ++i) x[i] = live ? p[(int64_t)(LPR * i) * lda] : 0.0;
     __syncthreads();
     int bad = NBD;   // warp 0: the first column with a pivot of the wrong sign
     auto pivot = [&](int j, double v) {   // warp 0: column j is final, v its entry of row j + lane
@@ -648,13 +650,13 @@ __global__ void __launch_bounds__(32 * PANEL_WARPS) panel32_kernel(const double*
     if (!__any_sync(0xffffffffu, live)) return;
 #pragma unroll
     for (int j = 0; j < NBD; ++j) {
-        const double xj = __shfl_sync(0xffffffffu, x[j / 4], (lane & ~3) | (j & 3));
+        const double xj = __shfl_sync(0xffffffffu, x[j / LPR], (lane & ~(LPR - 1)) | (j & (LPR - 1)));
 #pragma unroll
-        for (int i = j / 4 + (j % 4 == 3 ? 1 : 0); i < NBD / 4; ++i) x[i] = fma(-xj, T[j][4 * i + g], x[i]);
+        for (int i = j / LPR + (j % LPR == LPR - 1 ? 1 : 0); i < NBD / LPR; ++i) x[i] = fma(-xj, T[j][LPR * i + g], x[i]);
     }
     if (!live) return;
 #pragma unroll
-    for (int i = 0; i < NBD / 4; ++i) p[(int64_t)(4 * i) * lda] = x[i] * rs[4 * i + g];
+    for (int i = 0; i < NBD / LPR; ++i) p[(int64_t)(LPR * i) * lda] = x[i] * rs[LPR * i + g];
 }
 
 // C (m x nc) -= X Y^T, X the m x 32 sub-panel at the rows of C and Y its first nc rows (C starts at row and column
@@ -936,6 +938,17 @@ __global__ void sum_segments_kernel(int64_t M, int64_t N, int64_t kdim, int nseg
     }
 }
 
+int64_t sm_count() {
+    static int n_sm = 0;
+    if (!n_sm) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        n_sm = n > 0 ? n : 1;
+    }
+    return n_sm;
+}
+
 }  // namespace f64d
 
 
@@ -962,14 +975,12 @@ static void digit_product(int64_t M, int64_t Nc, int kpad, const void* A, int64_
     ProfScope prof_(name, s);
     static int n_sm = 0;
     if (!n_sm) {
+        const int n = (int)f64d::sm_count();
         for (auto k : {f64d::digit_update_kernel<128, true>, f64d::digit_update_kernel<64, true>, f64d::digit_update_kernel<32, true>,
                        f64d::digit_update_kernel<128, false>, f64d::digit_update_kernel<64, false>,
                        f64d::digit_update_kernel<32, false>})
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, f64d::SMEM_BYTES);
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        n_sm = n > 0 ? n : 1;
+        n_sm = n;
     }
     // Tile width: narrow tiles put a short product (a solve's right-hand sides, the next panel) on more SMs and leave a
     // shorter last epilogue, wide ones feed the tensor cores better.  Cycles of a tile's products (a K = 16 step takes
@@ -1093,8 +1104,15 @@ void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, in
 void panel32(double* A, int64_t lda, int w, int64_t m, double* Ld, int* err, int64_t* err_col, int64_t col_offset,
              cudaStream_t s) {
     ProfScope prof_("f64_panel", s);
-    f64d::launch(f64d::panel32_kernel, dim3((unsigned)std::max<int64_t>(1, (m + 31) / 32)), 32 * f64d::PANEL_WARPS, 0, s, (const double*)A, lda,
-                 w, m, A + w, Ld, err, err_col, col_offset);
+    // Few rows: more lanes per row, fewer rows per CTA, while one CTA per SM holds them all (the rows' substitution takes a
+    // quarter of the SM 144 / 80 / 48 FP64 instructions at 4 / 8 / 16 lanes per row: the smallest gain's 36 sub-panels 0.85 ->
+    // 0.71 ms).  With more rows than that, CTAs that share an SM would repeat the triangle.
+    const int64_t sms = f64d::sm_count();
+    const int lpr = m <= 8 * sms ? 16 : m <= 16 * sms ? 8 : 4;
+    auto kern = lpr == 16 ? f64d::panel32_kernel<16> : lpr == 8 ? f64d::panel32_kernel<8> : f64d::panel32_kernel<4>;
+    const int64_t rows = 128 / lpr;
+    f64d::launch(kern, dim3((unsigned)std::max<int64_t>(1, (m + rows - 1) / rows)), 32 * f64d::PANEL_WARPS, 0, s,
+                 (const double*)A, lda, w, m, A + w, Ld, err, err_col, col_offset);
     f64d::check("FP64 panel");
 }
 

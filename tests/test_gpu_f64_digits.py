@@ -106,6 +106,27 @@ def test_panel(cuda, w, m):
     assert np.linalg.norm(W @ L.T - P) <= 2.0**-52 * w * np.linalg.norm(W) * np.linalg.norm(L)
 
 
+@pytest.mark.parametrize("per_sm,more", [(8, 0), (8, 1), (16, 0), (16, 3), (32, 5)])
+def test_panel_rows_per_cta(cuda, per_sm, more):
+    """Both sides of the numbers of rows at which a row takes 16, 8 and 4 lanes."""
+    import torch
+    m = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + more
+    rng = np.random.default_rng(m)
+    X = rng.standard_normal((32, 32))
+    A, P = X @ X.T + 32 * np.eye(32), rng.standard_normal((m, 32))
+    L, W, status, _ = _panel(cuda, A, P)
+    assert status == 0
+    # the substitution's backward error, w eps
+    assert np.linalg.norm(W @ L.T - P) <= 2.0**-52 * 32 * np.linalg.norm(W) * np.linalg.norm(L)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_panel_reports_entries_that_are_not_finite(cuda, value):
+    A = 4.0 * np.eye(32)
+    A[12, 5] = A[5, 12] = value
+    assert _panel(cuda, A, np.ones((3, 32)))[2] == -3
+
+
 def test_panel_reports_the_wrong_sign(cuda):
     A = np.eye(32)
     A[9, 9] = -1.0
