@@ -1270,8 +1270,8 @@ void dsm_internal(omg_geometry g, const double* dip, int64_t nd, const omg_integ
         dperm = 1;
     }
     DevBuf sa((size_t)nd * g->h.nmesh * 8, s), dom((size_t)nd * sizeof(int), s);
-    // closed meshes, one per interface: only angles within 1 of 2 pi are summed in FP64 (the lookup asks which side of 2 pi a
-    // sum is on; away from it FP32 answers the same)
+    // closed meshes, one per interface: the lookup asks only which side of 2 pi a mesh's sum is on, so FP32 screens the sums
+    // and those it cannot be sure of are taken in FP64
     bool closed = true;
     for (const auto& f : g->h.ifaces) closed = closed && f.size() == 1;
     launch_mesh_solid_angles(dip, 6, nd, g->h.nmesh, g->tbeg, g->d.srec, sa.as<double>(), s,

@@ -1249,10 +1249,16 @@ __global__ void mesh_solid_angles_kernel(const double* __restrict__ pts, int64_t
     }
 }
 
-// Same, screened in FP32 for the domain lookup of the mixed path: a closed
-// mesh subtends 0 or +-4 pi, so only the classification |sum| > 2 pi matters;
-// a sum within 1 of 2 pi (a point at the surface, where FP32 could tip the
-// test) is recomputed in FP64, so the domains are those of the FP64 sums.
+// Same, screened in FP32 for the domain lookup: a closed mesh subtends 0 or
+// +-4 pi, so only the classification |sum| > 2 pi matters.  The FP64 sum is
+// taken where FP32 could tip that test:
+//  * a triangle whose angle FP32 cannot be sure of.  With u = 2^-24 the errors
+//    are at most 7 u 2A|r0| in num and 56 u d0 d1 d2 in den, together e below;
+//    the angle is within 2% when |num| or den exceeds 100 e.  With den < 0 and a
+//    smaller |num| (a point just off the triangle) even its sign is open, which
+//    moves the sum by 4 pi.  FP64 drops the angle when |num| < 1e-10, so here
+//    |num| has to be clear of that as well, or the angle below 2e-6 either way;
+//  * a sum within 1 of 2 pi.
 __global__ void mesh_solid_angles_screened_kernel(const double* __restrict__ pts, int64_t pstride, int nmesh,
                                                   const int64_t* __restrict__ tbeg, const double* __restrict__ srec,
                                                   double* out) {
@@ -1262,6 +1268,7 @@ __global__ void mesh_solid_angles_screened_kernel(const double* __restrict__ pts
     const d3 p = dev::ld3(pts + i * pstride);
     for (int m = 0; m < nmesh; ++m) {
         float acc = 0.f;
+        bool doubt = false;
         for (int64_t t = tbeg[m] + threadIdx.x; t < tbeg[m + 1]; t += blockDim.x) {
             const double* s = srec + t * SREC;
             const float ax = (float)(s[0] - p.x), ay = (float)(s[1] - p.y), az = (float)(s[2] - p.z);
@@ -1269,21 +1276,26 @@ __global__ void mesh_solid_angles_screened_kernel(const double* __restrict__ pts
             const float cx = (float)(s[6] - p.x), cy = (float)(s[7] - p.y), cz = (float)(s[8] - p.z);
             const float da = sqrtf(ax * ax + ay * ay + az * az), db = sqrtf(bx * bx + by * by + bz * bz),
                         dc = sqrtf(cx * cx + cy * cy + cz * cz);
-            const float num = 2.f * (float)s[12] * (ax * (float)s[9] + ay * (float)s[10] + az * (float)s[11]);
-            const float den = da * db * dc + da * (bx * cx + by * cy + bz * cz) + db * (cx * ax + cy * ay + cz * az) +
+            const float A2 = 2.f * (float)s[12], prod = da * db * dc;
+            const float num = A2 * (ax * (float)s[9] + ay * (float)s[10] + az * (float)s[11]);
+            const float den = prod + da * (bx * cx + by * cy + bz * cz) + db * (cx * ax + cy * ay + cz * az) +
                               dc * (ax * bx + ay * by + az * bz);
-            acc += 2.f * atan2f(num, den);
+            const float e = 4e-6f * prod + 5e-7f * (A2 * da), mag = fabsf(num);
+            if (mag > 1e-10f + 100.f * e || den > 1e-4f + 100.f * e)
+                acc += 2.f * atan2f(num, den);
+            else if (!(mag < 1e-10f - e))   // (so are infinities and NaN)
+                doubt = true;
         }
         redf[threadIdx.x] = acc;
-        __syncthreads();
+        doubt = __syncthreads_or(doubt);
         for (int w = blockDim.x / 2; w > 0; w >>= 1) {
             if (threadIdx.x < w) redf[threadIdx.x] += redf[threadIdx.x + w];
             __syncthreads();
         }
         const float sum = redf[0];
         __syncthreads();
-        if (fabsf(fabsf(sum) - 6.2831853f) > 1.f && sum == sum) {   // clear of the 2 pi boundary
-            if (threadIdx.x == 0) out[i * nmesh + m] = fabsf(sum) < 3.1415927f ? 0.0 : (sum > 0 ? 1.0 : -1.0) *
+        if (!doubt && fabsf(fabsf(sum) - 6.2831853f) > 1.f && sum == sum) {   // clear of the 2 pi boundary
+            if (threadIdx.x == 0) out[i * nmesh + m] = fabsf(sum) < 6.2831853f ? 0.0 : (sum > 0 ? 1.0 : -1.0) *
                                                                                           12.566370614359172;
             continue;
         }
