@@ -1033,9 +1033,16 @@ void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, in
               const std::vector<std::pair<int64_t, int64_t>>* ranges) {
     using namespace f64d;
     if (M <= 0 || N <= 0) return;
+    if (ranges && ranges->size() > (size_t)MAXRANGES) {   // (a kernel parameter lists MAXRANGES of them)
+        for (size_t q = 0; q < ranges->size(); q += MAXRANGES) {
+            const std::vector<std::pair<int64_t, int64_t>> part(ranges->begin() + q,
+                                                                ranges->begin() + std::min(q + MAXRANGES, ranges->size()));
+            gemm_f64(M, N, 0, alpha, A, lda, ta, B, ldb, tb, q == 0 ? beta : 1.0, C, ldc, err, s, &part);
+        }
+        return;
+    }
     RowRanges rr{};
     if (ranges) {
-        if (ranges->size() > (size_t)MAXRANGES) throw Error(OMG_ERR_UNSUPPORTED, "GEMM: too many row ranges");
         K = 0;
         for (const auto& r : *ranges) {
             rr.beg[rr.n] = r.first;
