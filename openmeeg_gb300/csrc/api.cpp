@@ -2224,6 +2224,7 @@ int omg_solver_solve_dev(omg_solver sv, double* b, int64_t ldb, int64_t nrhs) {
         OMG_REQUIRE(sv && b, "null argument");
         OMG_REQUIRE(ldb >= sv->geo->h.N && nrhs >= 0, "bad right-hand side shape");
         set_device(sv->ctx);
+        reset_err(sv->ctx);
         cudaStream_t s = sv->ctx->stream;
         const int64_t N = sv->N, nv = sv->geo->h.nvg, nP = sv->nP, nPt = sv->geo->d.nPt;
         // reference -> internal numbering: triangle rows [nv, nv+nPt) first, zero padding, then vertices [0, nv)
@@ -2239,7 +2240,7 @@ int omg_solver_solve_dev(omg_solver sv, double* b, int64_t ldb, int64_t nrhs) {
         solver_solve_internal(sv, x, N, nrhs);
         rows(b + nv, ldb, x, N, nPt);
         rows(b, ldb, x + nP, N, nv);
-        OMG_CUDA(cudaStreamSynchronize(s));
+        check_err(sv->ctx, "solve");   // (a bounded wait of the sweeps that gave up)
     });
 }
 
@@ -2429,3 +2430,6 @@ int omg_gain_host(omg_context ctx, omg_geometry geo, int32_t precision, const om
 }
 
 }  // extern "C"
+
+// Test hook (not part of the public header): the context's device-side status word.
+extern "C" int* omg_internal_status_dev(omg_context ctx) { return ctx ? ctx->d_err : nullptr; }
