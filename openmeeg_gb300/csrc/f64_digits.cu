@@ -1,35 +1,48 @@
-// FP64-accurate products on the bf16 tensor cores (sm_103a, tcgen05) for the FP64
-// factorization: C -= A B^T with the rows of A and B cut into exact fixed-point
-// digits (the scheme of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012):
+// FP64-accurate products on the bf16 tensor cores (sm_103a, tcgen05), for the FP64
+// factorization, its solves and general products: the rows of A and B are cut into
+// exact fixed-point digits (the scheme of Ozaki, Ogita, Oishi and Rump, Numer.
+// Algorithms 59, 2012):
 //
-//   A_ik = 2^(e_i) sum_{s=1..7} 2^(-8 s) a_s,ik,  |a_s| <= 128 integers (56 bits below the row's maximum),
-//   (A B^T)_ij = 2^(e_i + e_j) sum_l 2^(-8 l) v_l,  v_l = sum_{s+t=l} sum_k a_s,ik b_t,jk,  l = 2..9 (34 pairs).
+//   A_ik = 2^(e_i) sum_{s=1..ND} 2^(-8 s) a_s,ik,  a_s integers, |a_s| <= 128,
+//   (A B^T)_ij = 2^(e_i + e_j) sum_l 2^(-8 l) v_l,  v_l = sum_{s+t=l} sum_k a_s,ik b_t,jk.
 //
 // FP64's own pipe does 1.06 TFLOP/s here, the bf16 tensor cores 1.9 PFLOP/s, so 34
-// products are still ~50 times cheaper.  The seven digits hold more than FP64's 53
-// bits of the largest entry of a row, and the dropped pairs (l >= 10) are below 2^-58
-// of row maximum times row maximum each; with l = 9 left out (28 pairs) a solve
-// against a head matrix was three times further off than FP64 products, with it
-// it is level with them (N = 1126 and 4486, cond 4e3).
+// products are still ~50 times cheaper.
 //
-// Sums: a product of two digits is at most 2^14, K is at most 256, so the sums of the
-// levels 2..5 (1 to 4 pairs) stay within 2^24 and are exact in the FP32 accumulators.
-// The levels 6..9 weigh 2^-32 and less of the leading one; level 6 (5 pairs) is exact
-// up to the same limit, and 7, 8 and 9 share one accumulator (the digit planes carry
-// their power of two, so a product already has its level's scale): what FP32 rounds
-// there is below 2^-52 of the leading term's unit.
+// Updates of the factorization and the solves: ND = 7, levels l = 2..9 (34 pairs), an
+// entry held to 2^-57 of twice its row's maximum.  |L_i| <= sqrt(a_ii) for the rows of
+// a factor, so what is left out is of the size of the factorization's own rounding.
+// With l = 9 left out (28 pairs) a solve against a head matrix was three times further
+// off than FP64 products.
 //
-// One output tile of 128 x TN is three units of work, each with two accumulators
-// (a half of TMEM's 512 columns, the units alternate between the halves, so a unit's
-// products run while the one before is drained): levels {4, 5}, {2, 3}, {6, 7-9}.
+// General products: ND = 8, levels 2..10 (43 pairs), an entry held to 2^-65 of four
+// times the maximum of its row's segment of 256.  Rows of potentials and of sources have
+// peaks 100 and more above most of their entries, so with seven digits most entries of a
+// gain had a larger error bound than K 2^-53 sum |a||b|, FP64's.  With eight the
+// errors are below those of FP64 multiply-adds.  For operands graded beyond that, the
+// product of the leading digits' magnitudes (one more pair) bounds sum |a||b| from below,
+// and an entry whose bound is above FP64's is summed in FP64.
+//
+// Sums: a product of two digits is at most 2^14, K is at most 256, so the levels up to
+// the sixth (general: the eighth) are sums of integers within 2^24, or twice that where
+// all digits are as large as they can be, and exact in the FP32 accumulators.  The levels
+// 7-9 (9 and 10) share one (the digit planes carry their power of two, so a product
+// already has its level's scale): FP32 rounds there by about 2^-58 (2^-74) of the
+// exponents' unit in all.
+//
+// One output tile of 128 x TN is three units of work (general: five), each with two
+// accumulators (a half of TMEM's 512 columns, the units alternate between the halves, so
+// a unit's products run while the one before is drained): levels {6, 7-9}, {4, 5},
+// {2, 3} (general: the magnitudes, {8-10}, {6, 7}, {4, 5}, {2, 3}).
 // Within a unit, the K chunks of 64 stream their digit tiles through a ring of 13
-// slots of 16 KB, each digit tile of A and of B loaded once per chunk: for s = 1..7
-// the tiles B_t with lmin <= s + t <= lmax slide from high to low t, so four B tiles
-// and one A tile are live (26 tile loads per chunk and output tile against 68 when
-// every pair streams its own).  The epilogue keeps levels 2..5 as one 64-bit integer
-// per entry, adds the rest, and makes the FP64 value by integer operations: the FP64
-// pipe does one subtraction per entry (at three operations it took longer than the
-// products at K = 128).
+// slots of 16 KB, each digit tile of A and of B loaded once per chunk: for s = 1..ND
+// the tiles B_t with lmin <= s + t <= lmax slide from high to low t, so at most four B
+// tiles and one A tile are live (26 tile loads per chunk and output tile against 68 when
+// every pair streams its own).  The epilogue sums an entry from the lowest levels up in
+// one 64-bit integer, to 2^-61 (2^-69) of the unit or 2^-60 of the entry, and makes the
+// FP64 value by integer operations: the FP64 pipe does one subtraction per entry (at three
+// operations it took longer than the products at K = 128).  At 2^-53 of the unit this
+// rounding was the largest error of the whole product.
 // Output tiles run in super-columns of 12 tile columns, row by row, so the CTAs at
 // work at a time share their digit tiles in L2.
 #include <cuda_bf16.h>
@@ -56,7 +69,8 @@ namespace f64d {
 using tc::fence_after;
 using tc::fence_before;
 
-constexpr int ND = 7;                             // digits per entry, base 2^8
+constexpr int ND7 = 7, ND8 = 8;                   // digits per entry, base 2^8: updates, general products
+__host__ __device__ constexpr int planes(int nd) { return nd == ND8 ? 9 : nd; }   // ... and the magnitudes of the first digit
 constexpr int BT = 128;                           // tile rows and columns
 constexpr int BK = 64;                            // K per chunk: 128-byte swizzled rows
 constexpr int SLOT = BT * BK * 2;                 // 16 KB
@@ -98,32 +112,52 @@ static void launch(void (*kern)(KArgs...), dim3 grid, unsigned block, size_t sme
     cudaLaunchKernelEx(&cfg, kern, (KArgs)args...);
 }
 
+// Exponent and binary places of a row's digits, from the bits of its largest magnitude: x = 2^e sum_s 2^(-8 s) a_s with
+// |x| 2^-e below 1/2 (eight digits: 1/4, so that the integer of 64 places stays below 2^62).
+template <int ND>
+struct RowScale {
+    int e, sh;
+    bool finite;
+    __device__ __forceinline__ explicit RowScale(unsigned long long mb) {
+        const int be = (int)(mb >> 52);
+        finite = be < 0x7FF;
+        e = mb == 0 ? EXP_ZERO : (finite ? (be ? be : 1) - (ND == ND8 ? 1020 : 1021) : EXP_NAN);
+        sh = mb == 0 || !finite ? 0 : 8 * ND - e;
+    }
+    // the digits of x as one integer: balanced digits without carries by 128 sum_{j < ND - 1} 2^(8 j)
+    __device__ __forceinline__ long long digits(double x) const {
+        return (finite ? tcr::scaled_rn(x, sh) : 0ll) + (ND == ND8 ? 0x0080808080808080ll : 0x0000808080808080ll);
+    }
+    // digit s (from 0) of such an integer
+    __device__ __forceinline__ static int digit(long long Z, int s) {
+        const int bit = 8 * (ND - 1 - s);
+        return s == 0 ? (int)(Z >> bit) : (int)((unsigned)(Z >> bit) & 255u) - 128;
+    }
+};
+// 2^(-8 s) d, an FP32 value whose upper half is its bf16
+__device__ __forceinline__ unsigned digit_bits(int d, int s) {
+    return __float_as_uint((__int_as_float(0x4B400000 + d) - 12582912.0f) * __int_as_float((127 - 8 * s) << 23));
+}
+
 // Digits of PER consecutive entries of a row whose largest magnitude has the bits mb, at the entry's place in plane 0
 // (planes `plane` entries apart); the row's exponent to *ex.
-template <int PER>
+template <int ND, int PER>
 __device__ __forceinline__ void row_digits(const double (&x)[PER], unsigned long long mb, __nv_bfloat16* o, int64_t plane,
                                            int* ex) {
-    // |x| < 2^e0 for every entry; the digits represent x 2^-(e0 + 1), below one half, so the first stays within 128
-    const int be = (int)(mb >> 52);
-    const bool finite = be < 0x7FF;
-    const int e = mb == 0 ? EXP_ZERO : (finite ? (be ? be : 1) - 1021 : EXP_NAN);
-    if (ex) *ex = e;
-    const int sh = mb == 0 || !finite ? 0 : 8 * ND - e;
-    constexpr long long BIAS = 0x0000808080808080ll;   // 128 sum_{j < 6} 2^(8 j): balanced digits without carries
+    const RowScale<ND> R(mb);
+    if (ex) *ex = R.e;
 #pragma unroll
     for (int i0 = 0; i0 < PER; i0 += 8) {
         long long Z[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) Z[u] = (finite ? tcr::scaled_rn(x[i0 + u], sh) : 0ll) + BIAS;
+        for (int u = 0; u < 8; ++u) Z[u] = R.digits(x[i0 + u]);
 #pragma unroll
-        for (int s = 0; s < ND; ++s) {
-            const int bit = 8 * (ND - 1 - s);
-            const float scale = __int_as_float((127 - 8 * s) << 23);
+        for (int s = 0; s < planes(ND); ++s) {   // (plane 8: |a_1|)
             unsigned f[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const int d = s == 0 ? (int)(Z[u] >> bit) : (int)((unsigned)(Z[u] >> bit) & 255u) - 128;
-                f[u] = __float_as_uint((__int_as_float(0x4B400000 + d) - 12582912.0f) * scale);
+                const int d = R.digit(Z[u], s < ND ? s : 0);
+                f[u] = digit_bits(s < ND ? d : abs(d), s < ND ? s : 0);
             }
             *reinterpret_cast<uint4*>(o + (int64_t)s * plane + i0) =
                 make_uint4(__byte_perm(f[0], f[1], 0x7632), __byte_perm(f[2], f[3], 0x7632),
@@ -138,14 +172,14 @@ __device__ __forceinline__ void row_digits(const double (&x)[PER], unsigned long
 // entries; ex[i]: the row's exponent.  A CTA takes 32 rows, lanes along them
 // (coalesced reads of the columns), eight groups of K / 8 consecutive columns.
 // ---------------------------------------------------------------------------
-template <int K>
+template <int ND, int K>
 __global__ void __launch_bounds__(256) row_digits_kernel(const double* A, int64_t lda, int64_t m, int64_t k,
                                                          int64_t rows_per_plane, __nv_bfloat16* out, int* ex) {
     constexpr int PER = K / 8;
     __shared__ unsigned long long red[8][32];
     const int lane = threadIdx.x % 32, grp = threadIdx.x / 32;
     const int64_t row = (int64_t)blockIdx.x * 32 + lane, c0 = (int64_t)blockIdx.y * K;
-    out += (int64_t)blockIdx.y * ND * rows_per_plane * K;
+    out += (int64_t)blockIdx.y * planes(ND) * rows_per_plane * K;
     ex += (int64_t)blockIdx.y * rows_per_plane;
     double x[PER];
     unsigned long long mb = 0;
@@ -161,7 +195,7 @@ __global__ void __launch_bounds__(256) row_digits_kernel(const double* A, int64_
 #pragma unroll
     for (int g = 0; g < 8; ++g) mb = max(mb, red[g][lane]);
     if (row >= m) return;
-    row_digits<PER>(x, mb, out + row * K + grp * PER, rows_per_plane * K, grp == 0 ? ex + row : nullptr);
+    row_digits<ND, PER>(x, mb, out + row * K + grp * PER, rows_per_plane * K, grp == 0 ? ex + row : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -172,8 +206,8 @@ __host__ __device__ constexpr uint32_t idesc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BT >> 4) << 24);
 }
 
-// The four K = 16 steps of a 64-wide chunk, issued by the lane that holds `lead` (the other lanes only keep the operands
-// uniform: in a one-lane branch every operand of every MMA went through a register-to-uniform move, ~100 cycles a step).
+// The four K = 16 steps of a 64-wide chunk, issued by the lane that holds `lead`.  The whole warp computes the operands: with
+// a branch of one lane around each step a step took ~100 cycles.
 __device__ __forceinline__ void mma_chunk4(uint32_t tmem, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate, uint32_t lead) {
     asm volatile(
         "{\n .reg .pred p, q, t;\n .reg .b64 a1, a2, a3, b1, b2, b3;\n"
@@ -195,7 +229,7 @@ __device__ __forceinline__ void commit_by(uint64_t* bar, uint32_t lead) {
 }
 
 // T 2^e rounded to nearest even, by integer operations: the FP64 pipe (1/64 of the FP32 rate) is left one subtraction per
-// entry.  |T| < 2^62; an exponent past the range of normal numbers flushes to zero or infinity, EXP_NAN gives a NaN.
+// entry.  |T| < 2^63; an exponent past the range of normal numbers flushes to zero or infinity, EXP_NAN gives a NaN.
 __device__ __forceinline__ double scaled_double(long long T, int e) {
     if (e > (1 << 19)) return __longlong_as_double(0x7FF8000000000000ll);
     const unsigned long long u = (unsigned long long)(T < 0 ? -T : T);
@@ -213,7 +247,7 @@ __device__ __forceinline__ double scaled_double(long long T, int e) {
 
 // The order of a unit's tiles (levels LMIN..LMAX): step s = 1..smax loads the B_t not yet loaded, then A_s, and
 // multiplies A_s by B_t for t = tlo(s)..thi(s).
-template <int LMIN, int LMAX>
+template <int ND, int LMIN, int LMAX>
 struct Unit {
     __host__ __device__ static constexpr int least(int a, int b) { return a < b ? a : b; }
     static constexpr int smax = LMAX - 1 < ND ? LMAX - 1 : ND;
@@ -257,10 +291,11 @@ struct Shared {
     uint32_t issued;   // loads issued (load g goes to slot g % STAGES), written when the producer ends
 };
 
-template <int TN, int LMIN, int LMAX>
+// The loads of one chunk: unit LMIN..LMAX's digit tiles in their order, or (LMIN = 0) the tiles of plane ND, the magnitudes.
+template <int TN, int ND, int LMIN, int LMAX>
 __device__ __forceinline__ bool load_chunk(Shared& sh, Ring& r, uint32_t sbase, const CUtensorMap* tA,
                                            const CUtensorMap* tB, int x, int ya, int yb, int ra, int rb) {
-    using U = Unit<LMIN, LMAX>;
+    using U = Unit<ND, LMIN, LMAX>;
     auto load = [&](const CUtensorMap* map, int pos, int y, int bytes) -> bool {
         uint32_t s, ph;
         r.at(pos, s, ph);
@@ -270,6 +305,11 @@ __device__ __forceinline__ bool load_chunk(Shared& sh, Ring& r, uint32_t sbase, 
         ++r.count;
         return true;
     };
+    if (LMIN == 0) {
+        if (!load(tB, 0, ND * rb + yb, TN * BK * 2) || !load(tA, 1, ND * ra + ya, SLOT)) return false;
+        r.advance(2);
+        return true;
+    }
 #pragma unroll
     for (int s = 1; s <= U::smax; ++s) {
 #pragma unroll
@@ -283,14 +323,24 @@ __device__ __forceinline__ bool load_chunk(Shared& sh, Ring& r, uint32_t sbase, 
 
 // The products of one chunk (called by the whole warp); levels LMIN into accumulator 0, the others into accumulator 1.
 // FIRST: the unit's first chunk, whose first product of each accumulator overwrites it.
-template <int TN, int LMIN, int LMAX, bool FIRST>
+template <int TN, int ND, int LMIN, int LMAX, bool FIRST>
 __device__ __forceinline__ bool mma_chunk(Shared& sh, Ring& r, uint32_t sbase, uint32_t acc, uint32_t lead) {
-    using U = Unit<LMIN, LMAX>;
+    using U = Unit<ND, LMIN, LMAX>;
     auto wait = [&](int pos, uint32_t& s) -> bool {
         uint32_t ph;
         r.at(pos, s, ph);
         return tc::wait_or_abort(&sh.full[s], ph, &sh.abort);
     };
+    if (LMIN == 0) {
+        uint32_t sa, sb;
+        if (!wait(0, sb) || !wait(1, sa)) return false;
+        fence_after();
+        mma_chunk4(acc, tc::sdesc_sw128(sbase + sa * SLOT), tc::sdesc_sw128(sbase + sb * SLOT), idesc(TN), FIRST ? 0u : 1u, lead);
+        commit_by(&sh.empty[sa], lead);
+        commit_by(&sh.empty[sb], lead);
+        r.advance(2);
+        return true;
+    }
     bool fresh0 = FIRST, fresh1 = FIRST;   // resolved at compile time after unrolling
 #pragma unroll
     for (int s = 1; s <= U::smax; ++s) {
@@ -324,15 +374,15 @@ __device__ __forceinline__ bool mma_chunk(Shared& sh, Ring& r, uint32_t sbase, u
     return true;
 }
 
-template <int TN, int LMIN, int LMAX>
+template <int TN, int ND, int LMIN, int LMAX>
 __device__ __forceinline__ bool mma_unit(Shared& sh, Ring& r, uint32_t sbase, uint32_t tmem, uint32_t& lu, int nchunk,
                                          uint32_t lead) {
     const uint32_t half = lu & 1u, acc = tmem + half * 256;
     if (!tc::wait_or_abort(&sh.tempty[half], ((lu >> 1) & 1u) ^ 1u, &sh.abort)) return false;
     fence_after();
-    if (!mma_chunk<TN, LMIN, LMAX, true>(sh, r, sbase, acc, lead)) return false;
+    if (!mma_chunk<TN, ND, LMIN, LMAX, true>(sh, r, sbase, acc, lead)) return false;
     for (int c = 1; c < nchunk; ++c)
-        if (!mma_chunk<TN, LMIN, LMAX, false>(sh, r, sbase, acc, lead)) return false;
+        if (!mma_chunk<TN, ND, LMIN, LMAX, false>(sh, r, sbase, acc, lead)) return false;
     commit_by(&sh.tfull[half], lead);
     ++lu;
     return true;
@@ -376,13 +426,15 @@ struct Walk {
     }
 };
 
-// UPDATE: C -= A B^T; otherwise segment s of the products, C_s = A_s B_s^T, to the s-th of the M x Nc slices of C (operands:
-// ND planes per segment, exponents per segment; tile numbers run over the segments).
+// UPDATE: C -= A B^T; otherwise segment s of the products, C_s = A_s B_s^T, to the s-th of the M x Nc slices of C, and to the
+// s-th slice of `mag` the sum of the products of the first digits' magnitudes over 16, at most 255 (operands: 9 planes per
+// segment, exponents per segment; tile numbers run over the segments).
 template <int TN, bool UPDATE>
 __global__ void __launch_bounds__(THREADS, 1)
     digit_update_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, int64_t M,
                         int64_t Nc, int nchunk, int ra, int rb, const int* exA,
-                        const int* exB, double* C, int64_t ldc, int lower, int64_t ntiles, int* err) {
+                        const int* exB, double* C, int64_t ldc, uint8_t* mag, int lower, int64_t ntiles, int* err) {
+    constexpr int ND = UPDATE ? ND7 : ND8;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ __align__(8) Shared sh;
     const uint32_t sbase = (dev::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -425,10 +477,15 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const int seg = UPDATE ? 0 : (int)(t / per_seg);
                 if (!UPDATE) walk = walk0;
                 walk.tile(t - seg * per_seg, i, j);
-                const int ya = i * BT + seg * ND * ra, yb = j * TN + seg * ND * rb;
-                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 4, 5>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
-                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 2, 3>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
-                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, 6, 9>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                const int ya = i * BT + seg * planes(ND) * ra, yb = j * TN + seg * planes(ND) * rb;
+                if (!UPDATE) {
+                    for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, ND, 0, 0>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                    for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, ND, 8, 10>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                }
+                for (int c = 0; c < nchunk && ok; ++c)
+                    ok = load_chunk<TN, ND, 6, UPDATE ? 9 : 7>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, ND, 4, 5>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
+                for (int c = 0; c < nchunk && ok; ++c) ok = load_chunk<TN, ND, 2, 3>(sh, r, sbase, &tA, &tB, c * BK, ya, yb, ra, rb);
             }
             sh.issued = r.count;
             if (!ok) sh.abort = 1;
@@ -441,9 +498,11 @@ __global__ void __launch_bounds__(THREADS, 1)
         const uint32_t lead = lane == 0 ? 1u : 0u;
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
         for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x)
-            ok = mma_unit<TN, 4, 5>(sh, r, sbase, tm, lu, nchunk, lead) &&
-                 mma_unit<TN, 2, 3>(sh, r, sbase, tm, lu, nchunk, lead) &&
-                 mma_unit<TN, 6, 9>(sh, r, sbase, tm, lu, nchunk, lead);
+            ok = (UPDATE || (mma_unit<TN, ND, 0, 0>(sh, r, sbase, tm, lu, nchunk, lead) &&
+                             mma_unit<TN, ND, 8, 10>(sh, r, sbase, tm, lu, nchunk, lead))) &&
+                 mma_unit<TN, ND, 6, UPDATE ? 9 : 7>(sh, r, sbase, tm, lu, nchunk, lead) &&
+                 mma_unit<TN, ND, 4, 5>(sh, r, sbase, tm, lu, nchunk, lead) &&
+                 mma_unit<TN, ND, 2, 3>(sh, r, sbase, tm, lu, nchunk, lead);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) sh.abort = 1;
         commit_by(&sh.fin, lead);
@@ -472,61 +531,86 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (!UPDATE) walk = walk0;
             walk.tile(t - seg * per_seg, ti, tj);
             const int64_t row = (int64_t)ti * BT + q * 32 + lane, col0 = (int64_t)tj * TN + c0;
-            long long H[NCW];   // levels 2..5 in units of level 5, |H| < 2^47
-            if (!begin()) break;
+            // the two accumulators of the unit at hand, eight columns at a time
+            auto read = [&](int h, uint32_t (&a)[8], uint32_t (&b)[8]) {
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
+                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + TN + c0 + h * 8, b);
+            };
+            auto whole = [](uint32_t bits, float scale) { return __float2int_rn(__uint_as_float(bits) * scale); };
+            const int64_t j1 = min((int64_t)NCW, Nc - col0), jl = row < M ? (lower ? min(j1, row - col0 + 1) : j1) : 0;
+            // M: levels 4 and up in units of 2^-LOW, |M| < 2^61 (seven digits: 2^54)
+            constexpr int LOW = UPDATE ? 61 : 69;
+            long long M_[NCW];
+            if (!UPDATE) {
+                uint8_t* const mr = mag + (int64_t)seg * M * Nc + row + col0 * M;
+                if (!begin()) break;
+#pragma unroll
+                for (int h = 0; h < NCW / 8; ++h) {
+                    uint32_t a[8];
+                    tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (h * 8 + j < jl) mr[(h * 8 + j) * M] = (uint8_t)min((int)(__uint_as_float(a[j]) * 0.0625f), 255);
+                }
+                end();
+                if (!begin()) break;   // levels 8-10
+#pragma unroll
+                for (int h = 0; h < NCW / 8; ++h) {
+                    uint32_t a[8], b[8];
+                    read(h, a, b);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        M_[h * 8 + j] = __float2int_rn((__uint_as_float(a[j]) + __uint_as_float(b[j])) * 0x1p53f);
+                }
+                end();
+            }
+            if (!begin()) break;   // levels 6 and 7 (7-9)
 #pragma unroll
             for (int h = 0; h < NCW / 8; ++h) {
                 uint32_t a[8], b[8];
-                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
-                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + TN + c0 + h * 8, b);
+                read(h, a, b);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (UPDATE)
+                        M_[h * 8 + j] = ((long long)whole(a[j], 0x1p32f) << (LOW - 48)) + whole(b[j], 0x1p45f);
+                    else
+                        M_[h * 8 + j] += ((long long)whole(a[j], 0x1p32f) << (LOW - 48)) + ((long long)whole(b[j], 0x1p40f) << (LOW - 56));
+                }
+            }
+            end();
+            if (!begin()) break;   // levels 4 and 5
+#pragma unroll
+            for (int h = 0; h < NCW / 8; ++h) {
+                uint32_t a[8], b[8];
+                read(h, a, b);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    H[h * 8 + j] = ((long long)__float2int_rn(__uint_as_float(a[j]) * 0x1p16f) << 8) +
-                                   __float2int_rn(__uint_as_float(b[j]) * 0x1p24f);
+                    M_[h * 8 + j] += (((long long)whole(a[j], 0x1p16f) << 8) + whole(b[j], 0x1p24f)) << (LOW - 40);
             }
             end();
-            if (!begin()) break;
-#pragma unroll
-            for (int h = 0; h < NCW / 8; ++h) {
-                uint32_t a[8], b[8];
-                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
-                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + TN + c0 + h * 8, b);
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    H[h * 8 + j] += ((long long)__float2int_rn(__uint_as_float(a[j])) << 24) +
-                                    ((long long)__float2int_rn(__uint_as_float(b[j]) * 0x1p8f) << 16);
-            }
-            end();
-            if (!begin()) break;
-#pragma unroll
-            for (int h = 0; h < NCW / 8; ++h) {
-                uint32_t a[8], b[8];
-                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + c0 + h * 8, a);
-                tc::tmem_ld8(tmem + lanes + (lu & 1u) * 256 + TN + c0 + h * 8, b);
-#pragma unroll
-                for (int j = 0; j < 8; ++j)   // in units of 2^-13 of level 5 (levels 6..9 are below 2^30 of them)
-                    H[h * 8 + j] = (H[h * 8 + j] << 13) +
-                                   __float2int_rn((__uint_as_float(a[j]) + __uint_as_float(b[j])) * 0x1p37f);
-            }
-            end();
-            // (the integers' unit is 2^-53 of the exponents' product)
-            const int er = (row < M ? exA[row + (int64_t)seg * ra] : EXP_ZERO) - 53;
+            if (!begin()) break;   // levels 2 and 3: G in units of 2^-24, |G| < 2^31; then the value
+            const int er = row < M ? exA[row + (int64_t)seg * ra] : EXP_ZERO;
             const int* const eb = exB + (int64_t)seg * rb + col0;
             double* const Cr = C + (int64_t)seg * M * Nc + row + col0 * ldc;
-            const int64_t j1 = min((int64_t)NCW, Nc - col0), jl = lower ? min(j1, row - col0 + 1) : j1;
-            if (row >= M) continue;
 #pragma unroll
             for (int h = 0; h < NCW / 8; ++h) {
+                uint32_t a[8], b[8];
+                read(h, a, b);
                 double c[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) c[j] = UPDATE && h * 8 + j < jl ? Cr[(h * 8 + j) * ldc] : 0.0;
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     if (h * 8 + j < jl) {
-                        const double v = scaled_double(H[h * 8 + j], er + eb[h * 8 + j]);
+                        const int G = (whole(a[j], 1.0f) << 8) + whole(b[j], 0x1p8f);
+                        // k places fewer where G 2^(LOW - 24) would not stay below 2^61
+                        const int k = max(0, LOW - 24 + 32 - __clz(abs(G)) - 61);
+                        const long long T = ((long long)G << (LOW - 24 - k)) + (M_[h * 8 + j] >> k);
+                        const double v = scaled_double(T, er + eb[h * 8 + j] - LOW + k);
                         Cr[(h * 8 + j) * ldc] = UPDATE ? c[j] - v : v;
                     }
             }
+            end();
         }
     }
     __syncthreads();
@@ -714,24 +798,16 @@ constexpr int NBS = 128;
 // the planes.  mb: the largest magnitude's bits over the row.
 __device__ __forceinline__ void write_digits4(const double x[4], unsigned long long mb, __nv_bfloat16* out,
                                               int64_t rows_per_plane, int64_t row, int* ex, int lane) {
-    const int be = (int)(mb >> 52);
-    const bool finite = be < 0x7FF;
-    const int e = mb == 0 ? EXP_ZERO : (finite ? (be ? be : 1) - 1021 : EXP_NAN);
-    if (lane == 0) ex[row] = e;
-    const int sh = mb == 0 || !finite ? 0 : 8 * ND - e;
+    const RowScale<ND7> R(mb);
+    if (lane == 0) ex[row] = R.e;
     long long Z[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) Z[u] = (finite ? tcr::scaled_rn(x[u], sh) : 0ll) + 0x0000808080808080ll;
+    for (int u = 0; u < 4; ++u) Z[u] = R.digits(x[u]);
 #pragma unroll
-    for (int s = 0; s < ND; ++s) {
-        const int bit = 8 * (ND - 1 - s);
-        const float scale = __int_as_float((127 - 8 * s) << 23);
+    for (int s = 0; s < ND7; ++s) {
         unsigned f[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int d = s == 0 ? (int)(Z[u] >> bit) : (int)((unsigned)(Z[u] >> bit) & 255u) - 128;
-            f[u] = __float_as_uint((__int_as_float(0x4B400000 + d) - 12582912.0f) * scale);
-        }
+        for (int u = 0; u < 4; ++u) f[u] = digit_bits(R.digit(Z[u], s), s);
         *reinterpret_cast<uint2*>(out + ((int64_t)s * rows_per_plane + row) * NBS + 4 * lane) =
             make_uint2(__byte_perm(f[0], f[1], 0x7632), __byte_perm(f[2], f[3], 0x7632));
     }
@@ -771,7 +847,7 @@ __global__ void __launch_bounds__(256) panel_rows_kernel(const double* __restric
 #pragma unroll
     for (int g = 0; g < 8; ++g) mb = max(mb, red[g][lane]);
     if (row >= m) return;
-    row_digits<PER>(x, mb, out + (7 * before + row) * NBS + grp * PER, m * NBS, grp == 0 ? ex + before + row : nullptr);
+    row_digits<ND7, PER>(x, mb, out + (7 * before + row) * NBS + grp * PER, m * NBS, grp == 0 ? ex + before + row : nullptr);
 }
 
 // Digit rows of the block rows (rows 128 b .. , at most 128 of them, columns before) of blocks b0 + blockIdx.y: a warp per
@@ -904,37 +980,125 @@ __global__ void __launch_bounds__(256) col_segments_kernel(const double* __restr
         x[u] = k < kdim ? a[rr.row(k)] : 0.0;
         mb = max(mb, (unsigned long long)__double_as_longlong(x[u]) & 0x7FFFFFFFFFFFFFFFull);
     }
-    row_digits<8>(x, warp_max(mb), out + (seg * ND * n + c) * KS + 8 * lane, n * KS, lane == 0 ? ex + seg * n + c : nullptr);
+    row_digits<ND8, 8>(x, warp_max(mb), out + (seg * planes(ND8) * n + c) * KS + 8 * lane, n * KS,
+                       lane == 0 ? ex + seg * n + c : nullptr);
 }
 
-// C = alpha sum of the segments' products + beta C, in segment order.  An entry whose row of A or of B^T holds an infinity
-// or a NaN is summed directly, with IEEE arithmetic's result.
-struct Operand {   // element (i, k) of op(A): p[i * si + row(k) * sk]
-    const double* p;
-    int64_t si, sk;
-};
-__global__ void sum_segments_kernel(int64_t M, int64_t N, int64_t kdim, int nseg, const double* __restrict__ P,
-                                    const int* __restrict__ exA, const int* __restrict__ exB, Operand A, Operand B,
-                                    const __grid_constant__ RowRanges rr, int64_t k0, double alpha, double beta, double* C,
-                                    int64_t ldc) {
+// C = alpha sum of the segments' products + beta C, in segment order.
+//
+// With the exponents' unit u = 2^(e_i + e_j) of a segment, the digits leave out at most K 2^-65.5 u of its product, and FP64
+// multiply-adds may be off by K 2^-53 sum |a||b|.  `mag` bounds sum |a||b| from below, in units of 2^-12 u, rounded down:
+// where its sum over the segments is less than the sum of the units, the digits' bound is not below FP64's, and the entry
+// is left to direct_entries_kernel.  So is one whose row of A or of B^T holds an infinity or a NaN, and one in the range
+// of subnormal numbers, which the products flush.  These are listed, and marked in mag's first slice.
+__global__ void __launch_bounds__(128) sum_segments_kernel(int64_t M, int64_t N, int nseg, const double* __restrict__ P,
+                                                           uint8_t* mag, const int* __restrict__ exA,
+                                                           const int* __restrict__ exB, double alpha, double beta, double* C,
+                                                           int64_t ldc, int* list, int* count) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
     for (int64_t j = blockIdx.y; j < N; j += gridDim.y) {
         double v = 0.0;
-        bool special = false;
+        bool direct = false;
+        int top = 2 * EXP_ZERO;
         for (int g = 0; g < nseg; ++g) {
-            v += P[((int64_t)g * N + j) * M + i];
-            special |= exA[(int64_t)g * M + i] == EXP_NAN || exB[(int64_t)g * N + j] == EXP_NAN;
+            const int a = exA[(int64_t)g * M + i], b = exB[(int64_t)g * N + j];
+            direct |= a == EXP_NAN || b == EXP_NAN;
+            if (a != EXP_ZERO && b != EXP_ZERO) top = max(top, a + b);
         }
-        if (special) {
-            v = 0.0;
-            for (int64_t k = 0; k < kdim; ++k) {
-                const int64_t r = rr.row(k0 + k);
-                v = fma(A.p[i * A.si + r * A.sk], B.p[j * B.si + r * B.sk], v);
-            }
+        float units = 0.0f, sum = 0.0f;
+        for (int g = 0; g < nseg; ++g) {
+            const int a = exA[(int64_t)g * M + i], b = exB[(int64_t)g * N + j];
+            v += P[((int64_t)g * N + j) * M + i];
+            if (a == EXP_ZERO || b == EXP_ZERO) continue;
+            const float u = __int_as_float((127 + max(min(a + b - top, 0), -126)) << 23);
+            units += u;
+            sum += u * (float)mag[((int64_t)g * N + j) * M + i];
+        }
+        direct |= sum < units || (units > 0.0f && top < -960);
+        mag[j * M + i] = direct ? 1 : 0;
+        if (direct) {
+            list[atomicAdd(count, 1)] = (int)(j * M + i);
+            continue;
         }
         double* c = C + i + j * ldc;
         *c = beta == 0.0 ? alpha * v : fma(alpha, v, beta * *c);
+    }
+}
+
+// The entries of the list in FP64: a CTA each, its threads along K, while they are few (a handful per thousand of a
+// potential's rows); past one in 64, tiles of 32 x 32 that have any, which take at most what the FP64 kernel takes for the
+// whole product.
+struct Operand {   // element (i, k) of op(A): p[i * si + row(k) * sk]
+    const double* p;
+    int64_t si, sk;
+};
+__global__ void __launch_bounds__(256) direct_entries_kernel(int64_t M, int64_t N, int64_t kdim, Operand A, Operand B,
+                                                             const __grid_constant__ RowRanges rr, int64_t k0, double alpha,
+                                                             double beta, double* C, int64_t ldc, const uint8_t* mark,
+                                                             const int* list, const int* count) {
+    __shared__ double red[8], sa[16][33], sb[16][33];
+    const int n = *count, tid = threadIdx.x;
+    if (n == 0) return;
+    if ((int64_t)n * 64 <= M * N) {
+        for (int e = blockIdx.x; e < n; e += gridDim.x) {
+            const int64_t i = list[e] % M, j = list[e] / M;
+            const double* const a = A.p + i * A.si;
+            const double* const b = B.p + j * B.si;
+            double part[4] = {};
+            for (int64_t k = tid; k < kdim; k += 1024)
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (k + 256 * u < kdim) {
+                        const int64_t r = rr.row(k0 + k + 256 * u);
+                        part[u] = fma(a[r * A.sk], b[r * B.sk], part[u]);
+                    }
+            double v = (part[0] + part[1]) + (part[2] + part[3]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (tid % 32 == 0) red[tid / 32] = v;
+            __syncthreads();
+            if (tid == 0) {
+                v = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+                double* c = C + i + j * ldc;
+                *c = beta == 0.0 ? alpha * v : fma(alpha, v, beta * *c);
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    const int64_t mt = (M + 31) / 32, nt = (N + 31) / 32;
+    const int ti = tid % 32, tj = tid / 32;   // the thread's row and columns tj + 8 u of a tile
+    for (int64_t t = blockIdx.x; t < mt * nt; t += gridDim.x) {
+        const int64_t i0 = t % mt * 32, j0 = t / mt * 32;
+        bool mine[4], any = false;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            mine[u] = i0 + ti < M && j0 + tj + 8 * u < N && mark[(j0 + tj + 8 * u) * M + i0 + ti];
+            any |= mine[u];
+        }
+        if (!__syncthreads_or(any)) continue;
+        double v[4] = {};
+        for (int64_t kb = 0; kb < kdim; kb += 16) {
+            for (int e = tid; e < 512; e += 256) {   // the faster index along the operand's contiguous direction
+                const int ia = A.sk == 1 ? e / 16 : e % 32, ka = A.sk == 1 ? e % 16 : e / 32;
+                const int jb = B.sk == 1 ? e / 16 : e % 32, kc = B.sk == 1 ? e % 16 : e / 32;
+                sa[ka][ia] = kb + ka < kdim && i0 + ia < M ? A.p[(i0 + ia) * A.si + rr.row(k0 + kb + ka) * A.sk] : 0.0;
+                sb[kc][jb] = kb + kc < kdim && j0 + jb < N ? B.p[(j0 + jb) * B.si + rr.row(k0 + kb + kc) * B.sk] : 0.0;
+            }
+            __syncthreads();
+            const int nk = (int)(kdim - kb < 16 ? kdim - kb : 16);
+            for (int k = 0; k < nk; ++k)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = fma(sa[k][ti], sb[k][tj + 8 * u], v[u]);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (mine[u]) {
+                double* c = C + i0 + ti + (j0 + tj + 8 * u) * ldc;
+                *c = beta == 0.0 ? alpha * v[u] : fma(alpha, v[u], beta * *c);
+            }
     }
 }
 
@@ -959,18 +1123,18 @@ void row_digits_f64(const double* A, int64_t lda, int64_t m, int k, int kpad, in
     if ((kpad != 128 && kpad != 256) || k > kpad || rows_per_plane < m) throw Error(OMG_ERR_INVALID, "row digits: bad layout");
     ProfScope prof_("f64_digits", s);
     const unsigned grid = (unsigned)((m + 31) / 32);
-    auto kern = kpad == 128 ? f64d::row_digits_kernel<128> : f64d::row_digits_kernel<256>;
+    auto kern = kpad == 128 ? f64d::row_digits_kernel<f64d::ND7, 128> : f64d::row_digits_kernel<f64d::ND7, 256>;
     f64d::launch(kern, grid, 256, 0, s, A, lda, m, (int64_t)k, rows_per_plane, static_cast<__nv_bfloat16*>(out), ex);
     f64d::check("FP64 row digits");
 }
 
-// nseg > 0: the products of nseg segments, to slices of C; otherwise the update.
+// nseg > 0: the products of nseg segments, to slices of C and of mag; otherwise the update.
 static void digit_product(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
-                          const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, bool lower,
-                          int nseg, int* err, cudaStream_t s, const char* name) {
+                          const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, uint8_t* mag,
+                          bool lower, int nseg, int* err, cudaStream_t s, const char* name) {
     if (M <= 0 || Nc <= 0) return;
-    const int64_t segs = std::max(1, nseg);
-    if (kpad % f64d::BK || kpad > 256 || segs * f64d::ND * std::max(ra, rb) > (1ll << 30))
+    const int64_t segs = std::max(1, nseg), np = f64d::planes(nseg > 0 ? f64d::ND8 : f64d::ND7);
+    if (kpad % f64d::BK || kpad > 256 || segs * np * std::max(ra, rb) > (1ll << 30))
         throw Error(OMG_ERR_UNSUPPORTED, "digit update: bad sizes");
     ProfScope prof_(name, s);
     static int n_sm = 0;
@@ -992,7 +1156,7 @@ static void digit_product(int64_t M, int64_t Nc, int kpad, const void* A, int64_
         int64_t best = INT64_MAX;
         for (int w : {128, 64, 32}) {
             const int64_t waves = (segs * mt * ((Nc + w - 1) / w) + n_sm - 1) / n_sm;
-            const int64_t t = waves * 34 * (kpad / 16) * (w == 128 ? 64 : w == 64 ? 48 : 40) + 100 * w;
+            const int64_t t = waves * (nseg > 0 ? 44 : 34) * (kpad / 16) * (w == 128 ? 64 : w == 64 ? 48 : 40) + 100 * w;
             if (t < best) {
                 best = t;
                 tn = w;
@@ -1000,9 +1164,9 @@ static void digit_product(int64_t M, int64_t Nc, int kpad, const void* A, int64_
         }
     }
     const CUtensorMap mA = tc::make_map_2d(static_cast<const uint16_t*>(A) + a0 * kpad, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                                           2, segs * f64d::ND * ra - a0, kpad, kpad, f64d::BK, f64d::BT);
+                                           2, segs * np * ra - a0, kpad, kpad, f64d::BK, f64d::BT);
     const CUtensorMap mB = tc::make_map_2d(static_cast<const uint16_t*>(B) + b0 * kpad, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                                           2, segs * f64d::ND * rb - b0, kpad, kpad, f64d::BK, tn);
+                                           2, segs * np * rb - b0, kpad, kpad, f64d::BK, tn);
     const int64_t nt = (Nc + tn - 1) / tn;
     const int64_t ntiles = segs * (lower ? mt * nt - nt * (nt - 1) / 2 : mt * nt);
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, n_sm);
@@ -1013,7 +1177,7 @@ static void digit_product(int64_t M, int64_t Nc, int kpad, const void* A, int64_
                             : tn == 64 ? f64d::digit_update_kernel<64, true>
                                        : f64d::digit_update_kernel<32, true>);
     f64d::launch(kern, grid, f64d::THREADS, f64d::SMEM_BYTES, s, mA, mB, M, Nc, kpad / f64d::BK, (int)ra, (int)rb, exA + a0,
-                 exB + b0, C, ldc, lower ? 1 : 0, ntiles, err);
+                 exB + b0, C, ldc, mag, lower ? 1 : 0, ntiles, err);
     f64d::check(name);
 }
 
@@ -1022,12 +1186,13 @@ static void digit_product(int64_t M, int64_t Nc, int kpad, const void* A, int64_
 void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra, int64_t a0, const int* exA,
                       const void* B, int64_t rb, int64_t b0, const int* exB, double* C, int64_t ldc, bool lower,
                       int* err, cudaStream_t s, const char* name) {
-    digit_product(M, Nc, kpad, A, ra, a0, exA, B, rb, b0, exB, C, ldc, lower, 0, err, s, name);
+    digit_product(M, Nc, kpad, A, ra, a0, exA, B, rb, b0, exB, C, ldc, nullptr, lower, 0, err, s, name);
 }
 
-// C (M x N) = alpha op(A) op(B) + beta C over the K rows (columns) the ranges list (null: all K), FP64, column-major.
-// From about 60 us of FP64-pipe time on by FP64-accurate digit products, segment by segment of K (partial products of up to
-// 512 MB at a time); below that the operands' digits and the launches cost more than the FP64 kernel.
+// C (M x N) = alpha op(A) op(B) + beta C over the K rows (columns) the ranges list (null: all K), FP64, column-major, with an
+// error of at most K 2^-53 sum |a||b| per entry.
+// From about 60 us of FP64-pipe time on by digit products, segment by segment of K; below that the operands' digits and the
+// launches cost more than the FP64 kernel.
 void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t lda, bool ta, const double* B,
               int64_t ldb, bool tb, double beta, double* C, int64_t ldc, int* err, cudaStream_t s,
               const std::vector<std::pair<int64_t, int64_t>>* ranges) {
@@ -1063,48 +1228,62 @@ void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, in
                          ldc, s);
         return;
     }
-    // segments at a time: the partial products, and the operands' digits (14 bytes an entry), within 512 MB each
+    // segments at a time: the partial products with their bounds, and each operand's digits, within 512 MB
+    constexpr int64_t MOST = 512ll << 20, DIGIT_ROW = (int64_t)planes(ND8) * KS * 2;
     const int64_t nseg = (K + KS - 1) / KS;
-    const int64_t at_once = std::max<int64_t>(
-        1, std::min<int64_t>({nseg, (512ll << 20) / (M * N * 8), (512ll << 20) / (std::max(M, N) * KS * 14)}));
-    DevBuf P((size_t)at_once * M * N * 8, s), dA((size_t)at_once * ND * M * KS * 2, s),
-        dB((size_t)at_once * ND * N * KS * 2, s), ex((size_t)at_once * (M + N) * sizeof(int), s);
-    int* exA = ex.as<int>();
-    int* exB = exA + at_once * M;
-    for (int64_t g0 = 0; g0 < nseg; g0 += at_once) {
-        const int64_t ns = std::min(at_once, nseg - g0), k0 = g0 * KS, kk = std::min(K - k0, ns * KS);
-        RowRanges part = rr;   // the rows from k0 on
-        for (int64_t skip = k0; part.n > 0 && skip > 0;) {
-            const int64_t d = std::min(skip, part.len[0]);
-            part.beg[0] += d;
-            part.len[0] -= d;
-            skip -= d;
-            if (part.len[0] == 0 && part.n > 1) {
-                for (int q = 1; q < part.n; ++q) {
-                    part.beg[q - 1] = part.beg[q];
-                    part.len[q - 1] = part.len[q];
+    const int64_t mb = M, nb = N;
+    const int64_t at_once = std::max<int64_t>(1, std::min<int64_t>({nseg, MOST / (mb * nb * 9), MOST / (std::max(mb, nb) * DIGIT_ROW)}));
+    DevBuf P((size_t)at_once * mb * nb * 8, s), W((size_t)at_once * mb * nb, s), dA((size_t)at_once * mb * DIGIT_ROW, s),
+        dB((size_t)at_once * nb * DIGIT_ROW, s), left((size_t)(mb * nb + 1) * sizeof(int), s), ex((size_t)at_once * (mb + nb) * sizeof(int), s);
+    auto block = [&](int64_t M, int64_t N, const double* A, const double* B, double* C) {
+        int* exA = ex.as<int>();
+        int* exB = exA + at_once * M;
+        for (int64_t g0 = 0; g0 < nseg; g0 += at_once) {
+            const int64_t ns = std::min(at_once, nseg - g0), k0 = g0 * KS, kk = std::min(K - k0, ns * KS);
+            RowRanges part = rr;   // the rows from k0 on
+            for (int64_t skip = k0; part.n > 0 && skip > 0;) {
+                const int64_t d = std::min(skip, part.len[0]);
+                part.beg[0] += d;
+                part.len[0] -= d;
+                skip -= d;
+                if (part.len[0] == 0 && part.n > 1) {
+                    for (int q = 1; q < part.n; ++q) {
+                        part.beg[q - 1] = part.beg[q];
+                        part.len[q - 1] = part.len[q];
+                    }
+                    --part.n;
                 }
-                --part.n;
             }
+            auto digits = [&](const double* X, int64_t ldx, bool k_contiguous, int64_t n, void* out, int* e) {
+                ProfScope prof_("f64_digits", s);
+                if (k_contiguous)
+                    col_segments_kernel<<<dim3((unsigned)((n + 7) / 8), (unsigned)ns), 256, 0, s>>>(
+                        X + (part.n ? 0 : k0), ldx, n, kk, part, static_cast<__nv_bfloat16*>(out), e);
+                else
+                    launch(row_digits_kernel<ND8, KS>, dim3((unsigned)((n + 31) / 32), (unsigned)ns), 256, 0, s, X + k0 * ldx,
+                           ldx, n, kk, n, static_cast<__nv_bfloat16*>(out), e);
+                check("GEMM digits");
+            };
+            digits(A, lda, ta, M, dA.p, exA);
+            digits(B, ldb, !tb, N, dB.p, exB);
+            digit_product(M, N, KS, dA.p, M, 0, exA, dB.p, N, 0, exB, P.as<double>(), M, W.as<uint8_t>(), false, (int)ns, err,
+                          s, "f64_product");
+            ProfScope prof_("f64_segments", s);
+            OMG_CUDA(cudaMemsetAsync(left.p, 0, sizeof(int), s));
+            int* count = left.as<int>();
+            sum_segments_kernel<<<dim3((unsigned)((M + 127) / 128), (unsigned)std::min<int64_t>(N, 65535)), 128, 0, s>>>(
+                M, N, (int)ns, P.as<double>(), W.as<uint8_t>(), exA, exB, alpha, g0 == 0 ? beta : 1.0, C, ldc, count + 1,
+                count);
+            check("GEMM segments");
+            const Operand oa{A, ta ? lda : 1, ta ? 1 : lda}, ob{B, tb ? 1 : ldb, tb ? ldb : 1};
+            direct_entries_kernel<<<(unsigned)std::min<int64_t>((M * N + 63) / 64, 4 * sm_count()), 256, 0, s>>>(
+                M, N, kk, oa, ob, rr, k0, alpha, g0 == 0 ? beta : 1.0, C, ldc, W.as<uint8_t>(), count + 1, count);
+            check("GEMM entries");
         }
-        auto digits = [&](const double* X, int64_t ldx, bool k_contiguous, int64_t n, void* out, int* e) {
-            ProfScope prof_("f64_digits", s);
-            if (k_contiguous)
-                col_segments_kernel<<<dim3((unsigned)((n + 7) / 8), (unsigned)ns), 256, 0, s>>>(
-                    X + (part.n ? 0 : k0), ldx, n, kk, part, static_cast<__nv_bfloat16*>(out), e);
-            else
-                launch(row_digits_kernel<KS>, dim3((unsigned)((n + 31) / 32), (unsigned)ns), 256, 0, s, X + k0 * ldx, ldx, n,
-                       kk, n, static_cast<__nv_bfloat16*>(out), e);
-            check("GEMM digits");
-        };
-        digits(A, lda, ta, M, dA.p, exA);
-        digits(B, ldb, !tb, N, dB.p, exB);
-        digit_product(M, N, KS, dA.p, M, 0, exA, dB.p, N, 0, exB, P.as<double>(), M, false, (int)ns, err, s, "f64_product");
-        const Operand oa{A, ta ? lda : 1, ta ? 1 : lda}, ob{B, tb ? 1 : ldb, tb ? ldb : 1};
-        sum_segments_kernel<<<dim3((unsigned)((M + 127) / 128), (unsigned)std::min<int64_t>(N, 65535)), 128, 0, s>>>(
-            M, N, kk, (int)ns, P.as<double>(), exA, exB, oa, ob, rr, k0, alpha, g0 == 0 ? beta : 1.0, C, ldc);
-        check("GEMM segments");
-    }
+    };
+    for (int64_t i0 = 0; i0 < M; i0 += mb)
+        for (int64_t j0 = 0; j0 < N; j0 += nb)
+            block(std::min(mb, M - i0), std::min(nb, N - j0), A + i0 * (ta ? lda : 1), B + j0 * (tb ? 1 : ldb), C + i0 + j0 * ldc);
 }
 
 // Sub-panel at (k0, k0) of the matrix, w <= 32 columns: the diagonal block's factor to Ld, the rows below solved in place.
