@@ -1228,11 +1228,13 @@ void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, in
                          ldc, s);
         return;
     }
-    // segments at a time: the partial products with their bounds, and each operand's digits, within 512 MB
+    // Blocks of rows and columns, and segments at a time, for which the partial products with their bounds and each
+    // operand's digits take 512 MB at most.
     constexpr int64_t MOST = 512ll << 20, DIGIT_ROW = (int64_t)planes(ND8) * KS * 2;
     const int64_t nseg = (K + KS - 1) / KS;
-    const int64_t mb = M, nb = N;
-    const int64_t at_once = std::max<int64_t>(1, std::min<int64_t>({nseg, MOST / (mb * nb * 9), MOST / (std::max(mb, nb) * DIGIT_ROW)}));
+    const int64_t mb = std::min(M, MOST / DIGIT_ROW / BT * BT);
+    const int64_t nb = std::min({N, MOST / DIGIT_ROW / BT * BT, std::max<int64_t>(BT, MOST / (mb * 9) / BT * BT)});
+    const int64_t at_once = std::max<int64_t>(1, std::min<int64_t>({nseg, 65535, MOST / (mb * nb * 9), MOST / (std::max(mb, nb) * DIGIT_ROW)}));
     DevBuf P((size_t)at_once * mb * nb * 8, s), W((size_t)at_once * mb * nb, s), dA((size_t)at_once * mb * DIGIT_ROW, s),
         dB((size_t)at_once * nb * DIGIT_ROW, s), left((size_t)(mb * nb + 1) * sizeof(int), s), ex((size_t)at_once * (mb + nb) * sizeof(int), s);
     auto block = [&](int64_t M, int64_t N, const double* A, const double* B, double* C) {

@@ -76,6 +76,29 @@ def test_rows_with_peaks(cuda):
         assert np.all(err(out, axis) <= err(fma, axis))
 
 
+@pytest.mark.parametrize("M,N,K", [(116500, 3, 300), (2, 116600, 400), (7700, 7700, 130), (1, 1, 17_000_000)])
+def test_sizes_past_one_block(cuda, M, N, K):
+    """Rows, columns and output past one block of the scratch, and more segments than a grid's second dimension holds."""
+    import torch
+    from openmeeg_gb300 import _lib, api
+    g = torch.Generator(device=cuda).manual_seed(1)
+    A = torch.randn(M, K, dtype=torch.float64, device=cuda, generator=g)   # op(A) = A by its transpose
+    B = torch.randn(N, K, dtype=torch.float64, device=cuda, generator=g)
+    C = torch.empty(N, M, dtype=torch.float64, device=cuda)
+    ctx, p = api.Context.default(), lambda t: ctypes.c_void_p(t.data_ptr())
+    _lib.check(ctx.lib.omg_gemm_f64_dev(ctx.handle, 1, 0, M, N, K, 1.0, p(A), K, p(B), K, 0.0, p(C), M))
+    i = np.unique(np.r_[np.arange(min(M, 3)), M // 2, np.arange(max(M - 3, 0), M)])
+    j = np.unique(np.r_[np.arange(min(N, 3)), N // 2, np.arange(max(N - 3, 0), N)])
+    a, b = A.cpu().numpy()[i], B.cpu().numpy()[j].T
+    out = C.cpu().numpy().T[np.ix_(i, j)]
+    want = a.astype(L) @ b.astype(L)
+    mag = np.abs(a) @ np.abs(b)
+    assert np.all(np.abs(out - want).astype(float) <= 2.0**-53 * (min(K, 512) * mag + 2 * np.abs(want).astype(float)))
+    full = A @ B.T if M * N < 10**8 else None
+    if full is not None:   # every block was written
+        assert float((C.T - full).abs().max()) < 1e-9 * K**0.5
+
+
 def _update(cuda, A, B):
     import torch
     from openmeeg_gb300 import _lib
