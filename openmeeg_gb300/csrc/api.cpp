@@ -136,6 +136,7 @@ void digit_gemm(int64_t n, int64_t k, int64_t kdim, const void* Ad, int nda, con
                 int64_t kpad, const int* cexp, int beta, int lmax, const double* B, int64_t ldb, double sgn, double* R,
                 int64_t ldr, int* err, cudaStream_t s, const char* prof_name);
 // f64_digits.cu
+bool gemm_f64_by_digits(int64_t M, int64_t N, int64_t K);
 void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t lda, bool ta, const double* B,
               int64_t ldb, bool tb, double beta, double* C, int64_t ldc, int* err, cudaStream_t s,
               const std::vector<std::pair<int64_t, int64_t>>* ranges = nullptr);
@@ -2158,10 +2159,13 @@ int omg_gemm_f64_dev(omg_context ctx, int32_t trans_a, int32_t trans_b, int64_t 
             if (beta == 0.0)
                 for (int64_t j = 0; j < n; ++j) OMG_CUDA(cudaMemsetAsync(C + j * ldc, 0, (size_t)m * 8, ctx->stream));
         } else {
-            reset_err(ctx);
+            const bool digits = gemm_f64_by_digits(m, n, k);   // (their bounded waits report to the status word)
+            if (digits) reset_err(ctx);
             gemm_f64(m, n, k, alpha, A, lda, trans_a != 0, B, ldb, trans_b != 0, beta, C, ldc, ctx->d_err, ctx->stream);
-            check_err(ctx, "GEMM");
-            return;
+            if (digits) {
+                check_err(ctx, "GEMM");
+                return;
+            }
         }
         OMG_CUDA(cudaStreamSynchronize(ctx->stream));
     });

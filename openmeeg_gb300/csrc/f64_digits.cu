@@ -1189,10 +1189,21 @@ void digit_update_f64(int64_t M, int64_t Nc, int kpad, const void* A, int64_t ra
     digit_product(M, Nc, kpad, A, ra, a0, exA, B, rb, b0, exB, C, ldc, nullptr, lower, 0, err, s, name);
 }
 
+// Whether a general product goes by digit products: where they take less time than the FP64 kernel.  Measured in calls,
+// their fixed 16 us taken off: the FP64 kernel 0.29 us per K and wave of 32 x 32 tiles, 1.07 per K for an output within one
+// (a 64 x 64 tile on one SM); the digits 88 us (launches, the least product) and per segment of 256 29 us for a million
+// entries of C and 17 for a million entries of A and B.  E.g. 64 x 100 x 207: 59 us by FP64, 88 by digits; 64 x 100 x 600 176
+// and 88; 1 x 1 x 100 107 and 84; 4486 x 151 x 4486 9459 and 810.
+bool gemm_f64_by_digits(int64_t M, int64_t N, int64_t K) {
+    if (M <= 0 || N <= 0 || K <= 0) return false;
+    const double waves = std::ceil((double)((M + 31) / 32) * (double)((N + 31) / 32) / (double)f64d::sm_count());
+    const double fp64_us = (M <= 32 && N <= 32 ? 1.07 : 0.29 * waves) * (double)K;
+    const double nseg = (double)((K + f64d::KS - 1) / f64d::KS);
+    return fp64_us > 88.0 + nseg * (29e-6 * (double)M * (double)N + 17e-6 * (double)(M + N) * f64d::KS);
+}
+
 // C (M x N) = alpha op(A) op(B) + beta C over the K rows (columns) the ranges list (null: all K), FP64, column-major, with an
 // error of at most K 2^-53 sum |a||b| per entry.
-// From about 60 us of FP64-pipe time on by digit products, segment by segment of K; below that the operands' digits and the
-// launches cost more than the FP64 kernel.
 void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t lda, bool ta, const double* B,
               int64_t ldb, bool tb, double beta, double* C, int64_t ldc, int* err, cudaStream_t s,
               const std::vector<std::pair<int64_t, int64_t>>* ranges) {
@@ -1216,9 +1227,7 @@ void gemm_f64(int64_t M, int64_t N, int64_t K, double alpha, const double* A, in
         }
         if (rr.n > 0 && (!ta || tb)) throw Error(OMG_ERR_INVALID, "GEMM: row ranges need both operands K-contiguous");
     }
-    // the FP64 kernel: waves of 32 x 32 tiles, 0.29 us per K on an SM
-    const double us = std::ceil((double)((M + 31) / 32) * ((N + 31) / 32) / 152.0) * 0.29 * (double)K;
-    if (us < 60.0 || K <= 0) {
+    if (!gemm_f64_by_digits(M, N, K)) {
         if (K <= 0 || rr.n == 0) {
             gemm<double>(M, N, K, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, s);
             return;
