@@ -95,8 +95,20 @@ def ds2mm_torch(dipoles: torch.Tensor, squids: torch.Tensor) -> torch.Tensor:
 
 
 class _Gain(torch.autograd.Function):
+    # Library calls and torch's operations alternate on shared buffers, and torch gives a buffer out again as soon as its
+    # last use is queued: both passes keep the library on torch's stream.
     @staticmethod
     def forward(ctx, sigmas, dipoles, state):
+        with state["geo"].ctx.on_current_stream():
+            return _Gain._forward(ctx, sigmas, dipoles, state)
+
+    @staticmethod
+    def backward(ctx, Gbar):
+        with ctx.state["geo"].ctx.on_current_stream():
+            return _Gain._backward(ctx, Gbar)
+
+    @staticmethod
+    def _forward(ctx, sigmas, dipoles, state):
         geo = state["geo"]
         lib_ctx = geo.ctx
         sig = sigmas.detach().double().cpu().numpy()
@@ -132,7 +144,7 @@ class _Gain(torch.autograd.Function):
         return G
 
     @staticmethod
-    def backward(ctx, Gbar):
+    def _backward(ctx, Gbar):
         st = ctx.state
         geo, lib_ctx = st["geo"], st["geo"].ctx
         HM, Yc, Dc, sv, dip = st["HM"], st["Yc"], st["Dc"], st["sv"], st["dip"]

@@ -13,6 +13,7 @@ raise ``OMGError`` carrying the C status, where the reference raises its
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 import sys
@@ -53,6 +54,7 @@ class Context:
         h = ctypes.c_void_p()
         check(self.lib.omg_context_create(device, ctypes.byref(h)))
         self.handle = h
+        self.stream = 0   # the stream bound (0: the library's own, which follows the default stream)
 
     @classmethod
     def default(cls, device: Optional[int] = None) -> "Context":
@@ -64,8 +66,21 @@ class Context:
 
     def bind_current_stream(self):
         """Queue library work on torch's current stream of this device."""
-        s = torch.cuda.current_stream(self.device)
-        check(self.lib.omg_context_set_stream(self.handle, ctypes.c_void_p(s.cuda_stream)))
+        self._set_stream(torch.cuda.current_stream(self.device).cuda_stream)
+
+    def _set_stream(self, stream: int):
+        check(self.lib.omg_context_set_stream(self.handle, ctypes.c_void_p(stream)))
+        self.stream = stream
+
+    @contextlib.contextmanager
+    def on_current_stream(self):
+        """Within the scope, library work goes to torch's current stream of this device."""
+        bound = self.stream
+        self.bind_current_stream()
+        try:
+            yield
+        finally:
+            self._set_stream(bound)
 
     def synchronize(self):
         check(self.lib.omg_context_synchronize(self.handle))
