@@ -1543,6 +1543,10 @@ __global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, i
     }
 }
 
+// The tolerance at which a pair is settled by the first level: below tol by a margin that the rounding of the values (some
+// 1e-15 of them) cannot turn.  Where there is none left (tol under 1e-14, or negative: always refine) the pairs are listed.
+__device__ __forceinline__ double dsm_limit(double tol) { return tol * (1.0 - 1e-9) - 1e-14; }
+
 // The dipole's part in block fixed point: X and q (limbs with 0 <= l < 2^30), the exponent E of X + (point - c), that of q,
 // and how far the table's points shift.
 struct DsmFix {
@@ -1850,8 +1854,7 @@ __global__ void dsm_kernel(int64_t dip0, int64_t ndc, const double* __restrict__
 #pragma unroll
             for (int k = 0; k < 4; ++k) ref[k] = fma(0.25 * area, a[k], ref[k]);
         }
-        // settled with a margin of 1e-9 tol: rounding (1e-15) cannot turn the decision
-        const double lim = tol * (1.0 - 1e-9);
+        const double lim = dsm_limit(tol);
         double d2 = 0.0, c2 = 0.0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -1861,10 +1864,10 @@ __global__ void dsm_kernel(int64_t dip0, int64_t ndc, const double* __restrict__
                 d2 = fma(e, e, d2);
                 c2 = fma(v[k], v[k], c2);
             } else {
-                okp = fabs(e) <= lim * fabs(v[k]);
+                okp = lim >= 0.0 && fabs(e) <= lim * fabs(v[k]);
             }
         }
-        okv = d2 <= lim * lim * c2;
+        okv = lim >= 0.0 && d2 <= lim * lim * c2;
 #pragma unroll
         for (int k = 0; k < 4; ++k) v[k] = ref[k];
     }
@@ -2420,7 +2423,7 @@ __global__ void dsm_vjp_kernel(int64_t dip0, int64_t ndc, const double* __restri
     const double sub = levels > 0 ? 0.25 * area : area;
     if (levels > 0) {   // the test of dsm_kernel
         f[0] -= f[1] + f[2];
-        const double lim = tol * (1.0 - 1e-9);
+        const double lim = dsm_limit(tol);
         double d2 = 0.0, c2 = 0.0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -2429,10 +2432,10 @@ __global__ void dsm_vjp_kernel(int64_t dip0, int64_t ndc, const double* __restri
                 d2 = fma(e, e, d2);
                 c2 = fma(c, c, c2);
             } else {
-                okp = fabs(e) <= lim * fabs(c);
+                okp = lim >= 0.0 && fabs(e) <= lim * fabs(c);
             }
         }
-        okv = d2 <= lim * lim * c2;
+        okv = lim >= 0.0 && d2 <= lim * lim * c2;
     }
     double g[6] = {0, 0, 0, 0, 0, 0};
     if (okv) {
