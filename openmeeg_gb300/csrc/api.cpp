@@ -175,6 +175,14 @@ void set_last_error(const char* msg) { g_last_error = msg; }
 void set_device(omg_context ctx) {
     OMG_CUDA(cudaSetDevice(ctx->device));
     if (ctx->stream != ctx->own) return;
+    // While a blocking stream is being captured (by this thread in relaxed mode, or by another) the default stream may not
+    // be named: recording on it would fail and end that capture.  The query below says so and leaves the capture alone; what
+    // was queued on the default stream before it is then the caller's to wait for.
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(cudaStreamLegacy, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
     if (!ctx->ev_in) OMG_CUDA(cudaEventCreateWithFlags(&ctx->ev_in, cudaEventDisableTiming));
     OMG_CUDA(cudaEventRecord(ctx->ev_in, cudaStreamLegacy));
     OMG_CUDA(cudaStreamWaitEvent(ctx->own, ctx->ev_in, 0));
