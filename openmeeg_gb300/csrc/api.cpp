@@ -1253,6 +1253,15 @@ static std::vector<int> meshes_of_domains(omg_geometry g, const std::vector<int>
     return out;
 }
 
+// Whether every interface is one (closed) mesh.  The domain lookup then asks only which side of 2 pi a mesh's solid angle is
+// on: FP32 screens the sums and those it cannot be sure of are taken in FP64.  The angles of an interface's several open
+// meshes are added up, so they are needed themselves.
+static bool one_mesh_interfaces(omg_geometry g) {
+    for (const auto& f : g->h.ifaces)
+        if (f.size() != 1) return false;
+    return true;
+}
+
 void dsm_internal(omg_geometry g, const double* dip, int64_t nd, const omg_integrator& integ, int domain, int perm,
                   double* out, int64_t ldo, int precision, std::vector<int>* meshes_used, uint64_t allowed_domains,
                   DevBuf* dom_out) {
@@ -1279,12 +1288,7 @@ void dsm_internal(omg_geometry g, const double* dip, int64_t nd, const omg_integ
         dperm = 1;
     }
     DevBuf sa((size_t)nd * g->h.nmesh * 8, s), dom((size_t)nd * sizeof(int), s);
-    // closed meshes, one per interface: the lookup asks only which side of 2 pi a mesh's sum is on, so FP32 screens the sums
-    // and those it cannot be sure of are taken in FP64
-    bool closed = true;
-    for (const auto& f : g->h.ifaces) closed = closed && f.size() == 1;
-    launch_mesh_solid_angles(dip, 6, nd, g->h.nmesh, g->tbeg, g->d.srec, sa.as<double>(), s,
-                             precision == OMG_PREC_MIXED || closed);
+    launch_mesh_solid_angles(dip, 6, nd, g->h.nmesh, g->tbeg, g->d.srec, sa.as<double>(), s, one_mesh_interfaces(g));
     launch_domain_lookup(nd, g->h.nmesh, sa.as<double>(), g->ndom, g->maxb, g->dnb, g->bmesh, g->binside, g->orient,
                          g->bgrp, domain, dom.as<int>(), ctx->d_err, s);
     if (allowed_domains) launch_domain_check(nd, dom.as<int>(), allowed_domains, ctx->d_err, s);
@@ -1813,9 +1817,8 @@ static void keep_conducting_points(KeptPoints& kp, omg_geometry geo, const doubl
     kp.rows = DevBuf((size_t)std::max<int64_t>(n, 1) * sizeof(int64_t), s);
     kp.kept = 0;
     if (n == 0) return;
-    // FP32-screened solid angles: sums clear of the 2 pi boundary classify as in FP64, the rest are FP64 sums
     DevBuf sa((size_t)n * h.nmesh * 8, s);
-    launch_mesh_solid_angles(pts, 3, n, h.nmesh, geo->tbeg, geo->d.srec, sa.as<double>(), s, true);
+    launch_mesh_solid_angles(pts, 3, n, h.nmesh, geo->tbeg, geo->d.srec, sa.as<double>(), s, one_mesh_interfaces(geo));
     launch_domain_lookup(n, h.nmesh, sa.as<double>(), geo->ndom, geo->maxb, geo->dnb, geo->bmesh, geo->binside,
                          geo->orient, geo->bgrp, -1, kp.dom.as<int>(), geo->ctx->d_err, s);
     check_err(geo->ctx, "point domain lookup");
@@ -1890,7 +1893,7 @@ int omg_dipsource2internalpotmat_dev(omg_context ctx, omg_geometry geo, const do
         DevBuf sa((size_t)n_dipoles * h.nmesh * 8, s), ddom((size_t)n_dipoles * sizeof(int), s);
         if (domain < 0)
             launch_mesh_solid_angles(dipoles, 6, n_dipoles, h.nmesh, geo->tbeg, geo->d.srec, sa.as<double>(), s,
-                                     true);
+                                     one_mesh_interfaces(geo));
         launch_domain_lookup(n_dipoles, h.nmesh, sa.as<double>(), geo->ndom, geo->maxb, geo->dnb, geo->bmesh,
                              geo->binside, geo->orient, geo->bgrp, domain, ddom.as<int>(), ctx->d_err, s);
         launch_dipole_internal_pot(points, kp.dom.as<int>(), kp.rows.as<int64_t>(), n_points, dipoles, ddom.as<int>(),
