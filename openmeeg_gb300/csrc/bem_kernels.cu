@@ -1489,7 +1489,8 @@ __device__ __forceinline__ void dsm_adaptive_warp(int kind, int order, int level
 // FP64: the first adaptive level of both integrands of every (dipole, triangle)
 // pair, 80 points.  What depends on the triangle alone is tabled once per
 // launch, by rule point (the triangle's 16 and each child's 16), lanes along
-// the triangles: the point relative to the centroid c, the P1 values 1 and 2 and
+// the triangles: the point relative to the centroid c, the three P1 values (the
+// first as the sum's difference from the others' had three times their error) and
 // -3 n.(point - c).  With X = c - r0 (r0, q: the dipole) a point then takes 10
 // FP64 operations for the potential and its three P1-weighted derivatives:
 // r = X + (point - c), |r|^2, q.r, the reciprocal square root and its product with
@@ -1500,7 +1501,7 @@ __device__ __forceinline__ void dsm_adaptive_warp(int kind, int order, int level
 // A pair is settled here when |coarse - refined| <= tol |coarse| holds with a
 // margin far above the rounding; the others (and those decided by rounding) are
 // listed for dsm_fallback_kernel.
-constexpr int DSM_FL = 6;   // table values per point
+constexpr int DSM_FL = 7;   // table values per point
 
 // FIXED: the point relative to c in block fixed point, its exponent per triangle in te.
 template <bool FIXED>
@@ -1540,6 +1541,7 @@ __global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, i
         o[3 * nt] = inv_det * (c22 * a1 - c12 * a2);
         o[4 * nt] = inv_det * (c11 * a2 - c12 * a1);
         o[5 * nt] = -3.0 * dev::dot(n, d);   // (not 0: the rules' truncated digits do not sum to 1)
+        o[6 * nt] = 1.0 - o[3 * nt] - o[4 * nt];
     }
 }
 
@@ -1621,11 +1623,10 @@ __device__ __forceinline__ void dsm_set(const double* __restrict__ tab, int64_t 
         const double y2 = y * y, wy3 = y2 * wy;
         acc[3] = fma(qr, wy3, acc[3]);
         const double g = fma(h3 + tab[5 * nt], qr * y2, qn) * wy3;   // w (q.n - 3 (q.r) (n.r) / r^2) / r^3
-        acc[0] += g;
+        acc[0] = fma(tab[6 * nt], g, acc[0]);
         acc[1] = fma(tab[3 * nt], g, acc[1]);
         acc[2] = fma(tab[4 * nt], g, acc[2]);
     }
-    acc[0] -= acc[1] + acc[2];
 }
 
 // Mixed precision: the first adaptive level in FP32 with coordinates relative
