@@ -191,7 +191,8 @@ int omg_head2megmat_mesh_dev(omg_context ctx, omg_geometry geo, const double* sq
 int omg_dipsourcemat_vjp_dev(omg_context ctx, omg_geometry geo, const double* dipoles, int64_t n_dipoles,
                              const omg_integrator* integ, int32_t domain, const double* U, int64_t ldu,
                              double* out);
-/* C = alpha op(A) op(B) + beta C in FP64 (column-major; trans = 1 transposes). */
+/* C = alpha op(A) op(B) + beta C in FP64 (column-major; trans = 1 transposes).  The product's error is at most
+ * about k 2^-53 sum |a||b| per entry, the bound of FP64 multiply-adds, whichever kernels run. */
 int omg_gemm_f64_dev(omg_context ctx, int32_t trans_a, int32_t trans_b, int64_t m, int64_t n, int64_t k, double alpha,
                      const double* A, int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc);
 

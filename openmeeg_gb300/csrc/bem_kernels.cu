@@ -5,12 +5,12 @@
 // array in the solver's internal numbering -- triangle unknowns first, then
 // vertex unknowns (the reference's [V | P] order rotated by n_vertices) --
 // and only its lower triangle is written.  Per-triangle records (OperatorS
-// data, P1 single-layer data, quadrature points) are precomputed once and
-// staged tile by tile into shared memory with bulk (TMA) copies.
+// data, P1 single-layer data, quadrature points) are precomputed once; the
+// mixed far field stages them tile by tile into shared memory with bulk (TMA)
+// copies, the FP64 S and D blocks read tables of distances and edge integrals.
 //
-// Each kernel restates the reference loop it replaces; the per-pair work is
-// the reference's analytic inner integral times its Gauss outer rule, so the
-// FP64 results agree with the reference to rounding.
+// The integrals are the reference's: its analytic inner integral under its
+// Gauss outer rule, so the FP64 results agree with it to rounding.
 #include <algorithm>
 #include <cstdio>
 #include <string>
@@ -287,7 +287,7 @@ __global__ void sd_geometry_kernel(int64_t t0, int64_t nt, const double* __restr
     }
 }
 
-// 1/x to about an ulp: the hardware approximation and one third-order Newton step.
+// 1/x to about an ulp: the hardware approximation y times the geometric series 1 + e + e^2 of 1 / (1 - e), e = 1 - x y.
 __device__ __forceinline__ double sd_rcp(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -1390,7 +1390,7 @@ __device__ __forceinline__ void dsm_point(int kind, int order, const DsmTri& T, 
     const double n2 = dev::dot(x, x), qx = dev::dot(q, x);
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n2));
-    const double e = fma(-(n2 * y), y, 1.0);   // one third-order Newton step
+    const double e = fma(-(n2 * y), y, 1.0);   // (1 - e)^(-1/2) = 1 + e / 2 + 3 e^2 / 8: the binomial series
     y = fma(y * e, fma(0.375, e, 0.5), y);
     const double y2 = y * y, wy3 = w * (y2 * y);
     if (kind == 1) {

@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(32 * PANEL_WARPS) panel32_kernel(const double*
         bad = good ? bad : min(bad, j);
         const double d = __longlong_as_double(good ? bits : 0x3FF0000000000000ll);
         // v / d on the integer pipe (rounded once): the chain of dependent FP64 operations it takes there, three for the
-        // reciprocal's Newton step and the product, is twice as long
+        // reciprocal's correction and the product, is twice as long
         uint32_t ym;
         int ye;
         uint64_t c;
@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(32 * PANEL_WARPS) panel32_kernel(const double*
         }
         __syncthreads();
     }
-    if (warp == 0) {   // rs = 1 / sqrt(d): the approximation and one third-order Newton step
+    if (warp == 0) {   // rs = 1 / sqrt(d): the approximation times the binomial series 1 + e / 2 + 3 e^2 / 8, e = 1 - d y^2
         const double d0 = U[off(lane)];
         const double d = __double_as_longlong(d0) > 0 ? d0 : 1.0;
         double y;

@@ -16,8 +16,9 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 REF_BIN = os.path.join(HERE, "_ref", "bin")
 # Where the reference sources are read from (this recipe builds them where they
-# lie); OMG_REFERENCE_DIR overrides it.
-REFERENCE_DIR = os.environ.get("OMG_REFERENCE_DIR", "/root/reference")
+# lie): a folder beside this repository; OMG_REFERENCE_DIR overrides it.
+REFERENCE_DIR = os.environ.get("OMG_REFERENCE_DIR",
+                               os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference"))
 
 
 def available() -> bool:
