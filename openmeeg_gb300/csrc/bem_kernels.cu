@@ -1572,7 +1572,7 @@ __device__ __forceinline__ DsmFix dsm_fix(d3 X, d3 q, int te) {
     f.q[1] = dsm_limbs(fx::fix60(q.y, qm - qy));
     f.q[2] = dsm_limbs(fx::fix60(q.z, qm - qz));
     f.qe = qm - 1022;
-    f.use = abs(f.E) < 400 && qm < 1900;
+    f.use = abs(f.E) < 400 && qm > 100 && qm < 1900;   // (a moment of zero has no mantissa to cut)
     return f;
 }
 
