@@ -1503,7 +1503,8 @@ __device__ __forceinline__ void dsm_adaptive_warp(int kind, int order, int level
 // listed for dsm_fallback_kernel.
 constexpr int DSM_FL = 7;   // table values per point
 
-// FIXED: the point relative to c in block fixed point, its exponent per triangle in te.
+// FIXED: the point relative to c in block fixed point, its exponent per triangle in te.  Otherwise the point itself, so that
+// point - r0 is rounded once.
 template <bool FIXED>
 __global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, int order, double* tab, int32_t* te) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1534,9 +1535,9 @@ __global__ void dsm_points_kernel(int64_t nt, const double* __restrict__ srec, i
             f[nt] = fx::fix60(d.y, max(em - (int)fx::expo(d.y), 0));
             f[2 * nt] = fx::fix60(d.z, max(em - (int)fx::expo(d.z), 0));
         } else {
-            o[0] = d.x;
-            o[nt] = d.y;
-            o[2 * nt] = d.z;
+            o[0] = x.x;
+            o[nt] = x.y;
+            o[2 * nt] = x.z;
         }
         o[3 * nt] = inv_det * (c22 * a1 - c12 * a2);
         o[4 * nt] = inv_det * (c11 * a2 - c12 * a1);
@@ -2383,8 +2384,9 @@ __global__ void dsm_vjp_kernel(int64_t dip0, int64_t ndc, const double* __restri
     const VjpW w = dsm_vjp_weights(P, i, t, T32, tidx_ref, barrier, U, ldu);
     const double* s = srec + t * SREC;
     const d3 n = dev::ld3(s + 9), q = dev::ld3(dip + 6 * i + 3);
-    const d3 X = (dev::ld3(s) + dev::ld3(s + 3) + dev::ld3(s + 6)) * (1.0 / 3.0) - dev::ld3(dip + 6 * i);
-    const double qn = dev::dot(q, n), h3 = -3.0 * dev::dot(n, X), area = s[12], qn3 = -3.0 * qn;
+    const d3 r0 = dev::ld3(dip + 6 * i), X = r0 * -1.0;   // (added to the tabled points)
+    const double h3 = -3.0 * dev::dot(n, (dev::ld3(s) + dev::ld3(s + 3) + dev::ld3(s + 6)) * (1.0 / 3.0) - r0);
+    const double qn = dev::dot(q, n), area = s[12], qn3 = -3.0 * qn;
     const double W1 = w.W[1] - w.W[0], W2 = w.W[2] - w.W[0];
     const int np = c_nbpts[order];
     const int64_t set = (int64_t)np * DSM_FL * nt;

@@ -538,9 +538,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             };
             auto whole = [](uint32_t bits, float scale) { return __float2int_rn(__uint_as_float(bits) * scale); };
             const int64_t j1 = min((int64_t)NCW, Nc - col0), jl = row < M ? (lower ? min(j1, row - col0 + 1) : j1) : 0;
-            // M: levels 4 and up in units of 2^-LOW, |M| < 2^61 (seven digits: 2^54)
+            // low: levels 4 and up in units of 2^-LOW, below 2^61 (seven digits: 2^54) in magnitude
             constexpr int LOW = UPDATE ? 61 : 69;
-            long long M_[NCW];
+            long long low[NCW];
             if (!UPDATE) {
                 uint8_t* const mr = mag + (int64_t)seg * M * Nc + row + col0 * M;
                 if (!begin()) break;
@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     read(h, a, b);
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                        M_[h * 8 + j] = __float2int_rn((__uint_as_float(a[j]) + __uint_as_float(b[j])) * 0x1p53f);
+                        low[h * 8 + j] = __float2int_rn((__uint_as_float(a[j]) + __uint_as_float(b[j])) * 0x1p53f);
                 }
                 end();
             }
@@ -572,9 +572,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     if (UPDATE)
-                        M_[h * 8 + j] = ((long long)whole(a[j], 0x1p32f) << (LOW - 48)) + whole(b[j], 0x1p45f);
+                        low[h * 8 + j] = ((long long)whole(a[j], 0x1p32f) << (LOW - 48)) + whole(b[j], 0x1p45f);
                     else
-                        M_[h * 8 + j] += ((long long)whole(a[j], 0x1p32f) << (LOW - 48)) + ((long long)whole(b[j], 0x1p40f) << (LOW - 56));
+                        low[h * 8 + j] += ((long long)whole(a[j], 0x1p32f) << (LOW - 48)) + ((long long)whole(b[j], 0x1p40f) << (LOW - 56));
                 }
             }
             end();
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 read(h, a, b);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    M_[h * 8 + j] += (((long long)whole(a[j], 0x1p16f) << 8) + whole(b[j], 0x1p24f)) << (LOW - 40);
+                    low[h * 8 + j] += (((long long)whole(a[j], 0x1p16f) << 8) + whole(b[j], 0x1p24f)) << (LOW - 40);
             }
             end();
             if (!begin()) break;   // levels 2 and 3: G in units of 2^-24, |G| < 2^31; then the value
@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                         const int G = (whole(a[j], 1.0f) << 8) + whole(b[j], 0x1p8f);
                         // k places fewer where G 2^(LOW - 24) would not stay below 2^61
                         const int k = max(0, LOW - 24 + 32 - __clz(abs(G)) - 61);
-                        const long long T = ((long long)G << (LOW - 24 - k)) + (M_[h * 8 + j] >> k);
+                        const long long T = ((long long)G << (LOW - 24 - k)) + (low[h * 8 + j] >> k);
                         const double v = scaled_double(T, er + eb[h * 8 + j] - LOW + k);
                         Cr[(h * 8 + j) * ldc] = UPDATE ? c[j] - v : v;
                     }
